@@ -45,22 +45,22 @@ def listed():
     return [
         # a video-call thumbnail: the smallest calls, latency and launches count
         dict(name="call_176x144", kind="session", w=176, h=144, streams=1, me="full", search=16, qp=26, slices=1,
-             frames=5, resident=5, gop=5, src="host", out="nals"),
+             frames=5, gop=5, src="host", out="nals"),
         # VGA conference stream, the library's default search range, learned search, host frames to a bitstream
         dict(name="conference_640x480", kind="session", w=640, h=480, streams=1, me="learned", search=16, qp=30,
-             slices=1, frames=12, resident=6, gop=12, src="host", out="nals"),
+             slices=1, frames=12, gop=12, src="host", out="nals"),
         # the reference host encoder's own use: levels, DC, masks, modes and vectors staged for its entropy coder
         dict(name="staging_1080p", kind="session", w=1920, h=1080, streams=1, me="full", search=32, qp=27, slices=4,
-             frames=8, resident=8, gop=8, src="host", out="staging"),
+             frames=8, gop=8, src="host", out="staging"),
         # a streaming server: eight 1080p streams, pinned host frames to Annex B slices (the headline workload)
         dict(name="server_1080p_x8", kind="session", w=1920, h=1080, streams=8, me="learned_fp8", search=32, qp=27,
-             slices=4, frames=24, resident=6, gop=24, src="host", out="nals"),
+             slices=4, frames=16, gop=16, src="host", out="nals"),
         # transcoding a decoder's 2160p surfaces, outputs kept on the device
         dict(name="surfaces_2160p", kind="session", w=3840, h=2160, streams=1, me="learned_fp8", search=32, qp=32,
-             slices=4, frames=8, resident=4, gop=8, src="device", out="device"),
+             slices=4, frames=8, gop=8, src="device", out="device"),
         # an all-intra 720p contribution feed at a high rate
         dict(name="intra_720p", kind="session", w=1280, h=720, streams=1, me="full", search=16, qp=20, slices=4,
-             frames=4, resident=4, gop=1, src="host", out="nals"),
+             frames=4, gop=1, src="host", out="nals"),
         # the multi-stream batch: eight streams of four sizes, one launch a stage, a captured graph a step
         dict(name="batch_mixed_x8", kind="batch", streams=8, me="learned_fp8", search=32, qp=28, steps=6, gop=6,
              graph=True, size_shift=0),
@@ -94,7 +94,7 @@ def draw(rng):
         out = rng.choice(["nals", "nals", "staging", "device"])
         return dict(kind=kind, w=w, h=h, streams=rng.choice([1, 1, 2, 4] if small else [1, 1, 2]),
                     me=rng.choice(list(ME_MODE)), search=rng.choice([16, 32]), qp=qp,
-                    slices=rng.choice([1, 2, 4]) if h >= 128 else 1, frames=frames, resident=min(frames, 4),
+                    slices=rng.choice([1, 2, 4]) if h >= 128 else 1, frames=frames,
                     gop=rng.choice([1, frames, frames]), src="device" if out == "device" else "host", out=out)
     if kind == "batch":
         return dict(kind=kind, streams=rng.randint(2, 8), me=rng.choice(["full", "learned_fp8"]),
@@ -212,7 +212,7 @@ def _prepare_session(c, seed):
     S.hdr, S.hdr_bits = _slice_headers(c["slices"])
     for s in range(c["streams"]):
         st = _Stream()
-        frames, _ = _video(w, h, c["resident"], seed * 64 + s)
+        frames, _ = _video(w, h, c["frames"], seed * 64 + s)
         st.ctx = b200enc.Context()
         st.ctx.configure(search_range=c["search"], deblock=1)
         if c["me"] != "full":
@@ -237,12 +237,6 @@ def _prepare_session(c, seed):
     if c["streams"] > 1:
         S.pool = ThreadPoolExecutor(c["streams"])
     return S
-
-
-def _order(resident, t):
-    """The resident frames played forward and back, as long as the GOP lasts."""
-    k = t % (2 * resident - 2) if resident > 1 else 0
-    return k if k < resident else 2 * resident - 2 - k
 
 
 def _recon(ctx):
@@ -281,7 +275,7 @@ def _encode_stream(S, st):
             staged[slot] = ctx.staging(slot)
 
     for t in range(c["frames"]):
-        f = st.frames[_order(c["resident"], t)]
+        f = st.frames[t]
         idr = t % c["gop"] == 0
         if c["src"] == "device":
             ctx.encode_device(f, w, h, c["qp"], idr, num_slices=c["slices"])
@@ -316,7 +310,7 @@ def _prepare_batch(c, seed):
     S = _Stream()
     S.c = c
     S.sizes = [BATCH_SIZES[(k + c["size_shift"]) % len(BATCH_SIZES)] for k in range(c["streams"])]
-    S.frames = [[_nv12(*f) for f in _video(w, h, 2, seed * 64 + k)[0]] for k, (w, h) in enumerate(S.sizes)]
+    S.frames = [[_nv12(*f) for f in _video(w, h, c["steps"], seed * 64 + k)[0]] for k, (w, h) in enumerate(S.sizes)]
     S.qps = [c["qp"] + k % 5 - 2 for k in range(c["streams"])]
     S.batch = b200enc.Batch(S.sizes, search_range=c["search"], me_mode=ME_MODE[c["me"]], graph=c["graph"])
     return S
@@ -325,7 +319,7 @@ def _prepare_batch(c, seed):
 def _run_batch(S):
     n = len(S.sizes)
     for t in range(S.c["steps"]):
-        S.batch.encode([f[t & 1] for f in S.frames], S.qps, [t % S.c["gop"] == 0] * n)
+        S.batch.encode([f[t] for f in S.frames], S.qps, [t % S.c["gop"] == 0] * n)
     if S.batch.sync() != 0:
         raise RuntimeError("b200enc_batch_sync failed")
     out = []
