@@ -151,7 +151,7 @@ int enqueue_step(Batch* b, const uint8_t* htab, int np, int ni, int ng, int n_p,
   }
   if (n_irows > 0) rc |= b200enc_i_frame_batch_launch(bt, n_irows, kBatchMaxWaitUs, st) != 0;
   if (b->deblock && n_groups > 0)
-    rc |= b200enc_deblock_tiles_batch_launch(bt, n_groups, kBatchMaxWaitUs, st) != 0;
+    rc |= b200enc_deblock_tiles_batch_launch(bt, n_groups, st) != 0;
   // status: error words of every stream's two scratch regions
   rc |= cudaMemcpyAsync(b->status_host, b->scratch, b->scratch_words * 4, cudaMemcpyDeviceToHost, st) != cudaSuccess;
   return rc ? -1 : 0;
@@ -292,7 +292,7 @@ int b200enc_batch_encode(void* h, const b200enc_batch_frame_t* frames) {
   int* pg = reinterpret_cast<int*>(ht + b->lay.pre_g);
   int np = 0, ni = 0, ng = 0, n_p = 0, n_irows = 0, n_groups = 0;
   pp[0] = pi[0] = pg[0] = 0;
-  b200enc_deblock_tile_count(1, 1, &b->db_tw, &b->db_th);
+  b200enc_deblock_batch_tile(&b->db_tw, &b->db_th);
   for (int s = 0; s < b->n; ++s) {
     const b200enc_batch_frame_t& f = frames[s];
     StreamState& t = b->ss[s];
@@ -342,7 +342,7 @@ int b200enc_batch_encode(void* h, const b200enc_batch_frame_t* frames) {
       ++np;
       n_p += pad16(mbs);
     }
-    const int groups = b200enc_deblock_tile_count(t.mbw, t.mbh, nullptr, nullptr);
+    const int groups = ((t.mbw + b->db_tw - 1) / b->db_tw) * ((t.mbh + b->db_th - 1) / b->db_th);
     ig[ng] = s;
     pg[ng + 1] = pg[ng] + groups;
     ++ng;

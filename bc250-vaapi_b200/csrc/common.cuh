@@ -283,8 +283,8 @@ struct BatchTab {
   BatchSet i_rows;  // macroblock rows of the streams coding an I frame
   BatchSet groups;  // deblocking tiles of every stream
   MV* mvc;          // motion vectors by compact P index
-  uint32_t* ticket; // [0] intra rows, [1] deblocking groups
-  int db_rows;      // macroblock rows per deblocking group (tile deblocking: tile height)
+  uint32_t* ticket; // [0] intra rows
+  int db_rows;      // tile deblocking: tile height in macroblocks
   int db_cols;      // tile deblocking: tile width in macroblocks
 };
 

@@ -40,6 +40,7 @@
 
 #include "b200enc_internal.h"
 #include "common.cuh"
+#include "deblock_tile.cuh"
 
 namespace b200enc {
 
@@ -58,81 +59,6 @@ __constant__ uint8_t kTc0[52][3] = {
     {1, 1, 2}, {1, 1, 2}, {1, 1, 2}, {1, 1, 2}, {1, 2, 3}, {1, 2, 3}, {2, 2, 3},  {2, 2, 4},  {2, 3, 4},
     {2, 3, 4}, {3, 3, 5}, {3, 4, 6}, {3, 4, 6}, {4, 5, 7}, {4, 5, 8}, {4, 6, 9},  {5, 7, 10}, {6, 8, 11},
     {6, 8, 13}, {7, 10, 14}, {8, 11, 16}, {9, 12, 18}, {10, 13, 20}, {11, 15, 23}, {13, 17, 25}};
-
-// Line filters (clause 8.7.2.3 / 8.7.2.4) on samples held in registers; the
-// callers unroll the edge loop, so every index is a compile-time constant.
-// They are branch-free: every lane evaluates the whole filter and keeps the
-// result by selection, so lanes whose edges differ in bS or in the sample
-// tests never split the warp, and the dependent chain per edge stays short.
-// A line with bS 0 or a failed sample test is left as it is.
-//
-// This encoder's boundary strengths are 4 on the macroblock edges of intra
-// pictures, 3 on their internal edges and 0-2 in P pictures, so the strong
-// filter is taken on a warp-uniform condition (intra picture, macroblock
-// edge) and the normal filter elsewhere.
-__device__ __forceinline__ void luma_normal(int p2, int& p1, int& p0, int& q0, int& q1, int q2, int bs, int alpha,
-                                            int beta, int tc0) {
-  const int dqp = q0 - p0;
-  const bool f = (bs != 0) & (abs(dqp) < alpha) & (abs(p1 - p0) < beta) & (abs(q1 - q0) < beta);
-  const bool ap = abs(p2 - p0) < beta, aq = abs(q2 - q0) < beta;
-  const int tc = tc0 + (int)ap + (int)aq;
-  const int delta = clampi((dqp * 4 + (p1 - q1) + 4) >> 3, -tc, tc);
-  const int avg = (p0 + q0 + 1) >> 1;
-  const int np1 = p1 + clampi((p2 + avg - (p1 << 1)) >> 1, -tc0, tc0);
-  const int nq1 = q1 + clampi((q2 + avg - (q1 << 1)) >> 1, -tc0, tc0);
-  const int np0 = clip1(p0 + delta), nq0 = clip1(q0 - delta);
-  p1 = (f & ap) ? np1 : p1;
-  q1 = (f & aq) ? nq1 : q1;
-  p0 = f ? np0 : p0;
-  q0 = f ? nq0 : q0;
-}
-
-__device__ __forceinline__ void luma_strong(int p3, int& p2, int& p1, int& p0, int& q0, int& q1, int& q2, int q3, int bs,
-                                            int alpha, int beta) {
-  const int d0 = abs(p0 - q0);
-  const bool f = (bs != 0) & (d0 < alpha) & (abs(p1 - p0) < beta) & (abs(q1 - q0) < beta);
-  const bool small = d0 < ((alpha >> 2) + 2);
-  const bool sp = f & small & (abs(p2 - p0) < beta), sq = f & small & (abs(q2 - q0) < beta);
-  const int a0 = (p2 + 2 * p1 + 2 * p0 + 2 * q0 + q1 + 4) >> 3;
-  const int a1 = (p2 + p1 + p0 + q0 + 2) >> 2;
-  const int a2 = (2 * p3 + 3 * p2 + p1 + p0 + q0 + 4) >> 3;
-  const int aw = (2 * p1 + p0 + q1 + 2) >> 2;
-  const int b0 = (q2 + 2 * q1 + 2 * q0 + 2 * p0 + p1 + 4) >> 3;
-  const int b1 = (q2 + q1 + q0 + p0 + 2) >> 2;
-  const int b2 = (2 * q3 + 3 * q2 + q1 + q0 + p0 + 4) >> 3;
-  const int bw = (2 * q1 + q0 + p1 + 2) >> 2;
-  p0 = sp ? a0 : (f ? aw : p0);
-  p1 = sp ? a1 : p1;
-  p2 = sp ? a2 : p2;
-  q0 = sq ? b0 : (f ? bw : q0);
-  q1 = sq ? b1 : q1;
-  q2 = sq ? b2 : q2;
-}
-
-__device__ __forceinline__ void chroma_normal(int p1, int& p0, int& q0, int q1, int bs, int alpha, int beta, int tc0) {
-  const int dqp = q0 - p0;
-  const bool f = (bs != 0) & (abs(dqp) < alpha) & (abs(p1 - p0) < beta) & (abs(q1 - q0) < beta);
-  const int tc = tc0 + 1;
-  const int delta = clampi((dqp * 4 + (p1 - q1) + 4) >> 3, -tc, tc);
-  const int np0 = clip1(p0 + delta), nq0 = clip1(q0 - delta);
-  p0 = f ? np0 : p0;
-  q0 = f ? nq0 : q0;
-}
-
-__device__ __forceinline__ void chroma_strong(int p1, int& p0, int& q0, int q1, int bs, int alpha, int beta) {
-  const bool f = (bs != 0) & (abs(p0 - q0) < alpha) & (abs(p1 - p0) < beta) & (abs(q1 - q0) < beta);
-  const int np0 = (2 * p1 + p0 + q1 + 2) >> 2, nq0 = (2 * q1 + q0 + p1 + 2) >> 2;
-  p0 = f ? np0 : p0;
-  q0 = f ? nq0 : q0;
-}
-
-__device__ __forceinline__ int tc0_for(int bs, int t1, int t2, int t3) { return bs == 1 ? t1 : (bs == 2 ? t2 : t3); }
-
-// Filter thresholds of one picture (uniform QP): luma and chroma alpha/beta
-// and tC0 for bS 1..3.
-struct DbQ {
-  int al, be, alc, bec, tcl1, tcl2, tcl3, tcc1, tcc2, tcc3, is_intra;
-};
 
 __device__ __forceinline__ DbQ db_q(int qp, int is_intra) {
   const int qpc = chroma_qp(qp);
@@ -342,15 +268,9 @@ __device__ __forceinline__ bool wait_shared(const volatile uint32_t* flag, const
   return false;
 }
 
-// BATCH: the group tickets (bt.ticket[1]) run over the row groups of every
-// stream of a batch (bt.groups, R = bt.db_rows rows each); a group waits
-// only on its own stream's rows and scratch. Dynamic shared memory is sized
-// for the widest stream.
-template <bool BATCH>
-__global__ void deblock_kernel(int mbw_, int mbh_, int R, int qp_, int is_intra_,
-                                                      const uint32_t* __restrict__ nzm_, const MV* __restrict__ mvs_,
-                                                      uint8_t* rec_y_, uint8_t* rec_uv_, int rec_pitch_,
-                                                      uint32_t* scratch_, uint32_t max_wait, BatchTab bt) {  // max_wait in microseconds
+__global__ void deblock_kernel(int mbw, int mbh, int R, int qp, int is_intra, const uint32_t* __restrict__ nzm,
+                               const MV* __restrict__ mvs, uint8_t* rec_y, uint8_t* rec_uv, int rec_pitch,
+                               uint32_t* scratch, uint32_t max_wait) {  // max_wait in microseconds
   extern __shared__ __align__(16) uint8_t smem[];
   __shared__ int s_group, s_abort;
   const int tid = threadIdx.x, warp = tid >> 5, lane = tid & 31, nthr = blockDim.x;
@@ -359,32 +279,11 @@ __global__ void deblock_kernel(int mbw_, int mbh_, int R, int qp_, int is_intra_
 
   for (;;) {
     if (tid == 0) {
-      s_group = (int)atomicAdd(BATCH ? bt.ticket + 1 : Scratch{scratch_}.ticket(), 1u);
+      s_group = (int)atomicAdd(Scratch{scratch}.ticket(), 1u);
       s_abort = 0;
     }
     __syncthreads();
-    int mbw = mbw_, mbh = mbh_, qp = qp_, is_intra = is_intra_, rec_pitch = rec_pitch_;
-    const uint32_t* nzm = nzm_;
-    const MV* mvs = mvs_;
-    uint8_t *rec_y = rec_y_, *rec_uv = rec_uv_;
-    uint32_t* scratch = scratch_;
-    int group = s_group;
-    if (BATCH) {
-      if (group >= bt.groups.total()) return;
-      const int k = bt.groups.find(group);
-      const BatchStream& st = bt.groups.stream(k);
-      group -= bt.groups.prefix[k];
-      mbw = st.g.mbw;
-      mbh = st.g.mbh;
-      qp = st.qp;
-      is_intra = st.is_intra;
-      nzm = st.nz;
-      mvs = st.mv;
-      rec_y = st.rec_y;
-      rec_uv = st.rec_uv;
-      rec_pitch = st.rec_pitch;
-      scratch = st.scr_db;
-    }
+    const int group = s_group;
     const int y0 = group * R;
     if (y0 >= mbh) return;
     const DbPlan P = db_plan(mbw, R);
@@ -649,64 +548,80 @@ __global__ void deblock_kernel(int mbw_, int mbh_, int R, int qp_, int is_intra_
 
 
 // ---------------------------------------------------------------------------
-// Tile deblocking. Raster-order deblocking reaches only a short distance: a
-// filter changes at most three samples either side of an edge and reads at
-// most four, edges are four samples apart, and the value one edge hands to
-// the next (its q1, read back as the next edge's p2) depends on that edge's
-// own inputs only, so a change does not travel along a row or a column. As a
-// result the deblocked samples of a tile of macroblocks are those of the
-// raster-order deblocking of the tile with one macroblock of margin on every
-// side (clipped at the picture), treated as a picture of its own (no
-// filtering on the margin's outer edges). The oracle checks this against
-// whole-picture deblocking on random and adversarial content, intra and
-// inter, for several tile shapes (tests/test_deblock_tiles.py).
-//
-// So each CTA takes one tile: it loads the tile and its margin from the
-// unfiltered reconstruction (`src`) into shared memory, deblocks it there in
-// raster order (the row wavefront of the kernel above, one luma and one
-// chroma warp per macroblock row, rows a macroblock step apart), and stores
-// the tile alone to `dst`. CTAs never wait on one another; a picture is
-// mbw/TW x mbh/TH independent tiles of (TW + TH + 3) dependent steps each,
-// instead of one wavefront of mbw + mbh - 1 steps. `dst` must not overlap
+// Tile deblocking, out of place: each CTA takes one tile of macroblocks,
+// loads it with the few margin samples it depends on from the unfiltered
+// reconstruction (`src`) into shared memory, filters it there in the seven
+// phases of deblock_tile.cuh (raster order reproduced exactly; a barrier
+// between phases, every line of a phase independent), and stores the tile
+// alone to `dst`. CTAs never wait on one another; `dst` must not overlap
 // `src` (neighbouring tiles read each other's samples as their margin).
+//
+// What bounds it: the instructions of the line filters and the seven
+// barriers, not memory (a 1080p frame is 7 MB of traffic, ~1 us at HBM rate).
+// The form before this one ran each tile and a whole macroblock of margin as
+// a row wavefront in shared memory (TW + TH + 3 dependent macroblock steps of
+// ~1.8 us, 16 of 32 lanes active). P pictures, before and now, us: 176x144
+// 33 and 10.9, 640x480 37 and 12.1, 1920x1080 38 and 17 to 19, 3840x2160 111
+// and 41.
 // ---------------------------------------------------------------------------
-constexpr int kDbTileMax = 8;    // TH <= 8 (a luma and a chroma warp per region row)
-constexpr int kDbTileMaxW = 16;  // TW <= 16 (the width sets shared memory only: 78 KB at 16 x 8)
+constexpr int kDbTileMax = 8;    // TH <= 8
+constexpr int kDbTileMaxW = 16;  // TW <= 16
+constexpr int kDbTileThreads = 512;
 
 struct DbTilePlan {
-  int sp;  // shared-memory row stride: 16 * (TW + 2) + 4 bytes, an odd word count
-  size_t luma_off, chroma_off, bs_off, prog_off, bytes;
+  int sp;  // shared-memory row stride: 16 * (TW + 1) + 4 bytes, an odd word count (consecutive rows on
+           // different banks)
+  int mbs; // macroblocks of the tile with one of margin on every side
+  size_t luma_off, chroma_off, bs_off, save_off, mask_off, mv_off, bytes;
 };
 
 __host__ __device__ inline DbTilePlan db_tile_plan(int TW, int TH) {
   DbTilePlan p;
-  p.sp = 16 * (TW + 2) + 4;
-  p.luma_off = 0;                                                    // 4 margin rows + 16 (TH + 2) rows
-  p.chroma_off = (size_t)(16 * (TH + 2) + 4) * p.sp;                 // 2 margin rows + 8 (TH + 2) rows
-  p.bs_off = p.chroma_off + (size_t)(8 * (TH + 2) + 2) * p.sp;       // [MB][dir][edge][segment]
-  p.prog_off = (p.bs_off + (size_t)(TH + 2) * (TW + 2) * 32 + 15) & ~(size_t)15;
-  p.bytes = p.prog_off + 2 * (TH + 2) * sizeof(uint32_t);            // progress: luma rows, chroma rows
+  p.sp = 16 * (TW + 1) + 4;
+  p.mbs = (TW + 2) * (TH + 2);
+  p.luma_off = 0;
+  p.chroma_off = (size_t)(kDtTop + 16 * TH + kDtBottom) * p.sp;
+  p.bs_off = p.chroma_off + (size_t)(kDtTopC + 8 * TH + kDtBottomC) * p.sp;
+  p.save_off = p.bs_off + (size_t)p.mbs * 32;
+  p.mv_off = (p.save_off + (size_t)p.mbs * 64 + 7) & ~(size_t)7;
+  p.mask_off = p.mv_off + (size_t)p.mbs * sizeof(int2);
+  p.bytes = p.mask_off + (size_t)p.mbs * sizeof(uint32_t);
   return p;
+}
+
+// Threads of a tile's CTA: sixteen per macroblock (a phase has 7 to 18 lines
+// per macroblock), at most 512 (two CTAs per SM).
+static inline int db_tile_threads(int TW, int TH) {
+  const int n = (16 * TW * TH + 31) / 32 * 32;
+  return n < 64 ? 64 : (n > kDbTileThreads ? kDbTileThreads : n);
+}
+
+template <int PHASE>
+__device__ __forceinline__ void db_tile_phase(const DtTile& t, const DbQ& q, bool luma, bool chroma) {
+  const int nl = luma ? dt_luma_lines(t, PHASE) : 0, n = nl + (chroma ? dt_chroma_lines(t, PHASE) : 0);
+  for (int i = threadIdx.x; i < n; i += blockDim.x) {
+    if (i < nl) dt_luma_line(t, PHASE, i, q);
+    else dt_chroma_line(t, PHASE, i - nl, q);
+  }
+  __syncthreads();
 }
 
 // BATCH: one CTA per tile of every stream of a batch (bt.groups counts each
 // stream's tiles; bt.db_rows = TH, bt.db_cols = TW); the stream's unfiltered
 // reconstruction is rec_y/rec_uv, the deblocked one goes to db_y/db_uv.
 template <bool BATCH>
-__global__ void __launch_bounds__(64 * (kDbTileMax + 2), 2) deblock_tile_kernel(
+__global__ void __launch_bounds__(kDbTileThreads, 2) deblock_tile_kernel(
     int mbw_, int mbh_, int TW, int TH, int qp_, int is_intra_, const uint32_t* __restrict__ nzm_,
     const MV* __restrict__ mvs_, const uint8_t* __restrict__ t8_, const uint8_t* __restrict__ src_y_,
     const uint8_t* __restrict__ src_uv_,
-    uint8_t* __restrict__ dst_y_, uint8_t* __restrict__ dst_uv_, int pitch_, uint32_t* status_, uint32_t max_wait,
-    BatchTab bt) {
+    uint8_t* __restrict__ dst_y_, uint8_t* __restrict__ dst_uv_, int pitch_, uint32_t* status_, BatchTab bt) {
   extern __shared__ __align__(16) uint8_t smem[];
-  const int tid = threadIdx.x, warp = tid >> 5, lane = tid & 31, nthr = blockDim.x;
+  const int tid = threadIdx.x, nthr = blockDim.x;
   int mbw = mbw_, mbh = mbh_, qp = qp_, is_intra = is_intra_, pitch = pitch_;
   const uint32_t* nzm = nzm_;
   const MV* mvs = mvs_;
   const uint8_t *src_y = src_y_, *src_uv = src_uv_;
   uint8_t *dst_y = dst_y_, *dst_uv = dst_uv_;
-  uint32_t* status = status_;
   int tile = blockIdx.x;
   if (BATCH) {
     if (tile >= bt.groups.total()) return;
@@ -726,120 +641,126 @@ __global__ void __launch_bounds__(64 * (kDbTileMax + 2), 2) deblock_tile_kernel(
     dst_y = st.db_y;
     dst_uv = st.db_uv;
     pitch = st.rec_pitch;
-    status = st.scr_db;
+  } else if (tile == 0 && tid < 4) {
+    status_[tid] = 0u;  // nothing here can fail: the caller's status words are cleared
   }
+  const uint8_t* t8 = BATCH ? nullptr : t8_;
   const int ntx = (mbw + TW - 1) / TW;
   const int tx = tile % ntx, ty = tile / ntx;
   const int x0 = tx * TW, y0 = ty * TH;
   if (y0 >= mbh) return;
-  const int x1 = min(mbw, x0 + TW), y1 = min(mbh, y0 + TH);
-  // the deblocked region: the tile and its margin, clipped at the picture
-  const int rx0 = max(0, x0 - 1), ry0 = max(0, y0 - 1), rx1 = min(mbw, x1 + 1), ry1 = min(mbh, y1 + 1);
-  const int RWr = rx1 - rx0, RHr = ry1 - ry0;
   const DbTilePlan P = db_tile_plan(TW, TH);
-  uint8_t* ly = smem + P.luma_off;    // row 4 = picture row 16 * ry0, byte 0 = column 16 * rx0
-  uint8_t* cy = smem + P.chroma_off;  // row 2 = picture row 8 * ry0
+  DtTile t;
+  t.ly = smem + P.luma_off;
+  t.cy = smem + P.chroma_off;
+  t.sp = P.sp;
   uint8_t* bsm = smem + P.bs_off;
-  volatile uint32_t* prog = reinterpret_cast<volatile uint32_t*>(smem + P.prog_off);
-  const Scratch sc{status};
+  t.bs = bsm;
+  t.save = smem + P.save_off;
+  t.stride = TW + 2;
+  t.TW = min(TW, mbw - x0);
+  t.TH = min(TH, mbh - y0);
+  t.L = x0 > 0;
+  t.R = x0 + t.TW < mbw;
+  t.T = y0 > 0;
+  t.B = y0 + t.TH < mbh;
+  int2* mvm = reinterpret_cast<int2*>(smem + P.mv_off);
+  uint32_t* mask = reinterpret_cast<uint32_t*>(smem + P.mask_off);
   const DbQ q = db_q(qp, is_intra);
+  const bool luma = q.al && q.be, chroma = q.alc && q.bec;
 
-  // ---- load the region, boundary strengths, progress words -----------------
+  // ---- the tile and its margin; coefficient masks and vectors ---------------
   {
-    const int lrows = 16 * RHr, crows = 8 * RHr, n = (lrows + crows) * RWr;
+    // 16-byte units from the left margin (or the tile) to the tile's right
+    // end, then the right margin's 4 bytes
+    const int lr0 = -kDtTop * t.T, lrows = 16 * t.TH + kDtBottom * t.B - lr0;
+    const int cr0 = -kDtTopC * t.T, crows = 8 * t.TH + kDtBottomC * t.B - cr0;
+    const int nu = t.TW + t.L, n = (lrows + crows) * nu;
+    const uint8_t* gl = src_y + (size_t)(16 * y0 + lr0) * pitch + 16 * (x0 - t.L);
+    const uint8_t* gc = src_uv + (size_t)(8 * y0 + cr0) * pitch + 16 * (x0 - t.L);
+    uint8_t* sl = t.ly + (kDtTop + lr0) * P.sp + 16 * (1 - t.L);
+    uint8_t* sc = t.cy + (kDtTopC + cr0) * P.sp + 16 * (1 - t.L);
+#pragma unroll 4
     for (int i = tid; i < n; i += nthr) {
-      const int r = i / RWr, c = i - r * RWr;
+      const int r = i / nu, c = i - r * nu;
       const bool lu = r < lrows;
       const int rr = lu ? r : r - lrows;
-      const uint8_t* g = lu ? src_y + (size_t)(16 * ry0 + rr) * pitch + 16 * (rx0 + c)
-                            : src_uv + (size_t)(8 * ry0 + rr) * pitch + 16 * (rx0 + c);
-      const uint4 v = __ldg(reinterpret_cast<const uint4*>(g));
-      uint32_t* d = reinterpret_cast<uint32_t*>((lu ? ly + (size_t)(4 + rr) * P.sp : cy + (size_t)(2 + rr) * P.sp) +
-                                                16 * c);
+      const uint4 v = __ldg(reinterpret_cast<const uint4*>((lu ? gl : gc) + (size_t)rr * pitch + 16 * c));
+      uint32_t* d = reinterpret_cast<uint32_t*>((lu ? sl : sc) + rr * P.sp + 16 * c);
       d[0] = v.x;
       d[1] = v.y;
       d[2] = v.z;
       d[3] = v.w;
     }
-    // the margin rows above the region are read (never changed: the top
-    // edges of the region's first row have bS 0) by its first row's
-    // horizontal steps; give them defined contents
-    for (int i = tid; i < 6 * (P.sp / 4); i += nthr) {
-      const int r = i / (P.sp / 4), w = i - r * (P.sp / 4);
-      reinterpret_cast<uint32_t*>(r < 4 ? ly + (size_t)r * P.sp : cy + (size_t)(r - 4) * P.sp)[w] = 0u;
-    }
-    for (int i = tid; i < RHr * RWr * 32; i += nthr) {
-      const int k = i & 3, e = (i >> 2) & 3, dir = (i >> 4) & 1, m = i >> 5;
-      const int lyr = m / RWr, lxr = m - lyr * RWr;
-      bsm[i] = (uint8_t)db_bs(k, e, dir, (ry0 + lyr) * mbw + rx0 + lxr, mbw, dir == 0 ? lxr > 0 : lyr > 0, is_intra,
-                              nzm, mvs, BATCH ? nullptr : t8_);
-    }
-    for (int i = tid; i < 2 * (TH + 2); i += nthr) prog[i] = 0u;
-  }
-  __syncthreads();
-
-  // ---- the region's rows, one luma and one chroma warp each ----------------
-  {
-    const bool is_luma = warp < TH + 2;
-    const int wr = is_luma ? warp : warp - (TH + 2);
-    if (wr < RHr) {
-      const uint8_t* bsrow = bsm + (size_t)wr * RWr * 32;
-      volatile uint32_t* my_prog = prog + (is_luma ? 0 : TH + 2) + wr;
-      const volatile uint32_t* up_prog = my_prog - 1;
-      const bool on = is_luma ? (q.al && q.be) : (q.alc && q.bec);
-      uint8_t* vrow = is_luma ? ly + (size_t)(4 + 16 * wr) * P.sp : cy + (size_t)(2 + 8 * wr) * P.sp;
-      uint8_t* htop = is_luma ? ly + (size_t)(16 * wr) * P.sp : cy + (size_t)(8 * wr) * P.sp;
-      for (int mx = 0; mx < RWr; ++mx) {
-        const uint8_t* bs = bsrow + mx * 32;
-        // vertical edges: this row's own samples only
-        if (on && lane < 16) {
-          if (is_luma)
-            luma_v_step(vrow, P.sp, 16 * mx, 16 * (mx - 1), mx > 0, bs, lane, q);
-          else
-            chroma_v_step(vrow, P.sp, 16 * mx, 16 * (mx - 1), mx > 0, bs, lane, q);
-        }
-        __syncwarp();
-        if (mx > 0) {  // macroblock mx-1 of this row is final
-          __threadfence_block();
-          __syncwarp();
-          if (lane == 0) *my_prog = (uint32_t)mx;
-        }
-        // horizontal edges of mx: the row above has filtered the vertical
-        // edges of mx+1 (all of its row at the last macroblock)
-        if (wr > 0) {
-          if (!wait_shared(up_prog, sc, (uint32_t)(mx + 1), max_wait,
-                           (uint32_t)((ry0 + wr) * mbw + rx0 + mx)))
-            break;
-          __threadfence_block();
-        }
-        __syncwarp();
-        if (on && lane < 16) {
-          if (is_luma)
-            luma_h_step(htop, P.sp, 16 * mx, bs, lane, q);
-          else
-            chroma_h_step(htop, P.sp, 16 * mx, bs, lane, q);
-        }
-        if (mx == RWr - 1) {
-          __syncwarp();
-          __threadfence_block();
-          __syncwarp();
-          if (lane == 0) *my_prog = (uint32_t)RWr;
+    if (t.R)
+      for (int r = tid; r < lrows + crows; r += nthr) {
+        const bool lu = r < lrows;
+        const int rr = lu ? r : r - lrows;
+        *reinterpret_cast<uint32_t*>((lu ? sl : sc) + rr * P.sp + 16 * nu) =
+            __ldg(reinterpret_cast<const uint32_t*>((lu ? gl : gc) + (size_t)rr * pitch + 16 * nu));
+      }
+    if (!is_intra) {
+      // sixteen lanes per macroblock: one block's word each
+      const int nm = (t.TW + 2) * (t.TH + 2);
+      for (int i = tid; i < (nm * 16 + 31) / 32 * 32; i += nthr) {
+        const int m = i >> 4, b = i & 15, my = m / (t.TW + 2), mx = m - my * (t.TW + 2);
+        const int gx = x0 + mx - 1, gy = y0 + my - 1;
+        const bool in = m < nm && gx >= 0 && gx < mbw && gy >= 0 && gy < mbh;
+        const int mb = gy * mbw + gx;
+        const uint32_t w = in ? __ldg(nzm + (size_t)mb * 24 + b) & 0xffffu : 0u;
+        uint32_t bits = __ballot_sync(0xffffffffu, w != 0u);
+        if (b == 0 && in) {
+          bits = (bits >> (tid & 16)) & 0xffffu;
+          mask[my * t.stride + mx] = t8 && t8[mb] ? dt_mask_t8(bits) | 0x10000u : bits;
+          mvm[my * t.stride + mx] = __ldg(reinterpret_cast<const int2*>(mvs + mb));
         }
       }
     }
   }
+  if (!is_intra) __syncthreads();
+  // ---- boundary strengths -----------------------------------------------------
+  for (int i = tid; i < (t.TW + 2) * (t.TH + 2) * 8; i += nthr) {
+    const int m = i >> 3, dir = (i >> 2) & 1, e = i & 3, my = m / (t.TW + 2), mx = m - my * (t.TW + 2);
+    const int gx = x0 + mx - 1, gy = y0 + my - 1;
+    if (gx < 0 || gx >= mbw || gy < 0 || gy >= mbh) continue;
+    const int s = my * t.stride + mx, sn = dir == 0 ? s - 1 : s - t.stride;
+    // the margin's outer edges are never filtered here (and have no neighbour staged)
+    const bool edge0 = dir == 0 ? (gx > 0 && mx > 0) : (gy > 0 && my > 0);
+    uint32_t w;
+    if (is_intra) {
+      w = dt_strengths(dir, e, 0, 0, false, edge0, true, t8 && t8[gy * mbw + gx]);
+    } else {
+      const uint32_t mq = mask[s];
+      uint32_t mp = 0;
+      bool far = false;
+      if (e == 0 && edge0) {
+        const int2 a = mvm[s], b = mvm[sn];
+        mp = mask[sn];
+        far = abs(a.x - b.x) >= 4 || abs(a.y - b.y) >= 4;
+      }
+      w = dt_strengths(dir, e, mq & 0xffffu, mp, far, edge0, false, (mq & 0x10000u) != 0);
+    }
+    reinterpret_cast<uint32_t*>(bsm)[s * 8 + dir * 4 + e] = w;
+  }
   __syncthreads();
 
-  // ---- store the tile (whatever a failed wait left: the status says so) -----
+  db_tile_phase<1>(t, q, luma, chroma);
+  db_tile_phase<2>(t, q, luma, chroma);
+  db_tile_phase<3>(t, q, luma, chroma);
+  db_tile_phase<4>(t, q, luma, chroma);
+  db_tile_phase<5>(t, q, luma, chroma);
+  db_tile_phase<6>(t, q, luma, chroma);
+  db_tile_phase<7>(t, q, luma, chroma);
+
+  // ---- store the tile --------------------------------------------------------
   {
-    const int tw = x1 - x0, lrows = 16 * (y1 - y0), crows = 8 * (y1 - y0), n = (lrows + crows) * tw;
-    const int ox = x0 - rx0, oy = y0 - ry0;  // the tile's macroblock offset in the region
+    const int lrows = 16 * t.TH, n = (lrows + 8 * t.TH) * t.TW;
     for (int i = tid; i < n; i += nthr) {
-      const int r = i / tw, c = i - r * tw;
+      const int r = i / t.TW, c = i - r * t.TW;
       const bool lu = r < lrows;
       const int rr = lu ? r : r - lrows;
       const uint32_t* s4 = reinterpret_cast<const uint32_t*>(
-          (lu ? ly + (size_t)(4 + 16 * oy + rr) * P.sp : cy + (size_t)(2 + 8 * oy + rr) * P.sp) + 16 * (ox + c));
+          (lu ? t.ly + (kDtTop + rr) * P.sp : t.cy + (kDtTopC + rr) * P.sp) + 16 * (1 + c));
       uint8_t* g = lu ? dst_y + (size_t)(16 * y0 + rr) * pitch + 16 * (x0 + c)
                       : dst_uv + (size_t)(8 * y0 + rr) * pitch + 16 * (x0 + c);
       *reinterpret_cast<uint4*>(g) = make_uint4(s4[0], s4[1], s4[2], s4[3]);
@@ -877,31 +798,11 @@ extern "C" int b200enc_deblock_launch(int mbw, int mbh, int qp, int is_intra, co
   const DbPlan P = db_plan(mbw, R);
   const int groups = (mbh + R - 1) / R;
   if (ctas <= 0 || ctas > groups) ctas = groups;
-  if (cudaFuncSetAttribute(deblock_kernel<false>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)P.bytes) !=
+  if (cudaFuncSetAttribute(deblock_kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)P.bytes) !=
       cudaSuccess)
     return -1;
-  deblock_kernel<false><<<ctas, 64 * R + 128, P.bytes, (cudaStream_t)stream>>>(
-      mbw, mbh, R, qp, is_intra, nz, (const MV*)mv, rec_y, rec_uv, rec_pitch, scratch, max_wait, BatchTab{});
-  return cudaGetLastError() == cudaSuccess ? 0 : -1;
-}
-
-// Rows per group a batch's deblocking uses for streams up to max_mbw
-// macroblocks wide (0 if none fits).
-int b200enc_deblock_batch_rows(int max_mbw, int max_mbh) { return db_rows_per_cta(max_mbw, max_mbh); }
-
-// The deblocking of every stream of a batch: `ctas` persistent CTAs over
-// bt.groups (bt.db_rows rows per group; each stream's scratch zeroed and
-// bt.ticket[1] = 0 by the caller).
-int b200enc_deblock_batch_launch(const BatchTab& bt, int max_mbw, int ctas, uint32_t max_wait, cudaStream_t st) {
-  if (ctas <= 0) return 0;
-  const int R = bt.db_rows;
-  if (R <= 0) return -1;
-  const DbPlan P = db_plan(max_mbw, R);
-  if (cudaFuncSetAttribute(deblock_kernel<true>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)P.bytes) !=
-      cudaSuccess)
-    return -1;
-  deblock_kernel<true><<<ctas, 64 * R + 128, P.bytes, st>>>(0, 0, R, 0, 0, nullptr, nullptr, nullptr, nullptr, 0,
-                                                            nullptr, max_wait, bt);
+  deblock_kernel<<<ctas, 64 * R + 128, P.bytes, (cudaStream_t)stream>>>(
+      mbw, mbh, R, qp, is_intra, nz, (const MV*)mv, rec_y, rec_uv, rec_pitch, scratch, max_wait);
   return cudaGetLastError() == cudaSuccess ? 0 : -1;
 }
 
@@ -917,44 +818,41 @@ extern "C" int b200enc_deblock(int mbw, int mbh, int qp, int is_intra, const uin
                                 kMaxWaitUsDb, stream);
 }
 
-// Tile shape of the tile deblocking (TW x TH macroblocks): 8 x 8 unless the
-// autotuner chose otherwise.
-static void db_tile_shape(int* tw, int* th) {
+// Tile shape of the tile deblocking (TW x TH macroblocks) of a picture of
+// `mbs` macroblocks, unless the autotuner chose one: 4 x 4 up to 4,096
+// macroblocks, where the tiles do not fill the chip and a tile's own latency
+// is the kernel's (P picture, us, 4 x 4 against 8 x 8: 176x144 10.9 and 16.1,
+// 640x480 12.1 and 19.2, 1280x720 13.1 and 18.4), 8 x 8 above, where the
+// margin's share of the work counts (3840x2160 47.8 and 40.6).
+static void db_tile_shape(int mbs, int* tw, int* th) {
   const int w = b200enc_tuned(B200ENC_TUNE_DEBLOCK_TILE_W), h = b200enc_tuned(B200ENC_TUNE_DEBLOCK_TILE_H);
-  *tw = w > 0 ? std::min(w, kDbTileMaxW) : 8;
-  *th = h > 0 ? std::min(h, kDbTileMax) : 8;
+  const int d = mbs <= 4096 ? 4 : 8;
+  *tw = w > 0 ? std::min(w, kDbTileMaxW) : d;
+  *th = h > 0 ? std::min(h, kDbTileMax) : d;
 }
 
 int b200enc_deblock_tiles_launch(int mbw, int mbh, int qp, int is_intra, const uint32_t* nz, const void* mv,
                                  const uint8_t* src_y, const uint8_t* src_uv, uint8_t* dst_y, uint8_t* dst_uv,
-                                 int pitch, uint32_t* status, uint32_t max_wait, cudaStream_t stream,
-                                 const uint8_t* t8) {
+                                 int pitch, uint32_t* status, cudaStream_t stream, const uint8_t* t8) {
   int TW, TH;
-  db_tile_shape(&TW, &TH);
+  db_tile_shape(mbw * mbh, &TW, &TH);
   const DbTilePlan P = db_tile_plan(TW, TH);
   if (cudaFuncSetAttribute(deblock_tile_kernel<false>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)P.bytes) !=
       cudaSuccess)
     return -1;
   const int tiles = ((mbw + TW - 1) / TW) * ((mbh + TH - 1) / TH);
-  deblock_tile_kernel<false><<<tiles, 64 * (TH + 2), P.bytes, stream>>>(
-      mbw, mbh, TW, TH, qp, is_intra, nz, (const MV*)mv, t8, src_y, src_uv, dst_y, dst_uv, pitch, status,
-      max_wait, BatchTab{});
+  deblock_tile_kernel<false><<<tiles, db_tile_threads(TW, TH), P.bytes, stream>>>(
+      mbw, mbh, TW, TH, qp, is_intra, nz, (const MV*)mv, t8, src_y, src_uv, dst_y, dst_uv, pitch, status, BatchTab{});
   return cudaGetLastError() == cudaSuccess ? 0 : -1;
 }
 
-// Tiles of a stream of mbw x mbh macroblocks under the current tile shape,
-// and the shape itself (for a batch's table).
-int b200enc_deblock_tile_count(int mbw, int mbh, int* tw, int* th) {
-  int TW, TH;
-  db_tile_shape(&TW, &TH);
-  if (tw) *tw = TW;
-  if (th) *th = TH;
-  return ((mbw + TW - 1) / TW) * ((mbh + TH - 1) / TH);
-}
+// Tile shape of a batch's table: one shape for every stream, the large
+// picture's (a batch fills the chip with its streams).
+void b200enc_deblock_batch_tile(int* tw, int* th) { db_tile_shape(1 << 30, tw, th); }
 
 // The tile deblocking of every stream of a batch: one CTA per tile
 // (bt.groups over the streams' tiles, bt.db_cols x bt.db_rows each).
-int b200enc_deblock_tiles_batch_launch(const BatchTab& bt, int tiles, uint32_t max_wait, cudaStream_t st) {
+int b200enc_deblock_tiles_batch_launch(const BatchTab& bt, int tiles, cudaStream_t st) {
   if (tiles <= 0) return 0;
   const int TW = bt.db_cols, TH = bt.db_rows;
   if (TW < 1 || TH < 1 || TW > kDbTileMaxW || TH > kDbTileMax) return -1;
@@ -962,9 +860,8 @@ int b200enc_deblock_tiles_batch_launch(const BatchTab& bt, int tiles, uint32_t m
   if (cudaFuncSetAttribute(deblock_tile_kernel<true>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)P.bytes) !=
       cudaSuccess)
     return -1;
-  deblock_tile_kernel<true><<<tiles, 64 * (TH + 2), P.bytes, st>>>(0, 0, 0, 0, 0, 0, nullptr, nullptr, nullptr,
-                                                                   nullptr, nullptr, nullptr, nullptr, 0, nullptr,
-                                                                   max_wait, bt);
+  deblock_tile_kernel<true><<<tiles, db_tile_threads(TW, TH), P.bytes, st>>>(
+      0, 0, 0, 0, 0, 0, nullptr, nullptr, nullptr, nullptr, nullptr, nullptr, nullptr, 0, nullptr, bt);
   return cudaGetLastError() == cudaSuccess ? 0 : -1;
 }
 
@@ -996,7 +893,6 @@ extern "C" int b200enc_deblock_tiles_t8(int mbw, int mbh, int qp, int is_intra, 
   };
   if (overlap(d0, d1, s0, s1) || overlap(d0, d1, c0, c1) || overlap(e0, e1, s0, s1) || overlap(e0, e1, c0, c1))
     return -1;
-  if (cudaMemsetAsync(status, 0, 16, (cudaStream_t)stream) != cudaSuccess) return -1;
   return b200enc_deblock_tiles_launch(mbw, mbh, qp, is_intra, nz, mv, src_y, src_uv, dst_y, dst_uv, pitch, status,
-                                      kMaxWaitUsDb, (cudaStream_t)stream, t8);
+                                      (cudaStream_t)stream, t8);
 }

@@ -381,10 +381,9 @@ int encode_frame(gpu_context_t* ctx, Impl* m, const uint8_t* y, const uint8_t* u
     // Deblocked as independent tiles from the unfiltered reconstruction
     // into the other buffer: the previous reconstruction, which nothing
     // reads once the P chain (or the intra wavefront) has run.
-    rc |= cudaMemsetAsync(scr1, 0, m->scratch_words * 4, m->stream) == cudaSuccess ? 0 : -1;
     uint8_t* db_y = m->rec[m->cur];
     rc |= b200enc_deblock_tiles_launch(m->mbw, m->mbh, qp, is_intra, m->d_nz, m->d_mv, out_y, out_uv, db_y,
-                                       db_y + luma, m->pitch, scr1, kWavefrontMaxWaitUs, m->stream);
+                                       db_y + luma, m->pitch, scr1, m->stream);
   }
   perf_mark(m, 3);
   sl.num_slices = 0;

@@ -129,13 +129,13 @@ int b200enc_deblock(int mbw, int mbh, int qp, int is_intra,
 /* The same deblocking (identical output), from an unfiltered reconstruction
  * src_y/src_uv to a separate destination dst_y/dst_uv (same pitch; the
  * destination planes must not overlap the source planes), as independent
- * tiles: each tile of TW x TH macroblocks (8 x 8 unless tuned,
- * B200ENC_TUNE_DEBLOCK_TILE_W/_H) is deblocked in raster order together with
- * one macroblock of margin on every side and stored alone, which reproduces
+ * tiles: each tile of TW x TH macroblocks (4 x 4 up to 4,096 macroblocks and
+ * 8 x 8 above, unless tuned: B200ENC_TUNE_DEBLOCK_TILE_W/_H) is deblocked
+ * with the margin samples it depends on and stored alone, which reproduces
  * the whole picture's raster order on the tile. Replaces the same shader
  * dispatch as b200enc_deblock (src/gpu_compute.c:3261-3290). `status` is 16
- * bytes of device memory, zeroed here; word 1 is nonzero if a wait inside a
- * tile gave up. Pitch and bases must be multiples of 16. */
+ * bytes of device memory, zeroed here (no wait inside a tile can give up).
+ * Pitch and bases must be multiples of 16. */
 int b200enc_deblock_tiles(int mbw, int mbh, int qp, int is_intra,
                           const uint32_t *nz, const void *mv,
                           const uint8_t *src_y, const uint8_t *src_uv,
@@ -195,8 +195,8 @@ int b200enc_deblock_noalloc_status(uint32_t *status_host, void *stream);
  * launch per stage over all of them: ME over every P macroblock of every P
  * stream (me_mode 0 full search, 1 learned form with BF16 inference, 3 with
  * FP8), the P chain over the same macroblocks, the intra wavefront over
- * every I stream's macroblock rows, and the deblocking wavefront (deblock !=
- * 0) over every stream's row groups. Each stream's outputs and
+ * every I stream's macroblock rows, and the tile deblocking (deblock != 0)
+ * over every stream's tiles. Each stream's outputs and
  * reconstruction equal a single-stream context's (b200enc_ctx_*, same
  * search range, lambda 5, zero-MV threshold 512, clamping at the coded size,
  * the intra corner check) given the same frames, QPs and frame kinds.
@@ -240,8 +240,8 @@ int b200enc_batch_graph_stats(void *b, long *instantiations, long *updates);
 #define B200ENC_TUNE_FALLBACK_CTAS_PER_SM 3 /* fallback full-search grid, CTAs per SM, 1..16 (default 8) */
 #define B200ENC_TUNE_INTRA_CTAS 4           /* intra wavefront CTAs (rows in flight), >= 1 (default: one per row) */
 #define B200ENC_TUNE_ME_STAGE 5             /* full-search window staging: 1 word loads, 2 TMA (default TMA) */
-#define B200ENC_TUNE_DEBLOCK_TILE_W 6       /* tile deblocking: tile width in macroblocks, 1..16 (default 8) */
-#define B200ENC_TUNE_DEBLOCK_TILE_H 7       /* tile deblocking: tile height in macroblocks, 1..8 (default 8) */
+#define B200ENC_TUNE_DEBLOCK_TILE_W 6       /* tile deblocking: tile width in macroblocks, 1..16 (default 4 or 8, by size) */
+#define B200ENC_TUNE_DEBLOCK_TILE_H 7       /* tile deblocking: tile height in macroblocks, 1..8 (default 4 or 8, by size) */
 #define B200ENC_TUNE_COUNT 8
 /* Sets a knob (0 restores the default); -1 for an unknown key or a value
  * out of range. */
