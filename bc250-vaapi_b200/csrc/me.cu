@@ -10,15 +10,29 @@
 // reach of the refine) is staged once in shared memory, by one 2-D TMA load
 // (cp.async.bulk.tensor, no multicast) of a box that starts on the 16-byte
 // boundary 12 bytes left of the window when the window lies inside the
-// reference plane, by clamped word loads into the same layout at the
-// picture edges and in batched steps; the current MB sits
-// in 64 registers per thread. Thread t owns candidate column dx = t - R and
-// sweeps the window rows top to bottom: each row's 16 bytes (one funnel
-// shift per word off 5 aligned shared loads) feed the SADs of the 16
-// candidates that use that row, accumulated in a 16-slot ring, so every
-// window byte is read once per column. SAD is the byte-SIMD
-// vabsdiff4-with-add; the integer path uses no tensor cores. The column
-// dx = +R is scored directly, one candidate per thread, after the sweep.
+// reference plane, by clamped word loads into the same layout at the picture
+// edges and in batched steps. The search is exhaustive by elimination:
+//   1. a lower bound of every candidate's cost, thread t owning column
+//      dx = t - R: the SAD is at least the sum over the four 8x8 blocks of
+//      |difference of the blocks' sample sums| (successive elimination, Li and
+//      Salari 1995), formed from running 8-row sums of the column's samples
+//      (dp4a on masked words, sad.u32);
+//   2. an upper bound: the exact costs of the zero vector, of each column's
+//      candidate of smallest bound and of the column dx = +R;
+//   3. the exact SADs of every run of eight candidates of a column whose bound
+//      does not exceed it, listed and searched a run per thread: each window
+//      row's 16 bytes (one funnel shift per word off 5 aligned shared loads)
+//      feed the runs' candidates that use it (vabsdiff4 with add).
+// A candidate is dropped only when its bound exceeds a cost another candidate
+// has, so the winner and the raster tie-break are the exhaustive search's.
+//
+// What bounds it: the integer ALU (vabsdiff4, funnel shifts, sad at 64 lanes
+// per clock and SM) and the issue slots; a 1080p window set is 4 MB of DRAM.
+// Scoring every candidate in an 80-row sweep took 244 us for a 1080p frame at
+// R = 32 (ALU pipe 81 %, a fifth of it on rows outside the range) and 123 at
+// R = 16 with a scalar refine; now, on textured video with 10 % uniform noise,
+// 146 and 70 (30 and 50 % of the runs survive), 90 and 49 on smooth video
+// (2 %); on uniform noise, where every run survives, 243 and 83.
 #include <cuda.h>
 
 #include <algorithm>
@@ -30,6 +44,8 @@
 
 namespace b200enc {
 
+constexpr int kMeUnit = 8;  // candidates of a column searched (or ruled out) together
+
 template <int R>
 struct MeShared {
   static constexpr int WP = 2 * R + 24;                   // window side in pels
@@ -38,10 +54,13 @@ struct MeShared {
   static constexpr int BW = (4 * OFF + WP + 15) / 16 * 16;  // staged row: the TMA box width in bytes
   static constexpr int WS = BW / 4;                       // 32-bit words per staged row
   alignas(128) uint32_t win[WP * WS];
-  uint32_t cur[64];
+  alignas(16) uint32_t cur[64];
   uint32_t red[8];
+  uint16_t ubound[2 * R * (2 * R / kMeUnit)];  // half (rounded down) of each unit's smallest bound
+  uint32_t nlist;                          // units to search exactly
+  uint16_t list[2 * R * (2 * R / kMeUnit)];
   uint64_t bar;  // TMA completion
-  RefineShared rf;
+  RefineSimd rf;
 };
 static_assert(MeShared<16>::BW == 80 && MeShared<32>::BW == 112, "box widths");
 
@@ -55,8 +74,14 @@ enum : int { kMeGrid = 0, kMeList = 1, kMeBatch = 2, kMeBatchList = 3 };
 // Error word of launches given no scratch word (b200enc_me_wait_errors).
 __device__ uint32_t g_me_wait_err;
 
+// CTAs of one SM the kernel is compiled for: 30 warps of 64 registers (20
+// warps of 96, all of the current macroblock in registers: 152 us for the
+// 1080p frame that takes 149 at 30, before the smaller refine).
+template <int R>
+constexpr int kMeCtas = R == 32 ? 15 : 30;
+
 template <int R, int MODE>
-__global__ void __launch_bounds__(2 * R) me_full_search_kernel(const uint8_t* __restrict__ cur_, int cur_pitch_,
+__global__ void __launch_bounds__(2 * R, kMeCtas<R>) me_full_search_kernel(const uint8_t* __restrict__ cur_, int cur_pitch_,
                                                                const uint8_t* __restrict__ ref_, int ref_pitch_,
                                                                Geo g_, int lambda_, int zero_thresh_,
                                                                MV* __restrict__ out_, const int* __restrict__ mb_list,
@@ -68,7 +93,10 @@ __global__ void __launch_bounds__(2 * R) me_full_search_kernel(const uint8_t* __
   constexpr int WP = S::WP, WW = S::WW, WS = S::WS, OFF = S::OFF, SIDE = 2 * R + 1;
   constexpr uint64_t kWaitNs = 2000000000ull;
   __shared__ S sh;
-  const int tid = threadIdx.x;
+  // The refine, the corner candidate and a last partial round of units run on
+  // the first logical warp; every other CTA swaps its warps, so that this work
+  // does not always fall to the same two of an SM's four schedulers.
+  const int tid = NT > 32 ? (int)(threadIdx.x ^ (((blockIdx.x + blockIdx.y) & 1u) << 5)) : (int)threadIdx.x;
   // the map describes this launch's single reference plane; batched steps
   // read one plane per stream and stage with loads
   const bool tma_ok = (MODE == kMeGrid || MODE == kMeList) && use_tma;
@@ -179,77 +207,185 @@ __global__ void __launch_bounds__(2 * R) me_full_search_kernel(const uint8_t* __
     continue;
   }
 
-  // ---- integer full search: column sweep ---------------------------------
-  uint32_t cw[16][4];
+  // ---- integer full search ------------------------------------------------
+  // 1. Lower bounds of every candidate's cost, a column per thread: the SAD of
+  // a 16x16 block is at least the sum over its four 8x8 blocks of the
+  // difference of their sample sums. Each window row gives the column's two
+  // 8-sample sums (packed in halves of a word), a ring keeps the last eight.
+  const int lam = lambda;
+  const uint32_t lam_dx = (uint32_t)lam * (uint32_t)abs(tid - R);
+  const uint32_t* wcol = sh.win + 4 * WS + OFF + ((tid + 4) >> 2);  // window row 0 of this thread's column
+  const int wsh = ((tid + 4) & 3) * 8;
+  constexpr int NU = 2 * R / kMeUnit;  // units (runs of kMeUnit candidates) per column
+  uint32_t lkey, ckey = 0xffffffffu;   // smallest (bound << 14 | raster index) of the last row, of the column
+  {
+    uint32_t c00, c01, c10, c11;  // the current macroblock's 8x8 sums
+    {
+      const uint32_t w0 = sh.cur[2 * lane_id()], w1 = sh.cur[2 * lane_id() + 1];  // a lane per half row
+      uint32_t s8 = __dp4a(w1, 0x01010101u, __dp4a(w0, 0x01010101u, 0u));
 #pragma unroll
-  for (int r = 0; r < 16; ++r)
-#pragma unroll
-    for (int w = 0; w < 4; ++w) cw[r][w] = sh.cur[r * 4 + w];
-
-  const int dx = tid - R;
-  const int col = tid + 4;  // window byte column of candidate dx
-  const int wb = col >> 2, shft = (col & 3) * 8;
-  const uint32_t lam_dx = (uint32_t)lambda * (uint32_t)abs(dx);
-  uint32_t acc[16];
-#pragma unroll
-  for (int s = 0; s < 16; ++s) acc[s] = 0;
-  uint32_t best = 0xffffffffu;
-  constexpr int G = (2 * R + 16) / 16;
-  for (int gi = 0; gi < G; ++gi) {
-#pragma unroll
-    for (int k = 0; k < 16; ++k) {
-      const int wrow = gi * 16 + k;
-      const uint32_t* rowp = sh.win + (4 + wrow) * WS + OFF + wb;
-      const uint32_t w0 = rowp[0], w1 = rowp[1], w2 = rowp[2], w3 = rowp[3], w4 = rowp[4];
-      const uint32_t r0 = __funnelshift_r(w0, w1, shft), r1 = __funnelshift_r(w1, w2, shft);
-      const uint32_t r2 = __funnelshift_r(w2, w3, shft), r3 = __funnelshift_r(w3, w4, shft);
-#pragma unroll
-      for (int r = 0; r < 16; ++r) {
-        uint32_t a = acc[(k - r) & 15];
-        a = sad4_acc(r0, cw[r][0], a);
-        a = sad4_acc(r1, cw[r][1], a);
-        a = sad4_acc(r2, cw[r][2], a);
-        a = sad4_acc(r3, cw[r][3], a);
-        acc[(k - r) & 15] = a;
-      }
-      // slot (k+1)&15 now holds the finished candidate cy = wrow - 15
-      const int cy = wrow - 15;
-      const int sl = (k + 1) & 15;
-      if (cy >= 0) {
-        const uint32_t cost = acc[sl] + lam_dx + (uint32_t)lambda * (uint32_t)abs(cy - R);
-        best = min(best, (cost << 14) | (uint32_t)(cy * SIDE + tid));
-      }
-      acc[sl] = 0;
+      for (int o = 2; o < 16; o <<= 1) s8 += __shfl_xor_sync(0xffffffffu, s8, o);
+      c00 = __shfl_sync(0xffffffffu, s8, 0);
+      c01 = __shfl_sync(0xffffffffu, s8, 1);
+      c10 = __shfl_sync(0xffffffffu, s8, 16);
+      c11 = __shfl_sync(0xffffffffu, s8, 17);
     }
+    // Rings over the last eight rows: row sums, sums of the eight rows ending
+    // at a row, of the column's left and right eight samples. Candidate cy
+    // covers window rows cy .. cy + 15 of the column: its upper sums ended at
+    // row cy + 7, its lower ones end at cy + 15. The first two passes (rows
+    // -1 .. 14) only fill the rings.
+    uint32_t hl[8], hr[8], vl[8], vr[8], rl = 0, rr = 0;
+#pragma unroll
+    for (int k = 0; k < 8; ++k) hl[k] = hr[k] = vl[k] = vr[k] = 0;
+    // An unaligned run of eight bytes is the sum of three words' masked bytes.
+    const uint32_t m0 = 0x01010101u << wsh, m2 = wsh ? 0x01010101u >> (32 - wsh) : 0u;
+    auto bound = [&](int k, int cy) -> uint32_t {  // k = cy & 7, a constant
+      const uint32_t* rp = wcol + (cy + 15) * WS;
+      const uint32_t w0 = rp[0], w1 = rp[1], w2 = rp[2], w3 = rp[3], w4 = rp[4];
+      const uint32_t nl = __dp4a(w2, m2, __dp4a(w1, 0x01010101u, __dp4a(w0, m0, 0u)));
+      const uint32_t nr = __dp4a(w4, m2, __dp4a(w3, 0x01010101u, __dp4a(w2, m0, 0u)));
+      rl += nl - hl[k];
+      rr += nr - hr[k];
+      hl[k] = nl;
+      hr[k] = nr;
+      uint32_t lb = lam_dx + (uint32_t)(lam * abs(cy - R));
+      lb = __usad(rr, c11, __usad(rl, c10, __usad(vr[k], c01, __usad(vl[k], c00, lb))));
+      vl[k] = rl;
+      vr[k] = rr;
+      return (lb << 14) | (uint32_t)(cy * SIDE + tid);
+    };
+#pragma unroll 1
+    for (int u = -2; u < NU; ++u) {
+      uint32_t m = 0xffffffffu;
+#pragma unroll
+      for (int k = 0; k < kMeUnit; ++k) m = min(m, bound(k & 7, u * kMeUnit + k));
+      if (u >= 0) {
+        sh.ubound[u * NT + tid] = (uint16_t)(m >> 15);
+        ckey = min(ckey, m);
+      }
+    }
+    lkey = bound(0, 2 * R);
+    ckey = min(ckey, lkey);
   }
-  // column dx = +R (aligned), candidates cy = tid and, for thread 0, cy = 2R
-  for (int cy = tid; cy <= 2 * R; cy += NT) {
+
+  // 2. An upper bound: the exact costs of the zero vector, of each column's
+  // candidate of smallest bound and of the column dx = +R (aligned words).
+  auto key_of = [&](uint32_t sad, int cx, int cy) -> uint32_t {
+    return ((sad + (uint32_t)(lam * (abs(cx - R) + abs(cy - R)))) << 14) | (uint32_t)(cy * SIDE + cx);
+  };
+  auto exact = [&](int cx, int cy) -> uint32_t {
+    const uint32_t* rp = sh.win + (4 + cy) * WS + OFF + ((cx + 4) >> 2);
+    const int xs = ((cx + 4) & 3) * 8;
     uint32_t s = 0;
-#pragma unroll
-    for (int r = 0; r < 16; ++r) {
-      const uint32_t* rowp = sh.win + (4 + cy + r) * WS + OFF + (2 * R + 4) / 4;
-      s = sad4_acc(rowp[0], cw[r][0], s);
-      s = sad4_acc(rowp[1], cw[r][1], s);
-      s = sad4_acc(rowp[2], cw[r][2], s);
-      s = sad4_acc(rowp[3], cw[r][3], s);
+#pragma unroll 2
+    for (int r = 0; r < 16; ++r, rp += WS) {
+      const uint4 c = reinterpret_cast<const uint4*>(sh.cur)[r];
+      const uint32_t w0 = rp[0], w1 = rp[1], w2 = rp[2], w3 = rp[3], w4 = rp[4];
+      s = sad4_acc(__funnelshift_r(w0, w1, xs), c.x, s);
+      s = sad4_acc(__funnelshift_r(w1, w2, xs), c.y, s);
+      s = sad4_acc(__funnelshift_r(w2, w3, xs), c.z, s);
+      s = sad4_acc(__funnelshift_r(w3, w4, xs), c.w, s);
     }
-    const uint32_t cost = s + (uint32_t)lambda * (uint32_t)(R + abs(cy - R));
-    best = min(best, (cost << 14) | (uint32_t)(cy * SIDE + 2 * R));
+    return key_of(s, cx, cy);
+  };
+  uint32_t best = key_of(sad0, R, R);
+#pragma unroll 1
+  for (int j = 0; j < 2; ++j) best = min(best, j ? exact(2 * R, tid) : exact(tid, (int)(ckey & 0x3fffu) / SIDE));
+  if (tid < 32) {  // the corner (+R, +R): a row per lane
+    const uint32_t* rp = sh.win + (4 + 2 * R + (tid & 15)) * WS + OFF + (2 * R + 4) / 4;
+    const uint4 c = reinterpret_cast<const uint4*>(sh.cur)[tid & 15];
+    uint32_t s = sad4_acc(rp[3], c.w, sad4_acc(rp[2], c.z, sad4_acc(rp[1], c.y, sad4_acc(rp[0], c.x, 0u))));
+    s = __reduce_add_sync(0xffffffffu, tid < 16 ? s : 0u);
+    best = min(best, key_of(s, 2 * R, 2 * R));
+  }
+  best = block_min<NT>(best, sh.red);
+
+  // 3. The units whose bound does not exceed it, listed unit row by unit row
+  // (neighbouring columns stay neighbours: their window words are in
+  // different banks), and their exact costs, one unit per thread: kMeUnit
+  // candidates share the window rows they have in common.
+  const uint32_t ub = best >> 14;
+  {
+    uint32_t alive[NU], total = 0;
+#pragma unroll
+    for (int u = 0; u < NU; ++u) {
+      alive[u] = __ballot_sync(0xffffffffu, 2u * sh.ubound[u * NT + tid] <= ub);
+      total += (uint32_t)__popc(alive[u]);
+    }
+    const int lane = lane_id();
+    uint32_t base = 0;
+    if (NT > 32) {
+      if (tid == 0) sh.nlist = 0;
+      __syncthreads();
+      if (lane == 0 && total) base = atomicAdd(&sh.nlist, total);
+      base = __shfl_sync(0xffffffffu, base, 0);
+    } else if (lane == 0) {
+      sh.nlist = total;
+    }
+#pragma unroll
+    for (int u = 0; u < NU; ++u) {
+      if ((alive[u] >> lane) & 1u) sh.list[base + __popc(alive[u] & ((1u << lane) - 1u))] = (uint16_t)(u * NT + tid);
+      base += (uint32_t)__popc(alive[u]);
+    }
+    if ((lkey >> 14) <= ub) best = min(best, exact(tid, 2 * R));
+    if (NT > 32) __syncthreads();
+    else __syncwarp();
+  }
+  const int n_units = (int)sh.nlist;
+#pragma unroll 1
+  for (int i = tid; i < n_units; i += NT) {
+    const int e = sh.list[i], cx = e & (NT - 1), cy0 = (e / NT) * kMeUnit;
+    const uint32_t* up = sh.win + (4 + cy0) * WS + OFF + ((cx + 4) >> 2);
+    const int us = ((cx + 4) & 3) * 8;
+    uint32_t acc[kMeUnit];
+#pragma unroll
+    for (int c = 0; c < kMeUnit; ++c) acc[c] = 0;
+    // the macroblock's upper, then its lower eight rows: 32 registers of
+    // current samples instead of 64, which lets twice the CTAs share an SM
+#pragma unroll 1
+    for (int hb = 0; hb < 2; ++hb, up += 8 * WS) {
+      uint32_t cw[8][4];
+#pragma unroll
+      for (int r = 0; r < 8; ++r) {
+        const uint4 c = reinterpret_cast<const uint4*>(sh.cur)[8 * hb + r];
+        cw[r][0] = c.x;
+        cw[r][1] = c.y;
+        cw[r][2] = c.z;
+        cw[r][3] = c.w;
+      }
+#pragma unroll
+      for (int k = 0; k < kMeUnit + 7; ++k) {
+        const uint32_t* rp = up + k * WS;
+        const uint32_t w0 = rp[0], w1 = rp[1], w2 = rp[2], w3 = rp[3], w4 = rp[4];
+        const uint32_t r0 = __funnelshift_r(w0, w1, us), r1 = __funnelshift_r(w1, w2, us);
+        const uint32_t r2 = __funnelshift_r(w2, w3, us), r3 = __funnelshift_r(w3, w4, us);
+#pragma unroll
+        for (int c = 0; c < kMeUnit; ++c) {
+          const int r = k - c;
+          if (r < 0 || r > 7) continue;
+          acc[c] =
+              sad4_acc(r3, cw[r][3], sad4_acc(r2, cw[r][2], sad4_acc(r1, cw[r][1], sad4_acc(r0, cw[r][0], acc[c]))));
+        }
+      }
+    }
+#pragma unroll
+    for (int c = 0; c < kMeUnit; ++c) best = min(best, key_of(acc[c], cx, cy0 + c));
   }
   best = block_min<NT>(best, sh.red);
   const int idx = (int)(best & 0x3fffu);
   const int mx = idx % SIDE - R, my = idx / SIDE - R;
   const uint32_t int_sad = (best >> 14) - (uint32_t)lambda * (uint32_t)(abs(mx) + abs(my));
 
-  // ---- half/quarter-pel refine around the winner -------------------------
-  const uint8_t* wb8 = reinterpret_cast<const uint8_t*>(sh.win) + 4 * OFF;
-  const int px0 = mx + R + 4, py0 = my + R + 4;  // window coords of the winner
-  auto G8 = [&](int rx, int ry) -> int { return wb8[(py0 + ry) * S::BW + px0 + rx]; };
-  int qx, qy;
-  const uint32_t bsad =
-      qpel_refine<NT>(sh.rf, G8, reinterpret_cast<const uint8_t*>(sh.cur), int_sad, &qx, &qy);
-  if (tid == 0)
-    *o = MV{4 * mx + qx, 4 * my + qy, bsad, (flags & B200ENC_ME_LOG_INTEGER) ? me_log_word(mx, my, false) : 0u};
+  // ---- half/quarter-pel refine around the winner (one warp) ---------------
+  if (tid < 32) {
+    int qx, qy;
+    const uint32_t bsad =
+        qpel_refine_warp_simd(sh.rf, reinterpret_cast<const uint8_t*>(sh.win) + 4 * OFF, S::BW, my + R + 4, mx + R + 4,
+                              sh.cur, int_sad, &qx, &qy);
+    if (tid == 0)
+      *o = MV{4 * mx + qx, 4 * my + qy, bsad, (flags & B200ENC_ME_LOG_INTEGER) ? me_log_word(mx, my, false) : 0u};
+  }
   }
 }
 
@@ -339,9 +475,9 @@ int b200enc_me_full_search_err(const uint8_t* cur_y, int cur_pitch, const uint8_
   if (mb_list && (list_capacity <= 0 || list_capacity > g.mbw * g.mbh)) return -1;
   int sms = 148, dev = 0;
   if (mb_list && cudaGetDevice(&dev) == cudaSuccess) cudaDeviceGetAttribute(&sms, cudaDevAttrMultiProcessorCount, dev);
-  // list mode: a persistent grid of up to 8 CTAs per SM (or the tuned
+  // list mode: a persistent grid of up to 16 CTAs per SM (or the tuned
   // count) walks the list
-  const int per_sm = b200enc_tuned(B200ENC_TUNE_FALLBACK_CTAS_PER_SM) > 0 ? b200enc_tuned(B200ENC_TUNE_FALLBACK_CTAS_PER_SM) : 8;
+  const int per_sm = b200enc_tuned(B200ENC_TUNE_FALLBACK_CTAS_PER_SM) > 0 ? b200enc_tuned(B200ENC_TUNE_FALLBACK_CTAS_PER_SM) : 16;
   dim3 grid = mb_list ? dim3(std::min(list_capacity, per_sm * sms)) : dim3(g.mbw, g.mbh);
   const bool list = mb_list != nullptr;
   switch (range) {

@@ -14,6 +14,8 @@ __device__ __forceinline__ uint32_t sad4_acc(uint32_t a, uint32_t b, uint32_t c)
   return d;
 }
 
+__device__ __forceinline__ int lane_id() { return (int)(threadIdx.x & 31); }
+
 template <int NT>
 __device__ __forceinline__ uint32_t block_sum(uint32_t v, uint32_t* red) {
 #pragma unroll
@@ -61,141 +63,101 @@ __device__ __forceinline__ uint32_t load_word_clamped(const uint8_t* row, int gx
          ((uint32_t)__ldg(row + clampi(gx + 3, 0, RW - 1)) << 24);
 }
 
-// Refine planes over coordinates relative to the integer winner: columns
-// -1..16 and rows -1..16 (18 x 18); raw horizontal 6-tap sums for rows
-// -3..19 (23 x 18).
-struct RefineShared {
-  int16_t pb[18][18], ph[18][18], pj[18][18];
-  int32_t hr[23][18];
-  uint32_t part[8][4];
-};
-
-// Half- then quarter-pel refine around an integer winner whose integer SAD
-// is int_sad. G8(rx, ry) returns the reference pel at offset (rx, ry) from
-// the winner's top-left, for rx, ry in [-3, 19]. cur: the 256 current pels
-// in shared memory. Every thread of the NT-thread block calls it and gets
-// the same result: (*qx, *qy) the quarter-pel offset from the winner and
-// the winning SAD (strict improvement only, offsets tried in table order).
-// With NT == 32 the caller may be one warp of a larger block: only the warp
-// synchronises, and the sums come from shuffles alone.
-template <int NT, class G8F>
-__device__ __forceinline__ uint32_t qpel_refine(RefineShared& rf, G8F G8, const uint8_t* cur, uint32_t int_sad,
-                                                int* qx_out, int* qy_out) {
-  const int tid = NT == 32 ? (int)(threadIdx.x & 31) : (int)threadIdx.x;
-  for (int i = tid; i < 23 * 18; i += NT) {
-    const int ry = i / 18 - 3, rx = i % 18 - 1;
-    rf.hr[ry + 3][rx + 1] = G8(rx - 2, ry) - 5 * G8(rx - 1, ry) + 20 * G8(rx, ry) + 20 * G8(rx + 1, ry) -
-                             5 * G8(rx + 2, ry) + G8(rx + 3, ry);
-  }
-  if (NT == 32) __syncwarp(); else __syncthreads();
-  for (int i = tid; i < 18 * 18; i += NT) {
-    const int ry = i / 18 - 1, rx = i % 18 - 1;
-    rf.pb[ry + 1][rx + 1] = (int16_t)clip1((rf.hr[ry + 3][rx + 1] + 16) >> 5);
-    const int v = G8(rx, ry - 2) - 5 * G8(rx, ry - 1) + 20 * G8(rx, ry) + 20 * G8(rx, ry + 1) -
-                  5 * G8(rx, ry + 2) + G8(rx, ry + 3);
-    rf.ph[ry + 1][rx + 1] = (int16_t)clip1((v + 16) >> 5);
-    const int j1 = rf.hr[ry + 1][rx + 1] - 5 * rf.hr[ry + 2][rx + 1] + 20 * rf.hr[ry + 3][rx + 1] +
-                   20 * rf.hr[ry + 4][rx + 1] - 5 * rf.hr[ry + 5][rx + 1] + rf.hr[ry + 6][rx + 1];
-    rf.pj[ry + 1][rx + 1] = (int16_t)clip1((j1 + 512) >> 10);
-  }
-  if (NT == 32) __syncwarp(); else __syncthreads();
-
-  // One quarter-pel sample at offset (rx, ry) from the winner with phase
-  // (fy*4 + fx); the letters and averages of motion_estimation.comp:197-213,
-  // loading only the operands the phase uses (phase is uniform per call).
-  auto sample = [&](int phase, int rx, int ry) -> int {
-    switch (phase) {
-      case 0: return G8(rx, ry);
-      case 1: return (G8(rx, ry) + rf.pb[ry + 1][rx + 1] + 1) >> 1;
-      case 2: return rf.pb[ry + 1][rx + 1];
-      case 3: return (rf.pb[ry + 1][rx + 1] + G8(rx + 1, ry) + 1) >> 1;
-      case 4: return (G8(rx, ry) + rf.ph[ry + 1][rx + 1] + 1) >> 1;
-      case 5: return (rf.pb[ry + 1][rx + 1] + rf.ph[ry + 1][rx + 1] + 1) >> 1;
-      case 6: return (rf.pb[ry + 1][rx + 1] + rf.pj[ry + 1][rx + 1] + 1) >> 1;
-      case 7: return (rf.pb[ry + 1][rx + 1] + rf.ph[ry + 1][rx + 2] + 1) >> 1;
-      case 8: return rf.ph[ry + 1][rx + 1];
-      case 9: return (rf.ph[ry + 1][rx + 1] + rf.pj[ry + 1][rx + 1] + 1) >> 1;
-      case 10: return rf.pj[ry + 1][rx + 1];
-      case 11: return (rf.pj[ry + 1][rx + 1] + rf.ph[ry + 1][rx + 2] + 1) >> 1;
-      case 12: return (rf.ph[ry + 1][rx + 1] + G8(rx, ry + 1) + 1) >> 1;
-      case 13: return (rf.ph[ry + 1][rx + 1] + rf.pb[ry + 2][rx + 1] + 1) >> 1;
-      case 14: return (rf.pj[ry + 1][rx + 1] + rf.pb[ry + 2][rx + 1] + 1) >> 1;
-      default: return (rf.ph[ry + 1][rx + 2] + rf.pb[ry + 2][rx + 1] + 1) >> 1;
-    }
-  };
-
-  // Eight candidates, one at a time: per-thread partial SADs, then a block
-  // (or warp) reduction per candidate.
-  auto score8 = [&](const int8_t (*off)[2], int bx, int by, uint32_t* res) {
-    for (int c = 0; c < 8; ++c) {
-      const int ox_ = bx + off[c][0], oy_ = by + off[c][1];  // quarter-pel offset from the integer winner
-      const int dx = ox_ >> 2, dy = oy_ >> 2, phase = (oy_ & 3) * 4 + (ox_ & 3);
-      uint32_t p = 0;
-      for (int pix = tid; pix < 256; pix += NT) {
-        const int x = pix & 15, y = pix >> 4;
-        p += (uint32_t)abs((int)cur[pix] - sample(phase, x + dx, y + dy));
-      }
-#pragma unroll
-      for (int o2 = 16; o2 > 0; o2 >>= 1) p += __shfl_xor_sync(0xffffffffu, p, o2);
-      res[c] = p;
-      if (NT > 32 && (tid & 31) == 0) rf.part[c][tid >> 5] = p;
-    }
-    if (NT == 32) return;
-    __syncthreads();
-#pragma unroll
-    for (int c = 0; c < 8; ++c) {
-      uint32_t sum = 0;
-#pragma unroll
-      for (int w = 0; w < NT / 32; ++w) sum += rf.part[c][w];
-      res[c] = sum;
-    }
-    __syncthreads();  // part[] is rewritten by the next call
-  };
-
-  uint32_t cs[8];
-  score8(kHalfOff, 0, 0, cs);
-  uint32_t bsad = int_sad;
-  int hx = 0, hy = 0;
-#pragma unroll
-  for (int c = 0; c < 8; ++c)
-    if (cs[c] < bsad) { bsad = cs[c]; hx = kHalfOff[c][0]; hy = kHalfOff[c][1]; }
-  score8(kQtrOff, hx, hy, cs);
-  int qx = 0, qy = 0;
-#pragma unroll
-  for (int c = 0; c < 8; ++c)
-    if (cs[c] < bsad) { bsad = cs[c]; qx = kQtrOff[c][0]; qy = kQtrOff[c][1]; }
-  *qx_out = hx + qx;
-  *qy_out = hy + qy;
-  return bsad;
-}
-
 // ---------------------------------------------------------------------------
-// The same refine for one warp, on byte-SIMD words: the half-pel planes are
-// bytes (their values are clipped to 0..255), every quarter-pel sample is
-// either a plane value or the rounded byte average (a + b + 1) >> 1 of two,
-// which vavgu4 forms for 4 pels at once, and vabsdiff4 accumulates the SAD.
-// Results are identical to qpel_refine.
+// Half- then quarter-pel refine around an integer winner (strict improvement
+// only, offsets tried in table order), one warp, on byte-SIMD words: the
+// half-pel planes are bytes (their values are clipped to 0..255), every
+// quarter-pel sample is either a plane value or the rounded byte average
+// (a + b + 1) >> 1 of two, which vavgu4 forms for 4 pels at once, and
+// vabsdiff4 accumulates the SAD. Instructions bound it (one warp per
+// macroblock, no reuse between macroblocks): the planes take one pass of
+// packed 16-bit arithmetic instead of eleven passes of a sample per lane, the
+// positions one loop instead of sixteen unrolled bodies. Re-scoring a 640x480
+// frame: 13.8 -> 11.1 us; the fallback search of a few macroblocks: 31 -> 17.
 struct RefineSimd {
-  alignas(4) int16_t hr[23][18];  // 6-tap sums of 8-bit samples: -2550 .. 10710
   alignas(4) uint8_t pl[3][18][20];  // b, h, j at [ry+1][rx+1], ry, rx in -1..16
 };
 
 // The operands of each quarter-pel phase (fy*4+fx), motion_estimation.comp:
-// 197-213: {plane, sx, sy} twice (plane 0 G, 1 b, 2 h, 3 j, -1 none); the
-// sample is the first operand or the rounded average of both.
-__constant__ int8_t kQpelOp[16][6] = {
-    {0, 0, 0, -1, 0, 0}, {0, 0, 0, 1, 0, 0}, {1, 0, 0, -1, 0, 0}, {1, 0, 0, 0, 1, 0},
-    {0, 0, 0, 2, 0, 0},  {1, 0, 0, 2, 0, 0}, {1, 0, 0, 3, 0, 0},  {1, 0, 0, 2, 1, 0},
-    {2, 0, 0, -1, 0, 0}, {2, 0, 0, 3, 0, 0}, {3, 0, 0, -1, 0, 0}, {3, 0, 0, 2, 1, 0},
-    {2, 0, 0, 0, 0, 1},  {2, 0, 0, 1, 0, 1}, {3, 0, 0, 1, 0, 1},  {2, 1, 0, 1, 0, 1}};
+// 197-213: plane (0 G, 1 b, 2 h, 3 j) and extra shifts sx, sy of each; the
+// sample is the rounded average of both, which is the operand itself where a
+// phase has one (listed twice). Bits: plane a 0-1, sx a 2, sy a 3, plane b
+// 4-5, sx b 6, sy b 7.
+#define B200ENC_QOP(pa, xa, ya, pb, xb, yb) \
+  (uint8_t)((pa) | ((xa) << 2) | ((ya) << 3) | ((pb) << 4) | ((xb) << 6) | ((yb) << 7))
+__constant__ uint8_t kQpelOp[16] = {
+    B200ENC_QOP(0, 0, 0, 0, 0, 0), B200ENC_QOP(0, 0, 0, 1, 0, 0), B200ENC_QOP(1, 0, 0, 1, 0, 0),
+    B200ENC_QOP(1, 0, 0, 0, 1, 0), B200ENC_QOP(0, 0, 0, 2, 0, 0), B200ENC_QOP(1, 0, 0, 2, 0, 0),
+    B200ENC_QOP(1, 0, 0, 3, 0, 0), B200ENC_QOP(1, 0, 0, 2, 1, 0), B200ENC_QOP(2, 0, 0, 2, 0, 0),
+    B200ENC_QOP(2, 0, 0, 3, 0, 0), B200ENC_QOP(3, 0, 0, 3, 0, 0), B200ENC_QOP(3, 0, 0, 2, 1, 0),
+    B200ENC_QOP(2, 0, 0, 0, 0, 1), B200ENC_QOP(2, 0, 0, 1, 0, 1), B200ENC_QOP(3, 0, 0, 1, 0, 1),
+    B200ENC_QOP(2, 1, 0, 1, 0, 1)};
+#undef B200ENC_QOP
 
-// Two words (8 pels) of a byte row starting at byte offset c of a 4-aligned row.
-__device__ __forceinline__ void row8(const uint8_t* row, int c, uint32_t& w0, uint32_t& w1) {
-  const uint32_t* r = reinterpret_cast<const uint32_t*>(row) + (c >> 2);
-  const int sh = (c & 3) * 8;
-  const uint32_t a0 = r[0], a1 = r[1], a2 = r[2];
-  w0 = __funnelshift_r(a0, a1, sh);
-  w1 = __funnelshift_r(a1, a2, sh);
+// Two samples in the 16-bit halves of a word (each 0 .. 65535; sums and
+// multiples stay below 65536 per half, differences are biased to stay
+// non-negative, so plain 32-bit arithmetic never carries across).
+//
+// The 6-tap sum a - 5b + 20c + 20d - 5e + f of byte samples, plus kTapBias
+// (2560 = 80 * 32 > 2550): 10 .. 13270.
+constexpr uint32_t kTapBias = 2560u;
+__device__ __forceinline__ uint32_t tap6_pair(uint32_t a, uint32_t b, uint32_t c, uint32_t d, uint32_t e, uint32_t f) {
+  return (c + d) * 20u + (a + f + kTapBias * 0x10001u) - (b + e) * 5u;
+}
+// clip1((tap + 16) >> 5) of both halves of a biased sum.
+__device__ __forceinline__ uint32_t tap_round_pair(uint32_t t) {
+  const uint32_t v = ((t + 0x00100010u) >> 5) & 0x07ff07ffu;  // + 80
+  uint32_t lo, hi;
+  asm("max.u16x2 %0, %1, %2;" : "=r"(lo) : "r"(v), "r"(0x00500050u));
+  asm("min.u16x2 %0, %1, %2;" : "=r"(hi) : "r"(lo), "r"(0x014f014fu));
+  return hi - 0x00500050u;
+}
+
+// Half-pel planes b, h, j (motion_estimation.comp:154-215) of the 18 x 18
+// positions around the winner: lane = (group of three rows, four columns);
+// the lane reads the eight reference rows its rows reach (nine bytes each)
+// and keeps their horizontal sums in registers, so nothing but the planes is
+// written. g: 4-aligned rows, gstride bytes apart; the winner's top-left pel
+// is at row g_r0, byte g_c0.
+__device__ __forceinline__ void refine_planes(RefineSimd& rf, const uint8_t* g, int gstride, int g_r0, int g_c0,
+                                              int lane) {
+  if (lane < 30) {
+    const int grp = lane / 5, q = lane - 5 * grp;
+    const int bo = g_c0 + 4 * q - 3, sh = (bo & 3) * 8;  // byte of column rx - 2, rx = 4q - 1
+    const uint8_t* rows = g + (g_r0 + 3 * grp - 3) * gstride + (bo & ~3);
+    uint32_t t01[8], t23[8], g01[8], g23[8];  // horizontal sums (biased) and samples, rows 3 grp - 3 .. + 4
+#pragma unroll
+    for (int r = 0; r < 8; ++r) {
+      const uint32_t* wp = reinterpret_cast<const uint32_t*>(rows + r * gstride);
+      const uint32_t a0 = wp[0], a1 = wp[1], a2 = wp[2];
+      const uint32_t lo = __funnelshift_r(a0, a1, sh), hi = __funnelshift_r(a1, a2, sh);  // e0..e3, e4..e7
+      const uint32_t mid = __funnelshift_r(lo, hi, 16), up = __funnelshift_r(hi, a2 >> sh, 24);  // e2..e5, e7 e8 ..
+      const uint32_t p0 = __byte_perm(lo, 0, 0x4140), p1 = __byte_perm(lo, 0, 0x4241), p2 = __byte_perm(lo, 0, 0x4342);
+      const uint32_t p3 = __byte_perm(mid, 0, 0x4241), p4 = __byte_perm(hi, 0, 0x4140);
+      const uint32_t p5 = __byte_perm(hi, 0, 0x4241), p6 = __byte_perm(hi, 0, 0x4342), p7 = __byte_perm(up, 0, 0x4140);
+      t01[r] = tap6_pair(p0, p1, p2, p3, p4, p5);
+      t23[r] = tap6_pair(p2, p3, p4, p5, p6, p7);
+      g01[r] = p2;
+      g23[r] = p4;
+    }
+#pragma unroll
+    for (int k = 0; k < 3; ++k) {  // plane row 3 grp + k (ry = that - 1): reference rows k .. k + 5 of the eight
+      uint32_t* bp = reinterpret_cast<uint32_t*>(&rf.pl[0][3 * grp + k][4 * q]);
+      uint32_t* hp = reinterpret_cast<uint32_t*>(&rf.pl[1][3 * grp + k][4 * q]);
+      uint32_t* jp = reinterpret_cast<uint32_t*>(&rf.pl[2][3 * grp + k][4 * q]);
+      *bp = __byte_perm(tap_round_pair(t01[k + 2]), tap_round_pair(t23[k + 2]), 0x6420);
+      *hp = __byte_perm(tap_round_pair(tap6_pair(g01[k], g01[k + 1], g01[k + 2], g01[k + 3], g01[k + 4], g01[k + 5])),
+                        tap_round_pair(tap6_pair(g23[k], g23[k + 1], g23[k + 2], g23[k + 3], g23[k + 4], g23[k + 5])),
+                        0x6420);
+      // the taps' weights sum to 32, so the bias of the sums comes out as 32 * kTapBias
+      auto jval = [&](const uint32_t* t, int s) -> uint32_t {
+        auto at = [&](int i) -> int { return (int)(s ? t[k + i] >> 16 : t[k + i] & 0xffffu); };
+        const int v = (at(2) + at(3)) * 20 + (at(0) + at(5)) - (at(1) + at(4)) * 5;
+        return (uint32_t)clip1((v - 32 * (int)kTapBias + 512) >> 10);
+      };
+      *jp = __byte_perm(jval(t01, 0) | (jval(t01, 1) << 16), jval(t23, 0) | (jval(t23, 1) << 16), 0x6420);
+    }
+  }
 }
 
 // g: 4-aligned rows of the reference, gstride bytes apart; the integer
@@ -206,121 +168,59 @@ __device__ __forceinline__ uint32_t qpel_refine_warp_simd(RefineSimd& rf, const 
                                                           int g_c0, const uint32_t* cur, uint32_t int_sad,
                                                           int* qx_out, int* qy_out) {
   const int lane = threadIdx.x & 31;
-  auto G8 = [&](int rx, int ry) -> int { return g[(g_r0 + ry) * gstride + g_c0 + rx]; };
-  // horizontal sums, four columns (rx .. rx+3) per lane and pass: the nine
-  // bytes rx-2 .. rx+6 of the row come from three word loads; the pairs of
-  // 16-bit sums are stored as words (hr rows are 36 bytes, rx+1 is 0 mod 4)
-  for (int i = lane; i < 23 * 5; i += 32) {
-    const int q = i / 5, ry = q - 3, rx = (i - 5 * q) * 4 - 1;
-    const int bo = g_c0 + rx - 2;
-    const uint32_t* wp = reinterpret_cast<const uint32_t*>(g + (g_r0 + ry) * gstride) + (bo >> 2);
-    const int sh = (bo & 3) * 8;
-    const uint32_t a0 = wp[0], a1 = wp[1], a2 = wp[2];
-    const uint32_t lo = __funnelshift_r(a0, a1, sh), hi = __funnelshift_r(a1, a2, sh);
-    int e[9];
-#pragma unroll
-    for (int k = 0; k < 4; ++k) {
-      e[k] = (int)((lo >> (8 * k)) & 0xffu);
-      e[k + 4] = (int)((hi >> (8 * k)) & 0xffu);
-    }
-    e[8] = (int)((a2 >> sh) & 0xffu);
-    int v[4];
-#pragma unroll
-    for (int j = 0; j < 4; ++j) v[j] = e[j] - 5 * e[j + 1] + 20 * e[j + 2] + 20 * e[j + 3] - 5 * e[j + 4] + e[j + 5];
-    uint32_t* dst = reinterpret_cast<uint32_t*>(&rf.hr[ry + 3][rx + 1]);
-    dst[0] = (uint32_t)(uint16_t)v[0] | ((uint32_t)(uint16_t)v[1] << 16);
-    if (rx + 3 < 17) dst[1] = (uint32_t)(uint16_t)v[2] | ((uint32_t)(uint16_t)v[3] << 16);
-  }
-  __syncwarp();
-  for (int i = lane; i < 18 * 18; i += 32) {
-    const int ry = i / 18 - 1, rx = i % 18 - 1;
-    rf.pl[0][ry + 1][rx + 1] = (uint8_t)clip1((rf.hr[ry + 3][rx + 1] + 16) >> 5);
-    const int v = G8(rx, ry - 2) - 5 * G8(rx, ry - 1) + 20 * G8(rx, ry) + 20 * G8(rx, ry + 1) -
-                  5 * G8(rx, ry + 2) + G8(rx, ry + 3);
-    rf.pl[1][ry + 1][rx + 1] = (uint8_t)clip1((v + 16) >> 5);
-    const int j1 = rf.hr[ry + 1][rx + 1] - 5 * rf.hr[ry + 2][rx + 1] + 20 * rf.hr[ry + 3][rx + 1] +
-                   20 * rf.hr[ry + 4][rx + 1] - 5 * rf.hr[ry + 5][rx + 1] + rf.hr[ry + 6][rx + 1];
-    rf.pl[2][ry + 1][rx + 1] = (uint8_t)clip1((j1 + 512) >> 10);
-  }
+  refine_planes(rf, g, gstride, g_r0, g_c0, lane);
   __syncwarp();
 
-  const int y = lane >> 1, half = lane & 1;
-  const uint32_t c0 = cur[y * 4 + 2 * half], c1 = cur[y * 4 + 2 * half + 1];
-  // operand (plane p: 0 G, 1 b, 2 h, 3 j; extra shifts sx, sy) of the lane's
-  // 8 pels at integer offset (dx, dy) from the winner
-  auto operand = [&](int p, int dx, int dy, int sx, int sy, uint32_t& w0, uint32_t& w1) {
-    const int ry = y + dy + sy, rx = dx + sx + 8 * half;
-    if (p == 0) row8(g + (g_r0 + ry) * gstride, g_c0 + rx, w0, w1);
-    else row8(&rf.pl[p - 1][ry + 1][0], rx + 1, w0, w1);
-  };
-  auto part = [&](int ox, int oy) -> uint32_t {  // the lane's share of the SAD at quarter-pel (ox, oy)
-    const int dx = ox >> 2, dy = oy >> 2, ph = (oy & 3) * 4 + (ox & 3);
-    uint32_t a0, a1;
-    operand(kQpelOp[ph][0], dx, dy, kQpelOp[ph][1], kQpelOp[ph][2], a0, a1);
-    if (kQpelOp[ph][3] >= 0) {
-      uint32_t b0, b1;
-      operand(kQpelOp[ph][3], dx, dy, kQpelOp[ph][4], kQpelOp[ph][5], b0, b1);
-      a0 = __vavgu4(a0, b0);
-      a1 = __vavgu4(a1, b1);
-    }
-    return sad4_acc(a1, c1, sad4_acc(a0, c0, 0u));
-  };
-  // The 8 positions (bx, by) + off[c] summed over the warp together: the
-  // exchanges at distances 16, 8 and 4 each hand half of the lane's partial
-  // sums to its partner, so that lane L is left with position (L >> 2) & 7,
-  // and two more finish its sum. Returns min over c of (SAD_c << 3 | c): the
-  // smallest SAD, the earliest position among equal ones.
-  // Half-pel positions (kHalfOff order) each read one plane: b at (2,0) and
-  // (-2,0), h at (0,2) and (0,-2), j at the diagonals; the integer offset is
-  // -1 where the quarter-pel offset is -2. Plane and offsets are constants.
-  auto half_part = [&](int c) -> uint32_t {
-    const int p = c < 2 ? 1 : (c < 4 ? 2 : 3);
-    const int dx = (c == 1 || c == 6 || c == 7) ? -1 : 0;
-    const int dy = (c == 3 || c == 5 || c == 7) ? -1 : 0;
-    uint32_t a0, a1;
-    operand(p, dx, dy, 0, 0, a0, a1);
-    return sad4_acc(a1, c1, sad4_acc(a0, c0, 0u));
-  };
-  auto best8 = [&](const int8_t(*off)[2], int bx, int by) -> uint32_t {
-    uint32_t v[8];
-    if (off == nullptr) {
-#pragma unroll
-      for (int c = 0; c < 8; ++c) v[c] = half_part(c);
-    } else {
-#pragma unroll
-      for (int c = 0; c < 8; ++c) v[c] = part(bx + off[c][0], by + off[c][1]);
-    }
-    const bool h16 = lane & 16, h8 = lane & 8, h4 = lane & 4;
-    uint32_t w[4];
-#pragma unroll
-    for (int i = 0; i < 4; ++i)
-      w[i] = (h16 ? v[i + 4] : v[i]) + __shfl_xor_sync(0xffffffffu, h16 ? v[i] : v[i + 4], 16);
-    uint32_t x[2];
-#pragma unroll
-    for (int i = 0; i < 2; ++i)
-      x[i] = (h8 ? w[i + 2] : w[i]) + __shfl_xor_sync(0xffffffffu, h8 ? w[i] : w[i + 2], 8);
-    uint32_t t = (h4 ? x[1] : x[0]) + __shfl_xor_sync(0xffffffffu, h4 ? x[0] : x[1], 4);
-    t += __shfl_xor_sync(0xffffffffu, t, 2);
-    t += __shfl_xor_sync(0xffffffffu, t, 1);
-    return __reduce_min_sync(0xffffffffu, (t << 3) | (uint32_t)((lane >> 2) & 7));
-  };
+  // Each stage's eight positions at once: lane L scores four rows of position
+  // L >> 2 (rows (L & 3), + 4, ...), two shuffles finish the sums and one
+  // redux min over (SAD << 3 | position) picks the earliest smallest. Both
+  // stages run the same few instructions: the code of the eight positions
+  // written out (three times the instructions, most of them fetched cold by a
+  // launch of a few macroblocks) was the slower form.
+  const int pos = lane >> 2;
   uint32_t bsad = int_sad;
-  int hx = 0, hy = 0;
-  const uint32_t mh = best8(nullptr, 0, 0);  // the half-pel positions, kHalfOff order
-  if ((mh >> 3) < bsad) {
-    bsad = mh >> 3;
-    hx = kHalfOff[mh & 7][0];
-    hy = kHalfOff[mh & 7][1];
+  int bx = 0, by = 0;
+#pragma unroll 1
+  for (int stage = 0; stage < 2; ++stage) {
+    const int ox = bx + (stage ? kQtrOff[pos][0] : kHalfOff[pos][0]);
+    const int oy = by + (stage ? kQtrOff[pos][1] : kHalfOff[pos][1]);
+    const uint32_t op = kQpelOp[(oy & 3) * 4 + (ox & 3)];
+    // the first row of an operand: address of its word, bit shift, row pitch
+    auto operand = [&](uint32_t o, const uint32_t*& p, int& sh, int& pitch) {
+      const int rx = (ox >> 2) + (int)((o >> 2) & 1u), ry = (oy >> 2) + (int)((o >> 3) & 1u) + (lane & 3);
+      const int pl = (int)(o & 3u);
+      pitch = pl ? 20 : gstride;
+      const int c = pl ? rx + 1 : g_c0 + rx;
+      const uint8_t* base = pl ? &rf.pl[0][0][0] + (pl - 1) * 360 + (ry + 1) * 20 : g + (g_r0 + ry) * gstride;
+      p = reinterpret_cast<const uint32_t*>(base + (c & ~3));
+      sh = (c & 3) * 8;
+    };
+    const uint32_t *pa, *pb;
+    int sa, sb, ia, ib;
+    operand(op, pa, sa, ia);
+    operand(op >> 4, pb, sb, ib);
+    uint32_t sad = 0;
+#pragma unroll 1
+    for (int r = 0; r < 4; ++r, pa += ia, pb += ib) {  // every fourth row: word steps of 4 pitches / 4 bytes
+      const uint4 c = *reinterpret_cast<const uint4*>(cur + 4 * ((lane & 3) + 4 * r));
+      const uint32_t a0 = pa[0], a1 = pa[1], a2 = pa[2], a3 = pa[3], a4 = pa[4];
+      const uint32_t b0 = pb[0], b1 = pb[1], b2 = pb[2], b3 = pb[3], b4 = pb[4];
+      sad = sad4_acc(__vavgu4(__funnelshift_r(a0, a1, sa), __funnelshift_r(b0, b1, sb)), c.x, sad);
+      sad = sad4_acc(__vavgu4(__funnelshift_r(a1, a2, sa), __funnelshift_r(b1, b2, sb)), c.y, sad);
+      sad = sad4_acc(__vavgu4(__funnelshift_r(a2, a3, sa), __funnelshift_r(b2, b3, sb)), c.z, sad);
+      sad = sad4_acc(__vavgu4(__funnelshift_r(a3, a4, sa), __funnelshift_r(b3, b4, sb)), c.w, sad);
+    }
+    sad += __shfl_xor_sync(0xffffffffu, sad, 1);
+    sad += __shfl_xor_sync(0xffffffffu, sad, 2);
+    const uint32_t m = __reduce_min_sync(0xffffffffu, (sad << 3) | (uint32_t)pos);
+    if ((m >> 3) < bsad) {
+      bsad = m >> 3;
+      bx += stage ? kQtrOff[m & 7][0] : kHalfOff[m & 7][0];
+      by += stage ? kQtrOff[m & 7][1] : kHalfOff[m & 7][1];
+    }
   }
-  int qx = 0, qy = 0;
-  const uint32_t mq = best8(kQtrOff, hx, hy);
-  if ((mq >> 3) < bsad) {
-    bsad = mq >> 3;
-    qx = kQtrOff[mq & 7][0];
-    qy = kQtrOff[mq & 7][1];
-  }
-  *qx_out = hx + qx;
-  *qy_out = hy + qy;
+  *qx_out = bx;
+  *qy_out = by;
   return bsad;
 }
 

@@ -986,7 +986,7 @@ int b200enc_proposal_me_batch(void* h, const BatchTab& bt, int n, int range, int
   if (cudaGetDevice(&dev) == cudaSuccess) cudaDeviceGetAttribute(&sms, cudaDevAttrMultiProcessorCount, dev);
   if (cudaEventRecord(P->ev_sel, st) != cudaSuccess || cudaStreamWaitEvent(P->side, P->ev_sel, 0) != cudaSuccess)
     return -1;
-  const int fb_sm = b200enc_tuned(B200ENC_TUNE_FALLBACK_CTAS_PER_SM) > 0 ? b200enc_tuned(B200ENC_TUNE_FALLBACK_CTAS_PER_SM) : 8;
+  const int fb_sm = b200enc_tuned(B200ENC_TUNE_FALLBACK_CTAS_PER_SM) > 0 ? b200enc_tuned(B200ENC_TUNE_FALLBACK_CTAS_PER_SM) : 16;
   const int rc = b200enc_me_batch_launch(bt, range, P->b.lists + n, P->b.counters + 1, std::min(n, fb_sm * sms),
                                          P->side);
   const int rs_sm = b200enc_tuned(B200ENC_TUNE_RESCORE_CTAS_PER_SM) > 0 ? b200enc_tuned(B200ENC_TUNE_RESCORE_CTAS_PER_SM) : 8;
