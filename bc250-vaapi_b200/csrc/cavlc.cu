@@ -8,25 +8,30 @@
 // except two things: each block's nC is the neighbours' TotalCoeff, and each
 // coded macroblock is preceded by the run of skipped macroblocks before it.
 // Both are known up front: TotalCoeff is the number of nonzero levels the
-// block codes, and the skip decision depends only on the macroblock's own
-// levels and the vectors around it. So the slice data is built in four
-// launches over the picture's staged outputs (levels, DC, nz masks, modes,
-// vectors), all in device memory:
-//   1. cavlc_info_kernel: per macroblock, the skip decision, coded block
-//      pattern and every coded block's TotalCoeff;
-//   2. cavlc_mb_kernel: per macroblock, its header and residual bits (one
-//      warp per macroblock, a lane per block, into a private region of the
-//      scratch);
-//   3. cavlc_slice_kernel: per slice (one CTA), the skip runs and every
-//      coded macroblock's bit offset (two block-wide scans), the slice's
-//      length; it zeroes the slice's output words;
-//   4. cavlc_pack_kernel: each coded macroblock ORs ue(skip run) and its
-//      bits into the slice at its offset; each slice's first thread writes
-//      the caller's slice header bits, the trailing skip run and
-//      rbsp_trailing_bits;
-// then cavlc_bytes_kernel turns the MSB-first words into stream bytes. The
-// output is each slice's RBSP (header + slice data + trailing bits), ready
+// block codes (the staged nz masks), and the skip decision depends only on the
+// macroblock's own levels and the vectors around it. So the slice data is
+// built in three launches over the picture's staged outputs (levels, DC, nz
+// masks, modes, vectors), all in device memory:
+//   1. cavlc_mb_kernel: per macroblock (a warp, a lane per block), the skip
+//      decision, coded block pattern and nC, then its header and residual bits
+//      into a private region of the scratch;
+//   2. cavlc_slice_kernel: per slice (one CTA), the skip runs and every
+//      macroblock's bit offset (two block-wide scans), the slice's length;
+//   3. cavlc_gather_kernel: each output word collects the bits that fall into
+//      it (slice header, skip runs, macroblocks, trailing bits) and is stored
+//      as stream bytes.
+// The output is each slice's RBSP (header + slice data + trailing bits), ready
 // for emulation prevention and a NAL header, bit for bit the reference's.
+//
+// What bounds it: instruction issue in the serial symbol loop of the densest
+// block of each macroblock, and, below 640x480, the launches themselves. The
+// macroblock kernel keeps one copy of each writer (37 KB of code; with the
+// writers inlined at every call it was 152 KB, most of it fetched cold), and
+// the gather replaced clearing the words, atomics into them and a byte swap.
+// Before (five launches and a clear) and now, us: a 176x144 P picture 41 and
+// 19, 640x480 39 and 23, a 1280x720 I picture at QP 20 81 and 33 (its 360 KB
+// to mapped host memory take 7 at the bus's rate), a 1080p P picture at QP 22
+// 44 and 32.
 #include <algorithm>
 
 #include "b200enc_internal.h"
@@ -41,10 +46,40 @@ using namespace b200cavlc;
 constexpr int kCavlcMbWords = 640;  // 2560 bytes of bits per macroblock at most (the reference's CAVLC allowance)
 constexpr int kCavlcMaxSlices = 16;
 constexpr int kCavlcScanThreads = 1024;
+constexpr uint32_t kCavlcOver = 0xffffffffu;
+constexpr uint32_t kCavlcNoRun = 0xffffffffu;
+
+// The code tables as words of (length << 8 | code), in device memory (not
+// __constant__: lanes index them at different positions, which the constant
+// cache would serialise).
+struct CavlcTabs {
+  uint16_t ct[5][68];    // coeff_token: [nC class, 4 chroma DC][TotalCoeff * 4 + TrailingOnes]
+  uint16_t tz[15][16];   // total_zeros: [TotalCoeff - 1][total_zeros]
+  uint16_t cdtz[3][4];   // of chroma DC
+  uint16_t run[7][16];   // run_before: [min(zerosLeft, 7) - 1][run_before]
+};
+constexpr CavlcTabs make_cavlc_tabs() {
+  constexpr uint8_t ctl[5][68] = B200_CAVLC_COEFF_TOKEN_LEN, ctc[5][68] = B200_CAVLC_COEFF_TOKEN_CODE;
+  constexpr uint8_t tzl[15][16] = B200_CAVLC_TOTAL_ZEROS_LEN, tzc[15][16] = B200_CAVLC_TOTAL_ZEROS_CODE;
+  constexpr uint8_t cdl[3][4] = B200_CAVLC_CDC_TOTAL_ZEROS_LEN, cdc[3][4] = B200_CAVLC_CDC_TOTAL_ZEROS_CODE;
+  constexpr uint8_t rl[7][16] = B200_CAVLC_RUN_LEN, rc[7][16] = B200_CAVLC_RUN_CODE;
+  CavlcTabs t{};
+  for (int i = 0; i < 5; ++i)
+    for (int j = 0; j < 68; ++j) t.ct[i][j] = (uint16_t)(ctl[i][j] << 8 | ctc[i][j]);
+  for (int i = 0; i < 15; ++i)
+    for (int j = 0; j < 16; ++j) t.tz[i][j] = (uint16_t)(tzl[i][j] << 8 | tzc[i][j]);
+  for (int i = 0; i < 3; ++i)
+    for (int j = 0; j < 4; ++j) t.cdtz[i][j] = (uint16_t)(cdl[i][j] << 8 | cdc[i][j]);
+  for (int i = 0; i < 7; ++i)
+    for (int j = 0; j < 16; ++j) t.run[i][j] = (uint16_t)(rl[i][j] << 8 | rc[i][j]);
+  return t;
+}
+static __device__ const CavlcTabs d_cavlc = make_cavlc_tabs();
+static __device__ const uint8_t d_cbp_code[48] = B200_CAVLC_INTER_CBP_CODE;
 
 // spec luma block index (8x8 quadrants, then 4x4 within) -> block column / row
-__constant__ int8_t kBlkX4[16] = {0, 1, 0, 1, 2, 3, 2, 3, 0, 1, 0, 1, 2, 3, 2, 3};
-__constant__ int8_t kBlkY4[16] = {0, 0, 1, 1, 0, 0, 1, 1, 2, 2, 3, 3, 2, 2, 3, 3};
+__device__ __forceinline__ int blk_x4(int k) { return (k & 1) | ((k >> 1) & 2); }
+__device__ __forceinline__ int blk_y4(int k) { return ((k >> 1) & 1) | ((k >> 2) & 2); }
 __device__ __forceinline__ int spec_blk(int y4, int x4) { return ((y4 >> 1) << 3) | ((x4 >> 1) << 2) | ((y4 & 1) << 1) | (x4 & 1); }
 
 // Per-slice header bits (MSB first) of a launch, passed by value.
@@ -63,14 +98,12 @@ struct CavlcArgs {
   const uint32_t* pred_mode;
   const MV* mv;
   // scratch
-  uint32_t* info;    // [mbs] bit 0 skipped, bits 1..4 luma cbp quadrants (P) / bit 1 any luma AC (I), bits 8..9 cbp_chroma
-  uint8_t* tcs;      // [mbs][24] TotalCoeff of the coded blocks (luma in spec order, Cb, Cr; 0 when not coded)
-  uint32_t* nbits;   // [mbs] bits of the macroblock (header + residual, no skip run)
+  uint32_t* nbits;   // [mbs] bits of the macroblock (header + residual, no skip run); 0: skipped,
+                     // kCavlcOver: they outgrew its region
   uint32_t* words;   // [mbs][kCavlcMbWords]
-  uint32_t* off;     // [mbs] bit offset of a coded macroblock's skip run in its slice
-  uint32_t* run;     // [mbs] skip run before a coded macroblock (0xffffffff: none, I slices)
-  uint32_t* sl;      // [kCavlcMaxSlices * 4] per slice: total bits, trailing run, overflow, bytes
-  uint32_t* err;     // [1] nonzero: a macroblock's bits outgrew its region
+  uint4* place;      // [mbs] bit offset of the macroblock (of its skip run, if coded) in its slice; its bits;
+                     // the skip run before a coded macroblock (kCavlcNoRun: none, I slices); unused
+  uint32_t* sl;      // [kCavlcMaxSlices * 4] per slice: total bits, trailing run, did not fit, end of the data
   // output
   uint8_t* out;
   uint32_t slice_cap;  // bytes per slice region (multiple of 4)
@@ -128,101 +161,6 @@ __device__ void skip_pred(const MV* mv, int mbx, int mby, int mbw, uint32_t star
   mv_pred(mv, mbx, mby, mbw, start, px, py);
 }
 
-// Chroma DC of one plane: the 2x2 Hadamard of the four raw DC terms
-// (encoder_h264.c:791-797).
-__device__ __forceinline__ void chroma_dc(const int32_t* d, int out[4]) {
-  out[0] = d[0] + d[1] + d[2] + d[3];
-  out[1] = d[0] - d[1] + d[2] - d[3];
-  out[2] = d[0] + d[1] - d[2] - d[3];
-  out[3] = d[0] - d[1] - d[2] + d[3];
-}
-
-__device__ __forceinline__ bool any_nz(const uint32_t* nzm, int b0, int b1, uint32_t mask) {
-  uint32_t a = 0;
-  for (int b = b0; b < b1; ++b) a |= nzm[b];
-  return (a & mask) != 0;
-}
-
-// ---- 1. per macroblock: skip, coded block pattern, TotalCoeff ------------------
-__global__ void __launch_bounds__(128) cavlc_info_kernel(CavlcArgs a) {
-  const int mb = blockIdx.x * blockDim.x + threadIdx.x;
-  const int mbs = a.mbw * a.mbh;
-  if (mb >= mbs) return;
-  const int mbx = mb % a.mbw, mby = mb / a.mbw;
-  const uint32_t* nzm = a.nz + (size_t)mb * 24;
-  const int32_t* dcm = a.dc + (size_t)mb * 24;
-  uint8_t* tc = a.tcs + (size_t)mb * 24;
-  const QP qc = make_qp(chroma_qp(a.qp), a.is_intra != 0);
-  int cb[4], cr[4];
-  chroma_dc(dcm + 16, cb);
-  chroma_dc(dcm + 20, cr);
-  bool cdc_raw_nz = false, cdc_nz = false;
-  for (int i = 0; i < 4; ++i) {
-    cdc_raw_nz |= (cb[i] != 0) | (cr[i] != 0);
-    cdc_nz |= (quantize_dc(cb[i], qc) != 0) | (quantize_dc(cr[i], qc) != 0);
-  }
-  const bool cac_nz = any_nz(nzm, 16, 24, 0xfffeu);
-  const int cbp_c = cac_nz ? 2 : (cdc_nz ? 1 : 0);
-  uint32_t info = (uint32_t)cbp_c << 8;
-  if (a.is_intra) {
-    const bool lac = any_nz(nzm, 0, 16, 0xfffeu);
-    info |= lac ? 2u : 0u;
-    for (int b = 0; b < 16; ++b)
-      tc[b] = lac ? (uint8_t)__popc(nzm[kBlkY4[b] * 4 + kBlkX4[b]] & 0xfffeu) : 0;
-  } else {
-    // P_Skip (encoder_h264.c:3236-3255): no luma level, a zero chroma DC
-    // Hadamard and no chroma AC level, and the vector on the skip predictor
-    const uint32_t start = slice_start(slice_of(mb, mbs, a.ns), mbs, a.ns);
-    const bool zl = !any_nz(nzm, 0, 16, 0xffffu);
-    bool zc = !cdc_raw_nz && !cac_nz;
-    if (a.quality >= 5 && zl && !zc && abs(a.dc[mb * 2 + 0]) <= 1 && abs(a.dc[mb * 2 + 1]) <= 1) zc = true;
-    int px, py;
-    skip_pred(a.mv, mbx, mby, a.mbw, start, &px, &py);
-    const bool skip = zl && zc && a.mv[mb].mvx == px && a.mv[mb].mvy == py;
-    if (skip) {
-      info = 1u;
-      for (int b = 0; b < 24; ++b) tc[b] = 0;
-    } else {
-      for (int q = 0; q < 4; ++q) {
-        uint32_t m = 0;
-        for (int s = 0; s < 4; ++s) m |= nzm[kBlkY4[4 * q + s] * 4 + kBlkX4[4 * q + s]];
-        if (m & 0xffffu) info |= 2u << q;
-      }
-      for (int b = 0; b < 16; ++b)
-        tc[b] = (info >> (1 + (b >> 2)) & 1u) ? (uint8_t)__popc(nzm[kBlkY4[b] * 4 + kBlkX4[b]] & 0xffffu) : 0;
-    }
-  }
-  if (!(info & 1u))
-    for (int k = 0; k < 8; ++k) tc[16 + k] = cbp_c == 2 ? (uint8_t)__popc(nzm[16 + k] & 0xfffeu) : 0;
-  a.info[mb] = info;
-}
-
-// nC of luma block b (spec order) from the TotalCoeff of its left and upper
-// neighbours (encoder_h264.c:800-821).
-__device__ int luma_nc(const uint8_t* tcs, int mb, int mbx, int mby, int mbw, uint32_t start, int b) {
-  const int x4 = kBlkX4[b], y4 = kBlkY4[b];
-  int na = -1, nb = -1, n;
-  if (x4 > 0) na = tcs[mb * 24 + spec_blk(y4, x4 - 1)];
-  else if (nb_ok(mbx, mby, -1, 0, mbw, start, &n)) na = tcs[n * 24 + spec_blk(y4, 3)];
-  if (y4 > 0) nb = tcs[mb * 24 + spec_blk(y4 - 1, x4)];
-  else if (nb_ok(mbx, mby, 0, -1, mbw, start, &n)) nb = tcs[n * 24 + spec_blk(3, x4)];
-  if (na >= 0 && nb >= 0) return (na + nb + 1) >> 1;
-  return na >= 0 ? na : (nb >= 0 ? nb : 0);
-}
-
-// nC of chroma AC block k (raster in its 2x2 grid) of the plane whose
-// TotalCoeffs start at entry o (encoder_h264.c:823-841).
-__device__ int chroma_nc(const uint8_t* tcs, int mb, int mbx, int mby, int mbw, uint32_t start, int o, int k) {
-  const int x2 = k & 1, y2 = k >> 1;
-  int na = -1, nb = -1, n;
-  if (x2 > 0) na = tcs[mb * 24 + o + y2 * 2];
-  else if (nb_ok(mbx, mby, -1, 0, mbw, start, &n)) na = tcs[n * 24 + o + y2 * 2 + 1];
-  if (y2 > 0) nb = tcs[mb * 24 + o + x2];
-  else if (nb_ok(mbx, mby, 0, -1, mbw, start, &n)) nb = tcs[n * 24 + o + 2 + x2];
-  if (na >= 0 && nb >= 0) return (na + nb + 1) >> 1;
-  return na >= 0 ? na : (nb >= 0 ? nb : 0);
-}
-
 // Prediction modes the decoder can form at the slice and picture edges
 // (h264_sanitize_i16_mode / _chroma_mode, encoder_h264.c:919-946).
 __device__ __forceinline__ int sanitize_i16(int m, bool top, bool left) {
@@ -238,142 +176,362 @@ __device__ __forceinline__ int sanitize_chroma(int m, bool top, bool left) {
   return m;
 }
 
-// The luma DC block of an I16x16 macroblock: Hadamard of the 16 raw DC
-// terms with the reference's rounding, quantised, transposed
-// (h264_intra16_luma_dc_transform, encoder_h264.c:711-789).
-__device__ void luma_dc_levels(const int32_t* d, const QP& q, int16_t out[16]) {
-  int t[16], n[16];
-  for (int i = 0; i < 4; ++i) {
-    const int s01 = d[i * 4 + 0] + d[i * 4 + 1], d01 = d[i * 4 + 0] - d[i * 4 + 1];
-    const int s23 = d[i * 4 + 2] + d[i * 4 + 3], d23 = d[i * 4 + 2] - d[i * 4 + 3];
-    t[0 * 4 + i] = s01 + s23;
-    t[1 * 4 + i] = s01 - s23;
-    t[2 * 4 + i] = d01 - d23;
-    t[3 * 4 + i] = d01 + d23;
-  }
-  for (int i = 0; i < 4; ++i) {
-    const int s01 = t[i * 4 + 0] + t[i * 4 + 1], d01 = t[i * 4 + 0] - t[i * 4 + 1];
-    const int s23 = t[i * 4 + 2] + t[i * 4 + 3], d23 = t[i * 4 + 2] - t[i * 4 + 3];
-    n[i * 4 + 0] = quantize_dc((s01 + s23 + 1) >> 1, q);
-    n[i * 4 + 1] = quantize_dc((s01 - s23 + 1) >> 1, q);
-    n[i * 4 + 2] = quantize_dc((d01 - d23 + 1) >> 1, q);
-    n[i * 4 + 3] = quantize_dc((d01 + d23 + 1) >> 1, q);
-  }
-  for (int r = 0; r < 4; ++r)
-    for (int c = 0; c < 4; ++c) out[r * 4 + c] = (int16_t)n[c * 4 + r];
-}
-
-// ---- 2. per macroblock: header and residual bits --------------------------------
+// ---- 1. per macroblock: skip, coded block pattern, header and residual bits ----
 // One warp per macroblock; each lane writes one syntax element group into its
 // own bit buffer, in the order the reference writes them: lane 0 the header,
 // 1 the I16x16 luma DC block, 2..17 the luma blocks (spec order), 18 and 19 the
 // chroma DC blocks, 20..27 the chroma AC blocks (Cb then Cr). A warp scan of
 // the lanes' lengths places them; the lanes OR their words into the warp's
 // shared copy of the macroblock's region, which is then stored.
-constexpr int kCavlcLaneWords = 24;  // one block: at most 16 escaped levels (~36 bits each) + tokens
+constexpr int kCavlcLaneWords = 25;  // a block: at most 16 levels of 36 bits, token and runs < 24 words; odd
+                                     // stride: the lanes' words lie in different banks
 constexpr int kCavlcMbWarps = 4;
 
+struct CavlcWarp {
+  alignas(16) int16_t lev[24 * 16];
+  int16_t dcl[16];   // quantised luma DC, raster positions
+  int16_t cdl[8];    // quantised chroma DC (Cb, Cr)
+  uint32_t lane[28 * kCavlcLaneWords];
+  uint32_t out[kCavlcMbWords];
+};
+
+// MSB-first bit writer: `acc` ends in the nb < 32 pending bits.
+struct BitW {
+  uint64_t acc;
+  uint32_t* w;
+  uint32_t nb, pos;
+  __device__ __forceinline__ void put(uint32_t n, uint32_t v) {  // n <= 32 bits, v < 2^n
+    acc = (acc << n) | v;
+    nb += n;
+    pos += n;
+    if (nb >= 32u) {
+      nb -= 32u;
+      *w++ = (uint32_t)(acc >> nb);
+    }
+  }
+};
+
+// Raster mask of a 4x4 block's nonzero levels -> frame zig-zag scan positions
+// (scan position i holds raster position i + d; positions grouped by d), and
+// the raster position of scan position i.
+__device__ __forceinline__ uint32_t zigzag_mask(uint32_t m) {
+  return (m & 0xc003u) | ((m >> 2) & 0x0004u) | ((m >> 5) & 0x0008u) | ((m >> 1) & 0x0110u) | ((m << 3) & 0x0060u) |
+         ((m << 1) & 0x0880u) | ((m >> 3) & 0x0600u) | ((m << 5) & 0x1000u) | ((m << 2) & 0x2000u);
+}
+__device__ __forceinline__ int zigzag_pos(int i) { return (int)((0xFEB7ADC963258410ull >> (4 * i)) & 15u); }
+
+// P_Skip (encoder_h264.c:3236-3255): no luma level, a zero chroma DC Hadamard
+// (every raw term zero) and no chroma AC level, the vector on the skip
+// predictor; quality levels from 5 up also accept two tiny DC words.
+__device__ __forceinline__ bool p_skip(const CavlcArgs& a, int mb, int mbx, int mby, uint32_t start, bool luma,
+                                       bool cdc_raw, bool cac) {
+  if (luma) return false;
+  bool zc = !cdc_raw && !cac;
+  if (a.quality >= 5 && !zc && abs(a.dc[mb * 2 + 0]) <= 1 && abs(a.dc[mb * 2 + 1]) <= 1) zc = true;
+  if (!zc) return false;
+  int px, py;
+  skip_pred(a.mv, mbx, mby, a.mbw, start, &px, &py);
+  return a.mv[mb].mvx == px && a.mv[mb].mvy == py;
+}
+
 __global__ void __launch_bounds__(32 * kCavlcMbWarps) cavlc_mb_kernel(CavlcArgs a) {
-  __shared__ uint32_t shw[kCavlcMbWarps][kCavlcMbWords];
+  __shared__ CavlcWarp shw[kCavlcMbWarps];
+  const unsigned full = 0xffffffffu;
   const int lane = threadIdx.x & 31, wi = threadIdx.x >> 5;
   const int mb = blockIdx.x * kCavlcMbWarps + wi;
   const int mbs = a.mbw * a.mbh;
   if (mb >= mbs) return;
-  const uint32_t info = a.info[mb];
-  if (info & 1u) {  // skipped: its run is counted by the slice pass
+  CavlcWarp& sh = shw[wi];
+  const int mbx = mb % a.mbw, mby = mb / a.mbw;
+  const uint32_t start = slice_start(slice_of(mb, mbs, a.ns), mbs, a.ns);
+  const bool intra = a.is_intra != 0;
+  int nl, nt;
+  const bool left = nb_ok(mbx, mby, -1, 0, a.mbw, start, &nl), top = nb_ok(mbx, mby, 0, -1, a.mbw, start, &nt);
+
+  // lanes 2..17: luma block k (spec order), 20..27: chroma block k
+  const bool lu = lane >= 2 && lane < 18, ch = lane >= 20 && lane < 28;
+  const int k = lu ? lane - 2 : (lane & 3);
+  const int x4 = blk_x4(k), y4 = blk_y4(k);
+  const int blk = lu ? y4 * 4 + x4 : (ch ? lane - 4 : 0);  // staged block (raster luma, chroma from 16)
+  uint32_t zo = 0, zl = 0, zt = 0;
+  if (lu || ch) {
+    zo = __ldg(a.nz + (size_t)mb * 24 + blk);
+    if (left) zl = __ldg(a.nz + (size_t)nl * 24 + blk);
+    if (top) zt = __ldg(a.nz + (size_t)nt * 24 + blk);
+  }
+  const uint32_t used = ch || intra ? 0xfffeu : 0xffffu;  // levels the block codes (position 0 goes by the DC blocks)
+  zo &= used;
+  zl &= used;
+  zt &= used;
+  // raw DC terms: luma on the luma lanes, chroma on the chroma lanes
+  const int dcv = lu || ch ? __ldg(a.dc + (size_t)mb * 24 + blk) : 0;
+  // chroma DC: 2x2 Hadamard output of the lane, quantised (encoder_h264.c:791-797)
+  int cq;
+  {
+    const int g = lane & ~3;
+    const int c0 = __shfl_sync(full, dcv, g), c1 = __shfl_sync(full, dcv, g + 1);
+    const int c2 = __shfl_sync(full, dcv, g + 2), c3 = __shfl_sync(full, dcv, g + 3);
+    const int s1 = (lane & 1) ? -1 : 1, s2 = (lane & 2) ? -1 : 1;
+    cq = quantize_dc(c0 + s1 * c1 + s2 * c2 + s1 * s2 * c3, make_qp(chroma_qp(a.qp), intra));
+  }
+  const uint32_t bz = __ballot_sync(full, zo != 0u);
+  const uint32_t blu = (bz >> 2) & 0xffffu;  // luma blocks with levels, spec order
+  const bool cac = (bz >> 20) != 0u;
+  const bool cdc_raw = (__ballot_sync(full, ch && dcv != 0) != 0u);
+  const bool cdc = (__ballot_sync(full, ch && cq != 0) != 0u);
+  if (!intra && p_skip(a, mb, mbx, mby, start, blu != 0u, cdc_raw, cac)) {  // its run is counted by the slice pass
     if (lane == 0) a.nbits[mb] = 0;
     return;
   }
-  const int mbx = mb % a.mbw, mby = mb / a.mbw;
-  const uint32_t start = slice_start(slice_of(mb, mbs, a.ns), mbs, a.ns);
-  const int16_t* lv = a.levels + (size_t)mb * 384;
-  const int32_t* dcm = a.dc + (size_t)mb * 24;
-  const int cbp_c = (int)((info >> 8) & 3u);
-  const bool intra = a.is_intra != 0;
-  uint32_t lw[kCavlcLaneWords];
-  BitW b;
-  bw_init(b, lw, kCavlcLaneWords);
-  if (lane == 0) {
-    if (intra) {
-      int n;
-      const bool left = nb_ok(mbx, mby, -1, 0, a.mbw, start, &n), top = nb_ok(mbx, mby, 0, -1, a.mbw, start, &n);
-      const uint32_t pm = a.pred_mode[mb];
-      put_i16_header(b, sanitize_i16((int)(pm & 3u), top, left), sanitize_chroma((int)((pm >> 2) & 3u), top, left),
-                     cbp_c, (int)((info >> 1) & 1u));
+  // TotalCoeff of the lane's block and its neighbours. A skipped neighbour has
+  // none: no levels either, but for the quality rule's chroma AC.
+  int tl = __popc(zl), tt = __popc(zt);
+  const int tc_own = __popc(zo);
+  if (!intra && a.quality >= 5) {
+    auto nb_skip = [&](bool ok, int n, int nx, int ny, uint32_t z) -> bool {
+      const uint32_t b = __ballot_sync(full, z != 0u);
+      const int d = ok && ch ? a.dc[(size_t)n * 24 + blk] : 0;
+      const bool raw = __ballot_sync(full, d != 0) != 0u;
+      return ok && p_skip(a, n, nx, ny, start, (b & 0x3fffcu) != 0u, raw, (b >> 20) != 0u);
+    };
+    if (nb_skip(left, nl, mbx - 1, mby, zl)) tl = 0;
+    if (nb_skip(top, nt, mbx, mby - 1, zt)) tt = 0;
+  }
+  // nC (encoder_h264.c:800-841): the neighbours inside the macroblock are other lanes
+  int nc;
+  {
+    const int sl_in = lu ? 2 + spec_blk(y4, (x4 + 3) & 3) : lane ^ 1, st_in = lu ? 2 + spec_blk((y4 + 3) & 3, x4) : lane ^ 2;
+    const int o_l = __shfl_sync(full, tc_own, sl_in), o_t = __shfl_sync(full, tc_own, st_in);
+    const int n_l = __shfl_sync(full, tl, sl_in), n_t = __shfl_sync(full, tt, st_in);
+    const int xx = lu ? x4 : (lane & 1), yy = lu ? y4 : (lane & 2);
+    const int na = xx ? o_l : (left ? n_l : -1), nb = yy ? o_t : (top ? n_t : -1);
+    nc = na >= 0 && nb >= 0 ? (na + nb + 1) >> 1 : (na >= 0 ? na : (nb >= 0 ? nb : 0));
+  }
+  // coded block pattern: the 8x8 quadrants with levels (any luma AC in an I16x16)
+  uint32_t cbp_l = 0;
+  if (intra) cbp_l = blu ? 1u : 0u;
+  else cbp_l = (blu & 0xfu ? 1u : 0u) | (blu & 0xf0u ? 2u : 0u) | (blu & 0xf00u ? 4u : 0u) | (blu & 0xf000u ? 8u : 0u);
+  const int cbp_c = cac ? 2 : (cdc ? 1 : 0);
+  const bool use8 = a.t8 && !intra && (!a.t8f || a.t8f[mb]);
+
+  // ---- the levels, and the DC blocks, to shared memory ----------------------
+  {
+    const int16_t* lv = a.levels + (size_t)mb * 384;
+    if (((reinterpret_cast<uintptr_t>(lv)) & 15) == 0) {
+      const uint4* src = reinterpret_cast<const uint4*>(lv);
+      uint4* dst = reinterpret_cast<uint4*>(sh.lev);
+      dst[lane] = __ldg(src + lane);
+      if (lane < 16) dst[32 + lane] = __ldg(src + 32 + lane);
     } else {
-      int px, py;
-      mv_pred(a.mv, mbx, mby, a.mbw, start, &px, &py);
-      put_p16_header(b, a.mv[mb].mvx - px, a.mv[mb].mvy - py, (int)((info >> 1) & 15u) | (cbp_c << 4),
-                     a.t8, !a.t8f || a.t8f[mb]);
+#pragma unroll 1
+      for (int i = lane; i < 384; i += 32) sh.lev[i] = __ldg(lv + i);
     }
-  } else if (lane == 1) {
-    if (intra) {
-      int16_t ldc[16];
-      luma_dc_levels(dcm, make_qp(a.qp, true), ldc);
-      put_4x4(b, ldc, false, luma_nc(a.tcs, mb, mbx, mby, a.mbw, start, 0));
-    }
-  } else if (lane < 18) {
-    const int k = lane - 2;
-    const bool coded = intra ? ((info >> 1) & 1u) : ((info >> (1 + (k >> 2))) & 1u);
-    if (coded && a.t8 && !intra && (!a.t8f || a.t8f[mb])) {
-      // 8x8 block k >> 2 as its 4x4 block k & 3: scan positions (k & 3) + 4j (7.3.5.3.2)
-      int sc[16];
-      const int16_t* l8 = lv + 64 * (k >> 2);
-      for (int j = 0; j < 16; ++j) sc[j] = l8[kZigzag8[4 * j + (k & 3)]];
-      put_block(b, sc, 16, nc_class(luma_nc(a.tcs, mb, mbx, mby, a.mbw, start, k)));
-    } else if (coded) {
-      put_4x4(b, lv + (kBlkY4[k] * 4 + kBlkX4[k]) * 16, intra, luma_nc(a.tcs, mb, mbx, mby, a.mbw, start, k));
-    }
-  } else if (lane < 20) {
-    if (cbp_c >= 1) {
-      const QP qc = make_qp(chroma_qp(a.qp), intra);
-      int c[4];
-      chroma_dc(dcm + 16 + 4 * (lane - 18), c);
-      for (int i = 0; i < 4; ++i) c[i] = quantize_dc(c[i], qc);
-      put_block(b, c, 4, 4);
-    }
-  } else if (lane < 28) {
-    if (cbp_c == 2) {
-      const int p = (lane - 20) >> 2, k = (lane - 20) & 3;
-      put_4x4(b, lv + (16 + 4 * p + k) * 16, true, chroma_nc(a.tcs, mb, mbx, mby, a.mbw, start, 16 + 4 * p, k));
+    if (ch) sh.cdl[lane - 20] = (int16_t)cq;
+  }
+  uint32_t m = 0;          // nonzero levels in scan order
+  int vlc = 0, maxc = 16;  // nC class (4: chroma DC), levels the block may have
+  bool active = false;
+  const int16_t* src = sh.lev;  // level of scan position i: src[pos(i)]
+  if (intra) {
+    // Luma DC of an I16x16 macroblock: 2-D Hadamard of the 16 raw terms
+    // (rows + + + +, + + - -, + - - +, + - + -), (sum + 1) >> 1, quantised
+    // (h264_intra16_luma_dc_transform, encoder_h264.c:711-789); lane 4r + c
+    // forms frequency (r, c), first along rows, then down columns.
+    const int r = (lane >> 2) & 3, c = lane & 3;
+    auto sgn = [](int h, int i) -> int { return ((h == 1 ? 0xc : (h == 2 ? 0x6 : (h == 3 ? 0xa : 0))) >> i) & 1 ? -1 : 1; };
+    int t = 0, v = 0;
+#pragma unroll
+    for (int j = 0; j < 4; ++j) t += sgn(c, j) * __shfl_sync(full, dcv, 2 + spec_blk(r, j));
+#pragma unroll
+    for (int i = 0; i < 4; ++i) v += sgn(r, i) * __shfl_sync(full, t, 4 * i + c);
+    const int l = quantize_dc((v + 1) >> 1, make_qp(a.qp, true));
+    if (lane < 16) sh.dcl[lane] = (int16_t)l;
+    const uint32_t md = __ballot_sync(full, lane < 16 && (int16_t)l != 0);
+    const int nc0 = __shfl_sync(full, nc, 2);
+    if (lane == 1) {
+      active = true;
+      m = zigzag_mask(md);
+      vlc = nc0;
+      src = sh.dcl;
     }
   }
-  bw_flush(b);
-  // place the lanes' bits one after another
+  const uint32_t mc = __ballot_sync(full, ch && cq != 0) >> 20;  // chroma DC levels: Cb 0..3, Cr 4..7
+  bool raw_scan = false;  // positions are 8x8 scan positions (use8) or the levels are in scan order already (chroma DC)
+  if (lu) {
+    active = intra ? cbp_l != 0u : ((cbp_l >> (k >> 2)) & 1u) != 0u;
+    vlc = nc;
+    if (use8) {
+      m = zo;
+      src = sh.lev + 64 * (k >> 2);
+      raw_scan = true;
+    } else {
+      m = zigzag_mask(zo);
+      src = sh.lev + 16 * blk;
+    }
+  } else if (lane == 18 || lane == 19) {
+    active = cbp_c >= 1;
+    m = (mc >> (4 * (lane - 18))) & 15u;
+    src = sh.cdl + 4 * (lane - 18);
+    maxc = 4;
+  } else if (ch) {
+    active = cbp_c == 2;
+    m = zigzag_mask(zo);
+    vlc = nc;
+    src = sh.lev + 16 * blk;
+  }
+  vlc = maxc == 4 ? 4 : (vlc < 2 ? 0 : (vlc < 4 ? 1 : (vlc < 8 ? 2 : 3)));
+  const int first = (lu && intra) || ch ? 1 : 0;  // AC blocks: scan positions 1..15
+  m >>= first;
+  if (first) maxc = 15;
+  __syncwarp();
+  const bool cd = maxc == 4;
+  auto level = [&](int i) -> int {
+    const int pos = cd ? i : (raw_scan ? (int)kZigzag8[4 * i + (k & 3)] : zigzag_pos(i + first));
+    return src[pos];
+  };
+
+  BitW b;
+  b.acc = 0;
+  b.w = sh.lane + (lane < 28 ? lane : 27) * kCavlcLaneWords;
+  b.nb = b.pos = 0;
+  if (lane == 0) {
+    // macroblock header (clause 7.3.5): ue(v) values, one bit of
+    // transform_size_8x8_flag after the coded block pattern, mb_qp_delta 0
+    int px = 0, py = 0;
+    uint32_t v[4] = {0u, 0u, 0u, 0u};
+    int n;
+    if (intra) {
+      const uint32_t pm = a.pred_mode[mb];
+      v[0] = (uint32_t)(1 + sanitize_i16((int)(pm & 3u), top, left) + 4 * cbp_c) + 12u * cbp_l;
+      v[1] = (uint32_t)sanitize_chroma((int)((pm >> 2) & 3u), top, left);
+      n = 3;  // v[2] = 0: mb_qp_delta
+    } else {
+      mv_pred(a.mv, mbx, mby, a.mbw, start, &px, &py);
+      const int dx = a.mv[mb].mvx - px, dy = a.mv[mb].mvy - py;
+      v[1] = dx > 0 ? 2u * (uint32_t)dx - 1u : 2u * (0u - (uint32_t)dx);
+      v[2] = dy > 0 ? 2u * (uint32_t)dy - 1u : 2u * (0u - (uint32_t)dy);
+      v[3] = d_cbp_code[cbp_l | ((uint32_t)cbp_c << 4)];
+      n = 4;
+    }
+#pragma unroll 1
+    for (int i = 0; i < n; ++i) {
+      const uint32_t c = (i == 0 ? v[0] : (i == 1 ? v[1] : (i == 2 ? v[2] : v[3]))) + 1u;
+      const uint32_t l = 31u - (uint32_t)__clz((int)c);
+      b.put(l, 0u);
+      b.put(l + 1u, c);
+    }
+    if (!intra) {
+      if (a.t8 && cbp_l) b.put(1u, use8 ? 1u : 0u);
+      if (cbp_l || cbp_c) b.put(1u, 1u);
+    }
+  } else if (active) {
+    // ---- a residual block (clause 9.2): coeff_token and trailing-one signs,
+    //      levels from the highest frequency down, total_zeros, run_before -----
+    const int tc = __popc(m);
+    uint32_t rest = m, signs = 0, t1 = 0;
+#pragma unroll 1
+    while (t1 < 3u && rest) {  // trailing ones
+      const int i = 31 - __clz((int)rest), v = level(i);
+      if (v != 1 && v != -1) break;
+      signs = (signs << 1) | (v < 0 ? 1u : 0u);
+      ++t1;
+      rest ^= 1u << i;
+    }
+    {
+      const uint32_t e = d_cavlc.ct[vlc][tc * 4 + (int)t1];
+      b.put((e >> 8) + t1, ((e & 0xffu) << t1) | signs);
+    }
+    int sl = (tc > 10 && t1 < 3u) ? 1 : 0;
+    int sub = t1 < 3u ? 2 : 0;  // the first level after fewer than three trailing ones is not +-1
+#pragma unroll 1
+    while (rest) {
+      const int i = 31 - __clz((int)rest), v = level(i);
+      rest ^= 1u << i;
+      // level_prefix / level_suffix (9.2.2.1) with the reference's escape
+      // arithmetic for level_prefix >= 15 (cavlc.c:429-480)
+      const int code = (v > 0 ? 2 * v - 2 : -2 * v - 1) - sub;
+      sub = 0;
+      uint32_t zeros, ss, suf;
+      const int prefix = code >> sl;
+      if (sl == 0 && code >= 14 && code < 30) {
+        zeros = 14u;
+        ss = 4u;
+        suf = (uint32_t)(code - 14);
+      } else if (prefix < (sl == 0 ? 14 : 15)) {
+        zeros = (uint32_t)prefix;
+        ss = (uint32_t)sl;
+        suf = (uint32_t)(code & ((1 << sl) - 1));
+      } else {
+        const uint32_t total = (uint32_t)(sl == 0 ? code + 4066 : code - (15 << sl) + 4096);
+        ss = 31u - (uint32_t)__clz((int)total);
+        zeros = ss + 3u;
+        suf = total - (1u << ss);
+      }
+      uint32_t n = zeros + 1u + ss;
+      if (n > 32u) {  // at most 36 bits, the first ones zeros
+        b.put(n - 32u, 0u);
+        n = 32u;
+      }
+      b.put(n, (1u << ss) | suf);
+      if (sl == 0) sl = 1;
+      if (abs(v) > (3 << (sl - 1)) && sl < 6) ++sl;
+    }
+    if (tc) {
+      int i = 31 - __clz((int)m), zleft = i + 1 - tc;
+      if (tc < maxc) {
+        const uint32_t e = cd ? d_cavlc.cdtz[tc - 1][zleft] : d_cavlc.tz[tc - 1][zleft];
+        b.put(e >> 8, e & 0xffu);
+      }
+      rest = m ^ (1u << i);
+#pragma unroll 1
+      while (rest && zleft > 0) {
+        const int j = 31 - __clz((int)rest), r = i - j - 1;
+        const uint32_t e = d_cavlc.run[zleft <= 6 ? zleft - 1 : 6][r];
+        b.put(e >> 8, e & 0xffu);
+        rest ^= 1u << j;
+        zleft -= r;
+        i = j;
+      }
+    }
+  }
+  if (b.nb) *b.w = (uint32_t)(b.acc << (32u - b.nb));
+
+  // ---- place the lanes' bits one after another -------------------------------
+  __syncwarp();
   const uint32_t len = b.pos;
   uint32_t off = len;
+#pragma unroll
   for (int o = 1; o < 32; o <<= 1) {
-    const uint32_t y = __shfl_up_sync(0xffffffffu, off, o);
+    const uint32_t y = __shfl_up_sync(full, off, o);
     if (lane >= o) off += y;
   }
-  const uint32_t total = __shfl_sync(0xffffffffu, off, 31);
+  const uint32_t total = __shfl_sync(full, off, 31);
   off -= len;
-  const bool over = __any_sync(0xffffffffu, b.over) || total > 32u * kCavlcMbWords;
-  if (over) {
-    if (lane == 0) {
-      atomicExch(a.err, 1u);
-      a.nbits[mb] = 0;
-    }
+  if (total > 32u * kCavlcMbWords) {
+    if (lane == 0) a.nbits[mb] = kCavlcOver;
     return;
   }
-  uint32_t* sw = shw[wi];
   const uint32_t nw = (total + 31u) >> 5;
-  for (uint32_t k = lane; k < nw; k += 32) sw[k] = 0u;
+  for (uint32_t i = lane; i < nw; i += 32) sh.out[i] = 0u;
   __syncwarp();
-  for (uint32_t k = 0; 32u * k < len; ++k) {
-    const int m = (int)min(32u, len - 32u * k);
-    const uint32_t v = lw[k] >> (32 - m), left = m < 32 ? v << (32 - m) : v;
-    const uint32_t pos = off + 32u * k, wd = pos >> 5, sh = pos & 31u;
-    atomicOr(sw + wd, left >> sh);
-    if (sh + (uint32_t)m > 32u) atomicOr(sw + wd + 1, left << (32u - sh));
+  {
+    const uint32_t* w = sh.lane + (lane < 28 ? lane : 27) * kCavlcLaneWords;
+    uint32_t* d = sh.out + (off >> 5);
+    const uint32_t s = off & 31u;
+#pragma unroll 1
+    for (uint32_t i = 0; 32u * i < len; ++i) {  // the last word's unused low bits are zero
+      const uint32_t v = w[i];
+      atomicOr(d + i, v >> s);
+      if (s && (v << (32u - s))) atomicOr(d + i + 1, v << (32u - s));
+    }
   }
   __syncwarp();
   uint32_t* dst = a.words + (size_t)mb * kCavlcMbWords;
-  for (uint32_t k = lane; k < nw; k += 32) dst[k] = sw[k];
+  for (uint32_t i = lane; i < nw; i += 32) dst[i] = sh.out[i];
   if (lane == 0) a.nbits[mb] = total;
 }
 
-// ---- 3. per slice: skip runs, offsets, length --------------------------------------
+// ---- 2. per slice: skip runs, offsets, length --------------------------------------
 // A chunk of consecutive macroblocks seen from the run of skipped macroblocks:
 // `has` a coded one, R = the skips after its last coded macroblock (or all
 // of its macroblocks when none is coded). Chunks compose left to right.
@@ -435,20 +593,7 @@ __device__ uint32_t scan_sum(uint32_t v, uint32_t* sh, uint32_t* total) {
   return r;
 }
 
-// OR n <= 32 bits (the low n of v) into MSB-first words at bit position pos.
-__device__ __forceinline__ void or_bits(uint32_t* dst, uint32_t pos, uint32_t v, int n, bool atomic) {
-  if (n <= 0) return;
-  const uint32_t left = n < 32 ? v << (32 - n) : v;  // left-aligned
-  const uint32_t k = pos >> 5, sh = pos & 31u;
-  const uint32_t hi = left >> sh;
-  if (atomic) atomicOr(dst + k, hi);
-  else dst[k] |= hi;
-  if (sh + (uint32_t)n > 32u) {
-    const uint32_t lo = left << (32u - sh);
-    if (atomic) atomicOr(dst + k + 1, lo);
-    else dst[k + 1] |= lo;
-  }
-}
+__device__ __forceinline__ uint32_t ue_len(uint32_t v) { return 2u * (31u - (uint32_t)__clz((int)(v + 1u))) + 1u; }
 
 __global__ void __launch_bounds__(kCavlcScanThreads) cavlc_slice_kernel(CavlcArgs a, CavlcHdr h) {
   __shared__ RunState shr[32];
@@ -464,93 +609,137 @@ __global__ void __launch_bounds__(kCavlcScanThreads) cavlc_slice_kernel(CavlcArg
   const bool runs = !a.is_intra;
   uint32_t lead = 0, tail = 0, inner = 0, has = 0;
   for (uint32_t mb = i0; mb < i1; ++mb) {
-    if (a.info[mb] & 1u) {
+    const uint32_t n = a.nbits[mb];
+    if (n == 0u) {
       if (has) ++tail;
       else ++lead;
     } else {
-      inner += (has && runs ? (uint32_t)ue_bits(tail) : 0u) + a.nbits[mb];
+      inner += (has && runs ? ue_len(tail) : 0u) + n;
       tail = 0;
       has = 1;
     }
   }
+  // a macroblock of any slice that outgrew its region fails the picture
+  bool over = false;
+  for (uint32_t mb = t; mb < mbs; mb += kCavlcScanThreads) over |= a.nbits[mb] == kCavlcOver;
+  over = __syncthreads_or(over);
   RunState all;
   const RunState in = scan_run(RunState{has, has ? tail : lead}, shr, &all);
-  const uint32_t mine = has ? (runs ? (uint32_t)ue_bits(in.r + lead) : 0u) + inner : 0u;
+  const uint32_t mine = has ? (runs ? ue_len(in.r + lead) : 0u) + inner : 0u;
   uint32_t data = 0;
   const uint32_t base = (uint32_t)h.len[s] + scan_sum(mine, shs, &data);
   const uint32_t trail = all.r;  // skips after the slice's last coded macroblock
-  const uint32_t bits = (uint32_t)h.len[s] + data + (trail ? (uint32_t)ue_bits(trail) : 0u) + 1u;
+  const uint32_t bits = (uint32_t)h.len[s] + data + (trail ? ue_len(trail) : 0u) + 1u;
   const uint32_t bytes = (bits + 7u) >> 3;
-  const bool fits = bytes <= a.slice_cap && *a.err == 0u;
-  // offsets and runs of the coded macroblocks
+  const bool fits = bytes <= a.slice_cap && !over;
+  // offsets of the macroblocks, runs of the coded ones
   uint32_t pos = base, run = in.r;
   for (uint32_t mb = i0; mb < i1; ++mb) {
-    if (a.info[mb] & 1u) {
+    const uint32_t n = a.nbits[mb];
+    a.place[mb] = make_uint4(pos, n, runs ? run : kCavlcNoRun, 0u);
+    if (n == 0u) {
       ++run;
     } else {
-      a.off[mb] = pos;
-      a.run[mb] = runs ? run : 0xffffffffu;
-      pos += (runs ? (uint32_t)ue_bits(run) : 0u) + a.nbits[mb];
+      pos += (runs ? ue_len(run) : 0u) + n;
       run = 0;
     }
   }
-  uint32_t* dst = reinterpret_cast<uint32_t*>(a.out + (size_t)s * a.slice_cap);
-  const uint32_t nw = (bytes + 3u) >> 2;
-  if (fits)
-    for (uint32_t k = t; k < nw; k += kCavlcScanThreads) dst[k] = 0u;
-  __syncthreads();
   if (t == 0) {
     a.sl[4 * s + 0] = bits;
     a.sl[4 * s + 1] = trail;
     a.sl[4 * s + 2] = fits ? 0u : 1u;
+    a.sl[4 * s + 3] = (uint32_t)h.len[s] + data;
     a.out_bytes[s] = fits ? bytes : 0xffffffffu;
-    if (fits) {
-      for (int k = 0; k < 4 && 32 * k < h.len[s]; ++k)
-        or_bits(dst, 32u * k, h.bits[s][k] >> (32 - min(32, h.len[s] - 32 * k)), min(32, h.len[s] - 32 * k), false);
-      uint32_t p = (uint32_t)h.len[s] + data;
-      if (trail) {  // mb_skip_run of the slice's last macroblocks
-        const int l = ilog2(trail + 1u);
-        or_bits(dst, p + (uint32_t)l, trail + 1u, l + 1, false);
-        p += (uint32_t)(2 * l + 1);
-      }
-      or_bits(dst, p, 1u, 1, false);  // rbsp_stop_one_bit; the alignment zeros are the cleared words
-    }
   }
 }
 
-// ---- 4. place each coded macroblock's bits -------------------------------------
-__global__ void __launch_bounds__(128) cavlc_pack_kernel(CavlcArgs a) {
-  const int mb = blockIdx.x * blockDim.x + threadIdx.x;
-  const uint32_t mbs = (uint32_t)(a.mbw * a.mbh);
-  if (mb >= (int)mbs || (a.info[mb] & 1u)) return;
-  const uint32_t s = slice_of((uint32_t)mb, mbs, (uint32_t)a.ns);
-  if (a.sl[4 * s + 2]) return;  // the slice did not fit
-  uint32_t* dst = reinterpret_cast<uint32_t*>(a.out + (size_t)s * a.slice_cap);
-  const uint32_t run = a.run[mb];
-  uint32_t p = a.off[mb];
-  if (run != 0xffffffffu) {  // mb_skip_run (P slices)
-    const int l = ilog2(run + 1u);
-    or_bits(dst, p + (uint32_t)l, run + 1u, l + 1, true);
-    p += (uint32_t)(2 * l + 1);
-  }
-  const uint32_t n = a.nbits[mb];
-  const uint32_t* w = a.words + (size_t)mb * kCavlcMbWords;
-  for (uint32_t k = 0; 32u * k < n; ++k) {
-    const int m = (int)min(32u, n - 32u * k);
-    or_bits(dst, p + 32u * k, w[k] >> (32 - m), m, true);
-  }
-}
-
-// MSB-first words -> stream bytes (in place, or into out_copy: only the
-// slice's bytes cross to a host mapping).
-__global__ void cavlc_bytes_kernel(CavlcArgs a) {
+// ---- 3. every output word's bits -------------------------------------------------
+// A thread per 32-bit word of the slice: it finds the macroblock its first bit
+// falls into and collects the pieces that overlap the word, so no word is
+// cleared, shared or swapped afterwards. A warp's 32 words are found together:
+// a 32-way search over the offsets (three dependent loads for a 1080p frame
+// where a binary search takes thirteen) down to the first word's macroblock,
+// then the 32 macroblocks from there on in registers.
+__global__ void __launch_bounds__(256) cavlc_gather_kernel(CavlcArgs a, CavlcHdr h) {
   const int s = blockIdx.y;
-  const uint32_t nb = a.sl[4 * s + 2] ? 0xffffffffu : (a.sl[4 * s + 0] + 7u) >> 3;
-  if (nb == 0xffffffffu) return;
-  const uint32_t* src = reinterpret_cast<const uint32_t*>(a.out + (size_t)s * a.slice_cap);
+  if (a.sl[4 * s + 2]) return;  // the slice did not fit
+  const uint32_t bits = a.sl[4 * s + 0], trail = a.sl[4 * s + 1], end = a.sl[4 * s + 3];
+  const uint32_t nw = (((bits + 7u) >> 3) + 3u) >> 2, hl = (uint32_t)h.len[s];
+  const uint32_t mbs = (uint32_t)(a.mbw * a.mbh);
+  const uint32_t m0 = slice_start(s, mbs, a.ns), m1 = slice_start(s + 1, mbs, a.ns);
   uint32_t* dst = reinterpret_cast<uint32_t*>(a.out_copy + (size_t)s * a.slice_cap);
-  for (uint32_t k = blockIdx.x * blockDim.x + threadIdx.x; k < (nb + 3u) >> 2; k += gridDim.x * blockDim.x)
-    dst[k] = __byte_perm(src[k], 0u, 0x0123);
+  const uint32_t lane = threadIdx.x & 31u;
+  for (uint32_t k0 = blockIdx.x * blockDim.x + threadIdx.x - lane; k0 < nw; k0 += gridDim.x * blockDim.x) {
+    const uint32_t k = k0 + lane, p = 32u * k, p0 = 32u * k0;
+    // the last macroblock that starts at or before p0 (the first one, if none does)
+    uint32_t lo = m0, cnt = m1 - m0;
+    while (cnt > 1u) {
+      const uint32_t step = (cnt + 31u) >> 5, i = lo + lane * step;
+      const uint32_t le = __ballot_sync(0xffffffffu, lane * step < cnt && a.place[i].x <= p0);
+      const uint32_t j = le ? 31u - (uint32_t)__clz((int)le) : 0u;
+      cnt = min(step, cnt - j * step);
+      lo += j * step;
+    }
+    const uint32_t o = lo + lane < m1 ? a.place[lo + lane].x : 0xffffffffu;
+    uint32_t mb0 = 0;
+#pragma unroll
+    for (uint32_t st = 16u; st > 0u; st >>= 1) {
+      const uint32_t t = __shfl_sync(0xffffffffu, o, (int)(mb0 + st));
+      if (t <= p) mb0 += st;
+    }
+    const bool beyond = mb0 == 31u;  // words reaching past the 32 macroblocks (few bits each)
+    mb0 += lo;
+    if (k >= nw) continue;
+    uint32_t w = 0;
+    // n <= 32 bits v at stream position at (overlapping this word or not)
+    auto add = [&](uint32_t at, uint32_t n, uint32_t v) {
+      const uint32_t lft = n < 32u ? (n ? v << (32u - n) : 0u) : v;  // left-aligned
+      const int d = (int)(at - p);
+      if (d >= 0 && d < 32) w |= lft >> d;
+      else if (d < 0 && d > -32) w |= lft << -d;
+    };
+    if (p < hl) w |= h.bits[s][k] & (hl - p < 32u ? ~(0xffffffffu >> (hl - p)) : 0xffffffffu);
+    if (p + 32u > hl && p < end) {
+      if (beyond) {
+        uint32_t hi = m1 - 1u;
+        while (mb0 < hi) {
+          const uint32_t mid = (mb0 + hi + 1u) >> 1;
+          if (a.place[mid].x <= p) mb0 = mid;
+          else hi = mid - 1u;
+        }
+      }
+      uint4 next = a.place[mb0];
+      for (uint32_t mb = mb0; mb < m1; ++mb) {
+        const uint4 pl = next;
+        if (pl.x >= p + 32u) break;
+        if (mb + 1u < m1) next = a.place[mb + 1u];  // in flight while this one's words are read
+        uint32_t at = pl.x;
+        const uint32_t n = pl.y, run = pl.z;
+        if (n == 0u) continue;
+        if (run != kCavlcNoRun) {  // mb_skip_run (P slices): the last l + 1 bits of its 2l + 1
+          const uint32_t l = 31u - (uint32_t)__clz((int)(run + 1u));
+          add(at + l, l + 1u, run + 1u);
+          at += 2u * l + 1u;
+        }
+        // the macroblock's words that overlap [p, p + 32): at most two
+        const uint32_t* mw = a.words + (size_t)mb * kCavlcMbWords;
+        const uint32_t f = p > at ? (p - at) >> 5 : 0u;
+#pragma unroll
+        for (uint32_t i = 0; i < 2u; ++i)
+          if (32u * (f + i) < n) add(at + 32u * (f + i), 32u, mw[f + i]);  // unused low bits are zero
+      }
+    }
+    if (p + 32u > end) {  // trailing skips, rbsp_stop_one_bit; alignment zeros
+      uint32_t at = end;
+      if (trail) {
+        const uint32_t l = 31u - (uint32_t)__clz((int)(trail + 1u));
+        add(at + l, l + 1u, trail + 1u);
+        at += 2u * l + 1u;
+      }
+      add(at, 1u, 1u);
+    }
+    dst[k] = __byte_perm(w, 0u, 0x0123);
+  }
 }
 
 }  // namespace b200enc
@@ -560,7 +749,7 @@ using namespace b200enc;
 namespace {
 
 struct CavlcLayout {
-  size_t info, tcs, nbits, words, off, run, sl, err, bytes;
+  size_t nbits, words, place, sl, bytes;
 };
 
 size_t up256(size_t x) { return (x + 255) & ~(size_t)255; }
@@ -568,14 +757,10 @@ size_t up256(size_t x) { return (x + 255) & ~(size_t)255; }
 CavlcLayout cavlc_layout(int mbw, int mbh) {
   const size_t mbs = (size_t)mbw * mbh;
   CavlcLayout l;
-  l.err = 0;
-  l.sl = 256;
-  l.info = l.sl + up256(kCavlcMaxSlices * 16);
-  l.tcs = l.info + up256(mbs * 4);
-  l.nbits = l.tcs + up256(mbs * 24);
-  l.off = l.nbits + up256(mbs * 4);
-  l.run = l.off + up256(mbs * 4);
-  l.words = l.run + up256(mbs * 4);
+  l.sl = 0;
+  l.nbits = l.sl + up256(kCavlcMaxSlices * 16);
+  l.place = l.nbits + up256(mbs * 4);
+  l.words = l.place + up256(mbs * 16);
   l.bytes = l.words + mbs * kCavlcMbWords * 4;
   return l;
 }
@@ -625,25 +810,21 @@ extern "C" int b200enc_cavlc_slices(const b200enc_cavlc_t* p, void* stream) {
   a.nz = p->nz;
   a.pred_mode = p->pred_mode;
   a.mv = static_cast<const MV*>(p->mv);
-  a.info = reinterpret_cast<uint32_t*>(sc + L.info);
-  a.tcs = sc + L.tcs;
   a.nbits = reinterpret_cast<uint32_t*>(sc + L.nbits);
   a.words = reinterpret_cast<uint32_t*>(sc + L.words);
-  a.off = reinterpret_cast<uint32_t*>(sc + L.off);
-  a.run = reinterpret_cast<uint32_t*>(sc + L.run);
+  a.place = reinterpret_cast<uint4*>(sc + L.place);
   a.sl = reinterpret_cast<uint32_t*>(sc + L.sl);
-  a.err = reinterpret_cast<uint32_t*>(sc + L.err);
   a.out = p->out;
   a.slice_cap = (uint32_t)std::min<size_t>(p->slice_cap, 0xfffffffcu);
   a.out_bytes = p->out_bytes;
   a.out_copy = p->out_copy ? p->out_copy : p->out;
   cudaStream_t st = static_cast<cudaStream_t>(stream);
   const int mbs = p->mbw * p->mbh;
-  if (cudaMemsetAsync(a.err, 0, 4, st) != cudaSuccess) return -1;
-  cavlc_info_kernel<<<(mbs + 127) / 128, 128, 0, st>>>(a);
   cavlc_mb_kernel<<<(mbs + kCavlcMbWarps - 1) / kCavlcMbWarps, 32 * kCavlcMbWarps, 0, st>>>(a);
   cavlc_slice_kernel<<<p->num_slices, kCavlcScanThreads, 0, st>>>(a, h);
-  cavlc_pack_kernel<<<(mbs + 127) / 128, 128, 0, st>>>(a);
-  cavlc_bytes_kernel<<<dim3(16, p->num_slices), 256, 0, st>>>(a);
+  // words per slice are known on the device only: a CTA of 256 words per 16
+  // macroblocks (the share of a dense one), walking the rest in strides
+  const int ctas = std::max(1, std::min(128, mbs / p->num_slices / 16));
+  cavlc_gather_kernel<<<dim3(ctas, p->num_slices), 256, 0, st>>>(a, h);
   return cudaGetLastError() == cudaSuccess ? 0 : -1;
 }
