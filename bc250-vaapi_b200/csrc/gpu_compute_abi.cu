@@ -100,7 +100,6 @@ struct Impl {
   int entropy = 0, quality = 4;
   void* d_cavlc = nullptr;     // b200enc_cavlc_scratch_bytes
   size_t cavlc_bytes = 0;
-  uint8_t* d_slices = nullptr;  // the slices' bit words
   size_t slices_bytes = 0;
 };
 
@@ -126,9 +125,7 @@ void free_frame_buffers(Impl* m) {
   cudaFree(m->d_mv_prev);
   cudaFree(m->d_scratch);
   cudaFree(m->d_cavlc);
-  cudaFree(m->d_slices);
   m->d_cavlc = nullptr;
-  m->d_slices = nullptr;
   m->cavlc_bytes = m->slices_bytes = 0;
   if (m->prop) b200enc_proposal_destroy(m->prop);
   m->prop = nullptr;
@@ -289,16 +286,13 @@ int ensure_entropy(Impl* m) {
   const size_t mbs = (size_t)m->mbw * m->mbh;
   m->cavlc_bytes = b200enc_cavlc_scratch_bytes(m->mbw, m->mbh);
   m->slices_bytes = 16 * slice_cap_of(mbs, 16) + mbs * 2560;
-  bool ok = cudaMalloc(&m->d_cavlc, m->cavlc_bytes) == cudaSuccess &&
-            cudaMalloc(&m->d_slices, m->slices_bytes) == cudaSuccess;
+  bool ok = cudaMalloc(&m->d_cavlc, m->cavlc_bytes) == cudaSuccess;
   for (Slot& s : m->slot)
     ok = ok && cudaHostAlloc(&s.slices, m->slices_bytes, cudaHostAllocMapped) == cudaSuccess &&
          cudaHostAlloc(&s.slice_bytes, 16 * sizeof(uint32_t), cudaHostAllocMapped) == cudaSuccess;
   if (!ok) {
     cudaFree(m->d_cavlc);
-    cudaFree(m->d_slices);
     m->d_cavlc = nullptr;
-    m->d_slices = nullptr;
     for (Slot& s : m->slot) {
       cudaFreeHost(s.slices);
       cudaFreeHost(s.slice_bytes);
@@ -403,13 +397,12 @@ int encode_frame(gpu_context_t* ctx, Impl* m, const uint8_t* y, const uint8_t* u
     cp.nz = m->d_nz;
     cp.pred_mode = m->d_pred_mode;
     cp.mv = m->d_mv;
-    cp.out = m->d_slices;
     cp.slice_cap = slice_cap_of(mbs, cp.num_slices);
     uint8_t* dev_slices = nullptr;
     uint32_t* dev_bytes = nullptr;
     rc |= cudaHostGetDevicePointer((void**)&dev_slices, sl.slices, 0) == cudaSuccess ? 0 : -1;
     rc |= cudaHostGetDevicePointer((void**)&dev_bytes, sl.slice_bytes, 0) == cudaSuccess ? 0 : -1;
-    cp.out_copy = dev_slices;
+    cp.out = dev_slices;
     cp.out_bytes = dev_bytes;
     cp.scratch = m->d_cavlc;
     cp.scratch_bytes = m->cavlc_bytes;
@@ -860,6 +853,30 @@ struct NalOut {
     }
     acc &= nacc ? ((1ull << nacc) - 1ull) : 0ull;
   }
+  // n whole bytes behind the pending bits, eight at a time. A group without a
+  // zero byte that does not follow two zeros needs no emulation prevention
+  // (most of CAVLC data): it is stored as it is; the others go byte by byte.
+  // Assembling one 360 KB picture took ~1 ms a byte at a time.
+  void bytes(const uint8_t* d, size_t count) {
+    size_t k = 0;
+    for (; k + 8 <= count; k += 8) {
+      uint64_t v;
+      memcpy(&v, d + k, 8);
+      v = __builtin_bswap64(v);
+      const uint64_t x = nacc ? (acc << (64 - nacc)) | (v >> nacc) : v;
+      if (nacc) acc = v & ((1ull << nacc) - 1ull);
+      const bool has_zero = ((x - 0x0101010101010101ull) & ~x & 0x8080808080808080ull) != 0;
+      if (!has_zero && zeros < 2 && n + 8 <= cap) {
+        const uint64_t be = __builtin_bswap64(x);
+        memcpy(p + n, &be, 8);
+        n += 8;
+        zeros = 0;
+      } else {
+        for (int s = 56; s >= 0; s -= 8) byte((uint8_t)(x >> s));
+      }
+    }
+    for (; k < count; ++k) put(8, d[k]);
+  }
 };
 
 }  // namespace
@@ -893,7 +910,7 @@ int b200enc_ctx_slice_nals(gpu_context_t* ctx, int slot, const uint8_t* headers,
     const uint8_t* d = sl.slices + (size_t)s * slice_cap_of((size_t)m->mbw * m->mbh, sl.num_slices);
     const uint8_t last = d[nb - 1];
     const int data_bits_last = 7 - __builtin_ctz(last);  // bits before the stop bit in the last byte
-    for (uint32_t k = 0; k + 1 < nb; ++k) o.put(8, d[k]);
+    o.bytes(d, nb - 1);
     o.put(data_bits_last, (uint32_t)(last >> (8 - data_bits_last)));
     o.put(1, 1u);
     if (o.nacc) o.put(8 - o.nacc, 0u);

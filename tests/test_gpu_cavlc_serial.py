@@ -104,6 +104,49 @@ def test_transform8_and_quality_match_serial_writer(gpu, serial, choose, quality
         assert _gpu(gpu, *a, **kw) == serial(*a, **kw)
 
 
+def _nal(rbsp, ref_idc, kind):
+    out, zeros = bytearray([0, 0, 0, 1, ref_idc << 5 | kind]), 0
+    for b in rbsp:
+        if zeros == 2 and b <= 3:
+            out.append(3)
+            zeros = 0
+        out.append(b)
+        zeros = zeros + 1 if b == 0 else 0
+    return bytes(out)
+
+
+@pytest.mark.gpu
+@pytest.mark.parametrize("W,H,ns,qp", [(64, 48, 1, 30), (320, 192, 3, 14), (640, 480, 2, 38)])
+def test_slice_nals_match_serial_writer(gpu, serial, W, H, ns, qp):
+    """A context's NAL units: the serial writer's RBSP behind headers of 0 to
+    128 bits (every bit offset of the data, headers full of zeros, so that
+    emulation prevention acts), start codes, emulation prevention bytes."""
+    from b200enc import synth
+    seq = synth.Sequence(W, H, seed=W, pan=True)
+    ctx = gpu.Context()
+    ctx.configure(search_range=16, deblock=1)
+    ctx.set_entropy(1)
+    img, mem = ctx.create_image(W, H)
+    out = np.zeros(W * H * 4 + 65536, np.uint8)
+    try:
+        for t, bits in enumerate((0, 1, 26, 27, 60, 95, 128)):
+            y, uv = seq.frame(t)
+            ctx.upload(img, mem, y // 64 * 64 if t == 3 else y, uv)
+            slot = ctx.encode(img, W, H, qp, t % 4 == 0, ns)
+            assert ctx.sync(slot) == 0
+            g = {k: np.ascontiguousarray(v) for k, v in ctx.staging(slot).items()}
+            hdr, hb = np.zeros((ns, 16), np.uint8), np.full(ns, bits, np.int32)
+            hdr[:, 3] = 0x80
+            n = ctx.slice_nals(slot, hdr, hb, 2, 1, out)
+            heads = [(int.from_bytes(bytes(h), "big") >> (128 - bits), bits) for h in hdr]
+            want = serial((W + 15) // 16, (H + 15) // 16, qp, int(t % 4 == 0), ns, g["levels"], g["dc"], g["nz"],
+                          g["pred_mode"], g["mv"], headers=heads)
+            assert out[:n].tobytes() == b"".join(_nal(w, 2, 1) for w in want), f"frame {t}"
+    finally:
+        ctx.destroy_image(img, mem)
+        ctx.close()
+
+
 @pytest.mark.parametrize("intra", [1, 0])
 def test_serial_writer_matches_reference(oracle_mod, serial, intra):
     if not oracle_mod.cavlc_ref_available():
