@@ -22,6 +22,7 @@ int b200enc_me_full_search_err(const uint8_t* cur_y, int cur_pitch, const uint8_
 int b200enc_me_batch_launch(const b200enc::BatchTab& bt, int range, const int* list, const int* count, int ctas,
                             cudaStream_t st);
 int b200enc_p_frame_batch_launch(const b200enc::BatchTab& bt, int n, cudaStream_t st);
+int b200enc_i_frame_groups(int mbh);
 int b200enc_i_frame_batch_launch(const b200enc::BatchTab& bt, int ctas, uint32_t max_wait, cudaStream_t st);
 int b200enc_deblock_tiles_launch(int mbw, int mbh, int qp, int is_intra, const uint32_t* nz, const void* mv,
                                  const uint8_t* src_y, const uint8_t* src_uv, uint8_t* dst_y, uint8_t* dst_uv,

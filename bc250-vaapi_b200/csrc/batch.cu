@@ -330,9 +330,9 @@ int b200enc_batch_encode(void* h, const b200enc_batch_frame_t* frames) {
     const int mbs = t.mbw * t.mbh;
     if (f.is_intra) {
       ii[ni] = s;
-      pi[ni + 1] = pi[ni] + t.mbh;
+      pi[ni + 1] = pi[ni] + b200enc_i_frame_groups(t.mbh);
       ++ni;
-      n_irows += t.mbh;
+      n_irows = pi[ni];
     } else {
       // each P stream's range starts on a network tile (16 macroblocks), so
       // the FP8 network's per-tile activation scales see the same macroblocks

@@ -219,10 +219,9 @@ __device__ __forceinline__ uint64_t global_ns() {
 }
 
 // Scratch layout of the wavefront kernels (one region per launch):
-//   [0] ticket counter, [1] error code, [2] error detail, [3] reserved,
-//   [4 .. 4+mbh) per-row progress (luma rows for deblocking, the only rows
-//   of the intra wavefront), [4+mbh .. 4+2*mbh) chroma-row progress of the
-//   deblocking wavefront.
+//   [0] ticket counter (of the intra wavefront's luma rows), [1] error code,
+//   [2] error detail, [3] the intra wavefront's chroma tickets,
+//   [4 .. 4+mbh) luma-row progress, [4+mbh .. 4+2*mbh) chroma-row progress.
 struct Scratch {
   uint32_t* base;
   __device__ uint32_t* ticket() const { return base; }
@@ -280,10 +279,10 @@ struct BatchTab {
   BatchSet p_mbs;   // macroblocks of the streams coding a P frame (the compact P index); each
                     // stream's range is padded to a multiple of 16 items, the padding items
                     // (local index >= the stream's macroblock count) do no work
-  BatchSet i_rows;  // macroblock rows of the streams coding an I frame
+  BatchSet i_rows;  // intra row groups (b200enc_i_frame_groups) of the streams coding an I frame
   BatchSet groups;  // deblocking tiles of every stream
   MV* mvc;          // motion vectors by compact P index
-  uint32_t* ticket; // [0] intra rows
+  uint32_t* ticket; // intra row groups: [0] luma, [1] chroma
   int db_rows;      // tile deblocking: tile height in macroblocks
   int db_cols;      // tile deblocking: tile width in macroblocks
 };

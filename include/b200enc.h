@@ -86,7 +86,7 @@ int b200enc_p_frame(const uint8_t *cur_y, const uint8_t *cur_uv, int cur_pitch,
                     uint8_t *rec_y, uint8_t *rec_uv, int rec_pitch, void *stream);
 
 /* Bytes of scratch the wavefront kernels (intra, deblock) need for a frame
- * of mbh macroblock rows: a ticket, an error word and two progress words per
+ * of mbh macroblock rows: tickets, an error word and two progress words per
  * row (luma and chroma wavefronts). The scratch must be zeroed before each launch; the *_frame calls
  * below do that themselves on `stream`. */
 size_t b200enc_wavefront_scratch_bytes(int mbh);
@@ -103,9 +103,10 @@ size_t b200enc_wavefront_scratch_bytes(int mbh);
 
 /* I-frame intra wavefront: I16x16 4-mode decision from reconstructed
  * neighbours, chroma DC prediction, full transform/quant/DC/recon chain per
- * macroblock, in a persistent kernel whose CTAs take macroblock rows by
- * ticket and wait (bounded) on per-row progress words for the top
- * neighbour. Replaces the per-diagonal dispatch loop over
+ * macroblock, in a persistent kernel whose CTAs take groups of macroblock
+ * rows (luma and chroma apart) by ticket and wait (bounded) on per-row
+ * progress words for the top neighbour; at most `ctas` CTAs (0: two per
+ * group). Replaces the per-diagonal dispatch loop over
  * shaders/intra_wavefront.comp (src/gpu_compute.c:3217-3251). Writes
  * mv[] = 0. rec planes are read and written in place. */
 int b200enc_i_frame(const uint8_t *cur_y, const uint8_t *cur_uv, int cur_pitch,
@@ -238,7 +239,7 @@ int b200enc_batch_graph_stats(void *b, long *instantiations, long *updates);
 #define B200ENC_TUNE_PCHAIN_MBS_PER_CTA 1   /* macroblocks per P-chain CTA, 1, 2 or 4 (default 1) */
 #define B200ENC_TUNE_RESCORE_CTAS_PER_SM 2  /* learned re-scoring grid, CTAs per SM, 1..16 (default 8) */
 #define B200ENC_TUNE_FALLBACK_CTAS_PER_SM 3 /* fallback full-search grid, CTAs per SM, 1..16 (default 16) */
-#define B200ENC_TUNE_INTRA_CTAS 4           /* intra wavefront CTAs (rows in flight), >= 1 (default: one per row) */
+#define B200ENC_TUNE_INTRA_CTAS 4           /* intra wavefront CTAs (groups of four luma or chroma rows in flight), >= 1 (default: all) */
 #define B200ENC_TUNE_ME_STAGE 5             /* full-search window staging: 1 word loads, 2 TMA (default TMA) */
 #define B200ENC_TUNE_DEBLOCK_TILE_W 6       /* tile deblocking: tile width in macroblocks, 1..16 (default 4 or 8, by size) */
 #define B200ENC_TUNE_DEBLOCK_TILE_H 7       /* tile deblocking: tile height in macroblocks, 1..8 (default 4 or 8, by size) */
