@@ -499,55 +499,50 @@ __global__ void lp_loss_kernel(int mbs, LpBuf b, const int* __restrict__ label, 
                                const float* __restrict__ weight, __nv_bfloat16* __restrict__ g5,
                                float* __restrict__ loss) {
   const int mb = blockIdx.x * blockDim.x + threadIdx.x;
-  if (mb >= mbs) return;
-  const float nval = (float)max(b.counters[2], 1);
-  const float w = weight[mb] / nval;
-  const uint32_t dup = (b.state[mb] >> 8) & 0x3ffu;
-  float z[kClasses], p[kClasses];
-  for (int j = 0; j < kClasses; ++j) z[j] = b.logits[(size_t)mb * kOut + j];
-  masked_softmax(z, dup, p);
-  const uint32_t y = (uint32_t)label[mb];
-  float pset = 0.f;
-  for (int j = 0; j < kClasses; ++j)
-    if ((y >> j) & 1u) pset += p[j];
-  pset = fmaxf(pset, 1e-30f);
-  const float zs = b.logits[(size_t)mb * kOut + 11];
-  const float ps = 1.f / (1.f + expf(-zs));
-  const float t = norez[mb];
-  __nv_bfloat16* gr = g5 + (size_t)mb * kOut;
-  for (int j = 0; j < kClasses; ++j)
-    gr[j] = __float2bfloat16_rn(w * (p[j] - (((y >> j) & 1u) ? p[j] / pset : 0.f)));
-  gr[11] = __float2bfloat16_rn(w * 0.5f * (ps - t));
-  for (int j = 12; j < kOut; ++j) gr[j] = __float2bfloat16_rn(0.f);
-  if (weight[mb] > 0.f) {
-    // softplus forms of -log p_y and the BCE
-    const float ce = -logf(pset);
-    const float bce = fmaxf(zs, 0.f) - zs * t + log1pf(expf(-fabsf(zs)));
-    atomicAdd(loss, w * (ce + 0.5f * bce));
+  float term = 0.f;
+  if (mb < mbs) {
+    const float w = weight[mb] / (float)max(b.counters[2], 1);
+    const uint32_t dup = (b.state[mb] >> 8) & 0x3ffu;
+    float z[kOut], p[kClasses], gr[kOut];
+    const float4* zp = reinterpret_cast<const float4*>(b.logits + (size_t)mb * kOut);
+#pragma unroll
+    for (int j = 0; j < kOut / 4; ++j) {
+      const float4 v = zp[j];
+      z[4 * j] = v.x, z[4 * j + 1] = v.y, z[4 * j + 2] = v.z, z[4 * j + 3] = v.w;
+    }
+    masked_softmax(z, dup, p);
+    const uint32_t y = (uint32_t)label[mb];
+    float pset = 0.f;
+#pragma unroll
+    for (int j = 0; j < kClasses; ++j)
+      if ((y >> j) & 1u) pset += p[j];
+    pset = fmaxf(pset, 1e-30f);
+    const float zs = z[11];
+    const float ps = 1.f / (1.f + expf(-zs));
+    const float t = norez[mb];
+#pragma unroll
+    for (int j = 0; j < kOut; ++j)
+      gr[j] = j < kClasses ? w * (p[j < kClasses ? j : 0] - (((y >> j) & 1u) ? p[j < kClasses ? j : 0] / pset : 0.f))
+                           : (j == 11 ? w * 0.5f * (ps - t) : 0.f);
+    uint32_t o[kOut / 2];
+#pragma unroll
+    for (int j = 0; j < kOut / 2; ++j)
+      o[j] = (uint32_t)__bfloat16_as_ushort(__float2bfloat16_rn(gr[2 * j])) |
+             (uint32_t)__bfloat16_as_ushort(__float2bfloat16_rn(gr[2 * j + 1])) << 16;
+    uint4* dst = reinterpret_cast<uint4*>(g5 + (size_t)mb * kOut);
+    dst[0] = make_uint4(o[0], o[1], o[2], o[3]);
+    dst[1] = make_uint4(o[4], o[5], o[6], o[7]);
+    if (weight[mb] > 0.f) {
+      // softplus forms of -log p_y and the BCE
+      const float ce = -logf(pset);
+      const float bce = fmaxf(zs, 0.f) - zs * t + log1pf(expf(-fabsf(zs)));
+      term = w * (ce + 0.5f * bce);
+    }
   }
-}
-
-// G[r][c] = bf16(dA[r*lda + c] * (Y[r*ldy + c] > 0)), c < C
-__global__ void lp_relu_bwd_kernel(long long rows, int C, const float* __restrict__ dA, int lda,
-                                   const __nv_bfloat16* __restrict__ Y, int ldy, __nv_bfloat16* __restrict__ G) {
-  const long long i = (long long)blockIdx.x * blockDim.x + threadIdx.x;
-  if (i >= rows * C) return;
-  const long long r = i / C;
-  const int c = (int)(i - r * C);
-  const float y = __bfloat162float(Y[r * ldy + c]);
-  G[i] = __float2bfloat16_rn(y > 0.f ? dA[r * lda + c] : 0.f);
-}
-
-// out[c] += sum over rows of G[r][c] (G is [rows][C] BF16)
-__global__ void lp_colsum_kernel(long long rows, int C, const __nv_bfloat16* __restrict__ G, float* __restrict__ out) {
-  const int c = threadIdx.x % C;
-  const int lanes = blockDim.x / C;
-  const int sub = threadIdx.x / C;
-  if (sub >= lanes) return;
-  float s = 0.f;
-  for (long long r = (long long)blockIdx.x * lanes + sub; r < rows; r += (long long)gridDim.x * lanes)
-    s += __bfloat162float(G[r * C + c]);
-  atomicAdd(out + c, s);
+  // one addition per warp: one per macroblock to the same word took most of the kernel
+#pragma unroll
+  for (int o = 16; o > 0; o >>= 1) term += __shfl_xor_sync(0xffffffffu, term, o);
+  if ((threadIdx.x & 31) == 0 && term != 0.f) atomicAdd(loss, term);
 }
 
 __global__ void lp_adam_kernel(int n, float* __restrict__ p, const float* __restrict__ g, float* __restrict__ m,
@@ -590,7 +585,6 @@ struct Proposal {
   int *label = nullptr;
   float *norez = nullptr, *weight = nullptr, *loss = nullptr;
   __nv_bfloat16 *g5 = nullptr, *g4 = nullptr, *g3 = nullptr, *g2 = nullptr, *g1 = nullptr, *g0 = nullptr;
-  float *da5 = nullptr, *da4 = nullptr, *da3 = nullptr, *da2 = nullptr, *da1 = nullptr;
   std::vector<void*> allocs;
 
   template <class T>
@@ -629,15 +623,10 @@ struct Proposal {
     const size_t B = (size_t)max_mbs;
     train_ready = alloc(&label, B) && alloc(&norez, B) && alloc(&weight, B) && alloc(&loss, 1) &&
                   alloc(&g5, B * kOut) && alloc(&g4, B * 64) && alloc(&g3, B * 32) && alloc(&g2, B * 128) &&
-                  alloc(&g1, B * 512) && alloc(&g0, B * 2048) && alloc(&da5, B * 64) && alloc(&da4, B * kFIn) &&
-                  alloc(&da3, B * 128) && alloc(&da2, B * 512) && alloc(&da1, B * 2048) &&
+                  alloc(&g1, B * 512) && alloc(&g0, B * 2048) &&
                   cudaMemset(loss, 0, 4) == cudaSuccess;
     return train_ready;
   }
-  const __nv_bfloat16* W(int l) const { return wb + layer_woff(l); }
-  const float* bias(int l) const { return params + layer_boff(l); }
-  float* gW(int l) const { return grads + layer_woff(l); }
-  float* gb(int l) const { return grads + layer_boff(l); }
 };
 
 // SHA-256 (FIPS 180-4) for checkpoint integrity.
@@ -695,76 +684,16 @@ struct Sha256 {
   }
 };
 
-static int splits_for(long long k) {
-  const long long chunks = (k + 63) / 64;
-  long long s = chunks / 16;
-  return (int)(s < 1 ? 1 : (s > 255 ? 255 : s));
-}
-
-#define LP_TRY(x) \
-  do {            \
-    if ((x) != 0) return -1; \
-  } while (0)
-
 static int lp_forward(Proposal* P, int mbs, cudaStream_t st) {
-  const long long B = mbs;
-  const int relu_bf = B200ENC_GEMM_RELU | B200ENC_GEMM_OUT_BF16;
-  void* s = (void*)st;
-  LP_TRY(b200enc_gemm_bf16((int)(B * 64), 32, 8, P->b.x0, 8, 1, P->W(0), 8, 1, (float*)P->b.y1, 32, P->bias(0),
-                           relu_bf, P->err, s));
-  LP_TRY(b200enc_gemm_bf16((int)(B * 16), 32, 128, P->b.y1, 128, 1, P->W(1), 128, 1, (float*)P->b.y2, 32,
-                           P->bias(1), relu_bf, P->err, s));
-  LP_TRY(b200enc_gemm_bf16((int)(B * 4), 32, 128, P->b.y2, 128, 1, P->W(2), 128, 1, (float*)P->b.y3, 32, P->bias(2),
-                           relu_bf, P->err, s));
-  LP_TRY(b200enc_gemm_bf16((int)B, 32, 128, P->b.y3, 128, 1, P->W(3), 128, 1, (float*)P->b.f, kFIn, P->bias(3),
-                           relu_bf, P->err, s));
-  LP_TRY(b200enc_gemm_bf16((int)B, 64, kFIn, P->b.f, kFIn, 1, P->W(4), kFIn, 1, (float*)P->b.h, 64, P->bias(4),
-                           relu_bf, P->err, s));
-  LP_TRY(b200enc_gemm_bf16((int)B, kOut, 64, P->b.h, 64, 1, P->W(5), 64, 1, P->b.logits, kOut, P->bias(5), 0, P->err,
-                           s));
-  return 0;
-}
-
-// Gradient of one layer given its BF16 output gradient G [rows][out]:
-// dW += G^T A (split K over the rows), db += column sums of G, and, when dA
-// is non-null, dA = G W (FP32, [rows][in]).
-static int lp_layer_bwd(Proposal* P, int l, long long rows, const __nv_bfloat16* G, const __nv_bfloat16* A, int lda,
-                        float* dA, cudaStream_t st) {
-  const int in = layer_in(l), out = layer_out(l);
-  void* s = (void*)st;
-  LP_TRY(b200enc_gemm_bf16(out, in, (int)rows, G, 1, out, A, 1, lda, P->gW(l), in, nullptr,
-                           B200ENC_GEMM_SPLITK(splits_for(rows)), P->err, s));
-  const int lanes = 256 / out;
-  long long blocks = (rows + lanes * 64 - 1) / (lanes * 64);
-  if (blocks > 1184) blocks = 1184;
-  if (blocks < 1) blocks = 1;
-  lp_colsum_kernel<<<(int)blocks, lanes * out, 0, st>>>(rows, out, G, P->gb(l));
-  if (dA) LP_TRY(b200enc_gemm_bf16((int)rows, in, out, G, out, 1, P->W(l), 1, in, dA, in, nullptr, 0, P->err, s));
-  return cudaGetLastError() == cudaSuccess ? 0 : -1;
-}
-
-static void relu_bwd(long long rows, int C, const float* dA, int lda, const __nv_bfloat16* Y, int ldy,
-                     __nv_bfloat16* G, cudaStream_t st) {
-  const long long n = rows * C;
-  lp_relu_bwd_kernel<<<(unsigned)((n + 255) / 256), 256, 0, st>>>(rows, C, dA, lda, Y, ldy, G);
+  return lp_forward_layers(P->b, P->wb, P->params, mbs, P->err, st);
 }
 
 static int lp_backward(Proposal* P, int mbs, cudaStream_t st) {
-  const long long B = mbs;
   if (cudaMemsetAsync(P->grads, 0, kParams * 4, st) != cudaSuccess) return -1;
   lp_loss_kernel<<<(mbs + 127) / 128, 128, 0, st>>>(mbs, P->b, P->label, P->norez, P->weight, P->g5, P->loss);
-  LP_TRY(lp_layer_bwd(P, 5, B, P->g5, P->b.h, 64, P->da5, st));
-  relu_bwd(B, 64, P->da5, 64, P->b.h, 64, P->g4, st);
-  LP_TRY(lp_layer_bwd(P, 4, B, P->g4, P->b.f, kFIn, P->da4, st));
-  relu_bwd(B, 32, P->da4, kFIn, P->b.f, kFIn, P->g3, st);
-  LP_TRY(lp_layer_bwd(P, 3, B, P->g3, P->b.y3, 128, P->da3, st));
-  relu_bwd(B * 4, 32, P->da3, 32, P->b.y3, 32, P->g2, st);
-  LP_TRY(lp_layer_bwd(P, 2, B * 4, P->g2, P->b.y2, 128, P->da2, st));
-  relu_bwd(B * 16, 32, P->da2, 32, P->b.y2, 32, P->g1, st);
-  LP_TRY(lp_layer_bwd(P, 1, B * 16, P->g1, P->b.y1, 128, P->da1, st));
-  relu_bwd(B * 64, 32, P->da1, 32, P->b.y1, 32, P->g0, st);
-  LP_TRY(lp_layer_bwd(P, 0, B * 64, P->g0, P->b.x0, 8, nullptr, st));
-  return cudaGetLastError() == cudaSuccess ? 0 : -1;
+  if (cudaGetLastError() != cudaSuccess) return -1;
+  __nv_bfloat16* const g[6] = {P->g0, P->g1, P->g2, P->g3, P->g4, P->g5};
+  return lp_backward_layers(P->b, P->wb, P->grads, g, mbs, P->err, st);
 }
 
 }  // namespace b200enc

@@ -182,4 +182,10 @@ constexpr int kNet8PackBytes = 20480 + 6 * 64 * 4;
 int lp_net8_launch(int mbs, const LpBuf& b, const float* params, uint8_t* w8, bool* stale, float conf, int lambda,
                    MV* mv_out, uint32_t* err, cudaStream_t st);
 
+// lp_train.cu: the network layer by layer, forward and backward
+int lp_forward_layers(const LpBuf& b, const __nv_bfloat16* wb, const float* params, long long B, uint32_t* err,
+                      cudaStream_t st);
+int lp_backward_layers(const LpBuf& b, const __nv_bfloat16* wb, float* grads, __nv_bfloat16* const g[6], long long B,
+                       uint32_t* err, cudaStream_t st);
+
 }  // namespace b200enc

@@ -1,7 +1,7 @@
 // proposal_infer8.cu - the motion-proposal network's inference in FP8 (E4M3)
 // on the tcgen05 tensor cores (kind::f8f6f4, FP32 accumulation), as one
 // persistent kernel with the candidate selection fused into its last
-// epilogue. The network is trained in BF16 (proposal.cu, tc_gemm.cu); this
+// epilogue. The network is trained in BF16 (proposal.cu, lp_train.cu); this
 // is its FP8 inference form, selected by b200enc_proposal_me mode 3.
 //
 // Quantisation (the CPU oracle, oracle/proposal_ref.py forward_fp8, follows

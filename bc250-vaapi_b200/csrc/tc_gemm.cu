@@ -1,16 +1,16 @@
 // tc_gemm.cu - BF16 GEMM on the 5th-generation tensor cores (tcgen05).
 //
-// The one dense contraction in this project is the learned motion-proposal
-// network (convolutions as GEMMs over batches of macroblocks, forward and
-// backward). This kernel computes
+// The general GEMM of the library (the proposal network's own layers have
+// kernels for their shapes and layouts: lp_train.cu, proposal_infer*.cu). This
+// kernel computes
 //     C[m][n] = epilogue( sum_k A(m,k) * B(n,k) )
 // with A and B BF16 read through arbitrary (row, k) strides, so transposed
-// operands of the backward pass need no copies, FP32 accumulation in tensor
+// operands need no copies, FP32 accumulation in tensor
 // memory, and an epilogue of optional FP32 accumulate-into-C, bias and ReLU.
 //
 // Split K (grid z > 1) gives each z slice a range of 64-wide K chunks and
-// adds the slices' FP32 partial products into C with atomics, for the weight
-// gradients of the backward pass, whose reduction runs over every sample.
+// adds the slices' FP32 partial products into C with atomics, for reductions
+// much longer than the output (weight gradients).
 //
 // Per CTA: a 128 x BN output tile, 4 warps. For each 64-wide K chunk the
 // threads stage A (128 x 64) and B (BN x 64) in shared memory in the
