@@ -20,6 +20,7 @@
 // do; the quantiser divides by levelScale through the same reciprocal
 // multiply, which is exact over the reachable range.
 #include <algorithm>
+#include <type_traits>
 
 #include "b200enc_internal.h"
 #include "common.cuh"
@@ -303,9 +304,17 @@ __global__ void __launch_bounds__(256) hevc_hpel_kernel(const P* __restrict__ re
 }
 
 // ---- 8x8 CU motion search -------------------------------------------------
-// One warp per CU job, the reference's walk (hevc_enc_template.c:958-1043)
-// step for step: every lane follows the same (uniform) control flow and the
-// SADs are warp reductions, lane l scoring row l/4, columns 2(l%4), +1.
+// Half a warp per CU job, the reference's walk (hevc_enc_template.c:958-1043).
+// The walk compares its candidates against a fixed centre per step, in order,
+// strictly; so the lowest cost with the lowest candidate number is the same
+// choice, and four candidates are scored at a time: each of the four lanes of a
+// candidate holds two rows of the CU (read once) and scores them with packed
+// arithmetic, a step of the walk being one such pass, and each refinement two.
+// A job is a chain of about ten dependent passes of loads and shuffles, so the
+// kernel is bound by their latency and the instructions issued, not by bytes;
+// with two jobs in a warp each instruction serves both. 32,400 CUs of a 1080p
+// picture at 8 bits: 45 us; one job per warp, a row per lane, 75; one candidate
+// at a time, two samples per lane, 185.
 // Strides in samples. sad_shift brings a SAD back to eight-bit units (0 at
 // eight bits, 2 at ten: hevc_enc_template.c:484).
 template <typename P>
@@ -323,122 +332,205 @@ __device__ __forceinline__ int hevc_mvd_bits(int d) {
   return 3 + 2 * (31 - __clz((int)((a - 2) / 2 + 1))) + 2;
 }
 
-// SAD of the CU against the search planes at absolute quarter-sample
-// position (qx, qy) (search_sad, hevc_enc_template.c:463): positions are
-// clamped to the planes' margin; even/even reads one half-grid block, a
-// position odd in x, y or both averages (rounded) the two blocks beside it.
+// Eight samples from any address: the aligned words that hold them (none other
+// is read), shifted together.
 template <typename P>
-__device__ __forceinline__ uint32_t hevc_search_sad(const HevcSearch<P>& S, int cu_x, int cu_y, int qx, int qy,
-                                                    int lane) {
+struct HevcRow {
+  static constexpr int kWords = 2 * (int)sizeof(P);
+  uint32_t w[kWords];
+  __device__ __forceinline__ void load(const P* p) {
+    const uintptr_t a = reinterpret_cast<uintptr_t>(p);
+    const uint32_t* q = reinterpret_cast<const uint32_t*>(a & ~(uintptr_t)3);
+    const uint32_t off = (uint32_t)a & 3u;
+#pragma unroll
+    for (int i = 0; i < kWords; ++i) w[i] = __ldg(q + i);
+    const uint32_t last = __ldg(q + (off ? kWords : kWords - 1));
+#pragma unroll
+    for (int i = 0; i < kWords; ++i) w[i] = __funnelshift_r(w[i], i + 1 < kWords ? w[i + 1 < kWords ? i + 1 : i] : last, off * 8);
+  }
+  // rounded average of each sample with o's
+  __device__ __forceinline__ void average(const HevcRow& o) {
+    constexpr uint32_t m = sizeof(P) == 1 ? 0x7f7f7f7fu : 0x7fff7fffu;
+#pragma unroll
+    for (int i = 0; i < kWords; ++i) w[i] = (w[i] | o.w[i]) - (((w[i] ^ o.w[i]) >> 1) & m);
+  }
+  __device__ __forceinline__ uint32_t sad(const HevcRow& o) const {
+    uint32_t s = 0;
+#pragma unroll
+    for (int i = 0; i < kWords; ++i) {
+      if (sizeof(P) == 1) {
+        s += __vsadu4(w[i], o.w[i]);
+      } else {
+        s = __dp2a_lo(__vmaxu2(w[i], o.w[i]) - __vminu2(w[i], o.w[i]), 0x0101u, s);
+      }
+    }
+    return s;
+  }
+};
+
+// SAD of the CU (rows `row` and row + 4 in `cu`) against the search planes at
+// absolute quarter-sample position (qx, qy), the same for the four lanes of a
+// candidate (search_sad, hevc_enc_template.c:463): positions are clamped to the
+// planes' margin; even/even reads one half-grid block, a position odd in x, y or
+// both averages (rounded) the two blocks beside it. ODD false: the caller's
+// positions are all even.
+template <typename P, bool ODD>
+__device__ __forceinline__ uint32_t hevc_search_sad(const HevcSearch<P>& S, const HevcRow<P> (&cu)[2], int qx, int qy,
+                                                    int row) {
   const int lo = -(S.M - 2) * 4;
   const int hx = (S.w - 8 + S.M - 2) * 4, hy = (S.h - 8 + S.M - 2) * 4;
   qx = qx < lo ? lo : (qx > hx ? hx : qx);
   qy = qy < lo ? lo : (qy > hy ? hy : qy);
-  const int r = lane >> 2, c = (lane & 3) * 2;
-  auto sample = [&](int bqx, int bqy, int dc) -> int {
+  auto at = [&](int bqx, int bqy) -> const P* {
     const int ph = ((bqx & 2) ? 1 : 0) + ((bqy & 2) ? 2 : 0);
-    const int x = (bqx >> 2) + S.M + c + dc, y = (bqy >> 2) + S.M + r;
-    return S.plane[ph][(size_t)y * S.ppitch + x];
+    return S.plane[ph] + ((size_t)((bqy >> 2) + S.M + row) * S.ppitch + ((bqx >> 2) + S.M));
   };
-  uint32_t sad = 0;
-#pragma unroll
-  for (int dc = 0; dc < 2; ++dc) {
-    int v;
-    if (!(qx & 1) && !(qy & 1)) v = sample(qx, qy, dc);
-    else if ((qx & 1) && (qy & 1)) v = (sample(qx - 1, qy - 1, dc) + sample(qx + 1, qy + 1, dc) + 1) >> 1;
-    else if (qx & 1) v = (sample(qx - 1, qy, dc) + sample(qx + 1, qy, dc) + 1) >> 1;
-    else v = (sample(qx, qy - 1, dc) + sample(qx, qy + 1, dc) + 1) >> 1;
-    const int sv = S.src[(size_t)(cu_y + r) * S.src_pitch + cu_x + c + dc];
-    sad += (uint32_t)abs(sv - v);
+  const size_t down = (size_t)4 * S.ppitch;
+  HevcRow<P> a[2];
+  if (ODD) {
+    const int ox = qx & 1, oy = qy & 1;
+    HevcRow<P> b[2];  // even/even: the block itself twice, whose average it is
+    const P *pa = at(qx - ox, qy - oy), *pb = at(qx + ox, qy + oy);
+    a[0].load(pa);
+    a[1].load(pa + down);
+    b[0].load(pb);
+    b[1].load(pb + down);
+    a[0].average(b[0]);
+    a[1].average(b[1]);
+  } else {
+    const P* pa = at(qx, qy);
+    a[0].load(pa);
+    a[1].load(pa + down);
   }
-  return __reduce_add_sync(0xffffffffu, sad) >> S.sad_shift;
+  uint32_t sad = a[0].sad(cu[0]) + a[1].sad(cu[1]);
+  sad += __shfl_xor_sync(0xffffffffu, sad, 1);
+  sad += __shfl_xor_sync(0xffffffffu, sad, 2);
+  return sad >> S.sad_shift;
 }
 
 template <typename P>
-__global__ void __launch_bounds__(128) hevc_me_kernel(HevcSearch<P> S, const b200enc_hevc_me_job_t* __restrict__ jobs,
-                                                      int n, b200enc_hevc_me_result_t* __restrict__ out) {
-  const int lane = threadIdx.x & 31;
-  const int j = blockIdx.x * 4 + (threadIdx.x >> 5);
-  if (j >= n) return;
-  const b200enc_hevc_me_job_t job = jobs[j];
-  const int cu_x = job.cu_x, cu_y = job.cu_y;
-  if (cu_x < 0 || cu_y < 0 || cu_x > S.w - 8 || cu_y > S.h - 8) {  // not a CU of this picture
-    if (lane == 0) {
-      b200enc_hevc_me_result_t r{};
-      r.sad = 0xffffffffu;
-      r.cost_q8 = -1;
-      out[j] = r;
-    }
-    return;
-  }
+__global__ void __launch_bounds__(128) hevc_me_kernel(const __grid_constant__ HevcSearch<P> S,
+                                                      const b200enc_hevc_me_job_t* __restrict__ jobs, int n,
+                                                      b200enc_hevc_me_result_t* __restrict__ out) {
+  const int lane = threadIdx.x & 31, first = lane & 16, cand = (lane >> 2) & 3, row = lane & 3;
+  const int j = blockIdx.x * 8 + (threadIdx.x >> 4);
+  if (j - (first >> 4) >= n) return;  // neither half has a job
+  const b200enc_hevc_me_job_t& job = jobs[min(j, n - 1)];
+  int cu_x = job.cu_x, cu_y = job.cu_y;
+  const bool bad = cu_x < 0 || cu_y < 0 || cu_x > S.w - 8 || cu_y > S.h - 8;  // not a CU of this picture
+  if (bad) cu_x = cu_y = 0;  // searched with the other half's, then answered as invalid
+  HevcRow<P> cu[2];
+  cu[0].load(S.src + (size_t)(cu_y + row) * S.src_pitch + cu_x);
+  cu[1].load(S.src + (size_t)(cu_y + row + 4) * S.src_pitch + cu_x);
   const int min_dx = -cu_x - 8, max_dx = S.w - cu_x, min_dy = -cu_y - 8, max_dy = S.h - cu_y;
   const int range = 64, qx0 = cu_x * 4, qy0 = cu_y * 4;
-  auto mv_bits = [&](int qx, int qy) -> int {
-    const int b0 = hevc_mvd_bits(qx - job.mvp[0].x) + hevc_mvd_bits(qy - job.mvp[0].y);
-    const int b1 = hevc_mvd_bits(qx - job.mvp[1].x) + hevc_mvd_bits(qy - job.mvp[1].y);
-    return b0 <= b1 ? b0 : b1;
-  };
-  auto cost = [&](int qx, int qy, uint32_t sad) -> long long {
-    return (long long)sad * 256 + (long long)job.lambda_q8 * mv_bits(qx, qy);
-  };
-  int bx = 0, by = 0;
-  long long best = 0x7fffffffffffffffll;
+  const long long lambda = job.lambda_q8;
+  // this lane's share of the vector bits: one component against one predictor
+  const bool is_y = lane & 1;
+  const int pred = is_y ? job.mvp[(lane >> 1) & 1].y : job.mvp[(lane >> 1) & 1].x;
+  constexpr long long kNone = 0x7fffffffffffffffll;
+  long long best = kNone;
   uint32_t best_sad = 0;
-  int seen_x[16], seen_y[16], n_seen = 0;
-  const int ns = job.n_starts < 0 ? 0 : (job.n_starts > 16 ? 16 : job.n_starts);
-  for (int i = 0; i < ns; ++i) {
-    int dx = (job.starts[i].x + 2) >> 2, dy = (job.starts[i].y + 2) >> 2;
-    dx = dx < min_dx ? min_dx : (dx > max_dx ? max_dx : dx);
-    dy = dy < min_dy ? min_dy : (dy > max_dy ? max_dy : dy);
-    bool dup = false;
-    for (int k = 0; k < n_seen && !dup; ++k) dup = seen_x[k] == dx && seen_y[k] == dy;
-    if (dup) continue;
-    seen_x[n_seen] = dx;
-    seen_y[n_seen++] = dy;
-    const uint32_t sd = hevc_search_sad(S, cu_x, cu_y, qx0 + dx * 4, qy0 + dy * 4, lane);
-    const long long c = cost(dx * 4, dy * 4, sd);
-    if (c < best) { best = c; best_sad = sd; bx = dx; by = dy; }
+
+  // Scores four candidates per half, this lane's at (qx, qy) relative to its CU;
+  // returns the number of the one that beats the half's `best` (updated), or -1.
+  // Costs are far under 2^60, so the candidate number fits below them.
+  auto pass = [&](auto odd, int qx, int qy, bool valid) -> int {
+    const uint32_t sd = hevc_search_sad<P, decltype(odd)::value>(S, cu, qx0 + qx, qy0 + qy, row);
+    int bits = hevc_mvd_bits((is_y ? qy : qx) - pred);
+    bits += __shfl_xor_sync(0xffffffffu, bits, 1);
+    bits = min(bits, __shfl_xor_sync(0xffffffffu, bits, 2));
+    const long long c = (long long)sd * 256 + lambda * bits;
+    long long key = valid && c < best ? c * 4 + cand : kNone;
+#pragma unroll
+    for (int o = 4; o < 16; o <<= 1) {
+      const long long k = __shfl_xor_sync(0xffffffffu, key, o);
+      key = k < key ? k : key;
+    }
+    const int k = (int)(key & 3);
+    const uint32_t ks = __shfl_sync(0xffffffffu, sd, first + k * 4);
+    if (key == kNone) return -1;
+    best = key >> 2;
+    best_sad = ks;
+    return k;
+  };
+  using Even = std::false_type;
+  using Odd = std::true_type;
+
+  // start points, each distinct one once (a repeat cannot beat its first)
+  int bx = 0, by = 0;
+  {
+    const int i = lane & 15, ns = min(max(job.n_starts, 0), 16);
+    int dx = 0, dy = 0;
+    if (i < ns) {  // within +-8192: the limits lie on both sides of 0
+      dx = min(max((job.starts[i].x + 2) >> 2, min_dx), max_dx);
+      dy = min(max((job.starts[i].y + 2) >> 2, min_dy), max_dy);
+    }
+    const uint32_t key = i < ns ? (uint32_t)(dy + 8192) << 15 | (uint32_t)(dx + 8192) : 1u << 30 | i;
+    const uint32_t same = __match_any_sync(0xffffffffu, key | (uint32_t)first << 27);
+    uint32_t todo = __ballot_sync(0xffffffffu, i < ns && (same & ((1u << lane) - 1u)) == 0u) >> first & 0xffffu;
+    while (__any_sync(0xffffffffu, todo != 0)) {
+      uint32_t t = todo;  // this candidate's start: the cand-th of those left, or the last
+#pragma unroll
+      for (int q = 0; q < 3; ++q)
+        if (q < cand && (t & (t - 1))) t &= t - 1;
+      const int from = first + (t ? __ffs(t) - 1 : 0);
+      const int gx = __shfl_sync(0xffffffffu, dx, from), gy = __shfl_sync(0xffffffffu, dy, from);
+      const int k = pass(Even{}, gx * 4, gy * 4, cand < __popc(todo));
+      const int kx = __shfl_sync(0xffffffffu, gx, first + (k & 3) * 4), ky = __shfl_sync(0xffffffffu, gy, first + (k & 3) * 4);
+      if (k >= 0) bx = kx, by = ky;
+#pragma unroll
+      for (int q = 0; q < 4; ++q) todo &= todo - 1;
+    }
   }
   const int cx0 = bx, cy0 = by;
+  const int ddx = cand == 0 ? -1 : (cand == 1 ? 1 : 0), ddy = cand == 2 ? -1 : (cand == 3 ? 1 : 0);
   int back = -1;
-  for (int step = 0; step < 32; ++step) {
-    const int ddx[4] = {-1, 1, 0, 0}, ddy[4] = {0, 0, -1, 1};
-    int nbx = bx, nby = by, nk = -1;
-    for (int k = 0; k < 4; ++k) {
-      if (k == back) continue;
-      const int dx = bx + ddx[k], dy = by + ddy[k];
-      if (dx < min_dx || dx > max_dx || dy < min_dy || dy > max_dy) continue;
-      if (dx < cx0 - range || dx > cx0 + range || dy < cy0 - range || dy > cy0 + range) continue;
-      const uint32_t sd = hevc_search_sad(S, cu_x, cu_y, qx0 + dx * 4, qy0 + dy * 4, lane);
-      const long long c = cost(dx * 4, dy * 4, sd);
-      if (c < best) { best = c; best_sad = sd; nbx = dx; nby = dy; nk = k; }
+  bool walking = true;
+  for (int step = 0; step < 32 && __any_sync(0xffffffffu, walking); ++step) {
+    const int dx = bx + ddx, dy = by + ddy;
+    const bool valid = walking && cand != back && dx >= min_dx && dx <= max_dx && dy >= min_dy && dy <= max_dy &&
+                       dx >= cx0 - range && dx <= cx0 + range && dy >= cy0 - range && dy <= cy0 + range;
+    const int k = pass(Even{}, dx * 4, dy * 4, valid);
+    walking = k >= 0;
+    if (walking) {
+      bx += k == 0 ? -1 : (k == 1 ? 1 : 0);
+      by += k == 2 ? -1 : (k == 3 ? 1 : 0);
+      back = k ^ 1;
     }
-    if (nbx == bx && nby == by) break;
-    bx = nbx;
-    by = nby;
-    back = nk ^ 1;
   }
   int mx = bx * 4, my = by * 4;
-  for (int st = 2; st >= (S.qpel ? 1 : 2); st >>= 1) {
-    const int ox[8] = {-1, 0, 1, -1, 1, -1, 0, 1}, oy[8] = {-1, -1, -1, 0, 0, 1, 1, 1};
+  // the eight neighbours in raster order, four above and left, four right and below
+  auto refine = [&](auto odd, int st) {
     const int c0x = mx, c0y = my;
-    for (int k = 0; k < 8; ++k) {
-      const int tx = c0x + ox[k] * st, ty = c0y + oy[k] * st;
-      const uint32_t sd = hevc_search_sad(S, cu_x, cu_y, qx0 + tx, qy0 + ty, lane);
-      const long long c = cost(tx, ty, sd);
-      if (c < best) { best = c; best_sad = sd; mx = tx; my = ty; }
+#pragma unroll
+    for (int half = 0; half < 2; ++half) {
+      auto off_x = [&](int k) { return half == 0 ? (k == 3 ? -1 : k - 1) : (k == 0 ? 1 : k - 2); };
+      auto off_y = [&](int k) { return half == 0 ? (k == 3 ? 0 : -1) : (k == 0 ? 0 : 1); };
+      const int k = pass(odd, c0x + off_x(cand) * st, c0y + off_y(cand) * st, true);
+      if (k >= 0) {
+        mx = c0x + off_x(k) * st;
+        my = c0y + off_y(k) * st;
+      }
     }
-  }
-  if (lane == 0) {
-    const int b0 = hevc_mvd_bits(mx - job.mvp[0].x) + hevc_mvd_bits(my - job.mvp[0].y);
-    const int b1 = hevc_mvd_bits(mx - job.mvp[1].x) + hevc_mvd_bits(my - job.mvp[1].y);
-    b200enc_hevc_me_result_t r;
-    r.mv.x = (int16_t)mx;
-    r.mv.y = (int16_t)my;
-    r.mvp_idx = b1 < b0 ? 1 : 0;
-    r.cost_q8 = best;
-    r.sad = best_sad;
-    r.pad = 0;
+  };
+  refine(Even{}, 2);
+  if (S.qpel) refine(Odd{}, 1);
+  int bits = hevc_mvd_bits((is_y ? my : mx) - pred);
+  bits += __shfl_xor_sync(0xffffffffu, bits, 1);
+  const int b1 = __shfl_sync(0xffffffffu, bits, first + 2);
+  if (lane == first && j < n) {
+    b200enc_hevc_me_result_t r{};
+    if (bad) {
+      r.sad = 0xffffffffu;
+      r.cost_q8 = -1;
+    } else {
+      r.mv.x = (int16_t)mx;
+      r.mv.y = (int16_t)my;
+      r.mvp_idx = b1 < bits ? 1 : 0;
+      r.cost_q8 = best;
+      r.sad = best_sad;
+    }
     out[j] = r;
   }
 }
@@ -682,7 +774,7 @@ int b200enc_hevc_motion_search(const uint8_t* src_y, int src_pitch, int w, int h
   if (n == 0) return 0;
   HevcSearch<uint8_t> S{src_y, src_pitch, w, h, margin, qpel ? 1 : 0, {plane_i, plane_h, plane_v, plane_hv},
                         plane_pitch, 0};
-  hevc_me_kernel<uint8_t><<<(n + 3) / 4, 128, 0, (cudaStream_t)stream>>>(S, jobs, n, results);
+  hevc_me_kernel<uint8_t><<<(unsigned)(n / 8 + 1), 128, 0, (cudaStream_t)stream>>>(S, jobs, n, results);
   return cudaGetLastError() == cudaSuccess ? 0 : -1;
 }
 
@@ -695,7 +787,7 @@ int b200enc_hevc_motion_search_10(const uint16_t* src_y, int src_pitch, int w, i
   if (n == 0) return 0;
   HevcSearch<uint16_t> S{src_y, src_pitch, w, h, margin, qpel ? 1 : 0, {plane_i, plane_h, plane_v, plane_hv},
                          plane_pitch, 2};
-  hevc_me_kernel<uint16_t><<<(n + 3) / 4, 128, 0, (cudaStream_t)stream>>>(S, jobs, n, results);
+  hevc_me_kernel<uint16_t><<<(unsigned)(n / 8 + 1), 128, 0, (cudaStream_t)stream>>>(S, jobs, n, results);
   return cudaGetLastError() == cudaSuccess ? 0 : -1;
 }
 
