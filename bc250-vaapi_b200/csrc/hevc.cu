@@ -255,52 +255,170 @@ __global__ void __launch_bounds__(128) hevc_dqit8_kernel(const int16_t* __restri
 }
 
 // ---- half-sample planes ----------------------------------------------------
-// Output tile of 32 columns x 8 rows per 256-thread block. Plane coordinates
-// (r, c) are picture coordinates + margin; every reference read is clamped to
-// the picture (the reference's edge extension). With Y(k) = clampY(r - M - 3 + k)
-// and X(k) = clampX(c - M - 3 + k):
+// Plane coordinates (r, c) are picture coordinates + margin; every reference
+// read is clamped to the picture (the reference's edge extension). With
+// Y(k) = clampY(r - M - 3 + k) and X(k) = clampX(c - M - 3 + k):
 //   I  = ref[clampY(r - M)][clampX(c - M)]
 //   H  = clip((sum_k tap[k] * ref[clampY(r - M)][X(k)] + 32) >> 6)
 //   V  = clip((sum_k tap[k] * ref[Y(k)][clampX(c - M)] + 32) >> 6)
 //   HV = clip((sum_k tap[k] * T(Y(k)) + 2048) >> 12),  T(y) = sum_j tap[j] * ref[y][X(j)]
-constexpr int kHpTileW = 32, kHpTileH = 8;
+// A block makes a tile of 128 columns x 32 rows, a thread 4 columns x 8 rows of
+// it: the clamped samples are staged once, four at a time, in shared memory, and
+// each thread walks 15 of its rows with the last eight rows' column samples and
+// horizontal sums in registers. Horizontal sums are integer dot products (dp4a,
+// dp2a), vertical ones of 8-bit samples two columns to a register (a column's sum
+// is under 16 bits). Bound by instructions issued until the planes' four writes
+// per sample are what is left: 1080p at 8 bits 8.6 us, a thread per sample with
+// the sums staged in shared memory 17.5 (10.6 MB moved, 1.6 us).
+constexpr int kHpTileW = 128, kHpTileH = 32, kHpRows = 8;
 
-// P: the sample type (uint8_t at 8 bits, uint16_t at 10); maxv the largest
-// sample value, (1 << BitDepth) - 1 (hevc_enc_template.c:23-25).
+__device__ __forceinline__ int dot4(uint32_t samples, uint32_t taps, int acc) {
+  int d;
+  asm("dp4a.u32.s32 %0, %1, %2, %3;" : "=r"(d) : "r"(samples), "r"(taps), "r"(acc));
+  return d;
+}
+__device__ __forceinline__ int dot2(uint32_t samples, uint32_t taps, int acc) {
+  int d;
+  asm("dp2a.lo.u32.s32 %0, %1, %2, %3;" : "=r"(d) : "r"(samples), "r"(taps), "r"(acc));
+  return d;
+}
+template <class T>
+__device__ __forceinline__ T filter8(T a0, T a1, T a2, T a3, T a4, T a5, T a6, T a7) {
+  return (a3 + a4) * 40 - (a2 + a5) * 11 + (a1 + a6) * 4 - (a0 + a7);
+}
+
+// Four samples; P: the sample type (uint8_t at 8 bits, uint16_t at 10).
 template <typename P>
-__global__ void __launch_bounds__(256) hevc_hpel_kernel(const P* __restrict__ ref, int pitch, int w, int h, int M,
+struct Quad;
+template <>
+struct Quad<uint8_t> {
+  uint32_t w;
+  __device__ __forceinline__ void load(const uint8_t* p) {  // any alignment; only words holding the samples are read
+    const uintptr_t a = reinterpret_cast<uintptr_t>(p);
+    const uint32_t* q = reinterpret_cast<const uint32_t*>(a & ~(uintptr_t)3);
+    const uint32_t off = (uint32_t)a & 3u;
+    w = __funnelshift_r(__ldg(q), __ldg(q + (off ? 1 : 0)), off * 8);
+  }
+  __device__ __forceinline__ void set(int a, int b, int c, int d) { w = a | b << 8 | c << 16 | d << 24; }
+  __device__ __forceinline__ void store(uint8_t* p) const { *reinterpret_cast<uint32_t*>(p) = w; }
+  __device__ __forceinline__ uint8_t at(int i) const { return (uint8_t)(w >> (8 * i)); }
+  // horizontal sums of this quad's samples, given the quads on either side
+  __device__ __forceinline__ void sums(const Quad& l, const Quad& r, int (&t)[4]) const {
+    constexpr uint32_t ta = 0x28f504ffu, tb = 0xff04f528u;  // -1 4 -11 40, 40 -11 4 -1
+#pragma unroll
+    for (int j = 0; j < 4; ++j)
+      t[j] = dot4(j == 3 ? w : __funnelshift_r(l.w, w, 8 * (j + 1)), ta,
+                  dot4(j == 3 ? r.w : __funnelshift_r(w, r.w, 8 * (j + 1)), tb, 0));
+  }
+};
+template <>
+struct Quad<uint16_t> {
+  uint2 w;
+  __device__ __forceinline__ void load(const uint16_t* p) {
+    const uintptr_t a = reinterpret_cast<uintptr_t>(p);
+    const uint32_t* q = reinterpret_cast<const uint32_t*>(a & ~(uintptr_t)3);
+    const uint32_t off = (uint32_t)a & 3u, mid = __ldg(q + 1);
+    w.x = __funnelshift_r(__ldg(q), mid, off * 8);
+    w.y = __funnelshift_r(mid, __ldg(q + (off ? 2 : 1)), off * 8);
+  }
+  __device__ __forceinline__ void set(int a, int b, int c, int d) { w = make_uint2(a | b << 16, c | d << 16); }
+  __device__ __forceinline__ void store(uint16_t* p) const { *reinterpret_cast<uint2*>(p) = w; }
+  __device__ __forceinline__ uint16_t at(int i) const { return (uint16_t)((i < 2 ? w.x : w.y) >> (16 * (i & 1))); }
+  __device__ __forceinline__ void sums(const Quad& l, const Quad& r, int (&t)[4]) const {
+    const uint32_t e[6] = {l.w.x, l.w.y, w.x, w.y, r.w.x, r.w.y};  // pairs from even samples on
+    constexpr uint32_t tap[4] = {0x04ffu, 0x28f5u, 0xf528u, 0xff04u};
+#pragma unroll
+    for (int j = 0; j < 4; ++j) {
+      t[j] = 0;
+#pragma unroll
+      for (int k = 0; k < 4; ++k) {  // samples j + 1 + 2k of the twelve, and the next
+        const int i = (j + 1) / 2 + k;
+        t[j] = dot2((j & 1) ? e[i] : __funnelshift_r(e[i], e[i + 1 < 6 ? i + 1 : i], 16), tap[k], t[j]);
+      }
+    }
+  }
+};
+
+// maxv: the largest sample value, (1 << BitDepth) - 1 (hevc_enc_template.c:23-25);
+// vec: planes and their pitch aligned for four-sample stores.
+template <typename P>
+__global__ void __launch_bounds__(128) hevc_hpel_kernel(const P* __restrict__ ref, int pitch, int w, int h, int M,
                                                         P* __restrict__ pI, P* __restrict__ pH, P* __restrict__ pV,
-                                                        P* __restrict__ pHV, int opitch, int rows, int cols,
-                                                        int maxv) {
-  __shared__ P src[kHpTileH + 7][kHpTileW + 8];
-  __shared__ int32_t tsum[kHpTileH + 7][kHpTileW];
+                                                        P* __restrict__ pHV, int opitch, int rows, int cols, int maxv,
+                                                        int vec) {
+  constexpr int kQuads = kHpTileW / 4 + 2;
+  __shared__ Quad<P> src[kHpTileH + 7][kQuads];
   const int tx = threadIdx.x & 31, ty = threadIdx.x >> 5;
   const int c0 = blockIdx.x * kHpTileW, r0 = blockIdx.y * kHpTileH;
-  // source rows r0-M-3 .. r0-M+kHpTileH+3, columns c0-M-3 .. c0-M+kHpTileW+4
-  for (int i = threadIdx.x; i < (kHpTileH + 7) * (kHpTileW + 8); i += 256) {
-    const int sr = i / (kHpTileW + 8), sc = i - sr * (kHpTileW + 8);
-    const int y = clampi(r0 - M - 3 + sr, 0, h - 1), x = clampi(c0 - M - 3 + sc, 0, w - 1);
-    src[sr][sc] = ref[(size_t)y * pitch + x];
+  // source rows r0-M-3 .. r0-M+kHpTileH+3, columns c0-M-4 .. c0-M+kHpTileW+3
+  for (int i = threadIdx.x; i < (kHpTileH + 7) * kQuads; i += 128) {
+    const int sr = i / kQuads, sc = i - sr * kQuads;
+    const P* row = ref + (size_t)clampi(r0 - M - 3 + sr, 0, h - 1) * pitch;
+    const int x = c0 - M - 4 + 4 * sc;
+    Quad<P> q;
+    if (x >= 0 && x + 3 < w)
+      q.load(row + x);
+    else
+      q.set(row[clampi(x, 0, w - 1)], row[clampi(x + 1, 0, w - 1)], row[clampi(x + 2, 0, w - 1)],
+            row[clampi(x + 3, 0, w - 1)]);
+    src[sr][sc] = q;
   }
   __syncthreads();
-  for (int i = threadIdx.x; i < (kHpTileH + 7) * kHpTileW; i += 256) {
-    const int sr = i / kHpTileW, sc = i - sr * kHpTileW;
-    const P* p = &src[sr][sc];
-    tsum[sr][sc] = -p[0] + 4 * p[1] - 11 * p[2] + 40 * p[3] + 40 * p[4] - 11 * p[5] + 4 * p[6] - p[7];
+  const int c = c0 + 4 * tx, r1 = r0 + ty * kHpRows;
+  if (c >= cols || r1 >= rows) return;
+  const bool whole = vec && c + 3 < cols;
+  auto put = [&](P* plane, int r, const Quad<P>& q) {
+    P* p = plane + (size_t)r * opitch + c;
+    if (whole) {
+      q.store(p);
+    } else {
+#pragma unroll
+      for (int j = 0; j < 4; ++j)
+        if (c + j < cols) p[j] = q.at(j);
+    }
+  };
+  auto clip = [&](const int (&v)[4], int round, int shift) {
+    Quad<P> q;
+    q.set(clampi((v[0] + round) >> shift, 0, maxv), clampi((v[1] + round) >> shift, 0, maxv),
+          clampi((v[2] + round) >> shift, 0, maxv), clampi((v[3] + round) >> shift, 0, maxv));
+    return q;
+  };
+  int t[kHpRows][4];     // horizontal sums of the last eight rows
+  Quad<P> s[kHpRows];    // and their samples
+#pragma unroll
+  for (int k = 0; k < kHpRows + 7; ++k) {
+    const Quad<P>* q = &src[ty * kHpRows + k][tx];
+    s[k % 8] = q[1];
+    q[1].sums(q[0], q[2], t[k % 8]);
+    if (k < 7) continue;
+    const int r = r1 + k - 7;  // rows k - 7 .. k around it; its own is k - 4
+    if (r >= rows) return;
+    put(pI, r, s[(k - 4) % 8]);
+    put(pH, r, clip(t[(k - 4) % 8], 32, 6));
+    int v[4];
+    if constexpr (sizeof(P) == 1) {
+#pragma unroll
+      for (int p = 0; p < 2; ++p) {  // columns 2p and 2p + 1
+        uint32_t a[8];
+#pragma unroll
+        for (int i = 0; i < 8; ++i) a[i] = __byte_perm(s[(k - 7 + i) % 8].w, 0, p ? 0x4342 : 0x4140);
+        const uint32_t f = filter8(a[0], a[1], a[2], a[3], a[4], a[5], a[6], a[7]);
+        v[2 * p] = (int16_t)f;
+        v[2 * p + 1] = (int)(f + 0x8000u) >> 16;
+      }
+    } else {
+#pragma unroll
+      for (int j = 0; j < 4; ++j)
+        v[j] = filter8<int>(s[(k - 7) % 8].at(j), s[(k - 6) % 8].at(j), s[(k - 5) % 8].at(j), s[(k - 4) % 8].at(j),
+                            s[(k - 3) % 8].at(j), s[(k - 2) % 8].at(j), s[(k - 1) % 8].at(j), s[k % 8].at(j));
+    }
+    put(pV, r, clip(v, 32, 6));
+#pragma unroll
+    for (int j = 0; j < 4; ++j)
+      v[j] = filter8(t[(k - 7) % 8][j], t[(k - 6) % 8][j], t[(k - 5) % 8][j], t[(k - 4) % 8][j], t[(k - 3) % 8][j],
+                     t[(k - 2) % 8][j], t[(k - 1) % 8][j], t[k % 8][j]);
+    put(pHV, r, clip(v, 2048, 12));
   }
-  __syncthreads();
-  const int r = r0 + ty, c = c0 + tx;
-  if (r >= rows || c >= cols) return;
-  const int sr = ty + 3, sc = tx + 3;  // the sample (r - M, c - M) in the staged tile
-  const size_t o = (size_t)r * opitch + c;
-  pI[o] = src[sr][sc];
-  pH[o] = (P)clampi((tsum[sr][tx] + 32) >> 6, 0, maxv);
-  const int v = -src[ty][sc] + 4 * src[ty + 1][sc] - 11 * src[ty + 2][sc] + 40 * src[ty + 3][sc] +
-                40 * src[ty + 4][sc] - 11 * src[ty + 5][sc] + 4 * src[ty + 6][sc] - src[ty + 7][sc];
-  pV[o] = (P)clampi((v + 32) >> 6, 0, maxv);
-  const int hv = -tsum[ty][tx] + 4 * tsum[ty + 1][tx] - 11 * tsum[ty + 2][tx] + 40 * tsum[ty + 3][tx] +
-                 40 * tsum[ty + 4][tx] - 11 * tsum[ty + 5][tx] + 4 * tsum[ty + 6][tx] - tsum[ty + 7][tx];
-  pHV[o] = (P)clampi((hv + 2048) >> 12, 0, maxv);
 }
 
 // ---- 8x8 CU motion search -------------------------------------------------
@@ -687,6 +805,14 @@ __global__ void hevc_intra4_kernel(const P* __restrict__ src, int src_pitch, con
 bool aligned16(const void* p) { return (((uintptr_t)p) & 15) == 0; }
 int hclamp(int v, int lo, int hi) { return v < lo ? lo : (v > hi ? hi : v); }
 
+// Whether four samples of every plane row can be stored at once.
+template <typename P>
+static int quad_aligned(const P* a, const P* b, const P* c, const P* d, int pitch) {
+  const uintptr_t all = reinterpret_cast<uintptr_t>(a) | reinterpret_cast<uintptr_t>(b) |
+                        reinterpret_cast<uintptr_t>(c) | reinterpret_cast<uintptr_t>(d) | (uintptr_t)pitch * sizeof(P);
+  return all % (4 * sizeof(P)) == 0;
+}
+
 }  // namespace b200enc
 
 using namespace b200enc;
@@ -746,8 +872,9 @@ int b200enc_hevc_build_hpel(const uint8_t* recon, int pitch, int w, int h, int m
   const int rows = h + 2 * margin, cols = w + 2 * margin;
   if (plane_pitch < cols) return -1;
   dim3 grid((cols + kHpTileW - 1) / kHpTileW, (rows + kHpTileH - 1) / kHpTileH);
-  hevc_hpel_kernel<uint8_t><<<grid, 256, 0, (cudaStream_t)stream>>>(recon, pitch, w, h, margin, plane_i, plane_h,
-                                                                    plane_v, plane_hv, plane_pitch, rows, cols, 255);
+  hevc_hpel_kernel<uint8_t><<<grid, 128, 0, (cudaStream_t)stream>>>(
+      recon, pitch, w, h, margin, plane_i, plane_h, plane_v, plane_hv, plane_pitch, rows, cols, 255,
+      quad_aligned(plane_i, plane_h, plane_v, plane_hv, plane_pitch));
   return cudaGetLastError() == cudaSuccess ? 0 : -1;
 }
 
@@ -759,9 +886,9 @@ int b200enc_hevc_build_hpel_10(const uint16_t* recon, int pitch, int w, int h, i
   const int rows = h + 2 * margin, cols = w + 2 * margin;
   if (plane_pitch < cols) return -1;
   dim3 grid((cols + kHpTileW - 1) / kHpTileW, (rows + kHpTileH - 1) / kHpTileH);
-  hevc_hpel_kernel<uint16_t><<<grid, 256, 0, (cudaStream_t)stream>>>(recon, pitch, w, h, margin, plane_i, plane_h,
-                                                                     plane_v, plane_hv, plane_pitch, rows, cols,
-                                                                     1023);
+  hevc_hpel_kernel<uint16_t><<<grid, 128, 0, (cudaStream_t)stream>>>(
+      recon, pitch, w, h, margin, plane_i, plane_h, plane_v, plane_hv, plane_pitch, rows, cols, 1023,
+      quad_aligned(plane_i, plane_h, plane_v, plane_hv, plane_pitch));
   return cudaGetLastError() == cudaSuccess ? 0 : -1;
 }
 
