@@ -94,10 +94,10 @@ __device__ __forceinline__ int quant_ac(int c, int pos, const QP& q) {
   const int l = (a * qp_mf(q, pos_type(pos)) + q.f) >> q.f_shift;
   return c < 0 ? -l : l;
 }
+// (level * 16 V << per) >> 4, rounded (reconstruct.comp): the sixteen makes the
+// division exact and the rounding empty for every per.
 __device__ __forceinline__ int dequant_ac(int level, int pos, const QP& q) {
-  const int scale = 16 * qp_v(q, pos_type(pos));
-  if (q.per >= 4) return (level * scale) << (q.per - 4);
-  return (level * scale + (1 << (3 - q.per))) >> (4 - q.per);
+  return (level * qp_v(q, pos_type(pos))) << q.per;
 }
 
 __device__ __forceinline__ int quantize_dc(int v, const QP& q) {
