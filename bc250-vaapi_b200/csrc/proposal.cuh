@@ -50,14 +50,17 @@ __device__ __forceinline__ int cand_y(int32_t p) { return p >> 16; }
 
 __device__ __forceinline__ void masked_softmax(const float* z, uint32_t dup, float* p) {
   float mx = -INFINITY;
+#pragma unroll
   for (int j = 0; j < kClasses; ++j)
     if (!((dup >> j) & 1u)) mx = fmaxf(mx, z[j]);
   float s = 0.f;
+#pragma unroll
   for (int j = 0; j < kClasses; ++j) {
     p[j] = ((dup >> j) & 1u) ? 0.f : expf(z[j] - mx);
     s += p[j];
   }
   const float inv = 1.f / s;
+#pragma unroll
   for (int j = 0; j < kClasses; ++j) p[j] *= inv;
 }
 
@@ -138,13 +141,16 @@ __device__ __forceinline__ void lp_select_warp(int mb0, int nmb, int mbs, const 
       b.p_norez[mb] = 1.f / (1.f + expf(-logits[11]));
       uint32_t chosen = dup;
       float conf = 0.f;
-      for (int k = 0; k < 4; ++k) {
+#pragma unroll
+      for (int k = 0; k < 4; ++k) {  // unrolled: p stays in registers
         int best = -1;
+        float pb = 0.f;
+#pragma unroll
         for (int c = 0; c < kCand; ++c)
-          if (!((chosen >> c) & 1u) && (best < 0 || p[c] > p[best])) best = c;
+          if (!((chosen >> c) & 1u) && (best < 0 || p[c] > pb)) best = c, pb = p[c];
         if (best < 0) break;
         chosen |= 1u << best;
-        conf += p[best];
+        conf += pb;
         sel = (sel & ~(0xffu << (8 * k))) | ((uint32_t)best << (8 * k));
       }
       fall = conf < param;
