@@ -45,13 +45,6 @@ namespace b200enc {
 // Preparation: candidates, their SADs, the network input and side features.
 // 64 threads (two warps) per MB.
 // ---------------------------------------------------------------------------
-// Word i (0..7) of an 8-word register window, by selects (no local memory).
-__device__ __forceinline__ uint32_t pick8(const uint32_t (&w)[8], int i) {
-  const uint32_t lo = (i & 2) ? ((i & 1) ? w[3] : w[2]) : ((i & 1) ? w[1] : w[0]);
-  const uint32_t hi = (i & 2) ? ((i & 1) ? w[7] : w[6]) : ((i & 1) ? w[5] : w[4]);
-  return (i & 4) ? hi : lo;
-}
-
 // BATCH: one CTA per compact P macroblock of a batch (the buffers of b are
 // indexed by that compact index); geometry, planes, history and the early-out
 // threshold come from the macroblock's stream.
@@ -129,67 +122,76 @@ __global__ void __launch_bounds__(64) lp_prepare_kernel(const uint8_t* __restric
   }
   __syncthreads();
 
-  // exact SAD at each candidate: one warp per candidate, two lanes per
-  // reference row (lane pair h = 0, 1 scores the row's bytes 8h .. 8h+7),
-  // summed over the warp by shuffles. Where the plane's base and pitch are
-  // 16-byte aligned and the row's 32-byte aligned window lies inside the
-  // picture, each lane loads one 16-byte half of the window and the pair
-  // swaps halves: one load instruction covers 16 rows, where five word loads
-  // per row touched ~5x the L1 wavefronts. Other rows take clamped word
-  // loads (the same bytes).
+  // exact SAD at each candidate: five candidates per warp, two lanes per
+  // reference row (lane h = 0, 1 scores the row's bytes 8h .. 8h+7), summed over
+  // the warp. L1 lookups bound it (sixteen rows are sixteen lines an instruction),
+  // so where the plane's base and pitch are 16-byte aligned and the five blocks'
+  // aligned windows lie inside the picture's columns, one 16-byte load per lane
+  // covers the row, the pair swaps the two words each may need, and all five
+  // loads are issued before any is used; otherwise clamped word loads (the same
+  // bytes), a candidate at a time.
   {
-    const bool vec = ((ref_pitch & 15) == 0) && ((reinterpret_cast<uintptr_t>(ref) & 15) == 0);
     const int r = lane >> 1, h = lane & 1;
-    for (int c = warp; c < kCand; c += 2) {
-      const int x0 = X + scx[c];
-      const uint8_t* rp = ref + (size_t)clampi(Y + r + scy[c], 0, g.RH - 1) * ref_pitch;
-      const int x16 = x0 & ~15;
-      uint32_t w0, w1, w2;  // the words at (x0 & ~3) + 8h + 0, 4, 8
-      int shft;
-      if (vec && x16 >= 0 && x16 + 32 <= g.RW) {  // warp-uniform
-        const uint4 v = __ldg(reinterpret_cast<const uint4*>(rp + x16 + 16 * h));
-        const uint32_t o0 = __shfl_xor_sync(0xffffffffu, v.x, 1), o1 = __shfl_xor_sync(0xffffffffu, v.y, 1);
-        const uint32_t o2 = __shfl_xor_sync(0xffffffffu, v.z, 1), o3 = __shfl_xor_sync(0xffffffffu, v.w, 1);
-        const uint32_t win[8] = {h ? o0 : v.x, h ? o1 : v.y, h ? o2 : v.z, h ? o3 : v.w,
-                                 h ? v.x : o0, h ? v.y : o1, h ? v.z : o2, h ? v.w : o3};
-        const int q = ((x0 - x16) >> 2) + 2 * h;  // 0..5
-        w0 = pick8(win, q);
-        w1 = pick8(win, q + 1);
-        w2 = pick8(win, q + 2);
-        shft = (x0 & 3) * 8;
-      } else {
-        const int xa = x0 & ~3;
-        w0 = load_word_clamped(rp, xa + 8 * h, g.RW);
-        w1 = load_word_clamped(rp, xa + 8 * h + 4, g.RW);
-        w2 = load_word_clamped(rp, xa + 8 * h + 8, g.RW);
-        shft = (x0 - xa) * 8;
-      }
-      const uint32_t rv0 = __funnelshift_r(w0, w1, shft), rv1 = __funnelshift_r(w1, w2, shft);
-      uint32_t sad = sad4_acc(rv0, scw[r * 4 + 2 * h], 0u);
-      sad = sad4_acc(rv1, scw[r * 4 + 2 * h + 1], sad);
+    const uint32_t c0 = scw[r * 4 + 2 * h], c1 = scw[r * 4 + 2 * h + 1];
+    auto score = [&](int c, uint32_t rv0, uint32_t rv1) {
       if (c == 0) {
         rfw[r * 4 + 2 * h] = rv0;
         rfw[r * 4 + 2 * h + 1] = rv1;
       }
-#pragma unroll
-      for (int o = 16; o > 0; o >>= 1) sad += __shfl_xor_sync(0xffffffffu, sad, o);
+      const uint32_t sad = __reduce_add_sync(0xffffffffu, sad4_acc(rv1, c1, sad4_acc(rv0, c0, 0u)));
       if (lane == 0) ssad[c] = sad;
+    };
+    bool in = ((ref_pitch & 15) == 0) && ((reinterpret_cast<uintptr_t>(ref) & 15) == 0);
+#pragma unroll
+    for (int i = 0; i < 5; ++i) {
+      const int x0 = X + scx[warp + 2 * i];
+      in = in && x0 >= 0 && ((x0 + 31) & ~15) <= g.RW;
+    }
+    if (in) {  // warp-uniform
+      uint4 v[5];
+#pragma unroll
+      for (int i = 0; i < 5; ++i) {
+        const int x0 = X + scx[warp + 2 * i];  // an aligned block is in the first sixteen bytes
+        const uint8_t* rp = ref + (size_t)clampi(Y + r + scy[warp + 2 * i], 0, g.RH - 1) * ref_pitch + (x0 & ~15);
+        v[i] = __ldg(reinterpret_cast<const uint4*>(rp + ((x0 & 15) ? 16 * h : 0)));
+      }
+#pragma unroll
+      for (int i = 0; i < 5; ++i) {
+        const int x0 = X + scx[warp + 2 * i];
+        // words 2h .. 2h + 5 of the window, then the block's from there
+        const uint32_t o0 = __shfl_xor_sync(0xffffffffu, h ? v[i].x : v[i].z, 1);
+        const uint32_t o1 = __shfl_xor_sync(0xffffffffu, h ? v[i].y : v[i].w, 1);
+        uint32_t w[6] = {h ? o0 : v[i].x, h ? o1 : v[i].y, h ? v[i].x : v[i].z,
+                         h ? v[i].y : v[i].w, h ? v[i].z : o0, h ? v[i].w : o1};
+        if (x0 & 4) {
+#pragma unroll
+          for (int k = 0; k < 5; ++k) w[k] = w[k + 1];
+        }
+        if (x0 & 8) {
+#pragma unroll
+          for (int k = 0; k < 3; ++k) w[k] = w[k + 2];
+        }
+        score(warp + 2 * i, __funnelshift_r(w[0], w[1], (x0 & 3) * 8), __funnelshift_r(w[1], w[2], (x0 & 3) * 8));
+      }
+    } else {
+      for (int c = warp; c < kCand; c += 2) {
+        const int x0 = X + scx[c], xa = x0 & ~3, sh = (x0 - xa) * 8;
+        const uint8_t* rp = ref + (size_t)clampi(Y + r + scy[c], 0, g.RH - 1) * ref_pitch;
+        const uint32_t w0 = load_word_clamped(rp, xa + 8 * h, g.RW);
+        const uint32_t w1 = load_word_clamped(rp, xa + 8 * h + 4, g.RW);
+        const uint32_t w2 = load_word_clamped(rp, xa + 8 * h + 8, g.RW);
+        score(c, __funnelshift_r(w0, w1, sh), __funnelshift_r(w1, w2, sh));
+      }
     }
   }
-  // block gradients: sum |horizontal| and |vertical| neighbour differences
+  // block gradients: sum |horizontal| and |vertical| neighbour differences, a
+  // word of the block per thread
   {
-    const uint8_t* sc = reinterpret_cast<const uint8_t*>(scw);
-    uint32_t gh = 0, gv = 0;
-    for (int i = tid; i < 256; i += 64) {
-      const int y = i >> 4, x = i & 15;
-      if (x < 15) gh += (uint32_t)abs((int)sc[i] - (int)sc[i + 1]);
-      if (y < 15) gv += (uint32_t)abs((int)sc[i] - (int)sc[i + 16]);
-    }
-#pragma unroll
-    for (int o = 16; o > 0; o >>= 1) {
-      gh += __shfl_xor_sync(0xffffffffu, gh, o);
-      gv += __shfl_xor_sync(0xffffffffu, gv, o);
-    }
+    const uint32_t v = scw[tid], right = (tid & 3) < 3 ? scw[tid + 1] : v >> 24;
+    uint32_t gh = sad4_acc(v, __funnelshift_r(v, right, 8), 0u);
+    uint32_t gv = tid < 60 ? sad4_acc(v, scw[tid + 4], 0u) : 0u;
+    gh = __reduce_add_sync(0xffffffffu, gh);
+    gv = __reduce_add_sync(0xffffffffu, gv);
     if (lane == 0) {
       sgrad[warp][0] = gh;
       sgrad[warp][1] = gv;
@@ -197,35 +199,34 @@ __global__ void __launch_bounds__(64) lp_prepare_kernel(const uint8_t* __restric
   }
   __syncthreads();
 
-  uint32_t dup = 0;
-  uint32_t smin = 0xffffffffu;
-  for (int c = 0; c < kCand; ++c) {
-    for (int d = 0; d < c; ++d)
-      if (scx[d] == scx[c] && scy[d] == scy[c]) {
-        dup |= 1u << c;
-        break;
-      }
-    smin = min(smin, ssad[c]);
-  }
+  // candidates equal to an earlier one (lane c holds candidate c), lowest SAD
+  const uint32_t same =
+      __match_any_sync(0xffffffffu, lane < kCand ? (uint32_t)(scy[lane] << 16) | (scx[lane] & 0xffff) : 0x80000000u | lane);
+  const uint32_t dup = __ballot_sync(0xffffffffu, lane < kCand && (same & ((1u << lane) - 1u)) != 0u);
+  const uint32_t smin = __reduce_min_sync(0xffffffffu, lane < kCand ? ssad[lane] : 0xffffffffu);
   const bool early = zero_thresh >= 0 && ssad[9] <= (uint32_t)zero_thresh;
 
   // network input: row m (Morton cell (ox, oy) of the 8x8 grid) holds the
   // 2x2 pels (dy, dx) x (current, residual against c0) at k = (dy*2+dx)*2+ch
   {
-    const uint8_t* sc = reinterpret_cast<const uint8_t*>(scw);
-    const uint8_t* r0 = reinterpret_cast<const uint8_t*>(rfw);
+    // The values are whole numbers of at most eight bits over 64, exact in BF16; a
+    // byte becomes a float in the low bits of 2^23 + byte.
     const int m = tid, ox = morton_x(m), oy = morton_y(m);
-    __align__(16) __nv_bfloat16 v[8];
+    const uint16_t* sc = reinterpret_cast<const uint16_t*>(scw) + 16 * oy + ox;  // row 2 oy, column 2 ox
+    const uint16_t* r0 = reinterpret_cast<const uint16_t*>(rfw) + 16 * oy + ox;
+    uint32_t v[4];
 #pragma unroll
-    for (int dy = 0; dy < 2; ++dy)
+    for (int dy = 0; dy < 2; ++dy) {
+      const uint32_t cw = sc[8 * dy], rw = r0[8 * dy];
 #pragma unroll
       for (int dx = 0; dx < 2; ++dx) {
-        const int i = (2 * oy + dy) * 16 + 2 * ox + dx;
-        const int cv = sc[i], rv = r0[i];
-        v[(dy * 2 + dx) * 2 + 0] = __float2bfloat16_rn((float)(cv - 128) * 0.015625f);
-        v[(dy * 2 + dx) * 2 + 1] = __float2bfloat16_rn((float)(cv - rv) * 0.015625f);
+        const float cv = __uint_as_float(__byte_perm(cw, 0x4b000000u, 0x7650 + dx));
+        const float rv = __uint_as_float(__byte_perm(rw, 0x4b000000u, 0x7650 + dx));
+        const float x = fmaf(cv, 0.015625f, -(8388608.f + 128.f) * 0.015625f), y = (cv - rv) * 0.015625f;
+        asm("cvt.rn.bf16x2.f32 %0, %1, %2;" : "=r"(v[2 * dy + dx]) : "f"(y), "f"(x));
       }
-    *reinterpret_cast<uint4*>(b.x0 + ((size_t)mb * 64 + m) * 8) = *reinterpret_cast<const uint4*>(v);
+    }
+    *reinterpret_cast<uint4*>(b.x0 + ((size_t)mb * 64 + m) * 8) = make_uint4(v[0], v[1], v[2], v[3]);
   }
   // side features (64), columns 32..95 of the fc1 input row
   {
