@@ -190,6 +190,7 @@ int ensure_buffers(gpu_context_t* ctx, Impl* m, int W, int H) {
   cudaMemsetAsync(m->rec[0], 0, m->rec_bytes, m->stream);
   cudaMemsetAsync(m->rec[1], 0, m->rec_bytes, m->stream);
   cudaMemsetAsync(m->d_mv, 0, mbs * 16, m->stream);
+  cudaMemsetAsync(m->d_scratch, 0, m->scratch_words * 2 * 4, m->stream);
   for (Slot& s : m->slot) memset(s.status, 0, 16);
   m->cur = 0;
   ctx->has_recon_frame = false;
@@ -419,7 +420,8 @@ int encode_frame(gpu_context_t* ctx, Impl* m, const uint8_t* y, const uint8_t* u
     }
     rc |= cudaMemcpyAsync(sl.mv, m->d_mv, mbs * 16, cudaMemcpyDeviceToHost, st) == cudaSuccess ? 0 : -1;
     rc |= cudaMemcpyAsync(sl.status, scr0 + 1, 4, cudaMemcpyDeviceToHost, st) == cudaSuccess ? 0 : -1;
-    rc |= cudaMemcpyAsync(sl.status + 1, scr1 + 1, 4, cudaMemcpyDeviceToHost, st) == cudaSuccess ? 0 : -1;
+    sl.status[1] = 0;  // the deblocking pass's own word, where it runs
+    if (db) rc |= cudaMemcpyAsync(sl.status + 1, scr1 + 1, 4, cudaMemcpyDeviceToHost, st) == cudaSuccess ? 0 : -1;
   }
   perf_mark(m, 4);
   if (m->perf) {
