@@ -418,10 +418,11 @@ int encode_frame(gpu_context_t* ctx, Impl* m, const uint8_t* y, const uint8_t* u
       rc |= cudaMemcpyAsync(sl.pred_mode, m->d_pred_mode, mbs * 4, cudaMemcpyDeviceToHost, st) == cudaSuccess ? 0 : -1;
       rc |= cudaMemcpyAsync(sl.nz, m->d_nz, mbs * 96, cudaMemcpyDeviceToHost, st) == cudaSuccess ? 0 : -1;
     }
-    rc |= cudaMemcpyAsync(sl.mv, m->d_mv, mbs * 16, cudaMemcpyDeviceToHost, st) == cudaSuccess ? 0 : -1;
-    rc |= cudaMemcpyAsync(sl.status, scr0 + 1, 4, cudaMemcpyDeviceToHost, st) == cudaSuccess ? 0 : -1;
-    sl.status[1] = 0;  // the deblocking pass's own word, where it runs
-    if (db) rc |= cudaMemcpyAsync(sl.status + 1, scr1 + 1, 4, cudaMemcpyDeviceToHost, st) == cudaSuccess ? 0 : -1;
+    void *dev_mv = nullptr, *dev_status = nullptr;
+    rc |= cudaHostGetDevicePointer(&dev_mv, sl.mv, 0) == cudaSuccess ? 0 : -1;
+    rc |= cudaHostGetDevicePointer(&dev_status, sl.status, 0) == cudaSuccess ? 0 : -1;
+    if (rc == 0)
+      rc |= stage_mv_launch(m->d_mv, dev_mv, (int)mbs, scr0 + 1, db ? scr1 + 1 : nullptr, (uint32_t*)dev_status, st);
   }
   perf_mark(m, 4);
   if (m->perf) {
@@ -589,6 +590,18 @@ int gpu_compute_upload_nv12(gpu_context_t* ctx, gpu_image_t* image, gpu_memory_t
   (void)memory;
   if (!m || !image || !image->y_plane || !y_plane || !uv_plane || width <= 0 || height <= 0) return -1;
   if ((uint32_t)width > image->width || (uint32_t)height > image->height) return -1;
+  cudaPointerAttributes a{}, b{};
+  const bool locked = cudaPointerGetAttributes(&a, y_plane) == cudaSuccess && a.type == cudaMemoryTypeHost &&
+                      cudaPointerGetAttributes(&b, uv_plane) == cudaSuccess && b.type == cudaMemoryTypeHost;
+  if (!locked) cudaGetLastError();
+  // Rows apart on either side, page-locked and addressable: the row kernel
+  // (upload.cu says why the line lies there); else the copy engine.
+  const int dst_pitch = (int)image->pitch;
+  const bool apart = y_pitch != width || uv_pitch != width || dst_pitch != width;
+  if (locked && apart && a.devicePointer && b.devicePointer && y_pitch >= width && uv_pitch >= width)
+    return upload_nv12_launch((const uint8_t*)a.devicePointer, y_pitch, (const uint8_t*)b.devicePointer, uv_pitch,
+                                      (uint8_t*)image->y_plane, (uint8_t*)image->uv_plane, dst_pitch, width, height,
+                                      m->stream);
   if (cudaMemcpy2DAsync(image->y_plane, image->pitch, y_plane, y_pitch, width, height, cudaMemcpyHostToDevice,
                         m->stream) != cudaSuccess ||
       cudaMemcpy2DAsync(image->uv_plane, image->pitch, uv_plane, uv_pitch, width, height / 2,
@@ -597,12 +610,7 @@ int gpu_compute_upload_nv12(gpu_context_t* ctx, gpu_image_t* image, gpu_memory_t
   // Host buffers the caller may reuse on return: unless both planes are
   // page-locked (cudaMallocHost, or b200enc_host_register: then stream
   // order is enough), wait for the copy.
-  cudaPointerAttributes a{}, b{};
-  if (cudaPointerGetAttributes(&a, y_plane) != cudaSuccess || a.type != cudaMemoryTypeHost ||
-      cudaPointerGetAttributes(&b, uv_plane) != cudaSuccess || b.type != cudaMemoryTypeHost) {
-    cudaGetLastError();
-    return cudaStreamSynchronize(m->stream) == cudaSuccess ? 0 : -1;
-  }
+  if (!locked) return cudaStreamSynchronize(m->stream) == cudaSuccess ? 0 : -1;
   return 0;
 }
 
