@@ -31,6 +31,27 @@ struct Geo {
 __device__ __forceinline__ int clampi(int v, int lo, int hi) { return v < lo ? lo : (v > hi ? hi : v); }
 __device__ __forceinline__ int clip1(int v) { return clampi(v, 0, 255); }
 
+// Four unsigned bytes times four signed ones, summed onto acc.
+__device__ __forceinline__ int dot4(uint32_t samples, uint32_t taps, int acc) {
+  int d;
+  asm("dp4a.u32.s32 %0, %1, %2, %3;" : "=r"(d) : "r"(samples), "r"(taps), "r"(acc));
+  return d;
+}
+// Four values, each clipped to a byte; v[0] lowest.
+__device__ __forceinline__ uint32_t clip4(int v0, int v1, int v2, int v3) {
+  uint32_t d;
+  asm("{\n\t.reg .b32 t;\n\t"
+      "cvt.pack.sat.u8.s32.b32 t, %4, %3, 0;\n\t"
+      "cvt.pack.sat.u8.s32.b32 %0, %2, %1, t;\n\t}"
+      : "=r"(d)
+      : "r"(v0), "r"(v1), "r"(v2), "r"(v3));
+  return d;
+}
+// Rounded average of each byte.
+__device__ __forceinline__ uint32_t avg4(uint32_t a, uint32_t b) {
+  return (a | b) - (((a ^ b) >> 1) & 0x7f7f7f7fu);
+}
+
 __device__ __forceinline__ int chroma_qp(int qpy) {
   // A1/shaders/quantize.comp:182-187 (Table 8-15, offset 0)
   if (qpy < 30) return qpy;

@@ -272,11 +272,6 @@ __global__ void __launch_bounds__(128) hevc_dqit8_kernel(const int16_t* __restri
 // the sums staged in shared memory 17.5 (10.6 MB moved, 1.6 us).
 constexpr int kHpTileW = 128, kHpTileH = 32, kHpRows = 8;
 
-__device__ __forceinline__ int dot4(uint32_t samples, uint32_t taps, int acc) {
-  int d;
-  asm("dp4a.u32.s32 %0, %1, %2, %3;" : "=r"(d) : "r"(samples), "r"(taps), "r"(acc));
-  return d;
-}
 __device__ __forceinline__ int dot2(uint32_t samples, uint32_t taps, int acc) {
   int d;
   asm("dp2a.lo.u32.s32 %0, %1, %2, %3;" : "=r"(d) : "r"(samples), "r"(taps), "r"(acc));

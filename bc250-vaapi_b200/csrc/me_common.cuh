@@ -130,15 +130,16 @@ __device__ __forceinline__ void refine_planes(RefineSimd& rf, const uint8_t* g, 
     for (int r = 0; r < 8; ++r) {
       const uint32_t* wp = reinterpret_cast<const uint32_t*>(rows + r * gstride);
       const uint32_t a0 = wp[0], a1 = wp[1], a2 = wp[2];
-      const uint32_t lo = __funnelshift_r(a0, a1, sh), hi = __funnelshift_r(a1, a2, sh);  // e0..e3, e4..e7
-      const uint32_t mid = __funnelshift_r(lo, hi, 16), up = __funnelshift_r(hi, a2 >> sh, 24);  // e2..e5, e7 e8 ..
-      const uint32_t p0 = __byte_perm(lo, 0, 0x4140), p1 = __byte_perm(lo, 0, 0x4241), p2 = __byte_perm(lo, 0, 0x4342);
-      const uint32_t p3 = __byte_perm(mid, 0, 0x4241), p4 = __byte_perm(hi, 0, 0x4140);
-      const uint32_t p5 = __byte_perm(hi, 0, 0x4241), p6 = __byte_perm(hi, 0, 0x4342), p7 = __byte_perm(up, 0, 0x4140);
-      t01[r] = tap6_pair(p0, p1, p2, p3, p4, p5);
-      t23[r] = tap6_pair(p2, p3, p4, p5, p6, p7);
-      g01[r] = p2;
-      g23[r] = p4;
+      const uint32_t lo = __funnelshift_r(a0, a1, sh), hi = __funnelshift_r(a1, a2, sh), up = a2 >> sh;  // e0.., e4.., e8
+      constexpr uint32_t ta = 0x1414fb01u, tb = 0x000001fbu;  // 1 -5 20 20, -5 1
+      const int t0 = dot4(lo, ta, dot4(hi, tb, (int)kTapBias));
+      const int t1 = dot4(__funnelshift_r(lo, hi, 8), ta, dot4(__funnelshift_r(hi, up, 8), tb, (int)kTapBias));
+      const int t2 = dot4(__funnelshift_r(lo, hi, 16), ta, dot4(hi >> 16, tb, (int)kTapBias));
+      const int t3 = dot4(__funnelshift_r(lo, hi, 24), ta, dot4(__funnelshift_r(hi, up, 24), tb, (int)kTapBias));
+      t01[r] = __byte_perm(t0, t1, 0x5410);
+      t23[r] = __byte_perm(t2, t3, 0x5410);
+      g01[r] = __byte_perm(lo, 0, 0x4342);
+      g23[r] = __byte_perm(hi, 0, 0x4140);
     }
 #pragma unroll
     for (int k = 0; k < 3; ++k) {  // plane row 3 grp + k (ry = that - 1): reference rows k .. k + 5 of the eight
@@ -150,12 +151,14 @@ __device__ __forceinline__ void refine_planes(RefineSimd& rf, const uint8_t* g, 
                         tap_round_pair(tap6_pair(g23[k], g23[k + 1], g23[k + 2], g23[k + 3], g23[k + 4], g23[k + 5])),
                         0x6420);
       // the taps' weights sum to 32, so the bias of the sums comes out as 32 * kTapBias
-      auto jval = [&](const uint32_t* t, int s) -> uint32_t {
-        auto at = [&](int i) -> int { return (int)(s ? t[k + i] >> 16 : t[k + i] & 0xffffu); };
-        const int v = (at(2) + at(3)) * 20 + (at(0) + at(5)) - (at(1) + at(4)) * 5;
-        return (uint32_t)clip1((v - 32 * (int)kTapBias + 512) >> 10);
-      };
-      *jp = __byte_perm(jval(t01, 0) | (jval(t01, 1) << 16), jval(t23, 0) | (jval(t23, 1) << 16), 0x6420);
+      int v[4];
+#pragma unroll
+      for (int c = 0; c < 4; ++c) {  // a column's sums two rows to a word, three integer dot products
+        const uint32_t* t = c < 2 ? t01 : t23;
+        auto rows2 = [&](int i) -> int { return (int)__byte_perm(t[k + i], t[k + i + 1], (c & 1) ? 0x7632 : 0x5410); };
+        v[c] = __dp2a_lo(rows2(0), 0xfb01, __dp2a_lo(rows2(2), 0x1414, __dp2a_lo(rows2(4), 0x01fb, 512 - 32 * (int)kTapBias))) >> 10;
+      }
+      *jp = clip4(v[0], v[1], v[2], v[3]);
     }
   }
 }
@@ -200,15 +203,25 @@ __device__ __forceinline__ uint32_t qpel_refine_warp_simd(RefineSimd& rf, const 
     operand(op, pa, sa, ia);
     operand(op >> 4, pb, sb, ib);
     uint32_t sad = 0;
+    // every fourth row: word steps of 4 pitches / 4 bytes; the half positions
+    // are samples of one plane, not averages of two
 #pragma unroll 1
-    for (int r = 0; r < 4; ++r, pa += ia, pb += ib) {  // every fourth row: word steps of 4 pitches / 4 bytes
+    for (int r = 0; r < 4; ++r, pa += ia, pb += ib) {
       const uint4 c = *reinterpret_cast<const uint4*>(cur + 4 * ((lane & 3) + 4 * r));
       const uint32_t a0 = pa[0], a1 = pa[1], a2 = pa[2], a3 = pa[3], a4 = pa[4];
-      const uint32_t b0 = pb[0], b1 = pb[1], b2 = pb[2], b3 = pb[3], b4 = pb[4];
-      sad = sad4_acc(__vavgu4(__funnelshift_r(a0, a1, sa), __funnelshift_r(b0, b1, sb)), c.x, sad);
-      sad = sad4_acc(__vavgu4(__funnelshift_r(a1, a2, sa), __funnelshift_r(b1, b2, sb)), c.y, sad);
-      sad = sad4_acc(__vavgu4(__funnelshift_r(a2, a3, sa), __funnelshift_r(b2, b3, sb)), c.z, sad);
-      sad = sad4_acc(__vavgu4(__funnelshift_r(a3, a4, sa), __funnelshift_r(b3, b4, sb)), c.w, sad);
+      uint32_t v0 = __funnelshift_r(a0, a1, sa), v1 = __funnelshift_r(a1, a2, sa);
+      uint32_t v2 = __funnelshift_r(a2, a3, sa), v3 = __funnelshift_r(a3, a4, sa);
+      if (stage) {
+        const uint32_t b0 = pb[0], b1 = pb[1], b2 = pb[2], b3 = pb[3], b4 = pb[4];
+        v0 = avg4(v0, __funnelshift_r(b0, b1, sb));
+        v1 = avg4(v1, __funnelshift_r(b1, b2, sb));
+        v2 = avg4(v2, __funnelshift_r(b2, b3, sb));
+        v3 = avg4(v3, __funnelshift_r(b3, b4, sb));
+      }
+      sad = sad4_acc(v0, c.x, sad);
+      sad = sad4_acc(v1, c.y, sad);
+      sad = sad4_acc(v2, c.z, sad);
+      sad = sad4_acc(v3, c.w, sad);
     }
     sad += __shfl_xor_sync(0xffffffffu, sad, 1);
     sad += __shfl_xor_sync(0xffffffffu, sad, 2);

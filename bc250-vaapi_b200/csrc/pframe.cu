@@ -48,25 +48,6 @@ __device__ __forceinline__ uint32_t bytes4(const uint8_t* row, int o) {
   const uint32_t* w = reinterpret_cast<const uint32_t*>(row + (o & ~3));
   return __funnelshift_r(w[0], w[1], (o & 3) * 8);
 }
-__device__ __forceinline__ int dot4(uint32_t samples, uint32_t taps, int acc) {
-  int d;
-  asm("dp4a.u32.s32 %0, %1, %2, %3;" : "=r"(d) : "r"(samples), "r"(taps), "r"(acc));
-  return d;
-}
-// Four values, each clipped to a byte; v[0] lowest.
-__device__ __forceinline__ uint32_t clip4(int v0, int v1, int v2, int v3) {
-  uint32_t d;
-  asm("{\n\t.reg .b32 t;\n\t"
-      "cvt.pack.sat.u8.s32.b32 t, %4, %3, 0;\n\t"
-      "cvt.pack.sat.u8.s32.b32 %0, %2, %1, t;\n\t}"
-      : "=r"(d)
-      : "r"(v0), "r"(v1), "r"(v2), "r"(v3));
-  return d;
-}
-__device__ __forceinline__ uint32_t avg4(uint32_t a, uint32_t b) {
-  return (a | b) - (((a ^ b) >> 1) & 0x7f7f7f7fu);
-}
-
 // Horizontal 6-tap sums of four neighbouring samples: bytes o .. o + 8 of a row.
 __device__ __forceinline__ void tap6_row(const uint8_t* row, int o, int (&t)[4]) {
   const uint32_t* w = reinterpret_cast<const uint32_t*>(row + (o & ~3));
