@@ -263,7 +263,7 @@ __global__ void lp_select_kernel(int mbs, LpBuf b, int mode, float param, int la
 
 // ---------------------------------------------------------------------------
 // Exact re-scoring of the selected candidates' +-2 windows, then the refine.
-// 64 threads per MB, persistent over the learned list.
+// One warp per MB, persistent over the learned list.
 // ---------------------------------------------------------------------------
 // One warp per MB, four independent warps per block; every warp walks the
 // learned list on its own and synchronises only itself.
@@ -273,12 +273,11 @@ __global__ void lp_select_kernel(int mbs, LpBuf b, int mode, float param, int la
 // that window, so the refine reads no global memory. With the row starting
 // at that byte, integer offset ox of the window begins at byte 3+ox of every
 // patch row whatever the candidate, so the search's byte shifts are
-// compile-time constants. One lane scores a whole row of the window (the 5
-// offsets at one oy) from three 64-bit loads of the patch row and one
-// 128-bit load of the current row per macroblock row. Rows are kPatchStride
-// = 10 words apart (8 used) and candidates kCandWords = 274 words: the 20
-// lanes' 64-bit loads of one instruction then fall on distinct banks in
-// each half-warp phase.
+// compile-time constants. Rows are kPatchStride = 10 words apart (8 used) and
+// candidates kCandWords = 274 words: the 32 lanes' 64-bit loads of one
+// instruction (eight rows, two apart, of four candidates) fall on distinct banks
+// in each half-warp phase. Bound by instructions issued: 30,185 macroblocks of a
+// 2160p picture 97 us (117 with a row of the window per lane, 20 lanes at work).
 constexpr int kPatchRows = 27, kPatchStride = 10, kCandWords = 274;  // 8 words used per row
 struct RescoreWarp {
   alignas(16) uint32_t patch[4 * kCandWords];
@@ -290,8 +289,11 @@ struct RescoreWarp {
 // BATCH: the listed macroblocks are compact P indices of a batch; each
 // takes its stream's geometry, planes and lambda, and its vector goes to
 // mv_out at the compact index.
+// Nine CTAs per SM: with eight (64 registers) the driver gives the kernel a smaller
+// shared-memory carve-out than the fallback search running beside it, and the two
+// take turns on an SM instead of sharing it (640x480: the pair 28 us, not 19).
 template <bool BATCH>
-__global__ void __launch_bounds__(128) lp_rescore_kernel(const uint8_t* __restrict__ cur_, int cur_pitch_,
+__global__ void __launch_bounds__(128, 9) lp_rescore_kernel(const uint8_t* __restrict__ cur_, int cur_pitch_,
                                                          const uint8_t* __restrict__ ref_, int ref_pitch_, Geo g_,
                                                          int R, int lambda_, int mbs, LpBuf b,
                                                          MV* __restrict__ mv_out, BatchTab bt) {
@@ -393,48 +395,74 @@ __global__ void __launch_bounds__(128) lp_rescore_kernel(const uint8_t* __restri
     }
     __syncwarp();
 
-    // the 25 integer offsets of each candidate: lane k*5+oy scores the row
-    // of offsets (ox = 0..4, oy) of candidate k
+    // the 25 integer offsets of each candidate: lane 8k + i holds rows 2i and
+    // 2i + 1 of the current block and scores them against the six patch rows they
+    // meet, for every offset; the partial sums (a whole one is under 16 bits) are
+    // packed in pairs and dealt out over the candidate's eight lanes
     uint32_t best = 0xffffffffu;
-    if (lane < nk * 5) {
-      const int k = lane / 5, oy = lane - 5 * k;
-      const uint32_t* prow = sh.patch + k * kCandWords + (oy + 3) * kPatchStride;
-      uint32_t s0 = 0, s1 = 0, s2 = 0, s3 = 0, s4 = 0;
-#pragma unroll 4
-      for (int r = 0; r < 16; ++r) {
-        const uint2 p0 = *reinterpret_cast<const uint2*>(prow + r * kPatchStride);
-        const uint2 p1 = *reinterpret_cast<const uint2*>(prow + r * kPatchStride + 2);
-        const uint2 p2 = *reinterpret_cast<const uint2*>(prow + r * kPatchStride + 4);
-        const uint4 c = *reinterpret_cast<const uint4*>(sh.cur + 4 * r);
-        const uint32_t u0 = p0.x, u1 = p0.y, u2 = p1.x, u3 = p1.y, u4 = p2.x, u5 = p2.y;
-        s0 = sad4_acc(__funnelshift_r(u0, u1, 24), c.x, s0);  // ox 0: bytes 3..18
-        s0 = sad4_acc(__funnelshift_r(u1, u2, 24), c.y, s0);
-        s0 = sad4_acc(__funnelshift_r(u2, u3, 24), c.z, s0);
-        s0 = sad4_acc(__funnelshift_r(u3, u4, 24), c.w, s0);
-        s1 = sad4_acc(u1, c.x, s1);  // ox 1: bytes 4..19
-        s1 = sad4_acc(u2, c.y, s1);
-        s1 = sad4_acc(u3, c.z, s1);
-        s1 = sad4_acc(u4, c.w, s1);
-        s2 = sad4_acc(__funnelshift_r(u1, u2, 8), c.x, s2);  // ox 2: bytes 5..20
-        s2 = sad4_acc(__funnelshift_r(u2, u3, 8), c.y, s2);
-        s2 = sad4_acc(__funnelshift_r(u3, u4, 8), c.z, s2);
-        s2 = sad4_acc(__funnelshift_r(u4, u5, 8), c.w, s2);
-        s3 = sad4_acc(__funnelshift_r(u1, u2, 16), c.x, s3);  // ox 3: bytes 6..21
-        s3 = sad4_acc(__funnelshift_r(u2, u3, 16), c.y, s3);
-        s3 = sad4_acc(__funnelshift_r(u3, u4, 16), c.z, s3);
-        s3 = sad4_acc(__funnelshift_r(u4, u5, 16), c.w, s3);
-        s4 = sad4_acc(__funnelshift_r(u1, u2, 24), c.x, s4);  // ox 4: bytes 7..22
-        s4 = sad4_acc(__funnelshift_r(u2, u3, 24), c.y, s4);
-        s4 = sad4_acc(__funnelshift_r(u3, u4, 24), c.z, s4);
-        s4 = sad4_acc(__funnelshift_r(u4, u5, 24), c.w, s4);
-      }
-      const int dy = sh.ccy[k] - 2 + oy, dx0 = sh.ccx[k] - 2;
-      const uint32_t sads[5] = {s0, s1, s2, s3, s4};
+    {
+      const int k = lane >> 3, i = lane & 7;
+      const uint32_t* prow = sh.patch + k * kCandWords + (2 * i + 3) * kPatchStride;
+      const uint4 cr[2] = {*reinterpret_cast<const uint4*>(sh.cur + 8 * i), *reinterpret_cast<const uint4*>(sh.cur + 8 * i + 4)};
+      uint32_t sum[28];  // 5 oy + ox, then unused
 #pragma unroll
-      for (int ox = 0; ox < 5; ++ox) {
-        const int dx = dx0 + ox;
-        const uint32_t cost = sads[ox] + (uint32_t)lambda * (uint32_t)(abs(dx) + abs(dy));
-        best = min(best, (cost << 14) | (uint32_t)((dy + R) * SIDE + (dx + R)));
+      for (int j = 0; j < 28; ++j) sum[j] = 0;
+#pragma unroll
+      for (int p = 0; p < 6; ++p) {
+        const uint2 p0 = *reinterpret_cast<const uint2*>(prow + p * kPatchStride);
+        const uint2 p1 = *reinterpret_cast<const uint2*>(prow + p * kPatchStride + 2);
+        const uint2 p2 = *reinterpret_cast<const uint2*>(prow + p * kPatchStride + 4);
+        const uint32_t u[6] = {p0.x, p0.y, p1.x, p1.y, p2.x, p2.y};
+        // the row from bytes 3 + ox on (ox = 0 and 4 share words)
+        uint32_t v8[4], v16[4], v24[5];
+#pragma unroll
+        for (int j = 0; j < 5; ++j) v24[j] = __funnelshift_r(u[j], u[j + 1], 24);
+#pragma unroll
+        for (int j = 0; j < 4; ++j) {
+          v8[j] = __funnelshift_r(u[j + 1], u[j + 2], 8);
+          v16[j] = __funnelshift_r(u[j + 1], u[j + 2], 16);
+        }
+#pragma unroll
+        for (int c = 0; c < 2; ++c) {
+          const int oy = p - c;
+          if (oy < 0 || oy > 4) continue;
+          const uint32_t cw[4] = {cr[c].x, cr[c].y, cr[c].z, cr[c].w};
+#pragma unroll
+          for (int j = 0; j < 4; ++j) {
+            sum[5 * oy + 0] = sad4_acc(v24[j], cw[j], sum[5 * oy + 0]);
+            sum[5 * oy + 1] = sad4_acc(u[j + 1], cw[j], sum[5 * oy + 1]);
+            sum[5 * oy + 2] = sad4_acc(v8[j], cw[j], sum[5 * oy + 2]);
+            sum[5 * oy + 3] = sad4_acc(v16[j], cw[j], sum[5 * oy + 3]);
+            sum[5 * oy + 4] = sad4_acc(v24[j + 1], cw[j], sum[5 * oy + 4]);
+          }
+        }
+      }
+      // words 7 a + 0 .. 6 stay with the lanes of bit 4 = a, then 4 b + 0 .. 3 of
+      // those with bit 2 = b, then 2 c + 0 .. 1 with bit 1 = c
+      uint32_t w[8];
+      const bool ha = i & 4, hb = i & 2, hc = i & 1;
+#pragma unroll
+      for (int j = 0; j < 7; ++j) {
+        const uint32_t lo = sum[2 * j] | sum[2 * j + 1] << 16, hi = sum[14 + 2 * j] | sum[15 + 2 * j] << 16;
+        w[j] = (ha ? hi : lo) + __shfl_xor_sync(0xffffffffu, ha ? lo : hi, 4);
+      }
+      w[7] = 0;
+#pragma unroll
+      for (int j = 0; j < 4; ++j) w[j] = (hb ? w[4 + j] : w[j]) + __shfl_xor_sync(0xffffffffu, hb ? w[j] : w[4 + j], 2);
+#pragma unroll
+      for (int j = 0; j < 2; ++j) w[j] = (hc ? w[2 + j] : w[j]) + __shfl_xor_sync(0xffffffffu, hc ? w[j] : w[2 + j], 1);
+      if (k < nk) {
+        const int base = (hb ? 4 : 0) + (hc ? 2 : 0);
+        const int x0 = sh.ccx[k] - 2, y0 = sh.ccy[k] - 2;
+#pragma unroll
+        for (int j = 0; j < 4; ++j) {
+          const int s = 2 * ((ha ? 7 : 0) + base + (j >> 1)) + (j & 1);
+          if (base + (j >> 1) == 7 || s >= 25) continue;
+          const int oy = s / 5, dy = y0 + oy, dx = x0 + s - 5 * oy;
+          const uint32_t sad = (j & 1) ? w[j >> 1] >> 16 : w[j >> 1] & 0xffffu;
+          const uint32_t cost = sad + (uint32_t)lambda * (uint32_t)(abs(dx) + abs(dy));
+          best = min(best, (cost << 14) | (uint32_t)((dy + R) * SIDE + (dx + R)));
+        }
       }
     }
     best = __reduce_min_sync(0xffffffffu, best);
