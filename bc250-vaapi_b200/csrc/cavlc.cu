@@ -235,6 +235,7 @@ __device__ __forceinline__ bool p_skip(const CavlcArgs& a, int mb, int mbx, int 
 }
 
 __global__ void __launch_bounds__(32 * kCavlcMbWarps) cavlc_mb_kernel(CavlcArgs a) {
+  pdl_wait();
   __shared__ CavlcWarp shw[kCavlcMbWarps];
   const unsigned full = 0xffffffffu;
   const int lane = threadIdx.x & 31, wi = threadIdx.x >> 5;
@@ -596,6 +597,7 @@ __device__ uint32_t scan_sum(uint32_t v, uint32_t* sh, uint32_t* total) {
 __device__ __forceinline__ uint32_t ue_len(uint32_t v) { return 2u * (31u - (uint32_t)__clz((int)(v + 1u))) + 1u; }
 
 __global__ void __launch_bounds__(kCavlcScanThreads) cavlc_slice_kernel(CavlcArgs a, CavlcHdr h) {
+  pdl_wait();
   __shared__ RunState shr[32];
   __shared__ uint32_t shs[32];
   const int s = blockIdx.x, t = threadIdx.x;
@@ -661,6 +663,7 @@ __global__ void __launch_bounds__(kCavlcScanThreads) cavlc_slice_kernel(CavlcArg
 // where a binary search takes thirteen) down to the first word's macroblock,
 // then the 32 macroblocks from there on in registers.
 __global__ void __launch_bounds__(256) cavlc_gather_kernel(CavlcArgs a, CavlcHdr h) {
+  pdl_wait();
   const int s = blockIdx.y;
   if (a.sl[4 * s + 2]) return;  // the slice did not fit
   const uint32_t bits = a.sl[4 * s + 0], trail = a.sl[4 * s + 1], end = a.sl[4 * s + 3];
@@ -820,11 +823,11 @@ extern "C" int b200enc_cavlc_slices(const b200enc_cavlc_t* p, void* stream) {
   a.out_copy = p->out_copy ? p->out_copy : p->out;
   cudaStream_t st = static_cast<cudaStream_t>(stream);
   const int mbs = p->mbw * p->mbh;
-  cavlc_mb_kernel<<<(mbs + kCavlcMbWarps - 1) / kCavlcMbWarps, 32 * kCavlcMbWarps, 0, st>>>(a);
-  cavlc_slice_kernel<<<p->num_slices, kCavlcScanThreads, 0, st>>>(a, h);
+  launch_early(cavlc_mb_kernel, (mbs + kCavlcMbWarps - 1) / kCavlcMbWarps, 32 * kCavlcMbWarps, 0, st, a);
+  launch_early(cavlc_slice_kernel, p->num_slices, kCavlcScanThreads, 0, st, a, h);
   // words per slice are known on the device only: a CTA of 256 words per 16
   // macroblocks (the share of a dense one), walking the rest in strides
   const int ctas = std::max(1, std::min(128, mbs / p->num_slices / 16));
-  cavlc_gather_kernel<<<dim3(ctas, p->num_slices), 256, 0, st>>>(a, h);
+  launch_early(cavlc_gather_kernel, dim3(ctas, p->num_slices), 256, 0, st, a, h);
   return cudaGetLastError() == cudaSuccess ? 0 : -1;
 }

@@ -615,6 +615,7 @@ __global__ void __launch_bounds__(kDbTileThreads, 2) deblock_tile_kernel(
     const MV* __restrict__ mvs_, const uint8_t* __restrict__ t8_, const uint8_t* __restrict__ src_y_,
     const uint8_t* __restrict__ src_uv_,
     uint8_t* __restrict__ dst_y_, uint8_t* __restrict__ dst_uv_, int pitch_, uint32_t* status_, BatchTab bt) {
+  pdl_wait();
   extern __shared__ __align__(16) uint8_t smem[];
   const int tid = threadIdx.x, nthr = blockDim.x;
   int mbw = mbw_, mbh = mbh_, qp = qp_, is_intra = is_intra_, pitch = pitch_;
@@ -841,8 +842,8 @@ int b200enc_deblock_tiles_launch(int mbw, int mbh, int qp, int is_intra, const u
       cudaSuccess)
     return -1;
   const int tiles = ((mbw + TW - 1) / TW) * ((mbh + TH - 1) / TH);
-  deblock_tile_kernel<false><<<tiles, db_tile_threads(TW, TH), P.bytes, stream>>>(
-      mbw, mbh, TW, TH, qp, is_intra, nz, (const MV*)mv, t8, src_y, src_uv, dst_y, dst_uv, pitch, status, BatchTab{});
+  launch_early(deblock_tile_kernel<false>, tiles, db_tile_threads(TW, TH), P.bytes, stream, mbw, mbh, TW, TH, qp, is_intra, nz,
+               (const MV*)mv, t8, src_y, src_uv, dst_y, dst_uv, pitch, status, BatchTab{});
   return cudaGetLastError() == cudaSuccess ? 0 : -1;
 }
 

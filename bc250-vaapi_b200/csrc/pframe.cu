@@ -216,6 +216,7 @@ __global__ void __launch_bounds__(384, 3) p_mb_kernel(const uint8_t* __restrict_
                                                   uint32_t* __restrict__ pred_mode_, uint8_t* __restrict__ rec_y_,
                                                   uint8_t* __restrict__ rec_uv_, int rec_pitch_, BatchTab bt,
                                                   int t8 = 0, uint8_t* __restrict__ t8_flags = nullptr) {
+  pdl_wait();
   extern __shared__ __align__(16) uint8_t p_smem[];
   using Shared = typename std::conditional<T8, PShared8, PPatch>::type;
   Shared& s = reinterpret_cast<Shared*>(p_smem)[threadIdx.y];
@@ -591,13 +592,13 @@ extern "C" int b200enc_p_frame_t8(const uint8_t* cur_y, const uint8_t* cur_uv, i
   const dim3 grid((g.mbw + T - 1) / T, g.mbh), block(96, T);
   const cudaStream_t st = (cudaStream_t)stream;
   if (t8 != 0) {
-    p_mb_kernel<false, true><<<grid, block, T * sizeof(PShared8), st>>>(cur_y, cur_uv, cur_pitch, ref_y, ref_uv, ref_pitch, g,
-                                                                        qp, (const MV*)mv, levels, dc, nz, pred_mode, rec_y,
-                                                                        rec_uv, rec_pitch, BatchTab{}, t8, t8_flags);
+    launch_early(p_mb_kernel<false, true>, grid, block, T * sizeof(PShared8), st, cur_y, cur_uv, cur_pitch, ref_y, ref_uv,
+                 ref_pitch, g, qp, (const MV*)mv, levels, dc, nz, pred_mode, rec_y, rec_uv, rec_pitch, BatchTab{}, t8,
+                 t8_flags);
   } else {
-    p_mb_kernel<false, false><<<grid, block, T * sizeof(PPatch), st>>>(cur_y, cur_uv, cur_pitch, ref_y, ref_uv, ref_pitch, g,
-                                                                       qp, (const MV*)mv, levels, dc, nz, pred_mode, rec_y,
-                                                                       rec_uv, rec_pitch, BatchTab{}, 0, t8_flags);
+    launch_early(p_mb_kernel<false, false>, grid, block, T * sizeof(PPatch), st, cur_y, cur_uv, cur_pitch, ref_y, ref_uv,
+                 ref_pitch, g, qp, (const MV*)mv, levels, dc, nz, pred_mode, rec_y, rec_uv, rec_pitch, BatchTab{}, 0,
+                 t8_flags);
   }
   return cudaGetLastError() == cudaSuccess ? 0 : -1;
 }

@@ -53,6 +53,8 @@ __global__ void __launch_bounds__(64) lp_prepare_kernel(const uint8_t* __restric
                                                         const uint8_t* __restrict__ ref_, int ref_pitch_, Geo g_,
                                                         const MV* __restrict__ prev_, int R, int zero_thresh_,
                                                         LpBuf b, BatchTab bt) {
+  pdl_wait();
+  if (blockIdx.x == 0 && threadIdx.x < 8) b.counters[threadIdx.x] = 0;  // the selection's, after this kernel
   __shared__ uint32_t scw[64];   // current MB, 16 rows x 4 words (clamped to W, H)
   __shared__ uint32_t rfw[64];   // reference block at candidate 0
   __shared__ int scx[kCand], scy[kCand];
@@ -802,9 +804,8 @@ int b200enc_proposal_prepare(void* h, const uint8_t* cur_y, int cur_pitch, const
   const int mbs = g.mbw * g.mbh;
   if (mbs > P->max_mbs) return -1;
   cudaStream_t st = (cudaStream_t)stream;
-  if (cudaMemsetAsync(P->b.counters, 0, 32, st) != cudaSuccess) return -1;
-  lp_prepare_kernel<false><<<mbs, 64, 0, st>>>(cur_y, cur_pitch, ref_y, ref_pitch, g, (const MV*)prev_mv, range,
-                                               zero_thresh, P->b, BatchTab{});
+  launch_early(lp_prepare_kernel<false>, mbs, 64, 0, st, cur_y, cur_pitch, ref_y, ref_pitch, g, (const MV*)prev_mv, range,
+               zero_thresh, P->b, BatchTab{});
   return cudaGetLastError() == cudaSuccess ? 0 : -1;
 }
 
@@ -933,7 +934,6 @@ int b200enc_proposal_me_batch(void* h, const BatchTab& bt, int n, int range, int
                               cudaStream_t st) {
   Proposal* P = static_cast<Proposal*>(h);
   if (!P || n <= 0 || n > P->max_mbs || (mode != 1 && mode != 3) || (range != 16 && range != 32)) return -1;
-  if (cudaMemsetAsync(P->b.counters, 0, 32, st) != cudaSuccess) return -1;
   lp_prepare_kernel<true><<<n, 64, 0, st>>>(nullptr, 0, nullptr, 0, Geo{}, nullptr, range, 0, P->b, bt);
   if (mode == 1) {
     if (lp_net_launch(n, P->b, P->wb, P->params, param, lambda, bt.mvc, P->err, st) != 0) return -1;

@@ -84,6 +84,7 @@ constexpr int kNetThreads = 512;
 __global__ void __launch_bounds__(kNetThreads, 1) lp_net_kernel(int mbs, LpBuf b, const __nv_bfloat16* __restrict__ wb,
                                                        const float* __restrict__ params, float param, int lambda,
                                                        MV* __restrict__ mv_out, uint32_t* __restrict__ err) {
+  pdl_wait();
   extern __shared__ __align__(128) uint8_t smem_raw[];
   NetSmem& s = *reinterpret_cast<NetSmem*>(smem_raw);
   const int tid = threadIdx.x, warp = tid >> 5, lane = tid & 31;
@@ -326,7 +327,7 @@ int lp_net_launch(int mbs, const LpBuf& b, const __nv_bfloat16* wb, const float*
   int dev = 0;
   if (cudaGetDevice(&dev) == cudaSuccess) cudaDeviceGetAttribute(&sms, cudaDevAttrMultiProcessorCount, dev);
   const int ntiles = (mbs + kNetTileMbs - 1) / kNetTileMbs;
-  lp_net_kernel<<<std::min(ntiles, sms), kNetThreads, smem, st>>>(mbs, b, wb, params, conf, lambda, mv_out, err);
+  launch_early(lp_net_kernel, std::min(ntiles, sms), kNetThreads, smem, st, mbs, b, wb, params, conf, lambda, mv_out, err);
   return cudaGetLastError() == cudaSuccess ? 0 : -1;
 }
 

@@ -205,6 +205,7 @@ __device__ __forceinline__ float bf16_hi(uint32_t w) { return __uint_as_float(w 
 __global__ void __launch_bounds__(kNet8Block, 2) lp_net8_kernel(int mbs, LpBuf b, const float* __restrict__ params,
                                                          const uint8_t* __restrict__ w8, float param, int lambda,
                                                          MV* __restrict__ mv_out, uint32_t* __restrict__ err) {
+  pdl_wait();
   extern __shared__ __align__(128) uint8_t smem_raw[];
   Net8Smem& s = *reinterpret_cast<Net8Smem*>(smem_raw);
   const int tid = threadIdx.x, warp = tid >> 5, lane = tid & 31;
@@ -595,8 +596,7 @@ int lp_net8_launch(int mbs, const LpBuf& b, const float* params, uint8_t* w8, bo
   int dev = 0;
   if (cudaGetDevice(&dev) == cudaSuccess) cudaDeviceGetAttribute(&sms, cudaDevAttrMultiProcessorCount, dev);
   const int ntiles = (mbs + kNet8TileMbs - 1) / kNet8TileMbs;
-  lp_net8_kernel<<<std::min(ntiles, 2 * sms), kNet8Block, smem, st>>>(mbs, b, params, w8, conf, lambda, mv_out,
-                                                                       err);
+  launch_early(lp_net8_kernel, std::min(ntiles, 2 * sms), kNet8Block, smem, st, mbs, b, params, w8, conf, lambda, mv_out, err);
   return cudaGetLastError() == cudaSuccess ? 0 : -1;
 }
 

@@ -10,6 +10,7 @@
 #include <algorithm>
 
 #include "b200enc_internal.h"
+#include "common.cuh"
 
 namespace b200enc {
 
@@ -70,6 +71,7 @@ __global__ void __launch_bounds__(128) upload_nv12_kernel(UploadPlane y, UploadP
 __global__ void __launch_bounds__(256) stage_mv_kernel(const uint4* __restrict__ mv, uint4* __restrict__ mv_host, int mbs,
                                                        const uint32_t* __restrict__ s0, const uint32_t* __restrict__ s1,
                                                        uint32_t* __restrict__ status_host) {
+  pdl_wait();
   const int i = blockIdx.x * 256 + threadIdx.x;
   if (i < mbs) mv_host[i] = mv[i];
   if (i == 0) {
@@ -94,7 +96,7 @@ int upload_nv12_launch(const uint8_t* y, int y_pitch, const uint8_t* uv, int uv_
 
 int stage_mv_launch(const void* mv, void* mv_host, int mbs, const uint32_t* s0, const uint32_t* s1,
                     uint32_t* status_host, cudaStream_t st) {
-  stage_mv_kernel<<<(mbs + 255) / 256, 256, 0, st>>>(static_cast<const uint4*>(mv), static_cast<uint4*>(mv_host), mbs, s0,
-                                                     s1, status_host);
+  launch_early(stage_mv_kernel, (mbs + 255) / 256, 256, 0, st, static_cast<const uint4*>(mv), static_cast<uint4*>(mv_host),
+               mbs, s0, s1, status_host);
   return cudaGetLastError() == cudaSuccess ? 0 : -1;
 }
