@@ -78,6 +78,7 @@ __device__ __forceinline__ int hdequant(int c, int q, int bd_shift) {
 // ---- 4x4 -------------------------------------------------------------------
 __global__ void hevc_tq4_kernel(const int16_t* __restrict__ res, int16_t* __restrict__ out, int n, int q, int use_dst,
                                 int round_q12, int s1, int qshift) {
+  pdl_wait();
   const int b = blockIdx.x * blockDim.x + threadIdx.x;
   if (b >= n) return;
   const int16_t(*M)[4] = use_dst ? kHDst4 : kHDct4;
@@ -125,6 +126,7 @@ __global__ void hevc_tq4_kernel(const int16_t* __restrict__ res, int16_t* __rest
 
 __global__ void hevc_dqit4_kernel(const int16_t* __restrict__ coeff, int16_t* __restrict__ out, int n, int q,
                                   int use_dst, int bd_shift, int s2) {
+  pdl_wait();
   const int b = blockIdx.x * blockDim.x + threadIdx.x;
   if (b >= n) return;
   const int16_t(*M)[4] = use_dst ? kHDst4 : kHDct4;
@@ -165,6 +167,7 @@ __global__ void hevc_dqit4_kernel(const int16_t* __restrict__ coeff, int16_t* __
 // ---- 8x8 -------------------------------------------------------------------
 __global__ void __launch_bounds__(128) hevc_tq8_kernel(const int16_t* __restrict__ res, int16_t* __restrict__ out,
                                                        int n, int q, int round_q12, int s1, int qshift) {
+  pdl_wait();
   const int b = blockIdx.x * blockDim.x + threadIdx.x;
   if (b >= n) return;
   int x[64];
@@ -215,6 +218,7 @@ __global__ void __launch_bounds__(128) hevc_tq8_kernel(const int16_t* __restrict
 
 __global__ void __launch_bounds__(128) hevc_dqit8_kernel(const int16_t* __restrict__ coeff, int16_t* __restrict__ out,
                                                          int n, int q, int bd_shift, int s2) {
+  pdl_wait();
   const int b = blockIdx.x * blockDim.x + threadIdx.x;
   if (b >= n) return;
   int d[64];
@@ -341,6 +345,7 @@ __global__ void __launch_bounds__(128) hevc_hpel_kernel(const P* __restrict__ re
                                                         P* __restrict__ pI, P* __restrict__ pH, P* __restrict__ pV,
                                                         P* __restrict__ pHV, int opitch, int rows, int cols, int maxv,
                                                         int vec) {
+  pdl_wait();
   constexpr int kQuads = kHpTileW / 4 + 2;
   __shared__ Quad<P> src[kHpTileH + 7][kQuads];
   const int tx = threadIdx.x & 31, ty = threadIdx.x >> 5;
@@ -525,6 +530,7 @@ template <typename P>
 __global__ void __launch_bounds__(128) hevc_me_kernel(const __grid_constant__ HevcSearch<P> S,
                                                       const b200enc_hevc_me_job_t* __restrict__ jobs, int n,
                                                       b200enc_hevc_me_result_t* __restrict__ out) {
+  pdl_wait();
   const int lane = threadIdx.x & 31, first = lane & 16, cand = (lane >> 2) & 3, row = lane & 3;
   const int j = blockIdx.x * 8 + (threadIdx.x >> 4);
   if (j - (first >> 4) >= n) return;  // neither half has a job
@@ -705,6 +711,7 @@ template <typename P>
 __global__ void hevc_intra4_kernel(const P* __restrict__ src, int src_pitch, const P* __restrict__ rec,
                                    int rec_pitch, int width, int height, const int* __restrict__ jobs, int n,
                                    int* __restrict__ modes, P* __restrict__ preds, int bd) {
+  pdl_wait();
   const int maxv = (1 << bd) - 1;
   const int j = blockIdx.x * blockDim.x + threadIdx.x;
   if (j >= n) return;
@@ -820,9 +827,8 @@ int b200enc_hevc_transform_quant_4x4(const int16_t* residual, int16_t* coeff, in
   if (!aligned16(residual) || !aligned16(coeff) || round_q12 < 0 || round_q12 > 12) return -1;
   if (n == 0) return 0;
   const int q = bit_depth == 8 ? hclamp(qp, 0, 51) : hclamp(qp, 0, 63);
-  hevc_tq4_kernel<<<(n + 255) / 256, 256, 0, (cudaStream_t)stream>>>(residual, coeff, n, q, use_dst ? 1 : 0,
-                                                                       round_q12, bit_depth == 8 ? 1 : 3,
-                                                                       bit_depth == 8 ? 5 : 7);
+  launch_early(hevc_tq4_kernel, (n + 255) / 256, 256, 0, (cudaStream_t)stream, residual, coeff, n, q, use_dst ? 1 : 0,
+               round_q12, bit_depth == 8 ? 1 : 3, bit_depth == 8 ? 5 : 7);
   return cudaGetLastError() == cudaSuccess ? 0 : -1;
 }
 
@@ -834,9 +840,8 @@ int b200enc_hevc_dequant_itransform_4x4(const int16_t* coeff, int16_t* residual,
   if (bit_depth == 8 && (qp < 0 || qp > 51)) return -1;
   if (n == 0) return 0;
   const int q = bit_depth == 8 ? qp : hclamp(qp, 0, 63);
-  hevc_dqit4_kernel<<<(n + 255) / 256, 256, 0, (cudaStream_t)stream>>>(coeff, residual, n, q, use_dst ? 1 : 0,
-                                                                         bit_depth == 8 ? 5 : 7,
-                                                                         bit_depth == 8 ? 12 : 10);
+  launch_early(hevc_dqit4_kernel, (n + 255) / 256, 256, 0, (cudaStream_t)stream, coeff, residual, n, q, use_dst ? 1 : 0,
+               bit_depth == 8 ? 5 : 7, bit_depth == 8 ? 12 : 10);
   return cudaGetLastError() == cudaSuccess ? 0 : -1;
 }
 
@@ -845,8 +850,8 @@ int b200enc_hevc_transform_quant_8x8(const int16_t* residual, int16_t* coeff, in
   if (!residual || !coeff || n < 0 || (bit_depth != 8 && bit_depth != 10)) return -1;
   if (!aligned16(residual) || !aligned16(coeff) || round_q12 < 0 || round_q12 > 12) return -1;
   if (n == 0) return 0;
-  hevc_tq8_kernel<<<(n + 127) / 128, 128, 0, (cudaStream_t)stream>>>(residual, coeff, n, hclamp(qp, 0, 63),
-                                                                       round_q12, 3 + bit_depth - 9, bit_depth - 2);
+  launch_early(hevc_tq8_kernel, (n + 127) / 128, 128, 0, (cudaStream_t)stream, residual, coeff, n, hclamp(qp, 0, 63),
+               round_q12, 3 + bit_depth - 9, bit_depth - 2);
   return cudaGetLastError() == cudaSuccess ? 0 : -1;
 }
 
@@ -855,8 +860,8 @@ int b200enc_hevc_dequant_itransform_8x8(const int16_t* coeff, int16_t* residual,
   if (!residual || !coeff || n < 0 || (bit_depth != 8 && bit_depth != 10)) return -1;
   if (!aligned16(residual) || !aligned16(coeff)) return -1;
   if (n == 0) return 0;
-  hevc_dqit8_kernel<<<(n + 127) / 128, 128, 0, (cudaStream_t)stream>>>(coeff, residual, n, hclamp(qp, 0, 63),
-                                                                         bit_depth - 2, 20 - bit_depth);
+  launch_early(hevc_dqit8_kernel, (n + 127) / 128, 128, 0, (cudaStream_t)stream, coeff, residual, n, hclamp(qp, 0, 63),
+               bit_depth - 2, 20 - bit_depth);
   return cudaGetLastError() == cudaSuccess ? 0 : -1;
 }
 
@@ -867,9 +872,9 @@ int b200enc_hevc_build_hpel(const uint8_t* recon, int pitch, int w, int h, int m
   const int rows = h + 2 * margin, cols = w + 2 * margin;
   if (plane_pitch < cols) return -1;
   dim3 grid((cols + kHpTileW - 1) / kHpTileW, (rows + kHpTileH - 1) / kHpTileH);
-  hevc_hpel_kernel<uint8_t><<<grid, 128, 0, (cudaStream_t)stream>>>(
-      recon, pitch, w, h, margin, plane_i, plane_h, plane_v, plane_hv, plane_pitch, rows, cols, 255,
-      quad_aligned(plane_i, plane_h, plane_v, plane_hv, plane_pitch));
+  launch_early(hevc_hpel_kernel<uint8_t>, grid, 128, 0, (cudaStream_t)stream, recon, pitch, w, h, margin, plane_i,
+               plane_h, plane_v, plane_hv, plane_pitch, rows, cols, 255, quad_aligned(plane_i, plane_h, plane_v,
+               plane_hv, plane_pitch));
   return cudaGetLastError() == cudaSuccess ? 0 : -1;
 }
 
@@ -881,9 +886,9 @@ int b200enc_hevc_build_hpel_10(const uint16_t* recon, int pitch, int w, int h, i
   const int rows = h + 2 * margin, cols = w + 2 * margin;
   if (plane_pitch < cols) return -1;
   dim3 grid((cols + kHpTileW - 1) / kHpTileW, (rows + kHpTileH - 1) / kHpTileH);
-  hevc_hpel_kernel<uint16_t><<<grid, 128, 0, (cudaStream_t)stream>>>(
-      recon, pitch, w, h, margin, plane_i, plane_h, plane_v, plane_hv, plane_pitch, rows, cols, 1023,
-      quad_aligned(plane_i, plane_h, plane_v, plane_hv, plane_pitch));
+  launch_early(hevc_hpel_kernel<uint16_t>, grid, 128, 0, (cudaStream_t)stream, recon, pitch, w, h, margin, plane_i,
+               plane_h, plane_v, plane_hv, plane_pitch, rows, cols, 1023, quad_aligned(plane_i, plane_h, plane_v,
+               plane_hv, plane_pitch));
   return cudaGetLastError() == cudaSuccess ? 0 : -1;
 }
 
@@ -896,7 +901,7 @@ int b200enc_hevc_motion_search(const uint8_t* src_y, int src_pitch, int w, int h
   if (n == 0) return 0;
   HevcSearch<uint8_t> S{src_y, src_pitch, w, h, margin, qpel ? 1 : 0, {plane_i, plane_h, plane_v, plane_hv},
                         plane_pitch, 0};
-  hevc_me_kernel<uint8_t><<<(unsigned)(n / 8 + 1), 128, 0, (cudaStream_t)stream>>>(S, jobs, n, results);
+  launch_early(hevc_me_kernel<uint8_t>, (unsigned)(n / 8 + 1), 128, 0, (cudaStream_t)stream, S, jobs, n, results);
   return cudaGetLastError() == cudaSuccess ? 0 : -1;
 }
 
@@ -909,7 +914,7 @@ int b200enc_hevc_motion_search_10(const uint16_t* src_y, int src_pitch, int w, i
   if (n == 0) return 0;
   HevcSearch<uint16_t> S{src_y, src_pitch, w, h, margin, qpel ? 1 : 0, {plane_i, plane_h, plane_v, plane_hv},
                          plane_pitch, 2};
-  hevc_me_kernel<uint16_t><<<(unsigned)(n / 8 + 1), 128, 0, (cudaStream_t)stream>>>(S, jobs, n, results);
+  launch_early(hevc_me_kernel<uint16_t>, (unsigned)(n / 8 + 1), 128, 0, (cudaStream_t)stream, S, jobs, n, results);
   return cudaGetLastError() == cudaSuccess ? 0 : -1;
 }
 
@@ -919,8 +924,8 @@ int b200enc_hevc_choose_luma_mode(const uint8_t* src_y, int src_pitch, const uin
   if (!src_y || !recon_y || !jobs || !modes || !preds || n < 0 || width < 4 || height < 4) return -1;
   if (!aligned16(preds) || src_pitch < width || recon_pitch < width) return -1;
   if (n == 0) return 0;
-  hevc_intra4_kernel<uint8_t><<<(n + 127) / 128, 128, 0, (cudaStream_t)stream>>>(
-      src_y, src_pitch, recon_y, recon_pitch, width, height, jobs, n, modes, preds, 8);
+  launch_early(hevc_intra4_kernel<uint8_t>, (n + 127) / 128, 128, 0, (cudaStream_t)stream, src_y, src_pitch, recon_y,
+               recon_pitch, width, height, jobs, n, modes, preds, 8);
   return cudaGetLastError() == cudaSuccess ? 0 : -1;
 }
 
@@ -930,8 +935,8 @@ int b200enc_hevc_choose_luma_mode_10(const uint16_t* src_y, int src_pitch, const
   if (!src_y || !recon_y || !jobs || !modes || !preds || n < 0 || width < 4 || height < 4) return -1;
   if (!aligned16(preds) || src_pitch < width || recon_pitch < width) return -1;
   if (n == 0) return 0;
-  hevc_intra4_kernel<uint16_t><<<(n + 127) / 128, 128, 0, (cudaStream_t)stream>>>(
-      src_y, src_pitch, recon_y, recon_pitch, width, height, jobs, n, modes, preds, 10);
+  launch_early(hevc_intra4_kernel<uint16_t>, (n + 127) / 128, 128, 0, (cudaStream_t)stream, src_y, src_pitch, recon_y,
+               recon_pitch, width, height, jobs, n, modes, preds, 10);
   return cudaGetLastError() == cudaSuccess ? 0 : -1;
 }
 

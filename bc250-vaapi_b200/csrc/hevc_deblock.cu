@@ -32,6 +32,7 @@
 #include <type_traits>
 
 #include "b200enc_internal.h"
+#include "common.cuh"
 
 // The layouts the Python bindings mirror (b200enc/__init__.py).
 static_assert(sizeof(b200enc_hevc_mvf_t) == 20, "mvf record");
@@ -253,6 +254,7 @@ __device__ __forceinline__ int hdb_tc_chroma(const b200enc_hevc_deblock_t& p, co
 // lane (hevc_filter_template.c:298-335). VEC: see hdb_luma_line.
 template <typename T, bool VERT, bool VEC>
 __global__ void __launch_bounds__(kHdbThreads) hevc_deblock_kernel(const __grid_constant__ b200enc_hevc_deblock_t p) {
+  pdl_wait();
   const int per_row = VERT ? p.width >> 3 : p.width >> 2, rows = VERT ? p.height >> 2 : p.height >> 3;
   const int lane = threadIdx.x & 31;
   // ---- this lane's segment: its origin and what its lines need
@@ -310,10 +312,10 @@ static void hdb_launch(const b200enc_hevc_deblock_t& q, cudaStream_t st) {
   // four samples before and behind an edge start at a multiple of four of the row
   const bool vec = (reinterpret_cast<uintptr_t>(q.plane[0]) | (uintptr_t)q.stride[0] * sizeof(T)) % (4 * sizeof(T)) == 0;
   if (vec)
-    hevc_deblock_kernel<T, true, true><<<gv, kHdbThreads, 0, st>>>(q);
+    launch_early(hevc_deblock_kernel<T, true, true>, gv, kHdbThreads, 0, st, q);
   else
-    hevc_deblock_kernel<T, true, false><<<gv, kHdbThreads, 0, st>>>(q);
-  hevc_deblock_kernel<T, false, false><<<gh, kHdbThreads, 0, st>>>(q);
+    launch_early(hevc_deblock_kernel<T, true, false>, gv, kHdbThreads, 0, st, q);
+  launch_early(hevc_deblock_kernel<T, false, false>, gh, kHdbThreads, 0, st, q);
 }
 
 }  // namespace b200enc

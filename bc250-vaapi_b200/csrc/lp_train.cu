@@ -76,6 +76,7 @@ __global__ void __launch_bounds__(128) lp_row_gemm(int M, const __nv_bfloat16* _
                                                    const __nv_bfloat16* __restrict__ W, const float* __restrict__ bias,
                                                    const __nv_bfloat16* __restrict__ mask, int ldm,
                                                    void* __restrict__ C, int ldc, uint32_t* __restrict__ err) {
+  pdl_wait();
   using S = RowShared<K, N, EPI>;
   constexpr int KP = S::KP, NB = N < 32 ? 32 : N, KU = K / 8;  // KU: 16-byte units of a row
   constexpr uint32_t kCols = NB <= 32 ? 32 : (NB <= 64 ? 64 : 128);
@@ -210,6 +211,7 @@ template <int IN, int OUT>
 __global__ void __launch_bounds__(128) lp_wgrad(int rows, const __nv_bfloat16* __restrict__ G,
                                                 const __nv_bfloat16* __restrict__ A, int lda, float* __restrict__ gW,
                                                 float* __restrict__ gb, uint32_t* __restrict__ err) {
+  pdl_wait();
   using S = WgShared<IN, OUT>;
   constexpr int NB = OUT < 32 ? 32 : OUT, AU = IN / 8, BU = OUT / 8, kSumT = 128 / BU;
   constexpr uint32_t kCols = NB <= 32 ? 32 : 64;
@@ -337,8 +339,8 @@ int row_gemm(long long M, const __nv_bfloat16* A, int lda, const __nv_bfloat16* 
   if (cudaFuncSetAttribute(k, cudaFuncAttributeMaxDynamicSharedMemorySize, smem) != cudaSuccess) return -1;
   const int per_sm = std::max(1, std::min(N > 64 ? 4 : 6, 220 * 1024 / (smem + 1024)));
   const long long tiles = (M + 127) / 128;
-  k<<<(unsigned)std::min<long long>(tiles, (long long)per_sm * sm_count()), 128, smem, st>>>((int)M, A, lda, W, bias, mask, ldm,
-                                                                                          C, ldc, err);
+  launch_early(k, (unsigned)std::min<long long>(tiles, (long long)per_sm * sm_count()), 128, smem, st, (int)M, A, lda, W, bias,
+               mask, ldm, C, ldc, err);
   return cudaGetLastError() == cudaSuccess ? 0 : -1;
 }
 
@@ -351,7 +353,7 @@ int wgrad(long long rows, const __nv_bfloat16* G, const __nv_bfloat16* A, int ld
   const long long chunks = (rows + kWgRows - 1) / kWgRows;
   // two CTAs per SM; a CTA's share at least four chunks (its FP32 atomics cost as much as loading them)
   const long long ctas = std::max<long long>(1, std::min<long long>(2ll * sm_count(), chunks / 4));
-  k<<<(unsigned)ctas, 128, smem, st>>>((int)rows, G, A, lda, gW, gb, err);
+  launch_early(k, (unsigned)ctas, 128, smem, st, (int)rows, G, A, lda, gW, gb, err);
   return cudaGetLastError() == cudaSuccess ? 0 : -1;
 }
 

@@ -497,6 +497,7 @@ __global__ void __launch_bounds__(128, 9) lp_rescore_kernel(const uint8_t* __res
 // is 1 iff all 24 nz words of the plain encode are 0.
 __global__ void lp_label_kernel(int mbs, LpBuf b, const MV* __restrict__ logged, const uint32_t* __restrict__ nz,
                                 int* __restrict__ label, float* __restrict__ norez, float* __restrict__ weight) {
+  pdl_wait();
   const int mb = blockIdx.x * blockDim.x + threadIdx.x;
   if (mb >= mbs) return;
   const uint32_t st = b.state[mb];
@@ -579,6 +580,7 @@ __global__ void lp_loss_kernel(int mbs, LpBuf b, const int* __restrict__ label, 
 __global__ void lp_adam_kernel(int n, float* __restrict__ p, const float* __restrict__ g, float* __restrict__ m,
                                float* __restrict__ v, __nv_bfloat16* __restrict__ pb, float lr_t, float b1, float b2,
                                float eps) {
+  pdl_wait();
   const int i = blockIdx.x * blockDim.x + threadIdx.x;
   if (i >= n) return;
   const float gi = g[i];
@@ -819,8 +821,8 @@ int b200enc_proposal_labels(void* h, int mbs, const void* logged_mv, const uint3
   Proposal* P = static_cast<Proposal*>(h);
   if (!P || mbs <= 0 || mbs > P->max_mbs || !logged_mv || !P->init_train()) return -1;
   cudaStream_t st = (cudaStream_t)stream;
-  lp_label_kernel<<<(mbs + 127) / 128, 128, 0, st>>>(mbs, P->b, (const MV*)logged_mv, nz, P->label, P->norez,
-                                                     P->weight);
+  launch_early(lp_label_kernel, (mbs + 127) / 128, 128, 0, st, mbs, P->b, (const MV*)logged_mv, nz, P->label, P->norez,
+               P->weight);
   return cudaGetLastError() == cudaSuccess ? 0 : -1;
 }
 
@@ -836,8 +838,8 @@ int b200enc_proposal_adam(void* h, float lr, float beta1, float beta2, float eps
   const double c1 = 1.0 - std::pow((double)beta1, step), c2 = 1.0 - std::pow((double)beta2, step);
   const float lr_t = (float)(lr * std::sqrt(c2) / c1);
   P->w8_stale = true;
-  lp_adam_kernel<<<(kParams + 255) / 256, 256, 0, (cudaStream_t)stream>>>(kParams, P->params, P->grads, P->adam_m,
-                                                                         P->adam_v, P->wb, lr_t, beta1, beta2, eps);
+  launch_early(lp_adam_kernel, (kParams + 255) / 256, 256, 0, (cudaStream_t)stream, kParams, P->params, P->grads,
+               P->adam_m, P->adam_v, P->wb, lr_t, beta1, beta2, eps);
   return cudaGetLastError() == cudaSuccess ? 0 : -1;
 }
 
