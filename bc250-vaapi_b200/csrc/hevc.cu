@@ -31,10 +31,6 @@ namespace b200enc {
 // uses the same values).
 __constant__ int16_t kHDct4[4][4] = {{64, 64, 64, 64}, {83, 36, -36, -83}, {64, -64, -64, 64}, {36, -83, 83, -36}};
 __constant__ int16_t kHDst4[4][4] = {{29, 55, 74, 84}, {74, 74, 0, -74}, {84, -29, -74, 55}, {55, -84, 74, -29}};
-__constant__ int16_t kHDct8[8][8] = {{64, 64, 64, 64, 64, 64, 64, 64},     {89, 75, 50, 18, -18, -50, -75, -89},
-                                     {83, 36, -36, -83, -83, -36, 36, 83}, {75, -18, -89, -50, 50, 89, 18, -75},
-                                     {64, -64, -64, 64, 64, -64, -64, 64}, {50, -89, 18, 75, -75, -18, 89, -50},
-                                     {36, -83, 83, -36, -36, 83, -83, 36}, {18, -50, 75, -89, 89, -75, 50, -18}};
 __constant__ int kHLevelScale[6] = {40, 45, 51, 57, 64, 72};
 
 __device__ __forceinline__ int sat16(int v) { return v > 32767 ? 32767 : (v < -32768 ? -32768 : v); }
@@ -165,97 +161,107 @@ __global__ void hevc_dqit4_kernel(const int16_t* __restrict__ coeff, int16_t* __
 }
 
 // ---- 8x8 -------------------------------------------------------------------
-__global__ void __launch_bounds__(128) hevc_tq8_kernel(const int16_t* __restrict__ res, int16_t* __restrict__ out,
-                                                       int n, int q, int round_q12, int s1, int qshift) {
-  pdl_wait();
-  const int b = blockIdx.x * blockDim.x + threadIdx.x;
-  if (b >= n) return;
-  int x[64];
-  const int4* src = reinterpret_cast<const int4*>(res + (size_t)b * 64);
-  int any = 0;
+// Eight lanes per block: lane r loads row r (16 bytes; a warp's four blocks lie
+// together), the column pass follows a transpose across the lanes and the row pass
+// another, both as integer dot products of value pairs (the matrix fits in bytes).
+// 32,400 blocks 5.4 us, inverse 3.6; a thread per block, 128 bytes apart, 7.6 and
+// 6.9 (8.3 MB moved, 1.3 us).
+//
+// Entry (i, k) of the 8-point matrix: the standard's integer for
+// cos(i (2k + 1) pi / 16), which takes eight values and their negatives.
+__host__ __device__ constexpr int hdct8(int i, int k) {
+  const int turn = i * (2 * k + 1) % 32, half = turn > 16 ? 32 - turn : turn, a = half > 8 ? 16 - half : half;
+  const int c = a == 0 ? 64 : a == 1 ? 89 : a == 2 ? 83 : a == 3 ? 75 : a == 4 ? 64 : a == 5 ? 50 : a == 6 ? 36 : a == 7 ? 18 : 0;
+  return half > 8 ? -c : c;
+}
+__device__ __forceinline__ uint32_t pack_sat16(int lo, int hi) {
+  uint32_t d;
+  asm("cvt.pack.sat.s16.s32 %0, %1, %2;" : "=r"(d) : "r"(hi), "r"(lo));
+  return d;
+}
+// 8x8 transpose of 16-bit values over eight lanes: row r in, column r out, both
+// as pairs (0, 1), (2, 3), ...
+__device__ __forceinline__ void transpose8(uint32_t (&w)[4], int r) {
+  const bool odd = r & 1, b1 = r & 2, b2 = r & 4;
+#pragma unroll
+  for (int k = 0; k < 4; ++k) {  // two rows' values of one column to a word
+    const uint32_t o = __shfl_xor_sync(0xffffffffu, w[k], 1);
+    w[k] = __byte_perm(w[k], o, odd ? 0x3276 : 0x5410);
+  }
+#pragma unroll
+  for (int k = 0; k < 2; ++k) {  // a 4x4 transpose of those words over the row pairs
+    const uint32_t o = __shfl_xor_sync(0xffffffffu, b2 ? w[k] : w[k + 2], 4);
+    (b2 ? w[k] : w[k + 2]) = o;
+  }
+#pragma unroll
+  for (int k = 0; k < 4; k += 2) {
+    const uint32_t o = __shfl_xor_sync(0xffffffffu, b1 ? w[k] : w[k + 1], 2);
+    (b1 ? w[k] : w[k + 1]) = o;
+  }
+}
+// One pass over a lane's eight values: o[i] = (sum_k M[i][k] v[k] + round) >> shift,
+// M the matrix (FWD) or its transpose.
+template <bool FWD>
+__device__ __forceinline__ void dct8_pass(const uint32_t (&w)[4], int round, int shift, int (&o)[8]) {
 #pragma unroll
   for (int i = 0; i < 8; ++i) {
-    const int4 v = src[i];
-    any |= v.x | v.y | v.z | v.w;
-    const int w[4] = {v.x, v.y, v.z, v.w};
+    int s = round;
 #pragma unroll
     for (int k = 0; k < 4; ++k) {
-      x[8 * i + 2 * k] = (int)(int16_t)(w[k] & 0xffff);
-      x[8 * i + 2 * k + 1] = (int)(int16_t)((uint32_t)w[k] >> 16);
+      const int c0 = FWD ? hdct8(i, 2 * k) : hdct8(2 * k, i);
+      const int c1 = FWD ? hdct8(i, 2 * k + 1) : hdct8(2 * k + 1, i);
+      s = __dp2a_lo((int)w[k], (c0 & 0xff) | (c1 & 0xff) << 8, s);
     }
-  }
-  if (!any) {  // as for 4x4: an all-zero block gives all-zero levels
-    int4* dst = reinterpret_cast<int4*>(out + (size_t)b * 64);
-#pragma unroll
-    for (int i = 0; i < 8; ++i) dst[i] = make_int4(0, 0, 0, 0);
-    return;
-  }
-  int t[64];  // t[i*8+c]: column c, frequency i
-#pragma unroll
-  for (int i = 0; i < 8; ++i)
-#pragma unroll
-    for (int c = 0; c < 8; ++c) {
-      int s = 0;
-#pragma unroll
-      for (int r = 0; r < 8; ++r) s += kHDct8[i][r] * x[r * 8 + c];
-      t[i * 8 + c] = sat16((s + (1 << (s1 - 1))) >> s1);
-    }
-  const HQuant h = hquant(q, qshift, round_q12);
-  int4* dst = reinterpret_cast<int4*>(out + (size_t)b * 64);
-#pragma unroll
-  for (int i = 0; i < 8; ++i) {
-    __align__(16) int16_t o[8];
-#pragma unroll
-    for (int j = 0; j < 8; ++j) {
-      int s = 0;
-#pragma unroll
-      for (int c = 0; c < 8; ++c) s += kHDct8[j][c] * t[i * 8 + c];
-      o[j] = hquant_level(sat16((s + 256) >> 9), h);
-    }
-    dst[i] = *reinterpret_cast<const int4*>(o);
+    o[i] = s >> shift;
   }
 }
 
-__global__ void __launch_bounds__(128) hevc_dqit8_kernel(const int16_t* __restrict__ coeff, int16_t* __restrict__ out,
+__global__ void __launch_bounds__(256) hevc_tq8_kernel(const int16_t* __restrict__ res, int16_t* __restrict__ out,
+                                                       int n, int q, int round_q12, int s1, int qshift) {
+  pdl_wait();
+  const long long row = (long long)blockIdx.x * blockDim.x + threadIdx.x;  // of all blocks
+  const int r = threadIdx.x & 7;
+  const bool in = row < (long long)n * 8;
+  const uint4 v = in ? __ldg(reinterpret_cast<const uint4*>(res) + row) : make_uint4(0u, 0u, 0u, 0u);
+  uint32_t w[4] = {v.x, v.y, v.z, v.w};
+  // as for 4x4: an all-zero block gives all-zero levels
+  const uint32_t any = __ballot_sync(0xffffffffu, (v.x | v.y | v.z | v.w) != 0u) >> (threadIdx.x & 24) & 0xffu;
+  int o[8];
+  transpose8(w, r);
+  dct8_pass<true>(w, 1 << (s1 - 1), s1, o);
+#pragma unroll
+  for (int k = 0; k < 4; ++k) w[k] = pack_sat16(o[2 * k], o[2 * k + 1]);
+  transpose8(w, r);
+  dct8_pass<true>(w, 256, 9, o);
+  const HQuant h = hquant(q, qshift, round_q12);
+#pragma unroll
+  for (int k = 0; k < 4; ++k)
+    w[k] = any ? (uint32_t)(uint16_t)hquant_level(sat16(o[2 * k]), h) | (uint32_t)(uint16_t)hquant_level(sat16(o[2 * k + 1]), h) << 16
+               : 0u;
+  if (in) reinterpret_cast<uint4*>(out)[row] = make_uint4(w[0], w[1], w[2], w[3]);
+}
+
+__global__ void __launch_bounds__(256) hevc_dqit8_kernel(const int16_t* __restrict__ coeff, int16_t* __restrict__ out,
                                                          int n, int q, int bd_shift, int s2) {
   pdl_wait();
-  const int b = blockIdx.x * blockDim.x + threadIdx.x;
-  if (b >= n) return;
-  int d[64];
-  const int4* src = reinterpret_cast<const int4*>(coeff + (size_t)b * 64);
+  const long long row = (long long)blockIdx.x * blockDim.x + threadIdx.x;
+  const int r = threadIdx.x & 7;
+  const bool in = row < (long long)n * 8;
+  const uint4 v = in ? __ldg(reinterpret_cast<const uint4*>(coeff) + row) : make_uint4(0u, 0u, 0u, 0u);
+  uint32_t w[4] = {v.x, v.y, v.z, v.w};
 #pragma unroll
-  for (int i = 0; i < 8; ++i) {
-    const int4 v = src[i];
-    const int w[4] = {v.x, v.y, v.z, v.w};
+  for (int k = 0; k < 4; ++k)
+    w[k] = pack_sat16(hdequant((int)(int16_t)(w[k] & 0xffffu), q, bd_shift), hdequant((int)w[k] >> 16, q, bd_shift));
+  int o[8];
+  transpose8(w, r);
+  dct8_pass<false>(w, 64, 7, o);
 #pragma unroll
-    for (int k = 0; k < 4; ++k) {
-      d[8 * i + 2 * k] = hdequant((int)(int16_t)(w[k] & 0xffff), q, bd_shift);
-      d[8 * i + 2 * k + 1] = hdequant((int)(int16_t)((uint32_t)w[k] >> 16), q, bd_shift);
-    }
-  }
-  int g[64];  // g[r*8+c]
-#pragma unroll
-  for (int r = 0; r < 8; ++r)
-#pragma unroll
-    for (int c = 0; c < 8; ++c) {
-      int s = 0;
-#pragma unroll
-      for (int k = 0; k < 8; ++k) s += kHDct8[k][r] * d[k * 8 + c];
-      g[r * 8 + c] = sat16((s + 64) >> 7);
-    }
-  int4* dst = reinterpret_cast<int4*>(out + (size_t)b * 64);
-#pragma unroll
-  for (int r = 0; r < 8; ++r) {
-    __align__(16) int16_t o[8];
-#pragma unroll
-    for (int c = 0; c < 8; ++c) {
-      int s = 0;
-#pragma unroll
-      for (int k = 0; k < 8; ++k) s += kHDct8[k][c] * g[r * 8 + k];
-      o[c] = (int16_t)sat16((s + (1 << (s2 - 1))) >> s2);
-    }
-    dst[r] = *reinterpret_cast<const int4*>(o);
-  }
+  for (int k = 0; k < 4; ++k) w[k] = pack_sat16(o[2 * k], o[2 * k + 1]);
+  transpose8(w, r);
+  dct8_pass<false>(w, 1 << (s2 - 1), s2, o);
+  if (in)
+    reinterpret_cast<uint4*>(out)[row] =
+        make_uint4(pack_sat16(o[0], o[1]), pack_sat16(o[2], o[3]), pack_sat16(o[4], o[5]), pack_sat16(o[6], o[7]));
 }
 
 // ---- half-sample planes ----------------------------------------------------
@@ -850,7 +856,7 @@ int b200enc_hevc_transform_quant_8x8(const int16_t* residual, int16_t* coeff, in
   if (!residual || !coeff || n < 0 || (bit_depth != 8 && bit_depth != 10)) return -1;
   if (!aligned16(residual) || !aligned16(coeff) || round_q12 < 0 || round_q12 > 12) return -1;
   if (n == 0) return 0;
-  launch_early(hevc_tq8_kernel, (n + 127) / 128, 128, 0, (cudaStream_t)stream, residual, coeff, n, hclamp(qp, 0, 63),
+  launch_early(hevc_tq8_kernel, (unsigned)((n + 31ll) / 32), 256, 0, (cudaStream_t)stream, residual, coeff, n, hclamp(qp, 0, 63),
                round_q12, 3 + bit_depth - 9, bit_depth - 2);
   return cudaGetLastError() == cudaSuccess ? 0 : -1;
 }
@@ -860,7 +866,7 @@ int b200enc_hevc_dequant_itransform_8x8(const int16_t* coeff, int16_t* residual,
   if (!residual || !coeff || n < 0 || (bit_depth != 8 && bit_depth != 10)) return -1;
   if (!aligned16(residual) || !aligned16(coeff)) return -1;
   if (n == 0) return 0;
-  launch_early(hevc_dqit8_kernel, (n + 127) / 128, 128, 0, (cudaStream_t)stream, coeff, residual, n, hclamp(qp, 0, 63),
+  launch_early(hevc_dqit8_kernel, (unsigned)((n + 31ll) / 32), 256, 0, (cudaStream_t)stream, coeff, residual, n, hclamp(qp, 0, 63),
                bit_depth - 2, 20 - bit_depth);
   return cudaGetLastError() == cudaSuccess ? 0 : -1;
 }
