@@ -80,15 +80,32 @@ __device__ uint32_t g_me_wait_err;
 template <int R>
 constexpr int kMeCtas = R == 32 ? 15 : 30;
 
-template <int R, int MODE>
-__global__ void __launch_bounds__(2 * R, kMeCtas<R>) me_full_search_kernel(const uint8_t* __restrict__ cur_, int cur_pitch_,
+// Threads per macroblock. One per column of the search area (SEG = 1) does the
+// least work, and is what a picture that fills the chip takes; with few macroblocks
+// the chip idles while each is a serial chain, so SEG threads share a column: each
+// bounds its part of the rows (two fills of the rings more), and staging and the
+// exact costs have SEG times the threads. The line lies where both take the same
+// time (us, SEG = 1 / wide): at +-16 99 macroblocks 17.6 / 8.1, 396 17.9 / 11.3, 690
+// 20.1 / 14.5, 1,200 22.1 / 22.0, 1,900 27.6 / 30.0; at +-32 99 21.3 / 13.0, 690
+// 28.2 / 23.6, 2,304 55.2 / 53.1, 3,600 72.2 / 76.1: 8 and 16 macroblocks per SM. A
+// list's length is known on the device only: a learned search leaves a tenth of a
+// frame, beside the re-scoring of the rest (fallback alone / pair: 98 of 1,200
+// macroblocks 18.5 / 9.7 us, 583 of 8,160 pair 36.8 / 33.0, 898 of 14,400 56.6 / 53.3,
+// 2,215 of 32,400 108.9 / 112.0), so its line is 100 per SM. Batches, whose lists hold
+// whole frames without history, keep SEG = 1 (eight mixed streams 4.02 ms, not 4.10).
+template <int R>
+constexpr int kMeSeg = R == 16 ? 4 : 2;
+constexpr int kMeWideList = 100;
+
+template <int R, int MODE, int SEG>
+__global__ void __launch_bounds__(2 * R * SEG, kMeCtas<R> / SEG) me_full_search_kernel(const uint8_t* __restrict__ cur_, int cur_pitch_,
                                                                const uint8_t* __restrict__ ref_, int ref_pitch_,
                                                                Geo g_, int lambda_, int zero_thresh_,
                                                                MV* __restrict__ out_, const int* __restrict__ mb_list,
                                                                const int* __restrict__ mb_count, int flags,
                                                                BatchTab bt, const __grid_constant__ CUtensorMap tmap,
                                                                int use_tma, uint32_t* err) {
-  constexpr int NT = 2 * R;
+  constexpr int NT = 2 * R * SEG, COLS = 2 * R;
   using S = MeShared<R>;
   constexpr int WP = S::WP, WW = S::WW, WS = S::WS, OFF = S::OFF, SIDE = 2 * R + 1;
   constexpr uint64_t kWaitNs = 2000000000ull;
@@ -213,10 +230,12 @@ __global__ void __launch_bounds__(2 * R, kMeCtas<R>) me_full_search_kernel(const
   // difference of their sample sums. Each window row gives the column's two
   // 8-sample sums (packed in halves of a word), a ring keeps the last eight.
   const int lam = lambda;
-  const uint32_t lam_dx = (uint32_t)lam * (uint32_t)abs(tid - R);
-  const uint32_t* wcol = sh.win + 4 * WS + OFF + ((tid + 4) >> 2);  // window row 0 of this thread's column
-  const int wsh = ((tid + 4) & 3) * 8;
-  constexpr int NU = 2 * R / kMeUnit;  // units (runs of kMeUnit candidates) per column
+  const int col = tid & (COLS - 1), seg = tid / COLS;  // this thread's column and share of its rows
+  const uint32_t lam_dx = (uint32_t)lam * (uint32_t)abs(col - R);
+  const uint32_t* wcol = sh.win + 4 * WS + OFF + ((col + 4) >> 2);  // window row 0 of this thread's column
+  const int wsh = ((col + 4) & 3) * 8;
+  constexpr int NU = 2 * R / kMeUnit / SEG;  // units (runs of kMeUnit candidates) of a column per thread
+  const int u0 = seg * NU;
   uint32_t lkey, ckey = 0xffffffffu;   // smallest (bound << 14 | raster index) of the last row, of the column
   {
     uint32_t c00, c01, c10, c11;  // the current macroblock's 8x8 sums
@@ -253,23 +272,23 @@ __global__ void __launch_bounds__(2 * R, kMeCtas<R>) me_full_search_kernel(const
       lb = __usad(rr, c11, __usad(rl, c10, __usad(vr[k], c01, __usad(vl[k], c00, lb))));
       vl[k] = rl;
       vr[k] = rr;
-      return (lb << 14) | (uint32_t)(cy * SIDE + tid);
+      return (lb << 14) | (uint32_t)(cy * SIDE + col);
     };
 #pragma unroll 1
-    for (int u = -2; u < NU; ++u) {
+    for (int u = u0 - 2; u < u0 + NU; ++u) {
       uint32_t m = 0xffffffffu;
 #pragma unroll
       for (int k = 0; k < kMeUnit; ++k) m = min(m, bound(k & 7, u * kMeUnit + k));
-      if (u >= 0) {
-        sh.ubound[u * NT + tid] = (uint16_t)(m >> 15);
+      if (u >= u0) {
+        sh.ubound[u * COLS + col] = (uint16_t)(m >> 15);
         ckey = min(ckey, m);
       }
     }
-    lkey = bound(0, 2 * R);
+    lkey = seg == SEG - 1 ? bound(0, 2 * R) : 0xffffffffu;
     ckey = min(ckey, lkey);
   }
 
-  // 2. An upper bound: the exact costs of the zero vector, of each column's
+  // 2. An upper bound: the exact costs of the zero vector, of each thread's
   // candidate of smallest bound and of the column dx = +R (aligned words).
   auto key_of = [&](uint32_t sad, int cx, int cy) -> uint32_t {
     return ((sad + (uint32_t)(lam * (abs(cx - R) + abs(cy - R)))) << 14) | (uint32_t)(cy * SIDE + cx);
@@ -291,7 +310,8 @@ __global__ void __launch_bounds__(2 * R, kMeCtas<R>) me_full_search_kernel(const
   };
   uint32_t best = key_of(sad0, R, R);
 #pragma unroll 1
-  for (int j = 0; j < 2; ++j) best = min(best, j ? exact(2 * R, tid) : exact(tid, (int)(ckey & 0x3fffu) / SIDE));
+  for (int j = 0; j < (seg == SEG / 2 ? 2 : 1); ++j)
+    best = min(best, j ? exact(2 * R, col) : exact(col, (int)(ckey & 0x3fffu) / SIDE));
   if (tid < 32) {  // the corner (+R, +R): a row per lane
     const uint32_t* rp = sh.win + (4 + 2 * R + (tid & 15)) * WS + OFF + (2 * R + 4) / 4;
     const uint4 c = reinterpret_cast<const uint4*>(sh.cur)[tid & 15];
@@ -310,7 +330,7 @@ __global__ void __launch_bounds__(2 * R, kMeCtas<R>) me_full_search_kernel(const
     uint32_t alive[NU], total = 0;
 #pragma unroll
     for (int u = 0; u < NU; ++u) {
-      alive[u] = __ballot_sync(0xffffffffu, 2u * sh.ubound[u * NT + tid] <= ub);
+      alive[u] = __ballot_sync(0xffffffffu, 2u * sh.ubound[(u0 + u) * COLS + col] <= ub);
       total += (uint32_t)__popc(alive[u]);
     }
     const int lane = lane_id();
@@ -325,17 +345,17 @@ __global__ void __launch_bounds__(2 * R, kMeCtas<R>) me_full_search_kernel(const
     }
 #pragma unroll
     for (int u = 0; u < NU; ++u) {
-      if ((alive[u] >> lane) & 1u) sh.list[base + __popc(alive[u] & ((1u << lane) - 1u))] = (uint16_t)(u * NT + tid);
+      if ((alive[u] >> lane) & 1u) sh.list[base + __popc(alive[u] & ((1u << lane) - 1u))] = (uint16_t)((u0 + u) * COLS + col);
       base += (uint32_t)__popc(alive[u]);
     }
-    if ((lkey >> 14) <= ub) best = min(best, exact(tid, 2 * R));
+    if ((lkey >> 14) <= ub) best = min(best, exact(col, 2 * R));
     if (NT > 32) __syncthreads();
     else __syncwarp();
   }
   const int n_units = (int)sh.nlist;
 #pragma unroll 1
   for (int i = tid; i < n_units; i += NT) {
-    const int e = sh.list[i], cx = e & (NT - 1), cy0 = (e / NT) * kMeUnit;
+    const int e = sh.list[i], cx = e & (COLS - 1), cy0 = (e / COLS) * kMeUnit;
     const uint32_t* up = sh.win + (4 + cy0) * WS + OFF + ((cx + 4) >> 2);
     const int us = ((cx + 4) & 3) * 8;
     uint32_t acc[kMeUnit];
@@ -443,18 +463,26 @@ bool window_map(CUtensorMap* m, const uint8_t* ref, int pitch, int RW, int RH) {
 template <int R>
 void launch_frame(dim3 grid, bool list, const uint8_t* cur_y, int cur_pitch, const uint8_t* ref_y, int ref_pitch,
                   const Geo& g, int lambda, int zero_thresh, MV* out, const int* mb_list, const int* mb_count,
-                  int flags, uint32_t* err, cudaStream_t st) {
+                  int flags, int capacity, int sms, uint32_t* err, cudaStream_t st) {
   CUtensorMap map;
   const int use_tma = window_map<R>(&map, ref_y, ref_pitch, g.RW, g.RH) ? 1 : 0;
   const BatchTab none{};
-  if (list)
-    me_full_search_kernel<R, kMeList><<<grid, 2 * R, 0, st>>>(cur_y, cur_pitch, ref_y, ref_pitch, g, lambda,
-                                                              zero_thresh, out, mb_list, mb_count, flags, none, map,
-                                                              use_tma, err);
-  else
-    me_full_search_kernel<R, kMeGrid><<<grid, 2 * R, 0, st>>>(cur_y, cur_pitch, ref_y, ref_pitch, g, lambda,
-                                                              zero_thresh, out, mb_list, mb_count, flags, none, map,
-                                                              use_tma, err);
+  auto launch = [&](auto k, int threads) {
+    k<<<grid, threads, 0, st>>>(cur_y, cur_pitch, ref_y, ref_pitch, g, lambda, zero_thresh, out, mb_list, mb_count, flags, none,
+                                map, use_tma, err);
+  };
+  constexpr int kSeg = kMeSeg<R>;
+  if (list) {
+    if (capacity <= kMeWideList * sms)
+      launch(me_full_search_kernel<R, kMeList, kSeg>, 2 * R * kSeg);
+    else
+      launch(me_full_search_kernel<R, kMeList, 1>, 2 * R);
+  } else {
+    if (g.mbw * g.mbh <= (R == 16 ? 8 : 16) * sms)
+      launch(me_full_search_kernel<R, kMeGrid, kSeg>, 2 * R * kSeg);
+    else
+      launch(me_full_search_kernel<R, kMeGrid, 1>, 2 * R);
+  }
 }
 
 }  // namespace
@@ -474,7 +502,7 @@ int b200enc_me_full_search_err(const uint8_t* cur_y, int cur_pitch, const uint8_
   Geo g{W, H, RW, RH, (W + 15) / 16, (H + 15) / 16};
   if (mb_list && (list_capacity <= 0 || list_capacity > g.mbw * g.mbh)) return -1;
   int sms = 148, dev = 0;
-  if (mb_list && cudaGetDevice(&dev) == cudaSuccess) cudaDeviceGetAttribute(&sms, cudaDevAttrMultiProcessorCount, dev);
+  if (cudaGetDevice(&dev) == cudaSuccess) cudaDeviceGetAttribute(&sms, cudaDevAttrMultiProcessorCount, dev);
   // list mode: a persistent grid of up to 16 CTAs per SM (or the tuned
   // count) walks the list
   const int per_sm = b200enc_tuned(B200ENC_TUNE_FALLBACK_CTAS_PER_SM) > 0 ? b200enc_tuned(B200ENC_TUNE_FALLBACK_CTAS_PER_SM) : 16;
@@ -483,11 +511,11 @@ int b200enc_me_full_search_err(const uint8_t* cur_y, int cur_pitch, const uint8_
   switch (range) {
     case 16:
       launch_frame<16>(grid, list, cur_y, cur_pitch, ref_y, ref_pitch, g, lambda, zero_thresh, (MV*)mv_out, mb_list,
-                       mb_count, flags, err, st);
+                       mb_count, flags, list_capacity, sms, err, st);
       break;
     case 32:
       launch_frame<32>(grid, list, cur_y, cur_pitch, ref_y, ref_pitch, g, lambda, zero_thresh, (MV*)mv_out, mb_list,
-                       mb_count, flags, err, st);
+                       mb_count, flags, list_capacity, sms, err, st);
       break;
     default:
       return -1;
@@ -531,18 +559,18 @@ int b200enc_me_batch_launch(const BatchTab& bt, int range, const int* list, cons
   switch (range) {
     case 16:
       if (list)
-        me_full_search_kernel<16, kMeBatchList><<<ctas, 32, 0, st>>>(nullptr, 0, nullptr, 0, Geo{}, 0, 0, nullptr,
+        me_full_search_kernel<16, kMeBatchList, 1><<<ctas, 32, 0, st>>>(nullptr, 0, nullptr, 0, Geo{}, 0, 0, nullptr,
                                                                      list, count, 0, bt, none, 0, nullptr);
       else
-        me_full_search_kernel<16, kMeBatch><<<ctas, 32, 0, st>>>(nullptr, 0, nullptr, 0, Geo{}, 0, 0, nullptr, nullptr,
+        me_full_search_kernel<16, kMeBatch, 1><<<ctas, 32, 0, st>>>(nullptr, 0, nullptr, 0, Geo{}, 0, 0, nullptr, nullptr,
                                                                  nullptr, 0, bt, none, 0, nullptr);
       break;
     case 32:
       if (list)
-        me_full_search_kernel<32, kMeBatchList><<<ctas, 64, 0, st>>>(nullptr, 0, nullptr, 0, Geo{}, 0, 0, nullptr,
+        me_full_search_kernel<32, kMeBatchList, 1><<<ctas, 64, 0, st>>>(nullptr, 0, nullptr, 0, Geo{}, 0, 0, nullptr,
                                                                      list, count, 0, bt, none, 0, nullptr);
       else
-        me_full_search_kernel<32, kMeBatch><<<ctas, 64, 0, st>>>(nullptr, 0, nullptr, 0, Geo{}, 0, 0, nullptr, nullptr,
+        me_full_search_kernel<32, kMeBatch, 1><<<ctas, 64, 0, st>>>(nullptr, 0, nullptr, 0, Geo{}, 0, 0, nullptr, nullptr,
                                                                  nullptr, 0, bt, none, 0, nullptr);
       break;
     default:
