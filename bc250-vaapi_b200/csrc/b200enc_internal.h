@@ -36,3 +36,6 @@ int upload_nv12_launch(const uint8_t* y, int y_pitch, const uint8_t* uv, int uv_
                        uint8_t* dst_uv, int dst_pitch, int width, int height, cudaStream_t st);
 int stage_mv_launch(const void* mv, void* mv_host, int mbs, const uint32_t* s0, const uint32_t* s1,
                     uint32_t* status_host, cudaStream_t st);
+// cavlc.cu: b200enc_cavlc_slices, and on the way what stage_mv_launch does
+int cavlc_slices_and_stage(const b200enc_cavlc_t* p, void* mv_host, const uint32_t* s0, const uint32_t* s1,
+                           uint32_t* status_host, cudaStream_t st);

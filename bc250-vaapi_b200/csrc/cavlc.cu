@@ -88,7 +88,16 @@ struct CavlcHdr {
   int len[kCavlcMaxSlices];
 };
 
+// A frame's motion field and status words for the host, stored by the macroblock
+// kernel on its way (mv null: none; s1 null: no such word, 0).
+struct CavlcStage {
+  MV* mv;
+  const uint32_t *s0, *s1;
+  uint32_t* status;
+};
+
 struct CavlcArgs {
+  CavlcStage stage;
   int mbw, mbh, qp, is_intra, ns, quality;
   int t8;  // P macroblocks code their luma with the 8x8 transform (levels in 8x8 raster order)
   const uint8_t* t8f;  // NULL, or per macroblock: 0 = this one codes 4x4 blocks after all
@@ -242,6 +251,10 @@ __global__ void __launch_bounds__(32 * kCavlcMbWarps) cavlc_mb_kernel(CavlcArgs 
   const int mb = blockIdx.x * kCavlcMbWarps + wi;
   const int mbs = a.mbw * a.mbh;
   if (mb >= mbs) return;
+  if (a.stage.mv && lane < 4) {
+    reinterpret_cast<uint32_t*>(a.stage.mv + mb)[lane] = reinterpret_cast<const uint32_t*>(a.mv + mb)[lane];
+    if (mb == 0 && lane < 2) a.stage.status[lane] = lane == 0 ? *a.stage.s0 : (a.stage.s1 ? *a.stage.s1 : 0u);
+  }
   CavlcWarp& sh = shw[wi];
   const int mbx = mb % a.mbw, mby = mb / a.mbw;
   const uint32_t start = slice_start(slice_of(mb, mbs, a.ns), mbs, a.ns);
@@ -775,7 +788,7 @@ extern "C" size_t b200enc_cavlc_scratch_bytes(int mbw, int mbh) {
   return cavlc_layout(mbw, mbh).bytes;
 }
 
-extern "C" int b200enc_cavlc_slices(const b200enc_cavlc_t* p, void* stream) {
+static int cavlc_launch(const b200enc_cavlc_t* p, const CavlcStage& stage, cudaStream_t st) {
   if (!p || p->mbw <= 0 || p->mbh <= 0 || p->qp < 0 || p->qp > 51 || p->num_slices < 1 ||
       p->num_slices > kCavlcMaxSlices || p->num_slices > p->mbw * p->mbh)
     return -1;
@@ -800,6 +813,7 @@ extern "C" int b200enc_cavlc_slices(const b200enc_cavlc_t* p, void* stream) {
   }
   uint8_t* sc = static_cast<uint8_t*>(p->scratch);
   CavlcArgs a;
+  a.stage = stage;
   a.mbw = p->mbw;
   a.mbh = p->mbh;
   a.qp = p->qp;
@@ -821,7 +835,6 @@ extern "C" int b200enc_cavlc_slices(const b200enc_cavlc_t* p, void* stream) {
   a.slice_cap = (uint32_t)std::min<size_t>(p->slice_cap, 0xfffffffcu);
   a.out_bytes = p->out_bytes;
   a.out_copy = p->out_copy ? p->out_copy : p->out;
-  cudaStream_t st = static_cast<cudaStream_t>(stream);
   const int mbs = p->mbw * p->mbh;
   launch_early(cavlc_mb_kernel, (mbs + kCavlcMbWarps - 1) / kCavlcMbWarps, 32 * kCavlcMbWarps, 0, st, a);
   launch_early(cavlc_slice_kernel, p->num_slices, kCavlcScanThreads, 0, st, a, h);
@@ -830,4 +843,13 @@ extern "C" int b200enc_cavlc_slices(const b200enc_cavlc_t* p, void* stream) {
   const int ctas = std::max(1, std::min(128, mbs / p->num_slices / 16));
   launch_early(cavlc_gather_kernel, dim3(ctas, p->num_slices), 256, 0, st, a, h);
   return cudaGetLastError() == cudaSuccess ? 0 : -1;
+}
+
+extern "C" int b200enc_cavlc_slices(const b200enc_cavlc_t* p, void* stream) {
+  return cavlc_launch(p, CavlcStage{}, static_cast<cudaStream_t>(stream));
+}
+
+int cavlc_slices_and_stage(const b200enc_cavlc_t* p, void* mv_host, const uint32_t* s0, const uint32_t* s1,
+                           uint32_t* status_host, cudaStream_t st) {
+  return cavlc_launch(p, CavlcStage{static_cast<MV*>(mv_host), s0, s1, status_host}, st);
 }

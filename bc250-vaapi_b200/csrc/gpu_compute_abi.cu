@@ -381,6 +381,11 @@ int encode_frame(gpu_context_t* ctx, Impl* m, const uint8_t* y, const uint8_t* u
                                        db_y + luma, m->pitch, scr1, m->stream);
   }
   perf_mark(m, 3);
+  void *dev_mv = nullptr, *dev_status = nullptr;  // the slot's motion field and status words, for kernels to write
+  if (stage) {
+    rc |= cudaHostGetDevicePointer(&dev_mv, sl.mv, 0) == cudaSuccess ? 0 : -1;
+    rc |= cudaHostGetDevicePointer(&dev_status, sl.status, 0) == cudaSuccess ? 0 : -1;
+  }
   sl.num_slices = 0;
   if (m->entropy) {
     // the slice data of every slice, written by the GPU straight into the
@@ -407,7 +412,9 @@ int encode_frame(gpu_context_t* ctx, Impl* m, const uint8_t* y, const uint8_t* u
     cp.out_bytes = dev_bytes;
     cp.scratch = m->d_cavlc;
     cp.scratch_bytes = m->cavlc_bytes;
-    if (rc == 0) rc |= b200enc_cavlc_slices(&cp, m->stream);
+    if (rc == 0)
+      rc |= stage ? cavlc_slices_and_stage(&cp, dev_mv, scr0 + 1, db ? scr1 + 1 : nullptr, (uint32_t*)dev_status, m->stream)
+                  : b200enc_cavlc_slices(&cp, m->stream);
     sl.num_slices = cp.num_slices;
   }
   if (stage) {
@@ -418,10 +425,7 @@ int encode_frame(gpu_context_t* ctx, Impl* m, const uint8_t* y, const uint8_t* u
       rc |= cudaMemcpyAsync(sl.pred_mode, m->d_pred_mode, mbs * 4, cudaMemcpyDeviceToHost, st) == cudaSuccess ? 0 : -1;
       rc |= cudaMemcpyAsync(sl.nz, m->d_nz, mbs * 96, cudaMemcpyDeviceToHost, st) == cudaSuccess ? 0 : -1;
     }
-    void *dev_mv = nullptr, *dev_status = nullptr;
-    rc |= cudaHostGetDevicePointer(&dev_mv, sl.mv, 0) == cudaSuccess ? 0 : -1;
-    rc |= cudaHostGetDevicePointer(&dev_status, sl.status, 0) == cudaSuccess ? 0 : -1;
-    if (rc == 0)
+    if (!m->entropy && rc == 0)  // the entropy coder has stored them
       rc |= stage_mv_launch(m->d_mv, dev_mv, (int)mbs, scr0 + 1, db ? scr1 + 1 : nullptr, (uint32_t*)dev_status, st);
   }
   perf_mark(m, 4);

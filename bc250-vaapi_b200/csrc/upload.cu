@@ -66,8 +66,9 @@ __global__ void __launch_bounds__(128) upload_nv12_kernel(UploadPlane y, UploadP
   }
 }
 
-// A frame's motion field and its two status words to page-locked host memory:
-// three copy-engine commands of a few bytes each took 3.3 us apiece.
+// A frame's motion field and its two status words to page-locked host memory
+// (where no entropy coder runs, whose first kernel stores them on its way): three
+// copy-engine commands of a few bytes each took 3.3 us apiece.
 __global__ void __launch_bounds__(256) stage_mv_kernel(const uint4* __restrict__ mv, uint4* __restrict__ mv_host, int mbs,
                                                        const uint32_t* __restrict__ s0, const uint32_t* __restrict__ s1,
                                                        uint32_t* __restrict__ status_host) {
