@@ -589,10 +589,12 @@ __host__ __device__ inline DbTilePlan db_tile_plan(int TW, int TH) {
   return p;
 }
 
-// Threads of a tile's CTA: sixteen per macroblock (a phase has 7 to 18 lines
-// per macroblock), at most 512 (two CTAs per SM).
-static inline int db_tile_threads(int TW, int TH) {
-  const int n = (16 * TW * TH + 31) / 32 * 32;
+// Threads of a tile's CTA, at most 512 (two CTAs per SM): sixteen per macroblock
+// (a phase has 7 to 18 lines per macroblock), and where the tiles do not fill the
+// chip at two per SM, 64: nothing else would use the lanes, and a phase is one
+// round of lines (640x480: 10.7 us with sixteen, 9.0).
+static inline int db_tile_threads(int TW, int TH, int tiles) {
+  const int n = ((tiles <= 2 * 148 ? 64 : 16) * TW * TH + 31) / 32 * 32;
   return n < 64 ? 64 : (n > kDbTileThreads ? kDbTileThreads : n);
 }
 
@@ -820,14 +822,16 @@ extern "C" int b200enc_deblock(int mbw, int mbh, int qp, int is_intra, const uin
 }
 
 // Tile shape of the tile deblocking (TW x TH macroblocks) of a picture of
-// `mbs` macroblocks, unless the autotuner chose one: 4 x 4 up to 4,096
-// macroblocks, where the tiles do not fill the chip and a tile's own latency
-// is the kernel's (P picture, us, 4 x 4 against 8 x 8: 176x144 10.9 and 16.1,
-// 640x480 12.1 and 19.2, 1280x720 13.1 and 18.4), 8 x 8 above, where the
-// margin's share of the work counts (3840x2160 47.8 and 40.6).
-static void db_tile_shape(int mbs, int* tw, int* th) {
+// `mbs` macroblocks, unless the autotuner chose one. Small tiles where they do
+// not fill the chip and a tile's own latency is the kernel's; large ones where
+// the margin's share of the work counts. P pictures, us, 3 x 3 / 4 x 4 / 8 x 8:
+// 176x144 8.4 / 9.4 / 16.2, 640x480 9.0 / 10.5 / 19.3, 1280x720 13.3 / 12.4 / 18.7,
+// 1366x766 14.1 / 12.4 / 18.6, 1920x1080 20.9 / 16.4 / 19.5, 2560x1440 29.7 / 25.9 /
+// 23.7, 3840x2160 58.4 / 47.9 / 40.9; an intra picture, which filters every edge,
+// turns earlier (1920x1080 23.3 / 18.7 / 17.0).
+static void db_tile_shape(int mbs, bool intra, int* tw, int* th) {
   const int w = b200enc_tuned(B200ENC_TUNE_DEBLOCK_TILE_W), h = b200enc_tuned(B200ENC_TUNE_DEBLOCK_TILE_H);
-  const int d = mbs <= 4096 ? 4 : 8;
+  const int d = mbs <= 2048 ? 3 : (mbs <= (intra ? 6144 : 8192) ? 4 : 8);
   *tw = w > 0 ? std::min(w, kDbTileMaxW) : d;
   *th = h > 0 ? std::min(h, kDbTileMax) : d;
 }
@@ -836,20 +840,20 @@ int b200enc_deblock_tiles_launch(int mbw, int mbh, int qp, int is_intra, const u
                                  const uint8_t* src_y, const uint8_t* src_uv, uint8_t* dst_y, uint8_t* dst_uv,
                                  int pitch, uint32_t* status, cudaStream_t stream, const uint8_t* t8) {
   int TW, TH;
-  db_tile_shape(mbw * mbh, &TW, &TH);
+  db_tile_shape(mbw * mbh, is_intra != 0, &TW, &TH);
   const DbTilePlan P = db_tile_plan(TW, TH);
   if (cudaFuncSetAttribute(deblock_tile_kernel<false>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)P.bytes) !=
       cudaSuccess)
     return -1;
   const int tiles = ((mbw + TW - 1) / TW) * ((mbh + TH - 1) / TH);
-  launch_early(deblock_tile_kernel<false>, tiles, db_tile_threads(TW, TH), P.bytes, stream, mbw, mbh, TW, TH, qp, is_intra, nz,
+  launch_early(deblock_tile_kernel<false>, tiles, db_tile_threads(TW, TH, tiles), P.bytes, stream, mbw, mbh, TW, TH, qp, is_intra, nz,
                (const MV*)mv, t8, src_y, src_uv, dst_y, dst_uv, pitch, status, BatchTab{});
   return cudaGetLastError() == cudaSuccess ? 0 : -1;
 }
 
 // Tile shape of a batch's table: one shape for every stream, the large
 // picture's (a batch fills the chip with its streams).
-void b200enc_deblock_batch_tile(int* tw, int* th) { db_tile_shape(1 << 30, tw, th); }
+void b200enc_deblock_batch_tile(int* tw, int* th) { db_tile_shape(1 << 30, false, tw, th); }
 
 // The tile deblocking of every stream of a batch: one CTA per tile
 // (bt.groups over the streams' tiles, bt.db_cols x bt.db_rows each).
@@ -861,7 +865,7 @@ int b200enc_deblock_tiles_batch_launch(const BatchTab& bt, int tiles, cudaStream
   if (cudaFuncSetAttribute(deblock_tile_kernel<true>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)P.bytes) !=
       cudaSuccess)
     return -1;
-  deblock_tile_kernel<true><<<tiles, db_tile_threads(TW, TH), P.bytes, st>>>(
+  deblock_tile_kernel<true><<<tiles, db_tile_threads(TW, TH, tiles), P.bytes, st>>>(
       0, 0, 0, 0, 0, 0, nullptr, nullptr, nullptr, nullptr, nullptr, nullptr, nullptr, 0, nullptr, bt);
   return cudaGetLastError() == cudaSuccess ? 0 : -1;
 }

@@ -130,7 +130,8 @@ int b200enc_deblock(int mbw, int mbh, int qp, int is_intra,
 /* The same deblocking (identical output), from an unfiltered reconstruction
  * src_y/src_uv to a separate destination dst_y/dst_uv (same pitch; the
  * destination planes must not overlap the source planes), as independent
- * tiles: each tile of TW x TH macroblocks (4 x 4 up to 4,096 macroblocks and
+ * tiles: each tile of TW x TH macroblocks (3 x 3 up to 2,048 macroblocks, 4 x 4
+ * up to 8,192 of a P and 6,144 of an intra picture,
  * 8 x 8 above, unless tuned: B200ENC_TUNE_DEBLOCK_TILE_W/_H) is deblocked
  * with the margin samples it depends on and stored alone, which reproduces
  * the whole picture's raster order on the tile. Replaces the same shader
