@@ -293,9 +293,11 @@ struct RescoreWarp {
 // mv_out at the compact index.
 // Nine CTAs per SM: with eight (64 registers) the driver gives the kernel a smaller
 // shared-memory carve-out than the fallback search running beside it, and the two
-// take turns on an SM instead of sharing it (640x480: the pair 28 us, not 19).
+// take turns on an SM instead of sharing it (640x480: the pair 28 us, not 19). The
+// grid is nine per SM too (eight: a 2160p pair 110.4 us, nine 108.9).
+constexpr int kRescoreCtas = 9;
 template <bool BATCH>
-__global__ void __launch_bounds__(128, 9) lp_rescore_kernel(const uint8_t* __restrict__ cur_, int cur_pitch_,
+__global__ void __launch_bounds__(128, kRescoreCtas) lp_rescore_kernel(const uint8_t* __restrict__ cur_, int cur_pitch_,
                                                          const uint8_t* __restrict__ ref_, int ref_pitch_, Geo g_,
                                                          int R, int lambda_, int mbs, LpBuf b,
                                                          MV* __restrict__ mv_out, BatchTab bt) {
@@ -881,7 +883,7 @@ int b200enc_proposal_me(void* h, const uint8_t* cur_y, int cur_pitch, const uint
                                            (void*)P->side);
   int sms = 148, dev = 0;
   if (cudaGetDevice(&dev) == cudaSuccess) cudaDeviceGetAttribute(&sms, cudaDevAttrMultiProcessorCount, dev);
-  const int per_sm = b200enc_tuned(B200ENC_TUNE_RESCORE_CTAS_PER_SM) > 0 ? b200enc_tuned(B200ENC_TUNE_RESCORE_CTAS_PER_SM) : 8;
+  const int per_sm = b200enc_tuned(B200ENC_TUNE_RESCORE_CTAS_PER_SM) > 0 ? b200enc_tuned(B200ENC_TUNE_RESCORE_CTAS_PER_SM) : kRescoreCtas;
   lp_rescore_kernel<false><<<std::max(1, std::min((mbs + 3) / 4, per_sm * sms)), 128, 0, st>>>(
       cur_y, cur_pitch, ref_y, ref_pitch, g, range, lambda, mbs, P->b, (MV*)mv_out, BatchTab{});
   // join
@@ -949,7 +951,7 @@ int b200enc_proposal_me_batch(void* h, const BatchTab& bt, int n, int range, int
   const int fb_sm = b200enc_tuned(B200ENC_TUNE_FALLBACK_CTAS_PER_SM) > 0 ? b200enc_tuned(B200ENC_TUNE_FALLBACK_CTAS_PER_SM) : 16;
   const int rc = b200enc_me_batch_launch(bt, range, P->b.lists + n, P->b.counters + 1, std::min(n, fb_sm * sms),
                                          P->side);
-  const int rs_sm = b200enc_tuned(B200ENC_TUNE_RESCORE_CTAS_PER_SM) > 0 ? b200enc_tuned(B200ENC_TUNE_RESCORE_CTAS_PER_SM) : 8;
+  const int rs_sm = b200enc_tuned(B200ENC_TUNE_RESCORE_CTAS_PER_SM) > 0 ? b200enc_tuned(B200ENC_TUNE_RESCORE_CTAS_PER_SM) : kRescoreCtas;
   lp_rescore_kernel<true><<<std::max(1, std::min((n + 3) / 4, rs_sm * sms)), 128, 0, st>>>(
       nullptr, 0, nullptr, 0, Geo{}, range, 0, n, P->b, bt.mvc, bt);
   if (cudaEventRecord(P->ev_fb, P->side) != cudaSuccess || cudaStreamWaitEvent(st, P->ev_fb, 0) != cudaSuccess)

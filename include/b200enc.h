@@ -238,7 +238,7 @@ int b200enc_batch_graph_stats(void *b, long *instantiations, long *updates);
  * launch. */
 #define B200ENC_TUNE_DEBLOCK_ROWS 0         /* macroblock rows per deblocking CTA, 1..6 (default 4) */
 #define B200ENC_TUNE_PCHAIN_MBS_PER_CTA 1   /* macroblocks per P-chain CTA, 1, 2 or 4 (default 1) */
-#define B200ENC_TUNE_RESCORE_CTAS_PER_SM 2  /* learned re-scoring grid, CTAs per SM, 1..16 (default 8) */
+#define B200ENC_TUNE_RESCORE_CTAS_PER_SM 2  /* learned re-scoring grid, CTAs per SM, 1..16 (default 9) */
 #define B200ENC_TUNE_FALLBACK_CTAS_PER_SM 3 /* fallback full-search grid, CTAs per SM, 1..16 (default 16) */
 #define B200ENC_TUNE_INTRA_CTAS 4           /* intra wavefront CTAs (groups of four luma or chroma rows in flight), >= 1 (default: all) */
 #define B200ENC_TUNE_ME_STAGE 5             /* full-search window staging: 1 word loads, 2 TMA (default TMA) */
