@@ -780,11 +780,14 @@ static constexpr uint32_t kMaxWaitUsDb = 2000000u;  // 2 s
 // Rows per CTA: 4 unless the autotuner chose otherwise (one luma + one
 // chroma warp each, plus two IO and two halo warps: 64R + 128 threads). The ring must hold the 2*R columns a group's rows
 // span plus prefetch, so R stays well below kDbRing.
-static int db_rows_per_cta(int mbw, int mbh) {
+static int db_max_shared() {
   int dev = 0, maxsm = 0;
   cudaGetDevice(&dev);
   cudaDeviceGetAttribute(&maxsm, cudaDevAttrMaxSharedMemoryPerBlockOptin, dev);
-  if (maxsm <= 0) maxsm = 48 * 1024;
+  return maxsm > 0 ? maxsm : 48 * 1024;
+}
+static int db_rows_per_cta(int mbw, int mbh) {
+  const int maxsm = db_max_shared();
   const int tuned = b200enc_tuned(B200ENC_TUNE_DEBLOCK_ROWS);
   int R = tuned > 0 ? tuned : 4;
   while (R > 1 && db_plan(mbw, R).bytes + 64 > (size_t)maxsm) --R;
@@ -801,8 +804,8 @@ extern "C" int b200enc_deblock_launch(int mbw, int mbh, int qp, int is_intra, co
   const DbPlan P = db_plan(mbw, R);
   const int groups = (mbh + R - 1) / R;
   if (ctas <= 0 || ctas > groups) ctas = groups;
-  if (cudaFuncSetAttribute(deblock_kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)P.bytes) !=
-      cudaSuccess)
+  // one limit for every picture's plan: it is the process's
+  if (cudaFuncSetAttribute(deblock_kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, db_max_shared() - 64) != cudaSuccess)
     return -1;
   deblock_kernel<<<ctas, 64 * R + 128, P.bytes, (cudaStream_t)stream>>>(
       mbw, mbh, R, qp, is_intra, nz, (const MV*)mv, rec_y, rec_uv, rec_pitch, scratch, max_wait);
@@ -819,6 +822,15 @@ extern "C" int b200enc_deblock(int mbw, int mbh, int qp, int is_intra, const uin
   if (cudaMemsetAsync(scratch, 0, b200enc_wavefront_scratch_bytes(mbh), (cudaStream_t)stream) != cudaSuccess) return -1;
   return b200enc_deblock_launch(mbw, mbh, qp, is_intra, nz, mv, rec_y, rec_uv, rec_pitch, (uint32_t*)scratch, ctas,
                                 kMaxWaitUsDb, stream);
+}
+
+// Lets a tile kernel take the dynamic shared memory of the largest tile. The limit
+// is the process's, so it must not follow a launch's own tile: a thread that set it
+// for a small tile failed another thread's launch of a large one.
+template <bool BATCH>
+static bool db_tile_shared() {
+  return cudaFuncSetAttribute(deblock_tile_kernel<BATCH>, cudaFuncAttributeMaxDynamicSharedMemorySize,
+                              (int)db_tile_plan(kDbTileMaxW, kDbTileMax).bytes) == cudaSuccess;
 }
 
 // Tile shape of the tile deblocking (TW x TH macroblocks) of a picture of
@@ -842,9 +854,7 @@ int b200enc_deblock_tiles_launch(int mbw, int mbh, int qp, int is_intra, const u
   int TW, TH;
   db_tile_shape(mbw * mbh, is_intra != 0, &TW, &TH);
   const DbTilePlan P = db_tile_plan(TW, TH);
-  if (cudaFuncSetAttribute(deblock_tile_kernel<false>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)P.bytes) !=
-      cudaSuccess)
-    return -1;
+  if (!db_tile_shared<false>()) return -1;
   const int tiles = ((mbw + TW - 1) / TW) * ((mbh + TH - 1) / TH);
   launch_early(deblock_tile_kernel<false>, tiles, db_tile_threads(TW, TH, tiles), P.bytes, stream, mbw, mbh, TW, TH, qp, is_intra, nz,
                (const MV*)mv, t8, src_y, src_uv, dst_y, dst_uv, pitch, status, BatchTab{});
@@ -862,9 +872,7 @@ int b200enc_deblock_tiles_batch_launch(const BatchTab& bt, int tiles, cudaStream
   const int TW = bt.db_cols, TH = bt.db_rows;
   if (TW < 1 || TH < 1 || TW > kDbTileMaxW || TH > kDbTileMax) return -1;
   const DbTilePlan P = db_tile_plan(TW, TH);
-  if (cudaFuncSetAttribute(deblock_tile_kernel<true>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)P.bytes) !=
-      cudaSuccess)
-    return -1;
+  if (!db_tile_shared<true>()) return -1;
   deblock_tile_kernel<true><<<tiles, db_tile_threads(TW, TH, tiles), P.bytes, st>>>(
       0, 0, 0, 0, 0, 0, nullptr, nullptr, nullptr, nullptr, nullptr, nullptr, nullptr, 0, nullptr, bt);
   return cudaGetLastError() == cudaSuccess ? 0 : -1;
