@@ -32,6 +32,11 @@ int b200enc_deblock_tiles_batch_launch(const b200enc::BatchTab& bt, int tiles, c
 int b200enc_proposal_me_batch(void* h, const b200enc::BatchTab& bt, int n, int range, int lambda, int mode,
                               float param, cudaStream_t st);
 // upload.cu: transfers by kernels that address page-locked host memory
+struct HostRange {
+  bool locked;         // the first byte is page-locked (and not managed) host memory
+  const uint8_t* dev;  // its device address, if the whole range can be read there; else null
+};
+extern "C" HostRange b200enc_host_range(const void* p, size_t bytes);
 int upload_nv12_launch(const uint8_t* y, int y_pitch, const uint8_t* uv, int uv_pitch, uint8_t* dst_y,
                        uint8_t* dst_uv, int dst_pitch, int width, int height, cudaStream_t st);
 int stage_mv_launch(const void* mv, void* mv_host, int mbs, const uint32_t* s0, const uint32_t* s1,

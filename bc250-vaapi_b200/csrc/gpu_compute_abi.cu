@@ -592,25 +592,29 @@ int gpu_compute_upload_nv12(gpu_context_t* ctx, gpu_image_t* image, gpu_memory_t
                             int y_pitch, const uint8_t* uv_plane, int uv_pitch, int width, int height) {
   Impl* m = impl_of(ctx);
   (void)memory;
-  if (!m || !image || !image->y_plane || !y_plane || !uv_plane || width <= 0 || height <= 0) return -1;
+  if (!m || !image || !image->y_plane || !image->uv_plane || !y_plane || !uv_plane || width <= 0 || height <= 0) return -1;
   if ((uint32_t)width > image->width || (uint32_t)height > image->height) return -1;
-  cudaPointerAttributes a{}, b{};
-  const bool locked = cudaPointerGetAttributes(&a, y_plane) == cudaSuccess && a.type == cudaMemoryTypeHost &&
-                      cudaPointerGetAttributes(&b, uv_plane) == cudaSuccess && b.type == cudaMemoryTypeHost;
-  if (!locked) cudaGetLastError();
-  // Rows apart on either side, page-locked and addressable: the row kernel
-  // (upload.cu says why the line lies there); else the copy engine.
+  auto range = [&](const uint8_t* p, int pitch, int rows) {
+    const size_t span = rows > 0 && pitch >= width ? (size_t)(rows - 1) * pitch + width : 0;
+    return b200enc_host_range(p, span);
+  };
+  const HostRange ry = range(y_plane, y_pitch, height), ruv = range(uv_plane, uv_pitch, height / 2);
+  const bool locked = ry.locked && ruv.locked;
+  // Rows apart on either side, page-locked and addressable from the first to the
+  // last byte, planes that a pitched copy would take: the row kernel (upload.cu says
+  // why the line lies there); else the copy engine.
   const int dst_pitch = (int)image->pitch;
   const bool apart = y_pitch != width || uv_pitch != width || dst_pitch != width;
-  if (locked && apart && a.devicePointer && b.devicePointer && y_pitch >= width && uv_pitch >= width)
-    return upload_nv12_launch((const uint8_t*)a.devicePointer, y_pitch, (const uint8_t*)b.devicePointer, uv_pitch,
-                                      (uint8_t*)image->y_plane, (uint8_t*)image->uv_plane, dst_pitch, width, height,
-                                      m->stream);
+  if (apart && ry.dev && ruv.dev && y_pitch >= width && uv_pitch >= width && dst_pitch >= width)
+    return upload_nv12_launch(ry.dev, y_pitch, ruv.dev, uv_pitch, (uint8_t*)image->y_plane,
+                              (uint8_t*)image->uv_plane, dst_pitch, width, height, m->stream);
   if (cudaMemcpy2DAsync(image->y_plane, image->pitch, y_plane, y_pitch, width, height, cudaMemcpyHostToDevice,
                         m->stream) != cudaSuccess ||
       cudaMemcpy2DAsync(image->uv_plane, image->pitch, uv_plane, uv_pitch, width, height / 2,
-                        cudaMemcpyHostToDevice, m->stream) != cudaSuccess)
+                        cudaMemcpyHostToDevice, m->stream) != cudaSuccess) {
+    cudaGetLastError();  // refused: not the error of the next launch
     return -1;
+  }
   // Host buffers the caller may reuse on return: unless both planes are
   // page-locked (cudaMallocHost, or b200enc_host_register: then stream
   // order is enough), wait for the copy.

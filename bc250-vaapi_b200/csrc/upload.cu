@@ -7,6 +7,8 @@
 // rows one by one, and its time is the rows': 176x144 39 us, 720x576 109,
 // 1366x768 159, 2558x1440 320. Warps that read 512 bytes of a row each keep the
 // bus full at any pitch: 6.2, 18.6, 39 and 124 us.
+#include <cuda.h>
+
 #include <algorithm>
 
 #include "b200enc_internal.h"
@@ -84,6 +86,41 @@ __global__ void __launch_bounds__(256) stage_mv_kernel(const uint4* __restrict__
 
 using namespace b200enc;
 
+// What the driver knows of `bytes` bytes of memory from p on. The row kernel reads
+// them all, so the whole range has to lie in the object (a cudaHostAlloc, a
+// registration) its first byte lies in: a buffer registered in part, or in parts,
+// goes to the copy engine. One query per plane, as the type alone took.
+HostRange b200enc_host_range(const void* p, size_t bytes) {
+  using Fn = CUresult (*)(unsigned, CUpointer_attribute*, void**, CUdeviceptr);
+  static const Fn fn = []() -> Fn {
+    void* f = nullptr;
+    cudaDriverEntryPointQueryResult q;
+    if (cudaGetDriverEntryPoint("cuPointerGetAttributes", &f, cudaEnableDefault, &q) != cudaSuccess ||
+        q != cudaDriverEntryPointSuccess)
+      return nullptr;
+    return reinterpret_cast<Fn>(f);
+  }();
+  HostRange r{false, nullptr};
+  if (!fn) {
+    cudaPointerAttributes a{};
+    r.locked = cudaPointerGetAttributes(&a, p) == cudaSuccess && a.type == cudaMemoryTypeHost;
+    if (!r.locked) cudaGetLastError();
+    return r;
+  }
+  unsigned type = 0, managed = 0;
+  CUdeviceptr dev = 0, start = 0;
+  size_t size = 0;
+  CUpointer_attribute what[5] = {CU_POINTER_ATTRIBUTE_MEMORY_TYPE, CU_POINTER_ATTRIBUTE_IS_MANAGED,
+                                 CU_POINTER_ATTRIBUTE_DEVICE_POINTER, CU_POINTER_ATTRIBUTE_RANGE_START_ADDR,
+                                 CU_POINTER_ATTRIBUTE_RANGE_SIZE};
+  void* to[5] = {&type, &managed, &dev, &start, &size};
+  if (fn(5, what, to, reinterpret_cast<CUdeviceptr>(p)) != CUDA_SUCCESS) return r;
+  r.locked = type == CU_MEMORYTYPE_HOST && !managed;
+  const size_t off = (size_t)(reinterpret_cast<CUdeviceptr>(p) - start);
+  if (r.locked && dev && off <= size && bytes <= size - off) r.dev = reinterpret_cast<const uint8_t*>(dev);
+  return r;
+}
+
 // Both planes of an NV12 frame, `width` bytes of each row, from page-locked host
 // memory at device addresses y, uv. 148 CTAs keep the bus full.
 int upload_nv12_launch(const uint8_t* y, int y_pitch, const uint8_t* uv, int uv_pitch, uint8_t* dst_y,
@@ -91,13 +128,16 @@ int upload_nv12_launch(const uint8_t* y, int y_pitch, const uint8_t* uv, int uv_
   const int segs = (width + 511) / 512, rows = height + height / 2;
   const UploadPlane py{y, dst_y, y_pitch, dst_pitch, height}, pc{uv, dst_uv, uv_pitch, dst_pitch, height / 2};
   const long long warps = (long long)segs * rows;
-  upload_nv12_kernel<<<(unsigned)std::min<long long>((warps + 3) / 4, 148), 128, 0, st>>>(py, pc, width, segs);
-  return cudaGetLastError() == cudaSuccess ? 0 : -1;
+  // the launch's own result, as a copy's: an error another call left behind is not this one's
+  cudaLaunchConfig_t cfg{};
+  cfg.gridDim = (unsigned)std::min<long long>((warps + 3) / 4, 148);
+  cfg.blockDim = 128;
+  cfg.stream = st;
+  return cudaLaunchKernelEx(&cfg, upload_nv12_kernel, py, pc, width, segs) == cudaSuccess ? 0 : -1;
 }
 
 int stage_mv_launch(const void* mv, void* mv_host, int mbs, const uint32_t* s0, const uint32_t* s1,
                     uint32_t* status_host, cudaStream_t st) {
-  launch_early(stage_mv_kernel, (mbs + 255) / 256, 256, 0, st, static_cast<const uint4*>(mv), static_cast<uint4*>(mv_host),
-               mbs, s0, s1, status_host);
-  return cudaGetLastError() == cudaSuccess ? 0 : -1;
+  return launch_early(stage_mv_kernel, (mbs + 255) / 256, 256, 0, st, static_cast<const uint4*>(mv),
+                      static_cast<uint4*>(mv_host), mbs, s0, s1, status_host) == cudaSuccess ? 0 : -1;
 }
