@@ -165,6 +165,7 @@ struct Epi16 {
   }
 };
 
+// Barriers of the whole warp (.aligned): its lanes have to arrive together.
 __device__ __forceinline__ void bar_sync(int id, int threads) {
   asm volatile("bar.sync %0, %1;" ::"r"(id), "r"(threads) : "memory");
 }
@@ -254,10 +255,12 @@ __global__ void __launch_bounds__(kNet8Block, 2) lp_net8_kernel(int mbs, LpBuf b
     if (!mbar_wait(&s.bar, phase, kWaitNs)) s.failed = 1;
     phase ^= 1;
     tc_fence_after();
+    __syncwarp();
     bar_sync(kBarTile, kNet8Threads);
     return s.failed == 0;
   };
   auto publish = [&]() {  // generic smem writes and TMEM reads done -> next MMAs
+    __syncwarp();
     tmem_wait_ld();
     fence_async_smem();
     tc_fence_before();
@@ -272,6 +275,7 @@ __global__ void __launch_bounds__(kNet8Block, 2) lp_net8_kernel(int mbs, LpBuf b
     for (int tile = blockIdx.x; tile < ntiles; tile += gridDim.x) {
       const int mb0 = tile * kNet8TileMbs, nmb = min(kNet8TileMbs, mbs - mb0);
       const uint32_t st = lane < nmb ? b.state[mb0 + lane] : 0u;
+      __syncwarp();  // after the last tile's list appends
       bar_sync(kBarLogits, 64);
       if (s.failed) break;
       float z[kOut];
@@ -554,11 +558,13 @@ __global__ void __launch_bounds__(kNet8Block, 2) lp_net8_kernel(int mbs, LpBuf b
 #pragma unroll
         for (int j = 0; j < 4; ++j) lo[j] = make_float4(z[4 * j], z[4 * j + 1], z[4 * j + 2], z[4 * j + 3]);
       }
+      __syncwarp();
       if (done > 0) bar_sync(kBarTaken, 64);  // the tile before has been read
       if (lane < kNet8TileMbs) {
 #pragma unroll
         for (int j = 0; j < kOut; ++j) s.z[lane][j] = z[j];
       }
+      __syncwarp();
       bar_arrive(kBarLogits, 64);
     }
     ++done;

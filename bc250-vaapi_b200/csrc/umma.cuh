@@ -147,8 +147,11 @@ __device__ __forceinline__ void tmem_ld16(uint32_t taddr, uint32_t (&v)[16]) {
 
 __device__ __forceinline__ void tmem_wait_ld() { asm volatile("tcgen05.wait::ld.sync.aligned;" ::: "memory"); }
 // 16 accumulator columns of TMEM lane 32*quad + lane (a warp reads its own
-// lane quadrant), columns col .. col+15; waits for the load.
+// lane quadrant), columns col .. col+15; waits for the load. The load is one
+// instruction of the whole warp (.sync.aligned): lanes that part before it, in a
+// bounded wait or in stores that only some of them make, meet here again.
 __device__ __forceinline__ void tmem_row16(uint32_t tmem, int quad, int col, uint32_t (&v)[16]) {
+  __syncwarp();
   tmem_ld16(tmem + ((uint32_t)(quad * 32) << 16) + (uint32_t)col, v);
   tmem_wait_ld();
 }
