@@ -366,8 +366,8 @@ __global__ void __launch_bounds__(32 * kIWarps, 1)
           int raw_, mode_;
           const bool clamp_l = Y + 15 > rmy;  // rows past the clamp limit read its last row
           // lane and register (0: rows 0 and 1 of a block, 1: rows 2 and 3) holding the left sample of a row
-          auto left_lane = [&](int row) { const int c = min(row, rmy - Y), k = c & 3; return (((c >> 2) * 4 + 3) << 1) | ((k == 1 || k == 2) ? 1 : 0); };
-          auto left_reg = [&](int row) { return (min(row, rmy - Y) & 3) >> 1; };
+          auto left_lane = [&](int row) { const int c = clampi(rmy - Y, 0, row), k = c & 3; return (((c >> 2) * 4 + 3) << 1) | ((k == 1 || k == 2) ? 1 : 0); };
+          auto left_reg = [&](int row) { return (clampi(rmy - Y, 0, row) & 3) >> 1; };
           const int lla = left_lane(ra), llb = left_lane(rb), lra = left_reg(ra), lrb = left_reg(rb);
           const int l15_lane = left_lane(15), l15_reg = left_reg(15);
           uint32_t reca = 0x80808080u, recb = 0x80808080u;
@@ -402,7 +402,7 @@ __global__ void __launch_bounds__(32 * kIWarps, 1)
               prev_t15 = (int)lp[15];
               if (X + 15 > rmx) {  // columns past the clamp limit read its last one
                 tw = 0;
-                for (int k = 0; k < 4; ++k) tw |= (uint32_t)lp[min(4 * bx + k, rmx - X)] << (8 * k);
+                for (int k = 0; k < 4; ++k) tw |= (uint32_t)lp[clampi(rmx - X, 0, 4 * bx + k)] << (8 * k);
               }
             }
             const int t15 = (int)(__shfl_sync(full, tw, 6) >> 24);
@@ -541,8 +541,8 @@ __global__ void __launch_bounds__(32 * kIWarps, 1)
             nb = src_word(pb_row, 8 + 4 * bx);
           }
           const bool clamp_l = Yc + 7 > cmy;
-          auto left_lane = [&](int row) { const int c = min(row, cmy - Yc), k = c & 3; return ((pl * 4 + (c >> 2) * 2 + 1) << 1) | ((k == 1 || k == 2) ? 1 : 0); };
-          auto left_reg = [&](int row) { return (min(row, cmy - Yc) & 3) >> 1; };
+          auto left_lane = [&](int row) { const int c = clampi(cmy - Yc, 0, row), k = c & 3; return ((pl * 4 + (c >> 2) * 2 + 1) << 1) | ((k == 1 || k == 2) ? 1 : 0); };
+          auto left_reg = [&](int row) { return (clampi(cmy - Yc, 0, row) & 3) >> 1; };
           const int lla = left_lane(ra), llb = left_lane(rb), lra = left_reg(ra), lrb = left_reg(rb);
           uint32_t reca = 0x80808080u, recb = 0x80808080u;
           uint2 lva, lvb, px;
@@ -572,7 +572,7 @@ __global__ void __launch_bounds__(32 * kIWarps, 1)
                                         *reinterpret_cast<const uint32_t*>(lp + 8 * bx + 4), pick);
               if (Xc + 7 > cmx) {
                 tw = 0;
-                for (int k = 0; k < 4; ++k) tw |= (uint32_t)lp[2 * min(4 * bx + k, cmx - Xc) + pl] << (8 * k);
+                for (int k = 0; k < 4; ++k) tw |= (uint32_t)lp[2 * clampi(cmx - Xc, 0, 4 * bx + k) + pl] << (8 * k);
               }
               tsum = (int)__dp4a(tw, 0x01010101u, 0u);
             }
@@ -651,7 +651,8 @@ __global__ void __launch_bounds__(32 * kIWarps, 1)
       //      above has published them and a macroblock needs them ---------------
       if (row0 > 0) {
         const uint32_t* flag = flags_of + row0 - 1;
-        const uint8_t* src = is_luma ? rec_y + (size_t)(row0 * 16 - 1) * rec_pitch : rec_uv + (size_t)(row0 * 8 - 1) * rec_pitch;
+        const uint8_t* src = is_luma ? rec_y + (size_t)min(row0 * 16 - 1, rmy) * rec_pitch
+                                     : rec_uv + (size_t)min(row0 * 8 - 1, cmy) * rec_pitch;
         int m = 0, seen = 0, chunk = -1;
         unsigned needs = 0;  // of the chunk's 32 macroblocks
         uint64_t t0 = global_ns();
@@ -678,7 +679,7 @@ __global__ void __launch_bounds__(32 * kIWarps, 1)
           n = min(n, __shfl_sync(full, shared_acquire(s.prog[1]), 0) + kIRing - m);
           // their lines and the next progress word in one round trip
           uint4 v = make_uint4(0u, 0u, 0u, 0u);
-          const bool take = n > 0 && x >= m && x < m + n && need;
+          const bool take = n > 0 && x >= m && x < m + n && need && 16 * x < rec_pitch;
           if (take) v = __ldcg(reinterpret_cast<const uint4*>(src + 16 * x));
           int now = (int)load_acquire(flag);
           if (n > 0) {
@@ -708,7 +709,10 @@ __global__ void __launch_bounds__(32 * kIWarps, 1)
       if (row0 + rows < g.mbh) {
         uint8_t* dst = is_luma ? rec_y + (size_t)((row0 + rows) * 16 - 1) * rec_pitch
                                : rec_uv + (size_t)((row0 + rows) * 8 - 1) * rec_pitch;
-        const int limit = is_luma ? g.RW : 2 * (cmx + 1);  // bytes of the row
+        // bytes of the row to store; none of a row past the clamp limit (a macroblock
+        // wholly outside the limits is coded, as before, but not kept)
+        const bool kept = is_luma ? (row0 + rows) * 16 - 1 <= rmy : (row0 + rows) * 8 - 1 <= cmy;
+        const int limit = kept ? (is_luma ? g.RW : 2 * (cmx + 1)) : 0;
         int done = 0;
         while (done < g.mbw) {
           if (!wait_shared(s.prog[rows], done + 1, (uint32_t)((row0 + rows - 1) * g.mbw + done))) break;
@@ -775,8 +779,8 @@ extern "C" int b200enc_i_frame_launch(const uint8_t* cur_y, const uint8_t* cur_u
 int b200enc_i_frame_groups(int mbh) { return (mbh + kIRows - 1) / kIRows; }
 
 // The intra wavefront of every I-frame stream of a batch: `ctas` persistent
-// CTAs over the row groups of bt.i_rows (each stream's scratch zeroed and
-// bt.ticket[0] = 0 by the caller).
+// CTAs over the row groups of bt.i_rows (each stream's scratch and both
+// tickets of bt.ticket zeroed by the caller).
 int b200enc_i_frame_batch_launch(const BatchTab& bt, int ctas, uint32_t max_wait, cudaStream_t st) {
   if (ctas <= 0) return 0;
   i_frame_kernel<true><<<2 * ctas, 32 * kIWarps, 0, st>>>(nullptr, nullptr, 0, Geo{}, 0, 1, nullptr, nullptr, nullptr, nullptr,
