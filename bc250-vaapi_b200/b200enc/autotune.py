@@ -39,14 +39,15 @@ def candidates(name, mbh):
         return [1, 2, 4]
     if name in ("rescore_ctas_per_sm", "fallback_ctas_per_sm"):
         return [2, 4, 8, 12, 16]
-    if name == "intra_ctas":
-        return sorted({max(1, mbh // 2), mbh})
+    if name == "intra_ctas":  # of two CTAs (luma, chroma) for each group of four rows: all, half, a quarter
+        n = 2 * ((mbh + 3) // 4)
+        return sorted({max(1, n // 4), max(1, n // 2), n})
     if name == "me_stage":
         return [2, 1]
     if name == "deblock_tile_w":
-        return [4, 6, 8]
+        return [3, 4, 6, 8]
     if name == "deblock_tile_h":
-        return [2, 4, 6, 8]
+        return [2, 3, 4, 6, 8]
     raise KeyError(name)
 
 
@@ -60,6 +61,8 @@ def throughput_candidates(name, mbh):
         return [4, 8, 12, 16]
     if name == "deblock_tile_w":  # wider tiles: less margin work per frame, longer chains
         return [6, 8, 12, 16]
+    if name == "deblock_tile_h":
+        return [2, 4, 6, 8]
     return candidates(name, mbh)
 
 
