@@ -49,7 +49,7 @@ struct StreamState {
   uint32_t *nz, *pred_mode;
   MV* mv[2];
   int mv_cur;  // mv[mv_cur] is the latest field
-  uint32_t *scr_intra, *scr_db;
+  uint32_t* scr_intra;
 };
 
 // Device table layout (one allocation, mirrored by two pinned host copies):
@@ -74,7 +74,7 @@ struct Batch {
   cudaStream_t stream = nullptr;
   std::vector<StreamState> ss;
   uint8_t* arena = nullptr;
-  uint32_t* scratch = nullptr;  // every stream's two scratch regions + 2 tickets, contiguous
+  uint32_t* scratch = nullptr;  // every stream's intra scratch + 2 tickets, contiguous
   size_t scratch_words = 0;
   uint32_t* status_host = nullptr;
   MV* mvc = nullptr;
@@ -152,7 +152,7 @@ int enqueue_step(Batch* b, const uint8_t* htab, int np, int ni, int ng, int n_p,
   if (n_irows > 0) rc |= b200enc_i_frame_batch_launch(bt, n_irows, kBatchMaxWaitUs, st) != 0;
   if (b->deblock && n_groups > 0)
     rc |= b200enc_deblock_tiles_batch_launch(bt, n_groups, st) != 0;
-  // status: error words of every stream's two scratch regions
+  // status: error words of every stream's scratch (tile deblocking has no wait that can give up)
   rc |= cudaMemcpyAsync(b->status_host, b->scratch, b->scratch_words * 4, cudaMemcpyDeviceToHost, st) != cudaSuccess;
   return rc ? -1 : 0;
 }
@@ -195,7 +195,7 @@ void* b200enc_batch_create(int n_streams, const int* widths, const int* heights,
     const size_t mbs = (size_t)t.mbw * t.mbh;
     bytes += 2 * up(t.rec_bytes, 256) + up(mbs * 768, 256) + 2 * up(mbs * 96, 256) + up(mbs * 4, 256) +
              2 * up(mbs * 16, 256);
-    scr_words += 2 * scratch_words(t.mbh);
+    scr_words += scratch_words(t.mbh);
     b->total_mbs += pad16((int)mbs);  // the compact P index, tile-aligned per stream
     b->max_mbw = std::max(b->max_mbw, t.mbw);
     b->max_mbh = std::max(b->max_mbh, t.mbh);
@@ -233,8 +233,6 @@ void* b200enc_batch_create(int n_streams, const int* widths, const int* heights,
     t.mv[0] = reinterpret_cast<MV*>(take(mbs * 16));
     t.mv[1] = reinterpret_cast<MV*>(take(mbs * 16));
     t.scr_intra = sw;
-    sw += scratch_words(t.mbh);
-    t.scr_db = sw;
     sw += scratch_words(t.mbh);
     t.cur = 0;
     t.mv_cur = 0;
@@ -322,7 +320,6 @@ int b200enc_batch_encode(void* h, const b200enc_batch_frame_t* frames) {
     d.mv = t.mv[t.mv_cur ^ 1];
     d.mv_prev = t.mv[t.mv_cur];
     d.scr_intra = t.scr_intra;
-    d.scr_db = t.scr_db;
     // deblocked out of place into the previous reconstruction, which the
     // step's ME and P chain have read before the deblocking launch
     d.db_y = t.rec[t.cur];
@@ -403,10 +400,8 @@ int b200enc_batch_sync(void* h) {
   if (cudaEventSynchronize(b->done) != cudaSuccess) return -1;
   b->pending = false;
   // a wavefront that gave up leaves its stream's frame incomplete
-  for (const StreamState& t : b->ss) {
-    const size_t oi = (size_t)(t.scr_intra - b->scratch), od = (size_t)(t.scr_db - b->scratch);
-    if (b->status_host[oi + 1] | b->status_host[od + 1]) return -1;
-  }
+  for (const StreamState& t : b->ss)
+    if (b->status_host[(size_t)(t.scr_intra - b->scratch) + 1]) return -1;
   return 0;
 }
 

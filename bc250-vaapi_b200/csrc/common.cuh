@@ -91,16 +91,10 @@ __device__ __forceinline__ int chroma_qp(int qpy) {
   }
 }
 
-// Position class of raster index p in a 4x4 block: 0 both even, 1 both odd,
-// 2 mixed (A1/shaders/quantize.comp:160-168).
-__device__ __forceinline__ int pos_type(int p) {
-  const int r = (p >> 2) & 1, c = p & 1;
-  return (r & c) ? 1 : ((r | c) ? 2 : 0);
-}
-
 // MF (A1/shaders/quantize.comp:151-158), V (A1/shaders/reconstruct.comp:
 // 124-131) and the DC level scale (reconstruct.comp:92), indexed
-// [qp%6][position class].
+// [qp%6][position class: 0 row and column even, 1 both odd, 2 mixed
+// (quantize.comp:160-168)].
 static __constant__ int kMF[6][3] = {{13107, 5243, 8066}, {11916, 4660, 7490}, {10082, 4194, 6554},
                                      {9362, 3647, 5825},  {8192, 3355, 5243},  {7282, 2893, 4559}};
 static __constant__ int kV[6][3] = {{10, 16, 13}, {11, 18, 14}, {13, 20, 16},
@@ -133,19 +127,6 @@ __device__ __forceinline__ QP make_qp(int qp, bool intra) {
   q.v2 = v_of(q.rem, 2);
   return q;
 }
-__device__ __forceinline__ int qp_mf(const QP& q, int pt) { return pt == 0 ? q.mf0 : (pt == 1 ? q.mf1 : q.mf2); }
-__device__ __forceinline__ int qp_v(const QP& q, int pt) { return pt == 0 ? q.v0 : (pt == 1 ? q.v1 : q.v2); }
-
-__device__ __forceinline__ int quant_ac(int c, int pos, const QP& q) {
-  const int a = c < 0 ? -c : c;
-  const int l = (a * qp_mf(q, pos_type(pos)) + q.f) >> q.f_shift;
-  return c < 0 ? -l : l;
-}
-// (level * 16 V << per) >> 4, rounded (reconstruct.comp): the sixteen makes the
-// division exact and the rounding empty for every per.
-__device__ __forceinline__ int dequant_ac(int level, int pos, const QP& q) {
-  return (level * qp_v(q, pos_type(pos))) << q.per;
-}
 
 __device__ __forceinline__ int quantize_dc(int v, const QP& q) {
   // A1/src/encoder_h264.c:653-709 (luma and chroma bodies are identical)
@@ -156,11 +137,6 @@ __device__ __forceinline__ int quantize_dc(int v, const QP& q) {
   else { num = a << (5 - q.per); den = ls; }
   const int l = (num + den / 2) / den;
   return v < 0 ? -l : l;
-}
-__device__ __forceinline__ int dequant_dc_luma(int f, const QP& q) {
-  const int ls = dc_ls(q.rem);
-  if (q.per >= 6) return (f * ls) << (q.per - 6);
-  return (f * ls + (1 << (5 - q.per))) >> (6 - q.per);
 }
 __device__ __forceinline__ int dequant_dc_chroma(int f, const QP& q) {
   const int ls = dc_ls(q.rem);
@@ -220,15 +196,6 @@ __device__ __forceinline__ void quad_transpose(int x[4], int r) {
   t0 = __shfl_xor_sync(full, t0, 1);
   t1 = __shfl_xor_sync(full, t1, 1);
   if (odd) { x[0] = t0; x[2] = t1; } else { x[1] = t0; x[3] = t1; }
-}
-
-// Forward 4x4 of the residual row x[0..3] held by lane r. Returns column r
-// of the coefficients: c[i] = coef[i][r]. Rows then columns, like
-// dct_transform.comp; the forward transform is exact so order is moot.
-__device__ __forceinline__ void quad_forward(int x[4], int r) {
-  fwd4(x[0], x[1], x[2], x[3]);
-  quad_transpose(x, r);
-  fwd4(x[0], x[1], x[2], x[3]);
 }
 
 // Inverse 4x4 of the dequantized row d[0..3] (lane r holds row r, +32 already
@@ -299,7 +266,7 @@ struct BatchStream {
   uint32_t *nz, *pred_mode;
   MV* mv;             // this frame's field
   const MV* mv_prev;  // the previous P frame's field (the learned form's history)
-  uint32_t *scr_intra, *scr_db;  // wavefront scratch (scratch_words(mbh) words each)
+  uint32_t* scr_intra;  // wavefront scratch (scratch_words(mbh) words)
   uint8_t *db_y, *db_uv;          // the deblocked reconstruction (tile deblocking; not rec_y/rec_uv)
 };
 

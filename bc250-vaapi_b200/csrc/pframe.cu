@@ -421,6 +421,8 @@ __global__ void __launch_bounds__(384, 3) p_mb_kernel(const uint8_t* __restrict_
     if (active) reinterpret_cast<uint2*>(levels + (size_t)mb * 384)[4 * b + r] = row;
 
     // ---- dequant + inverse + recon ----------------------------------------
+    // (level * 16 V << per) >> 4, rounded (reconstruct.comp): the sixteen makes
+    // the division exact and the rounding empty for every per
     int d[4];
 #pragma unroll
     for (int i = 0; i < 4; ++i)
