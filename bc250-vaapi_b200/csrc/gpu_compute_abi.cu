@@ -602,10 +602,13 @@ int gpu_compute_upload_nv12(gpu_context_t* ctx, gpu_image_t* image, gpu_memory_t
   const bool locked = ry.locked && ruv.locked;
   // Rows apart on either side, page-locked and addressable from the first to the
   // last byte, planes that a pitched copy would take: the row kernel (upload.cu says
-  // why the line lies there); else the copy engine.
+  // why the line lies there); else the copy engine, which also serves a thread whose
+  // current device is not the context's.
+  int current = -1;
+  cudaGetDevice(&current);
   const int dst_pitch = (int)image->pitch;
   const bool apart = y_pitch != width || uv_pitch != width || dst_pitch != width;
-  if (apart && ry.dev && ruv.dev && y_pitch >= width && uv_pitch >= width && dst_pitch >= width)
+  if (apart && ry.dev && ruv.dev && y_pitch >= width && uv_pitch >= width && dst_pitch >= width && current == m->device)
     return upload_nv12_launch(ry.dev, y_pitch, ruv.dev, uv_pitch, (uint8_t*)image->y_plane,
                               (uint8_t*)image->uv_plane, dst_pitch, width, height, m->stream);
   if (cudaMemcpy2DAsync(image->y_plane, image->pitch, y_plane, y_pitch, width, height, cudaMemcpyHostToDevice,

@@ -101,12 +101,6 @@ HostRange b200enc_host_range(const void* p, size_t bytes) {
     return reinterpret_cast<Fn>(f);
   }();
   HostRange r{false, nullptr};
-  if (!fn) {
-    cudaPointerAttributes a{};
-    r.locked = cudaPointerGetAttributes(&a, p) == cudaSuccess && a.type == cudaMemoryTypeHost;
-    if (!r.locked) cudaGetLastError();
-    return r;
-  }
   unsigned type = 0, managed = 0;
   CUdeviceptr dev = 0, start = 0;
   size_t size = 0;
@@ -114,7 +108,13 @@ HostRange b200enc_host_range(const void* p, size_t bytes) {
                                  CU_POINTER_ATTRIBUTE_DEVICE_POINTER, CU_POINTER_ATTRIBUTE_RANGE_START_ADDR,
                                  CU_POINTER_ATTRIBUTE_RANGE_SIZE};
   void* to[5] = {&type, &managed, &dev, &start, &size};
-  if (fn(5, what, to, reinterpret_cast<CUdeviceptr>(p)) != CUDA_SUCCESS) return r;
+  if (!fn || fn(5, what, to, reinterpret_cast<CUdeviceptr>(p)) != CUDA_SUCCESS) {
+    // no driver query, or a thread that has made no runtime call yet
+    cudaPointerAttributes a{};
+    r.locked = cudaPointerGetAttributes(&a, p) == cudaSuccess && a.type == cudaMemoryTypeHost;
+    if (!r.locked) cudaGetLastError();
+    return r;
+  }
   r.locked = type == CU_MEMORYTYPE_HOST && !managed;
   const size_t off = (size_t)(reinterpret_cast<CUdeviceptr>(p) - start);
   if (r.locked && dev && off <= size && bytes <= size - off) r.dev = reinterpret_cast<const uint8_t*>(dev);

@@ -4,6 +4,7 @@ checked for ranges that do not (nothing is launched on them), the upload for pla
 registered apart and for surfaces it has to refuse.
 """
 import ctypes
+import threading
 
 import numpy as np
 import pytest
@@ -91,11 +92,22 @@ def test_planes_registered_apart(gpu):
         bad.pitch = W - 2
         assert ctx.L.gpu_compute_upload_nv12(c, ctypes.byref(bad), mem, vp(a.ctypes.data), P,
                                              vp(a.ctypes.data + uv_at), P, W, H) != 0
-        # and the refusal is not the next upload's
-        assert ctx.L.gpu_compute_upload_nv12(c, ctypes.byref(img), mem, vp(a.ctypes.data), P,
-                                             vp(a.ctypes.data + uv_at), P, W, H) == 0
-        assert ctx.L.gpu_compute_download_nv12(c, ctypes.byref(img), mem, vp(y.ctypes.data), W, vp(uv.ctypes.data), W,
-                                               W, H) == 0
+        # and the refusal is not the next upload's, here or in a thread that has made no call yet
+        for where in ("here", "thread"):
+            rc = []
+            up = lambda: rc.append(ctx.L.gpu_compute_upload_nv12(  # noqa: E731
+                c, ctypes.byref(img), mem, vp(a.ctypes.data), P, vp(a.ctypes.data + uv_at), P, W, H))
+            a[:y_bytes] ^= 0x55
+            if where == "thread":
+                t = threading.Thread(target=up)
+                t.start()
+                t.join()
+            else:
+                up()
+            assert rc == [0]
+            assert ctx.L.gpu_compute_download_nv12(c, ctypes.byref(img), mem, vp(y.ctypes.data), W,
+                                                   vp(uv.ctypes.data), W, W, H) == 0
+            np.testing.assert_array_equal(y, np.lib.stride_tricks.as_strided(a, (H, W), (P, 1)))
     finally:
         _unpin(gpu, a, 0)
         _unpin(gpu, a, uv_at)
