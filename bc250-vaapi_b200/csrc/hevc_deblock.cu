@@ -25,9 +25,14 @@
 // maps); then, eight segments at a time and only where one of the eight is
 // filtered, four lanes filter a segment's lines, the decision and the first and
 // last line's figures coming by shuffles. Bound by instructions issued and the
-// latency of the maps' chained reads: 2160p at 10 bits 16.3 us vertical, 14.8 us
-// horizontal (25 MB of samples each); with the decision made by each of a
-// segment's four lanes and a load per sample 18.0 and 18.7.
+// latency of the maps' chained reads. A picture that does not fill the chip with
+// such warps pays their four rounds one after another, so there (kHdbFew) a warp
+// takes eight segments, each of a segment's four lanes decides for itself and has its
+// samples on the way meanwhile. Several pictures of each size in turn, 8 / 10 bits, us,
+// with eight segments a warp and with 32: 1280x720 9.6 and 17.8, 1920x1080 16.2 / 17.5 and
+// 20.3 / 22.4, 2560x1440 22.7 / 24.1 and 22.5 / 24.8, 3840x2160 42.5 / 45.2 and 36.9 / 40.1.
+// (Eight segments a warp without early launches, a load per sample: 13.9, 18.4 / 20.5,
+// 24.8 / 26.7, 41.4 / 45.1.)
 #include <cstddef>
 #include <type_traits>
 
@@ -53,6 +58,9 @@ __constant__ uint8_t kHdbTc[54] = {0, 0, 0, 0, 0, 0, 0, 0, 0, 0, 0, 0, 0, 0, 0, 
 __constant__ uint8_t kHdbQpC[14] = {29, 30, 31, 32, 33, 33, 34, 34, 35, 35, 36, 36, 37, 37};
 
 constexpr int kHdbThreads = 256;
+// Segments of one direction up to which a warp takes eight instead of 32: the two
+// forms take the same time at 2560x1440 (115,200).
+constexpr int kHdbFew = 110000;
 
 __device__ __forceinline__ int hdb_clip(int v, int lo, int hi) { return v < lo ? lo : (v > hi ? hi : v); }
 
@@ -150,34 +158,43 @@ __device__ int hdb_strength(const b200enc_hevc_deblock_t& p, int xp, int yp, int
   return (straight || swapped) ? 0 : 1;
 }
 
-// One line of a 4-line luma segment (clauses 8.7.2.5.3, 8.7.2.5.6,
-// 8.7.2.5.7; hevc_filter_template.c:48-140). The four lanes 4k..4k+3 of a
-// warp hold the segment's four lines; the decisions read lines 0 and 3 only,
-// so those lanes' figures are shuffled to the other two. `q` points at this
-// line's q0 and `fw` steps from p to q. Every lane of the warp calls it
-// (the shuffles); `act` says that the segment is filtered. VEC: a line lies along
-// a row of aligned samples, and its eight are read and written as two words (its
-// outer two, which no edge of the pass changes, with their own values).
+// One line of a 4-line luma segment across an edge. `q` points at its q0 and `fw`
+// steps from p to q. VEC: the line lies along a row of aligned samples, and its
+// eight are read and written as two words (the outer two, which no edge of the
+// pass changes, with their own values).
 template <typename T, bool VEC>
-__device__ __forceinline__ void hdb_luma_line(T* q, int fw, bool act, int beta, int tc, bool keep_p, bool keep_q,
-                                              int maxv) {
+struct HdbLine {
   using Half = typename std::conditional<sizeof(T) == 1, uint32_t, uint2>::type;  // four samples
   int p3 = 0, p2 = 0, p1 = 0, p0 = 0, q0 = 0, q1 = 0, q2 = 0, q3 = 0;
-  if (act && VEC) {
-    alignas(8) T v[8];
-    *reinterpret_cast<Half*>(v) = *reinterpret_cast<const Half*>(q - 4);
-    *reinterpret_cast<Half*>(v + 4) = *reinterpret_cast<const Half*>(q);
-    p3 = v[0], p2 = v[1], p1 = v[2], p0 = v[3], q0 = v[4], q1 = v[5], q2 = v[6], q3 = v[7];
-  } else if (act) {
-    p3 = q[-4 * fw];
-    p2 = q[-3 * fw];
-    p1 = q[-2 * fw];
-    p0 = q[-fw];
-    q0 = q[0];
-    q1 = q[fw];
-    q2 = q[2 * fw];
-    q3 = q[3 * fw];
+  __device__ __forceinline__ void load(const T* q, int fw) {
+    if (VEC) {
+      alignas(8) T v[8];
+      *reinterpret_cast<Half*>(v) = *reinterpret_cast<const Half*>(q - 4);
+      *reinterpret_cast<Half*>(v + 4) = *reinterpret_cast<const Half*>(q);
+      p3 = v[0], p2 = v[1], p1 = v[2], p0 = v[3], q0 = v[4], q1 = v[5], q2 = v[6], q3 = v[7];
+    } else {
+      p3 = q[-4 * fw];
+      p2 = q[-3 * fw];
+      p1 = q[-2 * fw];
+      p0 = q[-fw];
+      q0 = q[0];
+      q1 = q[fw];
+      q2 = q[2 * fw];
+      q3 = q[3 * fw];
+    }
   }
+};
+
+// Filters a loaded line (clauses 8.7.2.5.3, 8.7.2.5.6, 8.7.2.5.7;
+// hevc_filter_template.c:48-140). The four lanes 4k..4k+3 of a warp hold a
+// segment's four lines; the decisions read lines 0 and 3 only, so those lanes'
+// figures are shuffled to the other two. Every lane of the warp calls it (the
+// shuffles); `act` says that the segment is filtered.
+template <typename T, bool VEC>
+__device__ __forceinline__ void hdb_luma_filter(const HdbLine<T, VEC>& s, T* q, int fw, bool act, int beta, int tc,
+                                                bool keep_p, bool keep_q, int maxv) {
+  using Half = typename HdbLine<T, VEC>::Half;
+  const int p3 = s.p3, p2 = s.p2, p1 = s.p1, p0 = s.p0, q0 = s.q0, q1 = s.q1, q2 = s.q2, q3 = s.q3;
   const int dp = abs(p2 - 2 * p1 + p0), dq = abs(q2 - 2 * q1 + q0);
   const int flat = abs(p3 - p0) + abs(q0 - q3), step = abs(p0 - q0);
   const int l0 = (threadIdx.x & 31) & ~3, l3 = l0 + 3;
@@ -248,51 +265,74 @@ __device__ __forceinline__ int hdb_tc_chroma(const b200enc_hevc_deblock_t& p, co
   return (int)kHdbTc[hdb_clip(qpc + 2 + ed.tc_offset, 0, 53)] << (p.bit_depth_chroma - 8);
 }
 
+// What a segment's lines need (x, y its first sample): strength, kept sides, tC and
+// beta in `luma`, 0 where it is not filtered, and the chroma planes' tC. Chroma goes
+// with the first segment of a cell on the 16-sample grid, one chroma line per lane
+// (hevc_filter_template.c:298-335).
+struct HdbSegment {
+  uint32_t luma = 0, chroma = 0;
+};
+template <bool VERT>
+__device__ __forceinline__ HdbSegment hdb_decide(const b200enc_hevc_deblock_t& p, int x, int y) {
+  HdbSegment s;
+  const int e = __ldg(p.edges + (size_t)(y >> 3) * p.edges_stride + (x >> 3));
+  const int ctb_w = (p.width + (1 << p.log2_ctb) - 1) >> p.log2_ctb;
+  const HdbEdge ed = hdb_edge(p, VERT ? x : x & ~7, VERT ? y & ~7 : y, VERT, ctb_w);
+  const int b = hdb_strength(p, VERT ? x - 1 : x, VERT ? y : y - 1, x, y, (e & (VERT ? 4 : 8)) != 0);
+  const int bs = ((e & (VERT ? 1 : 2)) && ed.on) ? b : 0;
+  if (bs) {
+    const int tc = (int)kHdbTc[hdb_clip(ed.qp + 2 * (bs - 1) + ed.tc_offset, 0, 53)] << (p.bit_depth_luma - 8);
+    s.luma = bs | (ed.keep_p ? 4u : 0u) | (ed.keep_q ? 8u : 0u) | (uint32_t)tc << 4 | (uint32_t)ed.beta << 11;
+    if (bs == 2 && !((VERT ? x : y) & 15) && !((VERT ? y : x) & 7))
+      s.chroma = (uint32_t)hdb_tc_chroma(p, ed, 0) | (uint32_t)hdb_tc_chroma(p, ed, 1) << 8;
+  }
+  return s;
+}
+
 // One direction's edges: 4-row segments of vertical ones (VERT; a cell column
-// each) or 4-column segments of horizontal ones (a cell row each). Chroma goes
-// with the first segment of a cell on the 16-sample grid, one chroma line per
-// lane (hevc_filter_template.c:298-335). VEC: see hdb_luma_line.
-template <typename T, bool VERT, bool VEC>
-__global__ void __launch_bounds__(kHdbThreads) hevc_deblock_kernel(const __grid_constant__ b200enc_hevc_deblock_t p) {
+// each) or 4-column segments of horizontal ones (a cell row each). ROUNDS: how many
+// times eight segments a warp takes; with one round every lane decides for itself,
+// its samples on the way meanwhile. VEC: see HdbLine.
+// Five CTAs per SM (48 registers; with 58 the 10-bit horizontal pass loses a fifth
+// of its warps).
+template <typename T, bool VERT, bool VEC, int ROUNDS>
+__global__ void __launch_bounds__(kHdbThreads, 5) hevc_deblock_kernel(const __grid_constant__ b200enc_hevc_deblock_t p) {
   pdl_wait();
   const int per_row = VERT ? p.width >> 3 : p.width >> 2, rows = VERT ? p.height >> 2 : p.height >> 3;
-  const int lane = threadIdx.x & 31;
-  // ---- this lane's segment: its origin and what its lines need
-  const int sid = blockIdx.x * kHdbThreads + threadIdx.x;
-  int x = 0, y = 0;
-  uint32_t luma = 0, chroma = 0;  // strength, kept sides, tC, beta; the chroma planes' tC
-  if (sid < per_row * rows) {
-    const int row = sid / per_row, col = sid - row * per_row;
-    x = VERT ? col << 3 : col << 2;
-    y = VERT ? row << 2 : row << 3;
-    if (VERT ? col > 0 : row > 0) {
-      const int e = __ldg(p.edges + (size_t)(y >> 3) * p.edges_stride + (x >> 3));
-      const int ctb_w = (p.width + (1 << p.log2_ctb) - 1) >> p.log2_ctb;
-      const HdbEdge ed = hdb_edge(p, VERT ? x : x & ~7, VERT ? y & ~7 : y, VERT, ctb_w);
-      const int b = hdb_strength(p, VERT ? x - 1 : x, VERT ? y : y - 1, x, y, (e & (VERT ? 4 : 8)) != 0);
-      const int bs = ((e & (VERT ? 1 : 2)) && ed.on) ? b : 0;
-      if (bs) {
-        const int tc = (int)kHdbTc[hdb_clip(ed.qp + 2 * (bs - 1) + ed.tc_offset, 0, 53)] << (p.bit_depth_luma - 8);
-        luma = bs | (ed.keep_p ? 4u : 0u) | (ed.keep_q ? 8u : 0u) | (uint32_t)tc << 4 | (uint32_t)ed.beta << 11;
-        if (bs == 2 && !((VERT ? x : y) & 15) && !((VERT ? y : x) & 7))
-          chroma = (uint32_t)hdb_tc_chroma(p, ed, 0) | (uint32_t)hdb_tc_chroma(p, ed, 1) << 8;
-      }
-    }
-  }
-  // ---- the warp's segments, eight at a time, a line per lane
-  const uint32_t active = __ballot_sync(0xffffffffu, luma != 0);
-  const int maxv = (int)(sizeof(T) == 1 ? 255 : 1023), line = lane & 3;
+  const int lane = threadIdx.x & 31, line = lane & 3;
+  const int maxv = (int)(sizeof(T) == 1 ? 255 : 1023), fw = VERT ? 1 : p.stride[0];
   T* Y = reinterpret_cast<T*>(p.plane[0]);
+  // ---- this lane's segment (of the warp's 8 x ROUNDS)
+  const int at = blockIdx.x * kHdbThreads + threadIdx.x, sid = ROUNDS == 1 ? at >> 2 : at;
+  const int row = sid / per_row, col = sid - row * per_row;
+  const bool inside = row < rows && (VERT ? col > 0 : row > 0);  // an edge of the picture's inside
+  const int x = VERT ? col << 3 : col << 2, y = VERT ? row << 2 : row << 3;
+  HdbSegment mine;
+  HdbLine<T, VEC> s;
+  if (ROUNDS == 1 && inside) s.load(Y + (size_t)(VERT ? y + line : y) * p.stride[0] + (VERT ? x : x + line), fw);
+  if (inside) mine = hdb_decide<VERT>(p, x, y);
+  // ---- the warp's segments, eight at a time and a line per lane, where one of the
+  //      eight is filtered
+  const uint32_t active = __ballot_sync(0xffffffffu, mine.luma != 0);
 #pragma unroll 1
-  for (int first = 0; first < 32; first += 8) {
-    if (!(active >> first & 0xffu)) continue;
-    const int from = first + (lane >> 2);
-    const uint32_t lw = __shfl_sync(0xffffffffu, luma, from), cw = __shfl_sync(0xffffffffu, chroma, from);
-    const int sx = __shfl_sync(0xffffffffu, x, from), sy = __shfl_sync(0xffffffffu, y, from);
+  for (int first = 0; first < (ROUNDS == 1 ? 1 : 32); first += 8) {
+    if (ROUNDS == 1 ? !active : !(active >> first & 0xffu)) continue;
+    uint32_t lw = mine.luma, cw = mine.chroma;
+    int sx = x, sy = y;
+    if (ROUNDS > 1) {
+      const int from = first + (lane >> 2);
+      lw = __shfl_sync(0xffffffffu, lw, from);
+      cw = __shfl_sync(0xffffffffu, cw, from);
+      sx = __shfl_sync(0xffffffffu, sx, from);
+      sy = __shfl_sync(0xffffffffu, sy, from);
+    }
     const bool keep_p = lw & 4u, keep_q = lw & 8u;
-    const int lx = VERT ? sx : sx + line, ly = VERT ? sy + line : sy;
-    hdb_luma_line<T, VEC>(Y + (size_t)ly * p.stride[0] + lx, VERT ? 1 : p.stride[0], lw != 0, (int)(lw >> 11),
-                          (int)(lw >> 4 & 127u), keep_p, keep_q, maxv);
+    T* q = Y + (size_t)(VERT ? sy + line : sy) * p.stride[0] + (VERT ? sx : sx + line);
+    if (ROUNDS > 1) {
+      s = HdbLine<T, VEC>();
+      if (lw) s.load(q, fw);
+    }
+    hdb_luma_filter<T, VEC>(s, q, fw, lw != 0, (int)(lw >> 11), (int)(lw >> 4 & 127u), keep_p, keep_q, maxv);
     if (!cw) continue;
     const int cx = VERT ? sx >> 1 : (sx >> 1) + line, cy = VERT ? (sy >> 1) + line : sy >> 1;
 #pragma unroll
@@ -305,17 +345,19 @@ __global__ void __launch_bounds__(kHdbThreads) hevc_deblock_kernel(const __grid_
   }
 }
 
-template <typename T>
+template <typename T, int ROUNDS>
 static void hdb_launch(const b200enc_hevc_deblock_t& q, cudaStream_t st) {
-  const int nv = (q.width >> 3) * (q.height >> 2), nh = (q.width >> 2) * (q.height >> 3);  // segments
-  const unsigned gv = (nv + kHdbThreads - 1) / kHdbThreads, gh = (nh + kHdbThreads - 1) / kHdbThreads;
+  // segments, and warps of 8 ROUNDS of them
+  const int nv = (q.width >> 3) * (q.height >> 2), nh = (q.width >> 2) * (q.height >> 3);
+  constexpr int kBlock = kHdbThreads / 32 * 8 * ROUNDS;
+  const unsigned gv = (nv + kBlock - 1) / kBlock, gh = (nh + kBlock - 1) / kBlock;
   // four samples before and behind an edge start at a multiple of four of the row
   const bool vec = (reinterpret_cast<uintptr_t>(q.plane[0]) | (uintptr_t)q.stride[0] * sizeof(T)) % (4 * sizeof(T)) == 0;
   if (vec)
-    launch_early(hevc_deblock_kernel<T, true, true>, gv, kHdbThreads, 0, st, q);
+    launch_early(hevc_deblock_kernel<T, true, true, ROUNDS>, gv, kHdbThreads, 0, st, q);
   else
-    launch_early(hevc_deblock_kernel<T, true, false>, gv, kHdbThreads, 0, st, q);
-  launch_early(hevc_deblock_kernel<T, false, false>, gh, kHdbThreads, 0, st, q);
+    launch_early(hevc_deblock_kernel<T, true, false, ROUNDS>, gv, kHdbThreads, 0, st, q);
+  launch_early(hevc_deblock_kernel<T, false, false, ROUNDS>, gh, kHdbThreads, 0, st, q);
 }
 
 }  // namespace b200enc
@@ -337,9 +379,10 @@ extern "C" int b200enc_hevc_deblock(const b200enc_hevc_deblock_t* p, void* strea
   if (((uintptr_t)q.mvf & 3) || ((uintptr_t)q.slice_filter & 3)) return -1;
   if (q.slice_filter && q.n_slice_filter <= 0) return -1;
   const cudaStream_t st = (cudaStream_t)stream;
+  const bool few = (q.width >> 3) * (q.height >> 2) <= kHdbFew;
   if (q.bit_depth_luma == 8)
-    hdb_launch<uint8_t>(q, st);
+    few ? hdb_launch<uint8_t, 1>(q, st) : hdb_launch<uint8_t, 4>(q, st);
   else
-    hdb_launch<uint16_t>(q, st);
+    few ? hdb_launch<uint16_t, 1>(q, st) : hdb_launch<uint16_t, 4>(q, st);
   return cudaGetLastError() == cudaSuccess ? 0 : -1;
 }
