@@ -39,9 +39,9 @@ def candidates(name, mbh):
         return [1, 2, 4]
     if name in ("rescore_ctas_per_sm", "fallback_ctas_per_sm"):
         return [2, 4, 8, 12, 16]
-    if name == "intra_ctas":  # of two CTAs (luma, chroma) for each group of four rows: all, half, a quarter
+    if name == "intra_ctas":  # of two CTAs (luma, chroma) for each group of four rows: all, half
         n = 2 * ((mbh + 3) // 4)
-        return sorted({max(1, n // 4), max(1, n // 2), n})
+        return [n // 2, n]
     if name == "me_stage":
         return [2, 1]
     if name == "deblock_tile_w":

@@ -647,8 +647,9 @@ def run_gpu(args):
 
     def one_stream(mode, vals):
         """The single-stream arm: the tuned values but the built-in deblocking
-        tile (8 x 8, the latency choice; the throughput choice is wider)."""
-        autotune.apply(dict(vals, deblock_tile_w=0, deblock_tile_h=0))
+        tile and wavefront grid (the latency choices: small tiles where a picture
+        does not fill the chip, every row group at once)."""
+        autotune.apply(dict(vals, deblock_tile_w=0, deblock_tile_h=0, intra_ctas=0))
         r = arm(mode, 1, k1, Wm, perf=True)
         autotune.apply(vals)
         return r
@@ -769,8 +770,8 @@ def run_gpu(args):
                               "plain_stage_ms_per_p_frame": {k2: round(v, 4) for k2, v in plain_stage_ms.items()},
                               "stage_ms_per_i_frame": {k2: round(v, 4) for k2, v in intra_ms.items()},
                               "last_p_frame_mbs": dict(zip(("learned", "fallback", "early"), me_counts)),
-                              "deblock_tile": "8 x 8 macroblocks (the latency choice); the 8-stream arms use the "
-                                              "tuned shape in `tune`"},
+                              "deblock_tile": "the library's own shape for one picture of this size; the 8-stream "
+                                              "arms use the tuned one in `tune`"},
             "me_int": {"value": round(me_abs / (plain_stage_ms["me"] / 1000.0), 1), "unit": "abs-diff/s",
                        "searched_mbs": searched,
                        "note": f"plain full search, one stream: ({2 * RANGE + 1}^2 + 16) x 256 abs-diffs per searched "

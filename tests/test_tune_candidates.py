@@ -15,9 +15,7 @@ from b200enc import autotune  # noqa: E402
 def test_intra_ctas_differ(mbh):
     all_ctas = 2 * -(-mbh // 4)  # the launch's own number and its limit (csrc/intra.cu)
     c = autotune.candidates("intra_ctas", mbh)
-    assert len({min(v, all_ctas) for v in c}) == len(c) and all_ctas in c
-    if mbh > 8:
-        assert len(c) == 3
+    assert len({min(v, all_ctas) for v in c}) == len(c) == 2 and all_ctas in c
 
 
 def test_library_tile_shapes_are_offered():
