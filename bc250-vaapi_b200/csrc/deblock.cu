@@ -561,8 +561,7 @@ __global__ void deblock_kernel(int mbw, int mbh, int R, int qp, int is_intra, co
 // The form before this one ran each tile and a whole macroblock of margin as
 // a row wavefront in shared memory (TW + TH + 3 dependent macroblock steps of
 // ~1.8 us, 16 of 32 lanes active). P pictures, before and now, us: 176x144
-// 33 and 10.9, 640x480 37 and 12.1, 1920x1080 38 and 17 to 19, 3840x2160 111
-// and 41.
+// 33 and 8.4, 640x480 37 and 9.0, 1920x1080 38 and 16.4, 3840x2160 111 and 41.
 // ---------------------------------------------------------------------------
 constexpr int kDbTileMax = 8;    // TH <= 8
 constexpr int kDbTileMaxW = 16;  // TW <= 16
@@ -840,7 +839,11 @@ static bool db_tile_shared() {
 // 176x144 8.4 / 9.4 / 16.2, 640x480 9.0 / 10.5 / 19.3, 1280x720 13.3 / 12.4 / 18.7,
 // 1366x766 14.1 / 12.4 / 18.6, 1920x1080 20.9 / 16.4 / 19.5, 2560x1440 29.7 / 25.9 /
 // 23.7, 3840x2160 58.4 / 47.9 / 40.9; an intra picture, which filters every edge,
-// turns earlier (1920x1080 23.3 / 18.7 / 17.0).
+// turns earlier (1920x1080 23.3 / 18.7 / 17.0). The 4 x 4 tiles' time steps with
+// their last wave, so the lines do not cross at one size: 4 x 4 / 8 x 8 at 9,216
+// macroblocks (2048x1152) 15.9 / 19.1, at 10,240 21.4 / 19.4, at 11,664 24.2 / 23.6.
+// One picture decides: eight 1080p streams at once, which fill the chip, would
+// take 8 x 8 (15.1 ms against 15.6) or the autotuner's 16 x 8.
 static void db_tile_shape(int mbs, bool intra, int* tw, int* th) {
   const int w = b200enc_tuned(B200ENC_TUNE_DEBLOCK_TILE_W), h = b200enc_tuned(B200ENC_TUNE_DEBLOCK_TILE_H);
   const int d = mbs <= 2048 ? 3 : (mbs <= (intra ? 6144 : 8192) ? 4 : 8);

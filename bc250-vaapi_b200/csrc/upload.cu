@@ -2,8 +2,9 @@
 // device by kernels that address the host memory directly.
 //
 // The copy engine moves a frame whose rows lie together on both sides at the
-// bus's rate, and then it is what gpu_compute_upload_nv12 uses (640x480: 15.9 us,
-// this kernel 14.5; 3840x2160: 232 and 248). With a pitch on either side it takes
+// bus's rate, and then it is what gpu_compute_upload_nv12 uses: the bus bounds
+// both (640x480: 15.9 us, this kernel 14.5; 3840x2160: 232 and 248), and the
+// engine leaves the SMs to the other streams. With a pitch on either side it takes
 // rows one by one, and its time is the rows': 176x144 39 us, 720x576 109,
 // 1366x768 159, 2558x1440 320. Warps that read 512 bytes of a row each keep the
 // bus full at any pitch: 6.2, 18.6, 39 and 124 us.
